@@ -50,18 +50,10 @@ METRIC = "DMRG sweep s & H_eff·x TFLOP/s, mixed vs FP64 on one GB300 at ΔE≤1
 # `bench.py --steps 2 --warmup 3`, averaged over its GEMM 1 and GEMM 2)
 NCU_TRAFFIC = {("bf16", 2048): {"bytes_per_launch": (88.77e6 + 134.09e6 + 334.29e6 + 106.94e6) / 2,
                                 "gemm1_bytes": 88.77e6 + 134.09e6, "gemm2_bytes": 334.29e6 + 106.94e6,
-                                "algorithmic_operand_bytes": {"gemm1": 76.0e6, "gemm2": 210.0e6}},
-               # dram__bytes_read + write of the two oz_gemm_pair launches of one application
-               # (ncu --set full, D=2048); the digit planes the GEMMs read are 0.68 GB (GEMM 1)
-               # and 1.89 GB (GEMM 2), the FP64 output tile's epilogue passes add their
-               # read-modify-write
-               ("fp64_tc", 2048): {"bytes_per_launch": (19.81e9 + 6.05e9 + 24.01e9 + 4.75e9) / 2,
-                                   "gemm1_bytes": 19.81e9 + 6.05e9, "gemm2_bytes": 24.01e9 + 4.75e9,
-                                   "algorithmic_digit_plane_bytes": {"gemm1": 0.68e9,
-                                                                     "gemm2": 1.89e9}}}
+                                "algorithmic_operand_bytes": {"gemm1": 76.0e6, "gemm2": 210.0e6}}}
 UNIT = "TFLOP/s"
 W_MPO, D_PHYS = 5, 2
-OZ_PRODUCTS = 45          # BF16 digit products per FP64 multiply-add of the fp64_tc GEMM
+OZ_PRODUCTS = 16          # BF16 residue products per FP64 multiply-add of the fp64_tc GEMM
 
 
 def flops_ac2(D, w=W_MPO, d=D_PHYS):
@@ -1071,10 +1063,10 @@ def main():
     if prec == "bf16":
         peak, peak_note = peaks.get("bf16_tflops", 1900.0), "bf16_tflops (burst) of measured"
     elif prec == "fp64_tc":
-        # the FP64-accurate GEMM forms 45 BF16 digit products per FP64 multiply-add: the FP64
-        # rate it can reach is the measured BF16 peak / 45
+        # the FP64-accurate GEMM forms 16 BF16 residue products per FP64 multiply-add (K > 1758):
+        # the FP64 rate it can reach is the measured BF16 peak / 16
         peak = peaks.get("bf16_tflops", 1900.0) / OZ_PRODUCTS
-        peak_note = "bf16_tflops (burst) of measured / %d digit products" % OZ_PRODUCTS
+        peak_note = "bf16_tflops (burst) of measured / %d residue products" % OZ_PRODUCTS
     elif prec in ("tf32", "tf32x3"):
         peak = peaks.get("bf16_tflops", 1900.0) / 2
         peak_note = "half of measured bf16_tflops (dense TF32 rate is half of BF16)"
@@ -1086,7 +1078,7 @@ def main():
         achieved = per_launch / (tc_ms / tc_n / 1e3) / 1e12
         if prec == "tf32x3":
             achieved *= 1.0          # algorithmic flops only (3 products are not credited)
-        kname = ("oz_gemm_pair (tcgen05 BF16 digit products of the FP64-accurate GEMM)"
+        kname = ("oz_gemm_pair (tcgen05 BF16 residue products of the FP64-accurate GEMM)"
                  if prec == "fp64_tc" else "tc_gemm (tcgen05 %s)" % prec)
         roof = {"bound": "tensor", "kernel": kname,
                 "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
@@ -1099,7 +1091,7 @@ def main():
         if prec == "fp64_tc":
             roof["bf16_mma_tflops"] = achieved * OZ_PRODUCTS
             roof["unit_note"] = ("achieved: algorithmic FP64 flops (2 w d^2 D^3 per launch) per "
-                                 "second; bf16_mma_tflops: the digit-product MMA work per second")
+                                 "second; bf16_mma_tflops: the residue-product MMA work per second")
         if prec == "bf16" and rank == 0:
             roof["cublas_same_shapes"] = cublas_same_shapes(D, stream)
 

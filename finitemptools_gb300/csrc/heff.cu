@@ -327,16 +327,22 @@ static GemmArgs gemm_args(int cplx, int ta, int tb, int m, int n, int k, const d
   return g;
 }
 
+// the environments' planes for the engine in use
+static OzCache* left_cache(fmpt_op* op) { return op->h->oz_digits ? &op->ozd_left : &op->oz_left; }
+static OzCache* right_cache(fmpt_op* op) {
+  return op->h->oz_digits ? &op->ozd_right : &op->oz_right;
+}
+
 int op_apply_fp64(fmpt_op* op, const double* x, double* y) {
   fmpt_handle* h = op->h;
-  // FP64_TC: the GEMMs go to the tensor-core FP64 engine wherever it is faster; the digit
+  // FP64_TC: the GEMMs go to the tensor-core FP64 engine wherever it is faster; the residue
   // planes of the environments (A of the first GEMM, B of the second) are kept in the
   // operator, since they do not change while it lives
   const int eng = op->precision == FMPT_PREC_FP64_TC ? 1 : 0;
   auto gemm_f64 = [&](fmpt_handle* hh, GemmArgs g) {
     g.engine = eng;
-    if (eng && g.A == op->hleft) g.cacheA = &op->oz_left;
-    if (eng && g.B == op->hright) g.cacheB = &op->oz_right;
+    if (eng && g.A == op->hleft) g.cacheA = left_cache(op);
+    if (eng && g.B == op->hright) g.cacheB = right_cache(op);
     return fmpt::gemm_f64(hh, g);
   };
   const int cp = op->dtype == FMPT_C128;
@@ -383,7 +389,7 @@ int op_fp64_head(fmpt_op* op, const double* x) {
   GemmArgs g1 = gemm_args(cp, FMPT_N, FMPT_N, Dl * wl, P * Dr, Dl, op->hleft, (int64_t)Dl * wl,
                           (int64_t)Dl * wl * Dl, x, Dl, nx, T1, (int64_t)Dl * wl, n1);
   g1.engine = eng;
-  if (eng) g1.cacheA = &op->oz_left;
+  if (eng) g1.cacheA = left_cache(op);
   FMPT_TRY(gemm_f64(h, g1));
   // 2. T3[a', s', w2, b] = sum_blocks O[s', s] T1[a', w, s, b]
   MidStrides si{1, (int64_t)Dl * wl * P, Dl, (int64_t)Dl * wl};
@@ -405,7 +411,7 @@ int op_fp64_tail(fmpt_op* op, double* y) {
   GemmArgs g2 = gemm_args(cp, FMPT_N, FMPT_T, Dl * P, Dr, wr * Dr, T3, (int64_t)Dl * P, n3,
                           op->hright, Dr, (int64_t)Dr * wr * Dr, y, (int64_t)Dl * P, nx);
   g2.engine = eng;
-  if (eng) g2.cacheB = &op->oz_right;
+  if (eng) g2.cacheB = right_cache(op);
   return gemm_f64(h, g2);
 }
 
@@ -495,6 +501,8 @@ int fmpt_op_destroy(fmpt_op* op) {
   mid_free(op->h, op->sched);
   oz_cache_free(op->h, op->oz_left);
   oz_cache_free(op->h, op->oz_right);
+  oz_cache_free(op->h, op->ozd_left);
+  oz_cache_free(op->h, op->ozd_right);
   op_tc_free(op);
   op_u1_free(op);
   if (op->proj_part) cudaFreeAsync(op->proj_part, op->h->stream);

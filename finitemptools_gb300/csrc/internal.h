@@ -54,10 +54,14 @@ struct fmpt_handle {
   // partial tiles and arrival counters of the BF16 pair GEMM's K-split last round
   void* tc_ws = nullptr;
   size_t tc_ws_bytes = 0;
-  // FP64 GEMMs on the BF16 tensor cores (Ozaki digit planes, exponents, split pieces):
+  // FP64 GEMMs on the BF16 tensor cores (Ozaki scheme: residue planes, exponents,
+  // the product's residues):
   // f64_tc 1 routes every FP64 GEMM of this handle there when its cost model says it is
   // faster than the CUDA-core kernel (fmpt_set_f64_engine)
   int f64_tc = 0;
+  // set while fmpt_lanczos_ground runs: its tensor-core FP64 GEMMs are the digit products of
+  // ozaki_digits.cu (see there), not the residue products of ozaki.cu
+  int oz_digits = 0;
   // failure-detection test hook (fmpt_set_wait_test): bound of the grouped kernel's barrier
   // waits (0: 2 s) and extra arrivals they wait for (0 in normal use)
   int64_t wait_test_ns = 0;
@@ -145,7 +149,7 @@ struct ProfScope {
   ~ProfScope();
 };
 
-// Digit planes and exponents of one FP64 GEMM operand for the tensor-core FP64 engine,
+// Residue planes and exponents of one FP64 GEMM operand for the tensor-core FP64 engine,
 // kept across calls by an owner whose operand does not change between them (a prepared
 // operator's environments): built on first use, reused while src and shape match.
 struct OzCache {
@@ -171,7 +175,7 @@ struct GemmArgs {
   int64_t strideA, strideB, strideC;
   int nosplit;              // 1: never split K (no workspace allocation)
   int engine;               // 0: the handle's FP64 engine, 1: tensor cores where faster
-  OzCache* cacheA;          // optional digit-plane caches of A / B (tensor-core engine)
+  OzCache* cacheA;          // optional residue-plane caches of A / B (tensor-core engine)
   OzCache* cacheB;
 };
 int gemm_f64(fmpt_handle* h, const GemmArgs& g);
@@ -179,6 +183,9 @@ int gemm_f64(fmpt_handle* h, const GemmArgs& g);
 // (engine requested, shape large enough to win), and the call itself
 int gemm_f64_ozaki_possible(fmpt_handle* h, const GemmArgs& g);
 int gemm_f64_ozaki(fmpt_handle* h, const GemmArgs& g);
+// the same by digit products (ozaki_digits.cu), inside the Lanczos solve
+int gemm_f64_digits_possible(fmpt_handle* h, const GemmArgs& g);
+int gemm_f64_digits(fmpt_handle* h, const GemmArgs& g);
 // the handle's device status word (1: a bounded device wait timed out), read and cleared by
 // gp_check_status / fmpt_synchronize
 int gp_status_word(fmpt_handle* h, int** out);
@@ -309,8 +316,9 @@ struct fmpt_op {
   bool defer_right = false;  // mixed precision: the right environment is converted later
   // FP64 intermediates of one application (T1/T3 or T), grown outside stream capture only
   double* scratch = nullptr;
-  // digit planes of the environments for the tensor-core FP64 engine (FP64_TC operators)
+  // residue planes of the environments for the tensor-core FP64 engine (FP64_TC operators)
   fmpt::OzCache oz_left, oz_right;
+  fmpt::OzCache ozd_left, ozd_right;   // digit planes (the Lanczos solve's engine)
   size_t scratch_bytes = 0;
   // projectors of the excited-state sweeps: after every application
   // y -= dot(y, p) p for each p in order (device vectors of n elements, not owned)

@@ -1290,6 +1290,12 @@ int fmpt_lanczos_ground(fmpt_op* op, const double* x0, int kmax, double btol, in
   fmpt_handle* h = op->h;
   if (!x0 || !xout || !eigval) return set_error(h, FMPT_ERR_ARG, "lanczos: null pointer");
   if (kmax < 1 || kmax > 128) return set_error(h, FMPT_ERR_ARG, "lanczos: kmax must be 1..128");
+  // the solve's tensor-core FP64 GEMMs are the digit products (ozaki_digits.cu says why)
+  struct DigitEngine {
+    fmpt_handle* h;
+    explicit DigitEngine(fmpt_handle* hh) : h(hh) { h->oz_digits = 1; }
+    ~DigitEngine() { h->oz_digits = 0; }
+  } digit_engine(h);
   if (op->u1 && h->graphs) {
     bool fallback = false;
     const int st = lanczos_graph(op, x0, kmax, btol, reorth, eigval, xout, info, niter, &fallback);

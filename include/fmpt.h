@@ -53,12 +53,13 @@ enum fmpt_dtype { FMPT_F64 = 0, FMPT_C128 = 1 };
 /* Arithmetic of the contractions (H_eff*x and environment updates).
  * FP64 is the plain form (CUDA-core FMA, or the handle's FP64 engine, see
  * fmpt_set_f64_engine).  FP64_TC is the same FP64 contraction with every GEMM
- * large enough to gain run on the BF16 tensor cores by the Ozaki scheme: each
- * FP64 operand row becomes 9 exact base-64 digit planes (every digit within 32,
- * 53 bits below the row maximum), the 45 digit products of levels up to 10 run
- * as tcgen05 MMAs whose FP32 sums over each K chunk are exact, and the level
- * sums are added in FP64 (Frobenius-relative error 1e-15 to 4e-15 against the
- * FP64 kernel on random data, the accuracy class of an FP64 GEMM).  TF32,
+ * large enough to gain run on the BF16 tensor cores by the Ozaki scheme
+ * in its modular form: the entries of an FP64 operand row become integers of at
+ * least 53 bits below the row maximum, their residues modulo 15 or 16 coprime
+ * numbers up to 256 are exact BF16 values, each modulus's product runs as tcgen05
+ * MMAs whose FP32 sums over a K chunk are exact, and the Chinese remainder theorem
+ * gives the exact integer product, rounded once to FP64 (Frobenius-relative error
+ * about 1e-15 against 64-bit references, no larger than the FP64 kernel's).  TF32,
  * 3xTF32 and BF16 run on tcgen05 with FP32 accumulation (3xTF32 = hi/lo split
  * products). */
 enum fmpt_precision {
