@@ -77,24 +77,32 @@ __global__ void mid_kernel(const double* __restrict__ in, int64_t plane_in, MidS
 // (wi, s, coefficient), in block order then s -- the order in which mid_kernel adds them,
 // so that both give the same sums.  It does only the nonzero multiply-adds (the two-site
 // blocks are Kronecker products of single-site operators, mostly zeros), which is what
-// bounds the step on GB300's FP64 pipe.  Passed by value.
+// bounds the step on GB300's FP64 pipe.  Passed by value; the small table holds every
+// two-site MPO of up to 8 channels with d = 2 in about 1 KB of parameters.
+template <int OUT, int TERMS>
 struct MidSparse {
   int n_out;                          // nw_out * p_out
-  short start[MS_MAX_OUT + 1];
-  short idx[MS_MAX_T];                // wi * 16 + s
-  double c[MS_MAX_T];                 // real coefficients; complex: re, im pairs
+  short start[OUT + 1];
+  short idx[TERMS];                   // wi * 16 + s
+  double c[TERMS];                    // real coefficients; complex: re, im pairs
 };
+constexpr int MS_SMALL_OUT = 32, MS_SMALL_T = 96;
 
-template <bool CPLX>
-__global__ void mid_sparse_kernel(const double* __restrict__ in, int64_t plane_in, MidStrides si,
-                                  double* __restrict__ out, int64_t plane_out, MidStrides so,
-                                  int n1, int n2, int p_out, const __grid_constant__ MidSparse ms) {
+// Thread = one (o1, o2), outputs blockIdx.y, blockIdx.y + gridDim.y, ..  A large problem
+// runs gridDim.y = 1 (one pass over the input, L1 serves the repeated reads; 4.6 TB/s at
+// D = 2048).  A small one gives every output its own threads: with all 20 outputs in one
+// thread a D = 32 step was 4 blocks and 13.3 us of dependent loads, spread out it is 3.
+template <bool CPLX, int OUT, int TERMS>
+__global__ void __launch_bounds__(128)
+    mid_sparse_kernel(const double* __restrict__ in, int64_t plane_in, MidStrides si,
+                      double* __restrict__ out, int64_t plane_out, MidStrides so, int n1, int n2,
+                      int p_out, const __grid_constant__ MidSparse<OUT, TERMS> ms) {
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)n1 * n2) return;
   const int o1 = (int)(t % n1), o2 = (int)(t / n1);
   const double* ib = in + o1 * si.o1 + o2 * si.o2;
   double* ob = out + o1 * so.o1 + o2 * so.o2;
-  for (int o = 0; o < ms.n_out; o++) {
+  for (int o = blockIdx.y; o < ms.n_out; o += gridDim.y) {
     const int wo = o / p_out, q = o - wo * p_out;
     double ar = 0.0, ai = 0.0;
     for (int e = ms.start[o]; e < ms.start[o + 1]; e++) {
@@ -276,6 +284,25 @@ void mid_free(fmpt_handle* h, MidSchedule& s) {
   s.d_win = nullptr; s.d_wstart = nullptr; s.d_coef = nullptr;
 }
 
+template <bool CPLX, int OUT, int TERMS>
+static int mid_sparse_launch(fmpt_handle* h, const MidSchedule& s, const double* in,
+                             int64_t plane_in, MidStrides si, double* out, int64_t plane_out,
+                             MidStrides so, int n1, int n2) {
+  MidSparse<OUT, TERMS> ms;
+  ms.n_out = (int)s.sp_start.size() - 1;
+  for (size_t i = 0; i < s.sp_start.size(); i++) ms.start[i] = (short)s.sp_start[i];
+  for (size_t i = 0; i < s.sp_idx.size(); i++) ms.idx[i] = (short)s.sp_idx[i];
+  for (size_t i = 0; i < s.sp_coef.size(); i++) ms.c[i] = s.sp_coef[i];
+  const int64_t blocks = ((int64_t)n1 * n2 + 127) / 128;
+  // below a few blocks per SM the outputs are spread over threads of their own (see the
+  // kernel); above, the input is read once
+  const int gy = blocks < 8LL * std::max(1, h->sm_count) ? ms.n_out : 1;
+  mid_sparse_kernel<CPLX, OUT, TERMS><<<dim3((unsigned)blocks, gy), 128, 0, h->stream>>>(
+      in, plane_in, si, out, plane_out, so, n1, n2, s.p_out, ms);
+  FMPT_LAUNCHED(h);
+  return FMPT_OK;
+}
+
 int mid_apply(fmpt_handle* h, const MidSchedule& s, const double* in, int64_t plane_in,
               MidStrides si, double* out, int64_t plane_out, MidStrides so, int n1, int n2) {
   int64_t nt = (int64_t)n1 * n2;
@@ -287,19 +314,15 @@ int mid_apply(fmpt_handle* h, const MidSchedule& s, const double* in, int64_t pl
   if (P > 16) return set_error(h, FMPT_ERR_UNSUPPORTED, "physical dimension product %d > 16", P);
   ProfScope prof(h, FMPT_K_MPO_STEP);
   if (!s.sp_start.empty()) {
-    MidSparse ms;
-    ms.n_out = (int)s.sp_start.size() - 1;
-    for (size_t i = 0; i < s.sp_start.size(); i++) ms.start[i] = (short)s.sp_start[i];
-    for (size_t i = 0; i < s.sp_idx.size(); i++) ms.idx[i] = (short)s.sp_idx[i];
-    for (size_t i = 0; i < s.sp_coef.size(); i++) ms.c[i] = s.sp_coef[i];
-    if (s.cplx)
-      mid_sparse_kernel<true><<<(unsigned)blocks, threads, 0, h->stream>>>(
-          in, plane_in, si, out, plane_out, so, n1, n2, s.p_out, ms);
-    else
-      mid_sparse_kernel<false><<<(unsigned)blocks, threads, 0, h->stream>>>(
-          in, plane_in, si, out, plane_out, so, n1, n2, s.p_out, ms);
-    FMPT_LAUNCHED(h);
-    return FMPT_OK;
+    const int n_out = (int)s.sp_start.size() - 1;
+    const bool small = n_out <= MS_SMALL_OUT && (int)s.sp_coef.size() <= MS_SMALL_T;
+#define MIDS(CP)                                                                              \
+  (small ? mid_sparse_launch<CP, MS_SMALL_OUT, MS_SMALL_T>(h, s, in, plane_in, si, out,       \
+                                                           plane_out, so, n1, n2)             \
+         : mid_sparse_launch<CP, MS_MAX_OUT, MS_MAX_T>(h, s, in, plane_in, si, out, plane_out, \
+                                                       so, n1, n2))
+    return s.cplx ? MIDS(true) : MIDS(false);
+#undef MIDS
   }
 #define MIDL(MP, CP)                                                                          \
   mid_kernel<MP, CP><<<(unsigned)blocks, threads, 0, h->stream>>>(                            \
