@@ -120,16 +120,15 @@ __global__ void __launch_bounds__(256, 4) oz_rowmax(SliceSrc src, int rows_out, 
 // loads in flight per thread and no shared-memory staging for the row maxima, the residues
 // of a K-contiguous operand straight from registers.  The generic kernels are bound by
 // memory latency (long-scoreboard stalls, 22-37% of DRAM bandwidth).
-constexpr int RM_KCH = 128;           // K columns per block, row-contiguous row maxima
 constexpr int RK_KCH = 1024;          // K columns per block, K-contiguous row maxima
 
 // rows r, r + 1 of a row-contiguous operand (element (r, c) at p[r + c ld])
-__global__ void __launch_bounds__(256) oz_rowmax_rowfast(const double* __restrict__ p, int64_t ld,
-                                                         int64_t bstride, int rows, int k,
+__global__ void __launch_bounds__(128) oz_rowmax_rowfast(const double* __restrict__ p, int64_t ld,
+                                                         int64_t bstride, int rows, int k, int kch,
                                                          unsigned long long* __restrict__ mx) {
   const int z = blockIdx.z;
-  const int r = (blockIdx.x * 256 + threadIdx.x) * 2;
-  const int c0 = blockIdx.y * RM_KCH, c1 = min(c0 + RM_KCH, k);
+  const int r = (blockIdx.x * 128 + threadIdx.x) * 2;
+  const int c0 = blockIdx.y * kch, c1 = min(c0 + kch, k);
   if (r >= rows) return;
   const double* b = p + (int64_t)z * bstride + r;
   uint64_t m0 = 0, m1 = 0;
@@ -213,9 +212,14 @@ inline bool oz_kfast(const SliceSrc& x, int k) {
 inline int oz_row_maxima(fmpt_handle* h, const SliceSrc& x, int rows, int k, int batch,
                          unsigned long long* mx) {
   if (x.sr == 1 && oz_aligned(x, x.sc) && (rows & 1) == 0) {
-    const dim3 g1((unsigned)((rows / 2 + 255) / 256), (unsigned)((k + RM_KCH - 1) / RM_KCH),
-                  (unsigned)batch);
-    oz_rowmax_rowfast<<<g1, 256, 0, h->stream>>>(x.p, x.sc, x.bstride, rows, k, mx);
+    // K columns per block (a multiple of the eight loads in flight): short enough for about
+    // 16 blocks per SM, so that a small operand is spread out (1024 x 1280: 35 us on 20
+    // blocks) and a large one ends evenly, at most 128
+    const int gx = (rows / 2 + 127) / 128;
+    const int64_t want = (int64_t)k * gx * batch / (16LL * std::max(1, h->sm_count));
+    const int kc = (int)std::max<int64_t>(8, std::min<int64_t>(128, want) / 8 * 8);
+    const dim3 g1((unsigned)gx, (unsigned)((k + kc - 1) / kc), (unsigned)batch);
+    oz_rowmax_rowfast<<<g1, 128, 0, h->stream>>>(x.p, x.sc, x.bstride, rows, k, kc, mx);
   } else if (oz_kfast(x, k)) {
     const dim3 g1((unsigned)((rows + 7) / 8), (unsigned)((k + RK_KCH - 1) / RK_KCH),
                   (unsigned)batch);

@@ -165,18 +165,18 @@ __device__ __forceinline__ void residues8_store(const uint64_t (&bits8)[8], int 
   }
 }
 
-// Residue planes: block (strip, K chunk, batch) writes NMOD BF16 planes of its 32 x SL_KCH
+// Residue planes: block (strip, K chunk, batch) writes NMOD BF16 planes of its 32 x kch
 // part (zeros in the padding up to ldk); the chunk-0 blocks write the row exponents.
 // S[(z NMOD + i) rows_out + r][ldk] (K-major), E[z rows_out + r].  Each 32 x 64 tile goes
 // through a double-buffered shared tile (one barrier per tile); thread (rr, part) then
 // turns 8 consecutive K entries of row rr into 16-byte stores, one per plane.
 template <int NMOD>
-__global__ void __launch_bounds__(256) oz_residues(SliceSrc src, int rows_out, int k_out, int ldk,
-                                                   int tbits,
+__global__ void __launch_bounds__(256, 2) oz_residues(SliceSrc src, int rows_out, int k_out, int ldk,
+                                                   int kch, int tbits,
                                                    const unsigned long long* __restrict__ mxa,
                                                    uint16_t* __restrict__ S, int* __restrict__ E) {
   __shared__ uint64_t tile[2][SL_ROWS][65];
-  const int r0 = blockIdx.x * SL_ROWS, kc0 = blockIdx.y * SL_KCH, z = blockIdx.z;
+  const int r0 = blockIdx.x * SL_ROWS, kc0 = blockIdx.y * kch, z = blockIdx.z;
   const int t = threadIdx.x, rr = t >> 3, part = t & 7;
   const bool rowfast = src.sr == 1;
   const int r = r0 + rr;
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(256) oz_residues(SliceSrc src, int rows_out, i
   if (blockIdx.y == 0 && part == 0 && r < rows_out) E[(int64_t)z * rows_out + r] = bad ? E_BAD : e;
   const int64_t plane_stride = (int64_t)rows_out * ldk;
   uint16_t* out = S + ((int64_t)z * NMOD * rows_out + r) * ldk;
-  const int c1 = min(kc0 + SL_KCH, ldk);
+  const int c1 = min(kc0 + kch, ldk);
   uint64_t v[8];
   if (kc0 < c1) fetch_tile(src, z, r0, kc0, rows_out, k_out, v);
   int buf = 0;
@@ -209,15 +209,15 @@ __global__ void __launch_bounds__(256) oz_residues(SliceSrc src, int rows_out, i
 }
 
 // Residues of a K-contiguous operand: thread (rr, part) of a block owns row r0 + rr and, per
-// 64-column tile, the 8 entries from part * 8; two tiles' loads are in flight at once.
+// 64-column tile, the 8 entries from part * 8.
 template <int NMOD>
-__global__ void __launch_bounds__(256) oz_residues_kfast(const double* __restrict__ p, int64_t ld,
+__global__ void __launch_bounds__(256, 2) oz_residues_kfast(const double* __restrict__ p, int64_t ld,
                                                        int64_t bstride, int rows_out, int k_out,
-                                                       int ldk, int tbits,
+                                                       int ldk, int kch, int tbits,
                                                        const unsigned long long* __restrict__ mxa,
                                                        uint16_t* __restrict__ S,
                                                        int* __restrict__ E) {
-  const int r0 = blockIdx.x * SL_ROWS, kc0 = blockIdx.y * SL_KCH, z = blockIdx.z;
+  const int r0 = blockIdx.x * SL_ROWS, kc0 = blockIdx.y * kch, z = blockIdx.z;
   const int t = threadIdx.x, rr = t >> 3, part = t & 7;
   const int r = r0 + rr;
   if (r >= rows_out) return;
@@ -227,29 +227,18 @@ __global__ void __launch_bounds__(256) oz_residues_kfast(const double* __restric
   const int64_t plane_stride = (int64_t)rows_out * ldk;
   uint16_t* out = S + ((int64_t)z * NMOD * rows_out + r) * ldk;
   const double* b = p + (int64_t)z * bstride + (int64_t)r * ld;
-  const int c1 = min(kc0 + SL_KCH, ldk);
-  for (int c0 = kc0; c0 < c1; c0 += 128) {
-    double2 v[2][4];
+  const int c1 = min(kc0 + kch, ldk);
+  for (int cb = kc0 + part * 8; cb < c1; cb += 64) {
+    uint64_t bits8[8];
 #pragma unroll
-    for (int hh = 0; hh < 2; hh++)
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const int cc = c0 + 64 * hh + part * 8 + 2 * u;
-        v[hh][u] = cc < k_out ? __ldg(reinterpret_cast<const double2*>(b + cc))
-                              : make_double2(0.0, 0.0);
-      }
-#pragma unroll
-    for (int hh = 0; hh < 2; hh++) {
-      const int cb = c0 + 64 * hh + part * 8;
-      if (cb >= c1) break;
-      uint64_t bits8[8];
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        bits8[2 * u] = (uint64_t)__double_as_longlong(v[hh][u].x);
-        bits8[2 * u + 1] = (uint64_t)__double_as_longlong(v[hh][u].y);
-      }
-      residues8_store<NMOD>(bits8, tbits - e, bad, out, plane_stride, cb);
+    for (int u = 0; u < 4; u++) {
+      const int cc = cb + 2 * u;
+      const double2 v = cc < k_out ? __ldg(reinterpret_cast<const double2*>(b + cc))
+                                   : make_double2(0.0, 0.0);
+      bits8[2 * u] = (uint64_t)__double_as_longlong(v.x);
+      bits8[2 * u + 1] = (uint64_t)__double_as_longlong(v.y);
     }
+    residues8_store<NMOD>(bits8, tbits - e, bad, out, plane_stride, cb);
   }
 }
 
@@ -258,9 +247,9 @@ __global__ void __launch_bounds__(256) oz_residues_kfast(const double* __restric
 // (two tiles in flight, no registers held for them), and thread (rr, part) turns 8
 // consecutive K entries of row rr into one 16-byte store per plane.
 template <int NMOD>
-__global__ void __launch_bounds__(256) oz_residues_rowfast(const double* __restrict__ p, int64_t ld,
+__global__ void __launch_bounds__(256, 2) oz_residues_rowfast(const double* __restrict__ p, int64_t ld,
                                                          int64_t bstride, int rows_out,
-                                                         int k_out, int ldk, int tbits,
+                                                         int k_out, int ldk, int kch, int tbits,
                                                          const unsigned long long* __restrict__ mxa,
                                                          uint16_t* __restrict__ S,
                                                          int* __restrict__ E) {
@@ -268,7 +257,7 @@ __global__ void __launch_bounds__(256) oz_residues_rowfast(const double* __restr
   auto tile = [&](int st, int lr, int lc) -> uint64_t& {
     return dr_smem[((size_t)st * SL_ROWS + lr) * 65 + lc];
   };
-  const int r0 = blockIdx.x * SL_ROWS, kc0 = blockIdx.y * SL_KCH, z = blockIdx.z;
+  const int r0 = blockIdx.x * SL_ROWS, kc0 = blockIdx.y * kch, z = blockIdx.z;
   const int t = threadIdx.x, rr = t >> 3, part = t & 7;
   const int r = r0 + rr;
   bool bad = false;
@@ -277,7 +266,7 @@ __global__ void __launch_bounds__(256) oz_residues_rowfast(const double* __restr
   const int64_t plane_stride = (int64_t)rows_out * ldk;
   uint16_t* out = S + ((int64_t)z * NMOD * rows_out + r) * ldk;
   const double* b = p + (int64_t)z * bstride;
-  const int c1 = min(kc0 + SL_KCH, ldk);
+  const int c1 = min(kc0 + kch, ldk);
   const int ntile = (c1 - kc0 + 63) / 64;
   // tile j of the chunk into stage j % DR_STAGES: lanes run along rows (contiguous)
   auto issue = [&](int j) {
@@ -314,7 +303,7 @@ __global__ void __launch_bounds__(256) oz_residues_rowfast(const double* __restr
 
 // ------------------------------------------------------------ GEMM kernel
 struct OzEpi {
-  uint8_t* res;         // residues [modulus][unit][16 column groups][256 rows][16 columns]
+  uint8_t* res;         // residues [modulus][unit][64 column groups][256 rows][4 columns]
   int M, N;
   int* err;
 };
@@ -494,7 +483,7 @@ __global__ void __launch_bounds__(NTHR, 1)
       const int i = item / units;
       const float p = (float)modulus(i), inv = 1.0f / p;
       uint32_t acc[64];                      // column pairs' chunk sums, each + 256 per chunk
-      uint8_t* out = ep.res + ((int64_t)item * 16 + 8 * half) * (TILE * 16) + rloc * 16;
+      uint8_t* out = ep.res + ((int64_t)item * 64 + 32 * half) * (TILE * 4) + rloc * 4;
       for (int ch = 0; ch < nch; ch++, local++) {
         const int buf = local & 1;
         const uint32_t use = (uint32_t)(local >> 1);
@@ -530,23 +519,17 @@ __global__ void __launch_bounds__(NTHR, 1)
       // total mod p in [0, 255]: the bias is taken out, a negative remainder lifted by p
       const float bias = 8388608.0f + 256.0f * (float)nch;
 #pragma unroll
-      for (int g = 0; g < 8; g++) {
-        uint32_t w[4];
+      for (int g = 0; g < 32; g++) {
+        uint32_t by[4];
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-          uint32_t by[4];
-#pragma unroll
-          for (int j = 0; j < 4; j++) {
-            const uint32_t pr = acc[8 * g + 2 * k + (j >> 1)];
-            const uint32_t lohi = __byte_perm(pr, 0x4B00u, (j & 1) ? 0x5432 : 0x5410);
-            const float v = mod_balanced(__uint_as_float(lohi) - bias, p, inv);
-            by[j] = __float_as_uint((v < 0.0f ? v + p : v) + 8388608.0f);
-          }
-          w[k] = __byte_perm(__byte_perm(by[0], by[1], 0x0040), __byte_perm(by[2], by[3], 0x0040),
-                             0x5410);
+        for (int j = 0; j < 4; j++) {
+          const uint32_t lohi = __byte_perm(acc[2 * g + (j >> 1)], 0x4B00u, (j & 1) ? 0x5432 : 0x5410);
+          const float v = mod_balanced(__uint_as_float(lohi) - bias, p, inv);
+          by[j] = __float_as_uint((v < 0.0f ? v + p : v) + 8388608.0f);
         }
-        *reinterpret_cast<uint4*>(out + (int64_t)g * (TILE * 16)) =
-            make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint32_t*>(out + (int64_t)g * (TILE * 4)) =
+            __byte_perm(__byte_perm(by[0], by[1], 0x0040), __byte_perm(by[2], by[3], 0x0040),
+                        0x5410);
       }
     }
   }
@@ -639,53 +622,45 @@ __device__ __forceinline__ double crt_value(const uint32_t (&c)[NMOD], int E) {
   return __hiloint2double((int)((uint32_t)(bits >> 32) | sgn), (int)(uint32_t)bits);
 }
 
-// Thread = one tile row of a 16-column group: one 16-byte load per modulus (a warp reads
-// 512 contiguous bytes), 16 outputs (a warp writes 256 contiguous bytes per column).  ALU
-// work of about 100-150 instructions per output (32 IMAD.WIDE among them); GENERAL applies
-// alpha / beta and the complex embedding in FP64.
+// Thread = one tile row of a 4-column group: one 4-byte load per modulus (a warp reads 128
+// contiguous bytes), 4 outputs (a warp writes 256 contiguous bytes per column).  Four
+// columns rather than sixteen keep the loaded residues in 16 registers, so that enough
+// warps are resident to hide the loads behind the integer work of the others; GENERAL
+// applies alpha / beta in FP64.
 template <int NMOD, bool GENERAL>
 __global__ void __launch_bounds__(256) oz_crt(CrtArgs a) {
-  const int u = blockIdx.x >> 4, cg = blockIdx.x & 15;
+  const int u = blockIdx.x >> 6, cg = blockIdx.x & 63;
   int mt2, nt, z;
   oz_tile(u, a.tiles_m2, a.tiles_n, mt2, nt, z);
-  const int row = mt2 * TILE + threadIdx.x, col0 = nt * TILE + cg * 16;
+  const int row = mt2 * TILE + threadIdx.x, col0 = nt * TILE + cg * 4;
   if (row >= a.M || col0 >= a.N) return;
-  const uint8_t* base = a.res + ((int64_t)blockIdx.x * TILE + threadIdx.x) * 16;
-  uint4 v[NMOD];
+  const uint8_t* base = a.res + ((int64_t)blockIdx.x * TILE + threadIdx.x) * 4;
+  uint32_t v[NMOD];
 #pragma unroll
   for (int i = 0; i < NMOD; i++)
-    v[i] = __ldcs(reinterpret_cast<const uint4*>(base + (int64_t)i * a.units * (TILE * TILE)));
+    v[i] = __ldcs(reinterpret_cast<const uint32_t*>(base + (int64_t)i * a.units * (TILE * TILE)));
   const int er = __ldg(a.ea + (int64_t)z * a.M + row);
   const int* eb = a.eb + (int64_t)z * a.N + col0;
   const bool im = row >= a.mh;
-  double* crow = a.C + (int64_t)z * a.strideC + (im ? a.planeC + row - a.mh : (int64_t)row);
-  const int lim = min(16, a.N - col0);
+  double* p = a.C + (int64_t)z * a.strideC + (im ? a.planeC + row - a.mh : (int64_t)row) +
+              (int64_t)col0 * a.ldc;
 #pragma unroll
-  for (int w = 0; w < 4; w++) {
+  for (int j = 0; j < 4; j++, p += a.ldc) {
+    if (col0 + j >= a.N) break;
+    uint32_t c[NMOD];
 #pragma unroll
-    for (int b = 0; b < 4; b++) {
-      const int j = 4 * w + b;
-      if (j < lim) {
-        uint32_t c[NMOD];
-#pragma unroll
-        for (int i = 0; i < NMOD; i++) {
-          const uint32_t word = w == 0 ? v[i].x : w == 1 ? v[i].y : w == 2 ? v[i].z : v[i].w;
-          c[i] = (word >> (8 * b)) & 0xffu;
-        }
-        const int ec = __ldg(eb + j);
-        double x;
-        if (er >= E_BAD || ec >= E_BAD)
-          x = __longlong_as_double(0x7ff8000000000000ll);
-        else
-          x = crt_value<NMOD>(c, er + ec - 2 * a.tbits);
-        double* p = crow + (int64_t)(col0 + j) * a.ldc;
-        if (GENERAL) {
-          x *= a.alpha[0];
-          if (a.beta[0] != 0.0) x += a.beta[0] * *p;
-        }
-        *p = x;
-      }
+    for (int i = 0; i < NMOD; i++) c[i] = (v[i] >> (8 * j)) & 0xffu;
+    const int ec = __ldg(eb + j);
+    double x;
+    if (er >= E_BAD || ec >= E_BAD)
+      x = __longlong_as_double(0x7ff8000000000000ll);
+    else
+      x = crt_value<NMOD>(c, er + ec - 2 * a.tbits);
+    if (GENERAL) {
+      x *= a.alpha[0];
+      if (a.beta[0] != 0.0) x += a.beta[0] * *p;
     }
+    *p = x;
   }
 }
 
@@ -765,8 +740,8 @@ int gemm_f64_ozaki_possible(fmpt_handle* h, const GemmArgs& g) {
 
 namespace oz {
 // kernels by modulus count
-typedef void (*ResGeneric)(SliceSrc, int, int, int, int, const unsigned long long*, uint16_t*, int*);
-typedef void (*ResFast)(const double*, int64_t, int64_t, int, int, int, int,
+typedef void (*ResGeneric)(SliceSrc, int, int, int, int, int, const unsigned long long*, uint16_t*, int*);
+typedef void (*ResFast)(const double*, int64_t, int64_t, int, int, int, int, int,
                         const unsigned long long*, uint16_t*, int*);
 static ResGeneric residues_kernel(int nmod) {
   return nmod == 15 ? oz_residues<15> : oz_residues<16>;
@@ -808,7 +783,7 @@ int gemm_f64_ozaki(fmpt_handle* h, const GemmArgs& g) {
   auto al = [](size_t b) { return (b + 255) / 256 * 256; };
   const int tiles_m2 = (M2 + TILE - 1) / TILE, tiles_n = (N + TILE - 1) / TILE;
   const int64_t units = (int64_t)tiles_m2 * tiles_n * batch;
-  if (units > INT32_MAX / 64) return set_error(h, FMPT_ERR_SHAPE, "ozaki: too many tiles");
+  if (units > INT32_MAX / 128) return set_error(h, FMPT_ERR_SHAPE, "ozaki: too many tiles");
   // resident clusters of the kernel
   static int clusters = -1;
   cudaLaunchConfig_t cfg{};
@@ -873,25 +848,30 @@ int gemm_f64_ozaki(fmpt_handle* h, const GemmArgs& g) {
   if (!hitA || !hitB) {
     ProfScope prof(h, FMPT_K_CONVERT);
     FMPT_CUDA(h, cudaMemsetAsync(MX, 0, (size_t)batch * (M2 + N) * sizeof(uint64_t), h->stream));
-    const unsigned kch = (unsigned)((ldk + SL_KCH - 1) / SL_KCH);
-    const dim3 ga((M2 + SL_ROWS - 1) / SL_ROWS, kch, batch), gb((N + SL_ROWS - 1) / SL_ROWS, kch, batch);
-    auto convert = [&](const SliceSrc& x, int rows, const dim3& grid, unsigned long long* mx,
-                       uint16_t* planes, int* ex) -> int {
+    auto convert = [&](const SliceSrc& x, int rows, unsigned long long* mx, uint16_t* planes,
+                       int* ex) -> int {
+      // K columns per block: 512 where that leaves four blocks per SM, else down to one
+      // 64-column tile (a 1024 x 256 operand on 32 blocks took 12 us, its FP64 data 0.3)
+      const int strips = (rows + SL_ROWS - 1) / SL_ROWS;
+      int kch = SL_KCH;
+      while (kch > 64 && (int64_t)strips * ((ldk + kch - 1) / kch) * batch < 4LL * h->sm_count)
+        kch /= 2;
+      const dim3 grid(strips, (ldk + kch - 1) / kch, batch);
       FMPT_TRY(oz_row_maxima(h, x, rows, K2, batch, mx));
       if (oz_kfast(x, K2))
         residues_kfast_kernel(nmod)<<<grid, 256, 0, h->stream>>>(
-            x.p, x.sr, x.bstride, rows, K2, ldk, plan.tbits, mx, planes, ex);
+            x.p, x.sr, x.bstride, rows, K2, ldk, kch, plan.tbits, mx, planes, ex);
       else if (x.sr == 1 && !x.cplx)
         residues_rowfast_kernel(nmod)<<<grid, 256, DR_SMEM, h->stream>>>(
-            x.p, x.sc, x.bstride, rows, K2, ldk, plan.tbits, mx, planes, ex);
+            x.p, x.sc, x.bstride, rows, K2, ldk, kch, plan.tbits, mx, planes, ex);
       else
-        residues_kernel(nmod)<<<grid, 256, 0, h->stream>>>(x, rows, K2, ldk, plan.tbits, mx,
+        residues_kernel(nmod)<<<grid, 256, 0, h->stream>>>(x, rows, K2, ldk, kch, plan.tbits, mx,
                                                            planes, ex);
       FMPT_LAUNCHED(h);
       return FMPT_OK;
     };
-    if (!hitA) FMPT_TRY(convert(sa, M2, ga, MX, SA, EA));
-    if (!hitB) FMPT_TRY(convert(sb, N, gb, MX + (size_t)batch * M2, SBp, EB));
+    if (!hitA) FMPT_TRY(convert(sa, M2, MX, SA, EA));
+    if (!hitB) FMPT_TRY(convert(sb, N, MX + (size_t)batch * M2, SBp, EB));
   }
   for (int side = 0; side < 2; side++) {
     OzCache* c = side == 0 ? g.cacheA : g.cacheB;
@@ -943,7 +923,7 @@ int gemm_f64_ozaki(fmpt_handle* h, const GemmArgs& g) {
   }
   const bool general = ca.alpha[0] != 1.0 || ca.beta[0] != 0.0;
   ProfScope prof(h, FMPT_K_CONVERT);
-  const unsigned blocks = (unsigned)(units * 16);
+  const unsigned blocks = (unsigned)(units * 64);
   if (nmod == 15) {
     if (general) oz_crt<15, true><<<blocks, 256, 0, h->stream>>>(ca);
     else oz_crt<15, false><<<blocks, 256, 0, h->stream>>>(ca);
