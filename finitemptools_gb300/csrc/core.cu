@@ -351,6 +351,9 @@ int fmpt_destroy(fmpt_handle* h) {
   if (h->tc_ws) cudaFree(h->tc_ws);
   if (h->oz_ws) cudaFree(h->oz_ws);
   if (h->gstatus) cudaFree(h->gstatus);
+  for (cudaEvent_t e : h->step_event)
+    if (e) cudaEventDestroy(e);
+  if (h->step_host) cudaFreeHost(h->step_host);
   if (h->pinned) cudaFreeHost(h->pinned);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
   delete h;

@@ -22,6 +22,11 @@ struct fmpt_handle {
   // small pinned host staging area for scalars read back by the solvers
   double* pinned = nullptr;
   size_t pinned_len = 0;
+  // Lanczos solve: the ends of its two latest steps, and pinned memory their kernels write
+  // (alpha, beta) pairs to; of its own, since a step thrown away on convergence may still
+  // be running when the solve returns (both created on first use)
+  cudaEvent_t step_event[2] = {nullptr, nullptr};
+  double* step_host = nullptr;
   int sm_count = 0;
   // device timers (fmpt_profile_*)
   bool prof = false;

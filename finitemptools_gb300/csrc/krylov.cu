@@ -121,15 +121,20 @@ __global__ void lanczos_axpy(int64_t n, double* __restrict__ y, const double* __
   if (threadIdx.x == 0) part_b[blockIdx.x] = s;
 }
 
-// b = sqrt(sum(part_b)); beta_out = b; if b != 0: y /= b
-__global__ void lanczos_scale(int64_t n, double* __restrict__ y, const double* __restrict__ part_b,
-                              int G, double* beta_out) {
+// b = sqrt(sum(part_b)); beta_out = b; vnext = y / b (y itself if b is 0); alpha and b also
+// go to pinned host memory, ab[0] and ab[1]
+__global__ void lanczos_scale(int64_t n, const double* __restrict__ y,
+                              const double* __restrict__ part_b, int G, const double* alpha,
+                              double* beta_out, double* __restrict__ vnext, double* ab) {
   const double b = sqrt(sum_parts(part_b, G));
-  if (blockIdx.x == 0 && threadIdx.x == 0) *beta_out = b;
-  if (b == 0.0) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *beta_out = b;
+    ab[0] = *alpha;
+    ab[1] = b;
+  }
   // Julia's qi /= b divides element-wise; so does this (no reciprocal)
   for (int64_t i = (int64_t)blockIdx.x * KT + threadIdx.x; i < n; i += (int64_t)gridDim.x * KT)
-    y[i] = y[i] / b;
+    vnext[i] = b == 0.0 ? y[i] : y[i] / b;
 }
 
 // ---- multi-vector kernels over the Krylov basis V (j vectors of length n,
@@ -305,15 +310,10 @@ __global__ void multi_axpy_sub(int cplx, int64_t n, int j, const double* __restr
 // out = sum_i c_i V_i (c complex when cplx, real otherwise); scale multiplies
 __global__ void combine_basis(int cplx, int64_t n, int j, const double* __restrict__ V,
                               int64_t vstride, const double* __restrict__ c, int cstride,
-                              double scale, int last_first, double* __restrict__ out,
-                              const int* j_dev = nullptr) {
-  if (j_dev) j = *j_dev;
+                              double scale, double* __restrict__ out) {
   for (int64_t e = (int64_t)blockIdx.x * KT + threadIdx.x; e < n; e += (int64_t)gridDim.x * KT) {
     double r = 0.0, im = 0.0;
-    // lanczos_linear_transformation_single (simple_lanczos.jl:70-78) adds the
-    // last basis vector first
-    for (int t = 0; t < j; t++) {
-      int i = last_first ? (t == 0 ? j - 1 : t - 1) : t;
+    for (int i = 0; i < j; i++) {
       const double* v = V + (int64_t)i * vstride;
       double cr = c[i * cstride], ci = cplx ? c[i * cstride + 1] : 0.0;
       double vr = v[e];
@@ -472,15 +472,19 @@ __global__ void scale_by(int64_t n, double* __restrict__ x, const double* a) {
 
 // Lowest eigenpair of the symmetric tridiagonal (alpha[0..k-1], beta[0..k-2])
 // by Sturm-sequence bisection and inverse iteration with a partially pivoted
-// tridiagonal solve (the LAPACK dgtsv elimination).  One thread: k <= 128.
-__device__ void tridiag_lowest_body(int k, const double* __restrict__ alpha,
-                                    const double* __restrict__ beta, double* eval_out,
-                                    double* __restrict__ evec_out) {
+// tridiagonal solve (the LAPACK dgtsv elimination), k <= 128, on the host: about 1400
+// dependent FP64 divisions at k = 20, which one GPU thread ran in 640 us (a quarter of a
+// D = 64 solve) and a host core runs in about 10, while alpha and beta are on the host for
+// the stopping test anyway.  The multiply-adds are fused explicitly, as the device compiler
+// fuses them: the eigenvector's sign hangs on the last bit of the eigenvalue, so another
+// rounding would flip it.
+void tridiag_lowest(int k, const double* alpha, const double* beta, double* eval_out,
+                    double* evec_out) {
   double lo = alpha[0], hi = alpha[0];
   for (int i = 0; i < k; i++) {
-    double r = (i > 0 ? fabs(beta[i - 1]) : 0.0) + (i < k - 1 ? fabs(beta[i]) : 0.0);
-    lo = fmin(lo, alpha[i] - r);
-    hi = fmax(hi, alpha[i] + r);
+    double r = (i > 0 ? std::fabs(beta[i - 1]) : 0.0) + (i < k - 1 ? std::fabs(beta[i]) : 0.0);
+    lo = std::fmin(lo, alpha[i] - r);
+    hi = std::fmax(hi, alpha[i] + r);
   }
   const double tiny = 1e-300;
   for (int it = 0; it < 200; it++) {
@@ -500,9 +504,9 @@ __device__ void tridiag_lowest_body(int k, const double* __restrict__ alpha,
   *eval_out = lam;
   if (k == 1) { evec_out[0] = 1.0; return; }
   double dl[128], dd[128], du[128], du2[128], x[128];
-  for (int i = 0; i < k; i++) x[i] = 1.0 / sqrt((double)k) * (1.0 + 0.01 * i);
+  for (int i = 0; i < k; i++) x[i] = 1.0 / std::sqrt((double)k) * std::fma(0.01, (double)i, 1.0);
   // a zero pivot is replaced by eps*|T| (the LAPACK dlagts perturbation idea)
-  const double pert = 2.2e-16 * (fmax(fabs(lo), fabs(hi)) + 1e-300);
+  const double pert = 2.2e-16 * (std::fmax(std::fabs(lo), std::fabs(hi)) + 1e-300);
   for (int iter = 0; iter < 3; iter++) {
     for (int i = 0; i < k; i++) {
       dd[i] = alpha[i] - lam;
@@ -511,17 +515,17 @@ __device__ void tridiag_lowest_body(int k, const double* __restrict__ alpha,
     }
     // forward elimination with row interchanges
     for (int i = 0; i < k - 1; i++) {
-      if (fabs(dd[i]) >= fabs(dl[i])) {
+      if (std::fabs(dd[i]) >= std::fabs(dl[i])) {
         if (dd[i] == 0.0) dd[i] = pert;
         double f = dl[i] / dd[i];
-        dd[i + 1] -= f * du[i];
-        x[i + 1] -= f * x[i];
+        dd[i + 1] = std::fma(-f, du[i], dd[i + 1]);
+        x[i + 1] = std::fma(-f, x[i], x[i + 1]);
         dl[i] = 0.0;
       } else {
         double f = dd[i] / dl[i];
         dd[i] = dl[i];
         double t = dd[i + 1];
-        dd[i + 1] = du[i] - f * t;
+        dd[i + 1] = std::fma(-f, t, du[i]);
         if (i < k - 2) {
           du2[i] = du[i + 1];
           du[i + 1] = -f * du2[i];
@@ -529,39 +533,41 @@ __device__ void tridiag_lowest_body(int k, const double* __restrict__ alpha,
         du[i] = t;
         double xt = x[i];
         x[i] = x[i + 1];
-        x[i + 1] = xt - f * x[i + 1];
+        x[i + 1] = std::fma(-f, x[i + 1], xt);
       }
     }
     if (dd[k - 1] == 0.0) dd[k - 1] = pert;
     // back substitution
     x[k - 1] = x[k - 1] / dd[k - 1];
-    x[k - 2] = (x[k - 2] - du[k - 2] * x[k - 1]) / dd[k - 2];
-    for (int i = k - 3; i >= 0; i--) x[i] = (x[i] - du[i] * x[i + 1] - du2[i] * x[i + 2]) / dd[i];
+    x[k - 2] = std::fma(-du[k - 2], x[k - 1], x[k - 2]) / dd[k - 2];
+    for (int i = k - 3; i >= 0; i--)
+      x[i] = std::fma(-du2[i], x[i + 2], std::fma(-du[i], x[i + 1], x[i])) / dd[i];
     // normalise without overflow: scale by the largest entry first
     double mx = 0.0;
-    for (int i = 0; i < k; i++) mx = fmax(mx, fabs(x[i]));
-    if (!(mx > 0.0) || !isfinite(mx)) { for (int i = 0; i < k; i++) x[i] = (i == 0); mx = 1.0; }
+    for (int i = 0; i < k; i++) mx = std::fmax(mx, std::fabs(x[i]));
+    if (!(mx > 0.0) || !std::isfinite(mx)) { for (int i = 0; i < k; i++) x[i] = (i == 0); mx = 1.0; }
     double nrm = 0.0;
-    for (int i = 0; i < k; i++) { x[i] /= mx; nrm += x[i] * x[i]; }
-    nrm = sqrt(nrm);
+    for (int i = 0; i < k; i++) { x[i] /= mx; nrm = std::fma(x[i], x[i], nrm); }
+    nrm = std::sqrt(nrm);
     for (int i = 0; i < k; i++) x[i] /= nrm;
   }
   for (int i = 0; i < k; i++) evec_out[i] = x[i];
 }
 
-__global__ void tridiag_lowest(int k, const double* __restrict__ alpha,
-                               const double* __restrict__ beta, double* eval_out,
-                               double* __restrict__ evec_out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  tridiag_lowest_body(k, alpha, beta, eval_out, evec_out);
-}
+// Ritz coefficients by value
+struct RitzCoef {
+  double c[128];
+};
 
-// the same with the Krylov dimension read from the device (graph-driven solve)
-__global__ void tridiag_lowest_dev(const int* __restrict__ k, const double* __restrict__ alpha,
-                                   const double* __restrict__ beta, double* eval_out,
-                                   double* __restrict__ evec_out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  tridiag_lowest_body(*k, alpha, beta, eval_out, evec_out);
+// out = sum_i c_i V_i in the order of lanczos_linear_transformation_single
+// (simple_lanczos.jl:70-78), which adds the last basis vector first
+__global__ void combine_ritz(int64_t n, int k, const double* __restrict__ V, int64_t vstride,
+                             const __grid_constant__ RitzCoef c, double* __restrict__ out) {
+  for (int64_t e = (int64_t)blockIdx.x * KT + threadIdx.x; e < n; e += (int64_t)gridDim.x * KT) {
+    double r = c.c[k - 1] * V[(int64_t)(k - 1) * vstride + e];
+    for (int i = 0; i < k - 1; i++) r = fma(c.c[i], V[(int64_t)i * vstride + e], r);
+    out[e] = r;
+  }
 }
 
 // Graph-driven Lanczos step closure.  ctl: [0] stop (converged or failed),
@@ -729,14 +735,12 @@ int lanczos_graph(fmpt_op* op, const double* x0, int kmax, double btol, int reor
   FMPT_TRY(coef.alloc(h, (size_t)(kmax + 1) * 2 * sizeof(double)));
   FMPT_TRY(ctlb.alloc(h, 4 * sizeof(int)));
   FMPT_TRY(gp_prepare(h));
-  FMPT_TRY(ensure_pinned(h, 4));
+  FMPT_TRY(ensure_pinned(h, (size_t)2 * kmax + 2));
   double* V = Vb.d();
   double* y = Yb.d();
   double* s_vm = scal.d();
   double* s_alpha = scal.d() + 1;
   double* s_beta = scal.d() + 1 + kmax;
-  double* s_eval = scal.d() + 1 + 2 * kmax;
-  double* s_evec = scal.d() + 2 + 2 * kmax;
   int* ctl = static_cast<int*>(ctlb.p);
   auto V_ = [&](int i) { return V + (int64_t)i * n; };
   cudaStream_t st = h->stream;
@@ -765,12 +769,11 @@ int lanczos_graph(fmpt_op* op, const double* x0, int kmax, double btol, int reor
       lanczos_close<<<G, KT, 0, st>>>(n, y, partB.d(), G, s_beta + j, ctl, btol, j, V_(j + 1));
       FMPT_LAUNCHED(h);
     }
-    tridiag_lowest_dev<<<1, 1, 0, st>>>(ctl + 1, s_alpha, s_beta, s_eval, s_evec);
-    FMPT_LAUNCHED(h);
-    combine_basis<<<G, KT, 0, st>>>(0, n, 0, V, n, s_evec, 1, 1.0, 1, xout, ctl + 1);
-    FMPT_LAUNCHED(h);
-    FMPT_CUDA(h, cudaMemcpyAsync(h->pinned, s_eval, sizeof(double), cudaMemcpyDeviceToHost, st));
-    FMPT_CUDA(h, cudaMemcpyAsync(h->pinned + 1, ctl, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    // alpha and beta are adjacent
+    FMPT_CUDA(h, cudaMemcpyAsync(h->pinned, s_alpha, (size_t)2 * kmax * sizeof(double),
+                                 cudaMemcpyDeviceToHost, st));
+    FMPT_CUDA(h, cudaMemcpyAsync(h->pinned + 2 * kmax, ctl, 4 * sizeof(int),
+                                 cudaMemcpyDeviceToHost, st));
     return FMPT_OK;
   };
   if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
@@ -808,11 +811,15 @@ int lanczos_graph(fmpt_op* op, const double* x0, int kmax, double btol, int reor
   h->graph_launches++;
   FMPT_CUDA(h, cudaStreamSynchronize(st));
   // read the staged results before anything else reuses the pinned buffer
-  const int* c = reinterpret_cast<const int*>(h->pinned + 1);
+  const int* c = reinterpret_cast<const int*>(h->pinned + 2 * kmax);
   const int k = c[1], bad = c[2], conv = c[3];
-  const double ev = h->pinned[0];
+  double ev = 0.0;
+  RitzCoef rc;
+  if (!bad && k > 0) tridiag_lowest(k, h->pinned, h->pinned + kmax, &ev, rc.c);
   FMPT_TRY(gp_check_status(h));
   if (bad) return set_error(h, FMPT_ERR_NONFINITE, "lanczos: beta is not finite");
+  combine_ritz<<<G, KT, 0, st>>>(n, k, V, n, rc, xout);
+  FMPT_LAUNCHED(h);
   *eigval = ev;
   if (info) *info = conv ? 0 : -1;
   if (niter) *niter = k;
@@ -1307,20 +1314,19 @@ int fmpt_lanczos_ground(fmpt_op* op, const double* x0, int kmax, double btol, in
   DevBuf Vb, Yb, scal, partA, partB, partM, coef;
   FMPT_TRY(Vb.alloc(h, (size_t)(kmax + 1) * n * sizeof(double)));
   FMPT_TRY(Yb.alloc(h, (size_t)n * sizeof(double)));
-  // scal: [0] vm, [1..kmax] alpha, [kmax+1 .. 2kmax] beta, [2kmax+1] eval, then evec (kmax)
-  FMPT_TRY(scal.alloc(h, (size_t)(3 * kmax + 8) * sizeof(double)));
+  FMPT_TRY(scal.alloc(h, (size_t)(2 * kmax + 1) * sizeof(double)));   // vm, alpha, beta
   FMPT_TRY(partA.alloc(h, (size_t)G * sizeof(double)));
   FMPT_TRY(partB.alloc(h, (size_t)G * sizeof(double)));
   FMPT_TRY(partM.alloc(h, (size_t)G * (kmax + 1) * 2 * sizeof(double)));
   FMPT_TRY(coef.alloc(h, (size_t)(kmax + 1) * 2 * sizeof(double)));
-  FMPT_TRY(ensure_pinned(h, 4));
+  if (!h->step_host) FMPT_CUDA(h, cudaMallocHost((void**)&h->step_host, 256 * sizeof(double)));
+  for (cudaEvent_t& e : h->step_event)
+    if (!e) FMPT_CUDA(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   double* V = Vb.d();
   double* y = Yb.d();
   double* s_vm = scal.d();
   double* s_alpha = scal.d() + 1;
   double* s_beta = scal.d() + 1 + kmax;
-  double* s_eval = scal.d() + 1 + 2 * kmax;
-  double* s_evec = scal.d() + 2 + 2 * kmax;
   auto V_ = [&](int i) { return V + (int64_t)i * n; };
 
   // reorthogonalise y against V_0..V_{j-1} (classical Gram-Schmidt, one pass)
@@ -1334,77 +1340,59 @@ int fmpt_lanczos_ground(fmpt_op* op, const double* x0, int kmax, double btol, in
     return FMPT_OK;
   };
 
-  // ---- lanczos_make_first_step (simple_lanczos.jl:27-42)
+  // step j: lanczos_make_first_step / lanczos_make_step (simple_lanczos.jl:27-68), from V_j
+  // to alpha_j, beta_j and V_{j+1}; alpha_j and beta_j are in step_host[2 j], [2 j + 1] once
+  // step_event[j & 1] has passed
+  double* ab = h->step_host;
+  auto launch_step = [&](int j) -> int {
+    FMPT_TRY(fmpt_op_apply(op, V_(j), y));
+    rdot_partial<<<G, KT, 0, h->stream>>>(n, V_(j), y, partA.d());
+    FMPT_LAUNCHED(h);
+    lanczos_axpy<<<G, KT, 0, h->stream>>>(n, y, V_(j), j ? V_(j - 1) : nullptr, partA.d(), G,
+                                          j ? s_beta + (j - 1) : nullptr, s_alpha + j, partB.d());
+    FMPT_LAUNCHED(h);
+    if (reorth) FMPT_TRY(reorthogonalise(j + 1));
+    lanczos_scale<<<G, KT, 0, h->stream>>>(n, y, partB.d(), G, s_alpha + j, s_beta + j, V_(j + 1),
+                                           ab + 2 * j);
+    FMPT_LAUNCHED(h);
+    FMPT_CUDA(h, cudaEventRecord(h->step_event[j & 1], h->stream));
+    return FMPT_OK;
+  };
   rdot_partial<<<G, KT, 0, h->stream>>>(n, x0, x0, partA.d());
   FMPT_LAUNCHED(h);
   normalize_from_parts<<<G, KT, 0, h->stream>>>(n, x0, V_(0), partA.d(), G, s_vm);
   FMPT_LAUNCHED(h);
-  FMPT_TRY(fmpt_op_apply(op, V_(0), y));
-  rdot_partial<<<G, KT, 0, h->stream>>>(n, V_(0), y, partA.d());
-  FMPT_LAUNCHED(h);
-  lanczos_axpy<<<G, KT, 0, h->stream>>>(n, y, V_(0), nullptr, partA.d(), G, nullptr, s_alpha,
-                                        partB.d());
-  FMPT_LAUNCHED(h);
-  if (reorth) FMPT_TRY(reorthogonalise(1));
-  lanczos_scale<<<G, KT, 0, h->stream>>>(n, y, partB.d(), G, s_beta);
-  FMPT_LAUNCHED(h);
-  FMPT_CUDA(h, cudaMemcpyAsync(h->pinned, s_beta, sizeof(double), cudaMemcpyDeviceToHost,
-                               h->stream));
-  FMPT_CUDA(h, cudaStreamSynchronize(h->stream));
-  double b = h->pinned[0];
-  int k = 1;
-  int inf = 0;
-  if (!std::isfinite(b)) return set_error(h, FMPT_ERR_NONFINITE, "lanczos: beta is not finite");
-  if (b < btol) {
+  // Step j + 1 is queued before beta_j is looked at, so the device does not wait for the
+  // host's test (25 us per step at D = 64); one step past convergence is thrown away.
+  double al[128], be[128];
+  int k = 0;
+  bool converged = false;
+  FMPT_TRY(launch_step(0));
+  while (k < kmax && !converged) {
+    if (k + 1 < kmax) FMPT_TRY(launch_step(k + 1));
+    FMPT_CUDA(h, cudaEventSynchronize(h->step_event[k & 1]));
+    al[k] = ab[2 * k];
+    be[k] = ab[2 * k + 1];
+    if (!std::isfinite(be[k]))
+      return set_error(h, FMPT_ERR_NONFINITE, "lanczos: beta is not finite");
+    converged = be[k] < btol;
+    k++;
+  }
+  if (converged && k == 1) {
     // converged after the first step: Rayleigh quotient and the start vector
-    FMPT_CUDA(h, cudaMemcpyAsync(h->pinned, s_alpha, sizeof(double), cudaMemcpyDeviceToHost,
-                                 h->stream));
     FMPT_CUDA(h, cudaMemcpyAsync(xout, V_(0), n * sizeof(double), cudaMemcpyDeviceToDevice,
                                  h->stream));
-    FMPT_CUDA(h, cudaStreamSynchronize(h->stream));
-    *eigval = h->pinned[0];
-    if (info) *info = 0;
-    if (niter) *niter = 1;
-    return FMPT_OK;
+    *eigval = al[0];
+  } else {
+    // eigen(Symmetric(T[1:k,1:k])), lowest pair (find_lanczos "SR")
+    RitzCoef rc;
+    tridiag_lowest(k, al, be, eigval, rc.c);
+    combine_ritz<<<G, KT, 0, h->stream>>>(n, k, V, n, rc, xout);
+    FMPT_LAUNCHED(h);
   }
-  // y holds q_1 (normalised); move it into V_1
-  FMPT_CUDA(h, cudaMemcpyAsync(V_(1), y, n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-  bool converged = false;
-  while (k < kmax) {
-    // lanczos_make_step(A, V[k-1], V[k], beta[k-1])  (simple_lanczos.jl:49-68)
-    FMPT_TRY(fmpt_op_apply(op, V_(k), y));
-    rdot_partial<<<G, KT, 0, h->stream>>>(n, V_(k), y, partA.d());
-    FMPT_LAUNCHED(h);
-    lanczos_axpy<<<G, KT, 0, h->stream>>>(n, y, V_(k), V_(k - 1), partA.d(), G, s_beta + (k - 1),
-                                          s_alpha + k, partB.d());
-    FMPT_LAUNCHED(h);
-    if (reorth) FMPT_TRY(reorthogonalise(k + 1));
-    lanczos_scale<<<G, KT, 0, h->stream>>>(n, y, partB.d(), G, s_beta + k);
-    FMPT_LAUNCHED(h);
-    FMPT_CUDA(h, cudaMemcpyAsync(h->pinned, s_beta + k, sizeof(double), cudaMemcpyDeviceToHost,
-                                 h->stream));
-    FMPT_CUDA(h, cudaStreamSynchronize(h->stream));
-    b = h->pinned[0];
-    k += 1;
-    if (!std::isfinite(b)) return set_error(h, FMPT_ERR_NONFINITE, "lanczos: beta is not finite");
-    if (b < btol) { converged = true; break; }
-    if (k < kmax)
-      FMPT_CUDA(h, cudaMemcpyAsync(V_(k), y, n * sizeof(double), cudaMemcpyDeviceToDevice,
-                                   h->stream));
-  }
-  if (!converged) inf = -1;
-  // eigen(Symmetric(T[1:k,1:k])) on the device, lowest pair (find_lanczos "SR")
-  tridiag_lowest<<<1, 1, 0, h->stream>>>(k, s_alpha, s_beta, s_eval, s_evec);
-  FMPT_LAUNCHED(h);
-  combine_basis<<<G, KT, 0, h->stream>>>(0, n, k, V, n, s_evec, 1, 1.0, 1, xout);
-  FMPT_LAUNCHED(h);
-  FMPT_CUDA(h, cudaMemcpyAsync(h->pinned, s_eval, sizeof(double), cudaMemcpyDeviceToHost,
-                               h->stream));
-  FMPT_CUDA(h, cudaStreamSynchronize(h->stream));
-  *eigval = h->pinned[0];
   if (!prec_is_f64(op->precision)) FMPT_TRY(op_tc_check(op));
   if (op->u1) FMPT_TRY(gp_check_status(op->h));
-  if (info) *info = inf;
+  if (info) *info = converged ? 0 : -1;
   if (niter) *niter = k;
   return FMPT_OK;
 }
@@ -1505,7 +1493,7 @@ int fmpt_exponentiate(fmpt_op* op, double t_re, double t_im, const double* x, do
     FMPT_CUDA(h, cudaMemcpyAsync(Ed.d(), colbuf.data(), (size_t)2 * m * sizeof(double),
                                  cudaMemcpyHostToDevice, h->stream));
     // w = sum_i E[i, 0] V_i, renormalised into V_0; acc *= ||w||
-    combine_basis<<<G, KT, 0, h->stream>>>(cp, n, m, V, nr, Ed.d(), 2, 1.0, 0, zb.d());
+    combine_basis<<<G, KT, 0, h->stream>>>(cp, n, m, V, nr, Ed.d(), 2, 1.0, zb.d());
     FMPT_LAUNCHED(h);
     rdot_partial<<<G, KT, 0, h->stream>>>(nr, zb.d(), zb.d(), part.d());
     FMPT_LAUNCHED(h);
@@ -1607,7 +1595,7 @@ int fmpt_expm_nodes(fmpt_op* op, double t_re, double t_im, const double* x, int 
   for (int q = 0; q < nnodes; q++) {
     double* oq = out + (int64_t)q * nr;
     combine_basis<<<G, KT, 0, h->stream>>>(cp, n, m, V, nr, Ed.d() + (size_t)2 * m * q, 2, 1.0,
-                                           0, oq);
+                                             oq);
     FMPT_LAUNCHED(h);
     scale_by<<<G, KT, 0, h->stream>>>(nr, oq, acc.d());
     FMPT_LAUNCHED(h);
