@@ -43,7 +43,7 @@ struct fmpt_handle {
   // CUDA graphs for the Krylov solvers of block-sparse operators (fmpt_set_graphs)
   bool graphs = true;
   // Krylov exponentials: one cooperative launch per Arnoldi orthogonalisation step
-  // (fmpt_set_fused_krylov; the seven separate launches give bit-identical results)
+  // (fmpt_set_fused_krylov; the six separate launches give bit-identical results)
   int fused_gs = 1;
   // thin QR of small tall panels on one thread-block cluster (fmpt_set_cluster_qr)
   int cluster_qr = 1;

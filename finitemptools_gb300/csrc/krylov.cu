@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cmath>
 #include <complex>
+#include <mutex>
 #include <vector>
 
 #include "internal.h"
@@ -144,12 +145,10 @@ __global__ void lanczos_scale(int64_t n, const double* __restrict__ y,
 // shared-memory pass per chunk -- instead of one full block reduction per vector.  Fixed
 // summation order throughout (deterministic).
 constexpr int MD_CH = 8;
-template <int CH = MD_CH>
-__device__ __forceinline__ void multidot_body(int cplx, int64_t n, int j,
-                                              const double* __restrict__ V, int64_t vstride,
-                                              const double* __restrict__ z,
-                                              double* __restrict__ part, int epb = KT) {
-  constexpr int MD_CH = CH;       // vectors per pass over z (the sums do not depend on it)
+__global__ void multidot_partial(int cplx, int64_t n, int j, const double* __restrict__ V,
+                                 int64_t vstride, const double* __restrict__ z,
+                                 double* __restrict__ part, const int* gate = nullptr) {
+  if (gate && *gate) return;
   __shared__ double red[KT / 32][2 * MD_CH];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   for (int i0 = 0; i0 < j; i0 += MD_CH) {
@@ -159,8 +158,7 @@ __device__ __forceinline__ void multidot_body(int cplx, int64_t n, int j,
       sr[c] = 0.0;
       si[c] = 0.0;
     }
-    for (int64_t e = (int64_t)blockIdx.x * epb + threadIdx.x; threadIdx.x < epb && e < n;
-         e += (int64_t)gridDim.x * epb) {
+    for (int64_t e = (int64_t)blockIdx.x * KT + threadIdx.x; e < n; e += (int64_t)gridDim.x * KT) {
       const double zr = z[e], zi = cplx ? z[n + e] : 0.0;
 #pragma unroll
       for (int c = 0; c < MD_CH; c++) {
@@ -183,13 +181,8 @@ __device__ __forceinline__ void multidot_body(int cplx, int64_t n, int j,
       v[2 * c] = sr[c];
       v[2 * c + 1] = si[c];
     }
-    // warps past the block's elements hold zeros: they store them without the shuffle sums
-    const bool holds = wid * 32 < epb;
-    if (holds) warp_sum_many<2 * MD_CH>(v);
-    {
-      constexpr int sh = MD_CH == 16 ? 0 : (MD_CH == 8 ? 1 : (MD_CH == 4 ? 2 : 3));
-      if ((lane & ((1 << sh) - 1)) == 0) red[wid][lane >> sh] = holds ? v[0] : 0.0;
-    }
+    warp_sum_many<2 * MD_CH>(v);
+    if ((lane & 1) == 0) red[wid][lane >> 1] = v[0];        // 2 MD_CH = 16 values
     __syncthreads();
     if (threadIdx.x < 2 * MD_CH) {
       const int c = threadIdx.x >> 1;
@@ -201,21 +194,12 @@ __device__ __forceinline__ void multidot_body(int cplx, int64_t n, int j,
   }
 }
 
-__global__ void multidot_partial(int cplx, int64_t n, int j, const double* __restrict__ V,
-                                 int64_t vstride, const double* __restrict__ z,
-                                 double* __restrict__ part, const int* gate = nullptr,
-                                 int epb = KT) {
-  if (gate && *gate) return;
-  multidot_body<>(cplx, n, j, V, vstride, z, part, epb);
-}
-
 // coef[i] (re, im) = sum over the G partials, one warp per value (lanes stride over the
 // partials in a fixed order, then a shuffle sum); launched with one block of KT threads
 // Coefficients t0 .. t0 + 63 (t = 2 i + re/im) of the sums over the G partials [G][j][2]:
 // warp w takes t = t0 + w + 8 u (u < 8); a lane adds its partials g = lane, lane + 32, ...
 // in g order, then the warp sums its 8 values with warp_sum_many.  out[t] = the sum
-// (accum[t] += it when given).  QMAX > 0: at most QMAX partials per lane, loads unrolled.
-template <int QMAX>
+// (accum[t] += it when given).
 __device__ __forceinline__ void coef_group(int j, int G, const double* __restrict__ part, int t0,
                                            double* out, double* accum) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -226,15 +210,7 @@ __device__ __forceinline__ void coef_group(int j, int G, const double* __restric
     double sum = 0.0;
     if (t < 2 * j) {
       const int i = t >> 1, comp = t & 1;
-      if (QMAX > 0) {
-#pragma unroll
-        for (int q = 0; q < QMAX; q++) {
-          const int g = lane + 32 * q;
-          if (g < G) sum += part[((int64_t)g * j + i) * 2 + comp];
-        }
-      } else {
-        for (int g = lane; g < G; g += 32) sum += part[((int64_t)g * j + i) * 2 + comp];
-      }
+      for (int g = lane; g < G; g += 32) sum += part[((int64_t)g * j + i) * 2 + comp];
     }
     acc[u] = sum;
   }
@@ -251,17 +227,16 @@ __global__ void multidot_finalize(int j, int G, const double* __restrict__ part,
                                   double* __restrict__ coef, double* __restrict__ accum,
                                   const int* gate = nullptr) {
   if (gate && *gate) return;
-  for (int t0 = 0; t0 < 2 * j; t0 += 64) coef_group<0>(j, G, part, t0, coef, accum);
+  for (int t0 = 0; t0 < 2 * j; t0 += 64) coef_group(j, G, part, t0, coef, accum);
 }
 
-__device__ __forceinline__ void multi_axpy_body(int cplx, int64_t n, int j,
-                                                const double* __restrict__ V, int64_t vstride,
-                                                const double* __restrict__ coef,
-                                                double* __restrict__ z, double* __restrict__ part,
-                                                int epb = KT) {
+__global__ void multi_axpy_sub(int cplx, int64_t n, int j, const double* __restrict__ V,
+                               int64_t vstride, const double* __restrict__ coef,
+                               double* __restrict__ z, double* __restrict__ part,
+                               const int* gate = nullptr) {
+  if (gate && *gate) return;
   double s = 0.0;
-  for (int64_t e = (int64_t)blockIdx.x * epb + threadIdx.x; threadIdx.x < epb && e < n;
-       e += (int64_t)gridDim.x * epb) {
+  for (int64_t e = (int64_t)blockIdx.x * KT + threadIdx.x; e < n; e += (int64_t)gridDim.x * KT) {
     double zr = z[e], zi = cplx ? z[n + e] : 0.0;
     // MD_CH vectors' elements are loaded together (their L2 latencies overlap), then
     // subtracted in vector order
@@ -295,81 +270,328 @@ __device__ __forceinline__ void multi_axpy_body(int cplx, int64_t n, int j,
     s = fma(zr, zr, s);
     if (cplx) s = fma(zi, zi, s);
   }
-  s = block_sum(s, (epb + 31) / 32);
+  s = block_sum(s);
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
-__global__ void multi_axpy_sub(int cplx, int64_t n, int j, const double* __restrict__ V,
-                               int64_t vstride, const double* __restrict__ coef,
-                               double* __restrict__ z, double* __restrict__ part,
-                               const int* gate = nullptr, int epb = KT) {
-  if (gate && *gate) return;
-  multi_axpy_body(cplx, n, j, V, vstride, coef, z, part, epb);
-}
-
-// out = sum_i c_i V_i (c complex when cplx, real otherwise); scale multiplies
+// out_q = scale sum_i c_qi V_i for q = blockIdx.y (coefficients (re, im) pairs, cq = their
+// stride per q; scale a device scalar, or 1).  Eight vectors' elements are loaded together:
+// one at a time the sum is a chain of L2 latencies (21 us at 30 vectors, now 5).
 __global__ void combine_basis(int cplx, int64_t n, int j, const double* __restrict__ V,
-                              int64_t vstride, const double* __restrict__ c, int cstride,
-                              double scale, double* __restrict__ out) {
+                              int64_t vstride, const double* __restrict__ c, int64_t cq,
+                              const double* scale, double* __restrict__ out, int64_t oq) {
+  constexpr int U = 8;
+  c += blockIdx.y * cq;
+  out += blockIdx.y * oq;
+  const double f = scale ? *scale : 1.0;
   for (int64_t e = (int64_t)blockIdx.x * KT + threadIdx.x; e < n; e += (int64_t)gridDim.x * KT) {
     double r = 0.0, im = 0.0;
-    for (int i = 0; i < j; i++) {
-      const double* v = V + (int64_t)i * vstride;
-      double cr = c[i * cstride], ci = cplx ? c[i * cstride + 1] : 0.0;
-      double vr = v[e];
-      if (cplx) {
-        double vi = v[n + e];
-        r += cr * vr - ci * vi;
-        im += cr * vi + ci * vr;
-      } else {
-        r += cr * vr;
+    for (int i0 = 0; i0 < j; i0 += U) {
+      double vr[U], vi[U], cr[U], ci[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const bool in = i0 + u < j;
+        const double* v = V + (int64_t)(i0 + u) * vstride;
+        vr[u] = in ? v[e] : 0.0;
+        vi[u] = in && cplx ? v[n + e] : 0.0;
+        cr[u] = in ? c[2 * (i0 + u)] : 0.0;
+        ci[u] = in && cplx ? c[2 * (i0 + u) + 1] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        if (i0 + u >= j) break;
+        r = fma(cr[u], vr[u], r);
+        if (cplx) {
+          r = fma(-ci[u], vi[u], r);
+          im = fma(cr[u], vi[u], im);
+          im = fma(ci[u], vr[u], im);
+        }
       }
     }
-    out[e] = r * scale;
-    if (cplx) out[n + e] = im * scale;
+    out[e] = r * f;
+    if (cplx) out[n + e] = im * f;
   }
 }
 
-// Arnoldi step closure on the device: s = ||z|| after orthogonalisation; the
-// norm before it is sqrt(s^2 + sum_i |H[i][j]|^2).  If s is below 1e-12 of
-// that (the Krylov space is exhausted: happy breakdown) the next basis vector
-// and H[j+1][j] are zero, otherwise V_{j+1} = z / s and H[j+1][j] = s.
-__device__ __forceinline__ void arnoldi_normalize_body(int64_t n_real,
-                                                       const double* __restrict__ z,
-                                                       const double* __restrict__ part, int G,
-                                                       const double* hc, double* __restrict__ Hcol,
-                                                       int j, double* __restrict__ vnext,
-                                                       int epb = KT) {
-  const double s = sqrt(sum_parts(part, G));
-  double ref = s * s;
-  for (int i = 0; i <= j; i++) ref += hc[2 * i] * hc[2 * i] + hc[2 * i + 1] * hc[2 * i + 1];
-  const bool breakdown = !(s > 1e-12 * sqrt(ref));
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    Hcol[2 * (j + 1)] = breakdown ? 0.0 : s;
-    Hcol[2 * (j + 1) + 1] = 0.0;
+// ---- orthogonalisation step of one Arnoldi vector: two Gram-Schmidt passes of z against
+// V_0..V_j and the normalisation V_{j+1} = z / s.
+//
+// On GB300 an FP64 warp instruction occupies its SM sub-partition for about 60 cycles and a
+// dependent one waits about 200, so the step is bound by its chains of dependent FP64
+// instructions and by its grid-wide waits, not by the loads.  Hence
+// - a warp's unit is a chunk of 32 elements of ONE component (real or imaginary plane): two
+//   multiply-adds per lane and vector instead of four, twice as many warps at work;
+// - a block of 8 working warps holds cpb chunks (1, 2, 4 or 8), and 8 / cpb warps share a
+//   chunk, each taking every (8 / cpb)-th vector;
+// - sums run as independent chains or trees, over the values that exist;
+// - |z|^2 is one more value of each pass's dots: s^2 = |z|^2 - sum |c2|^2 after the second
+//   (c2 is of rounding size), which saves a third grid-wide wait;
+// - s and 1 / s are found by a ninth warp while the others form sum c_i V_i.
+// One step at n = 8192 complex, 16 vectors (D = 64, 128 blocks of 4 chunks): 26 us, half of it
+// the FP64 pipe, 1.4 us in each grid-wide wait; the form it replaces (both components of an
+// element per thread, a plain warp sum per block, three waits) took 38 us, and 45 on any
+// small vector, now about 15.
+constexpr int GS_T = 288;                      // 8 working warps and the closing one
+constexpr int GS_NV = 64;                      // values per pass: (re, im) per vector, |z|^2
+struct GsArgs {
+  int cplx, j;                                 // orthogonalise against V_0..V_j
+  int64_t n;                                   // elements (complex ones if cplx)
+  int cpb;                                     // chunks per block: 1, 2, 4, 8
+  const double* V;
+  int64_t vstride;
+  double* z;
+  double* part;                                // [2][GS_NV][G] block sums
+  double* Hcol;
+  double* vnext;
+};
+
+struct GsWarp {
+  int lane, wid, cs, vg, VG;
+  int64_t nch, S, step;
+  __device__ GsWarp(const GsArgs& a) {
+    lane = threadIdx.x & 31;
+    wid = threadIdx.x >> 5;
+    cs = wid % a.cpb;
+    vg = wid / a.cpb;
+    VG = 8 / a.cpb;
+    nch = (a.n + 31) / 32;
+    S = a.cplx ? 2 * nch : nch;
+    step = (int64_t)gridDim.x * a.cpb;
   }
-  const double inv = breakdown ? 0.0 : 1.0 / s;
-  for (int64_t e = (int64_t)blockIdx.x * epb + threadIdx.x; threadIdx.x < epb && e < n_real;
-       e += (int64_t)gridDim.x * epb)
-    vnext[e] = z[e] * inv;
+  // this warp's first chunk
+  __device__ int64_t first(const GsArgs& a) const { return (int64_t)blockIdx.x * a.cpb + cs; }
+  __device__ void locate(const GsArgs& a, int64_t ch, int& comp, int64_t& e, bool& in) const {
+    comp = ch >= nch ? 1 : 0;
+    e = (ch - (comp ? nch : 0)) * 32 + lane;
+    in = ch < S && e < a.n;
+  }
+};
+
+// r[0] + r[stride] + .. (n = 1, 2, 4, 8 terms) as a tree
+__device__ __forceinline__ double gs_tree(const double* r, int stride, int n) {
+  double x[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) x[k] = k < n ? r[k * stride] : 0.0;
+  if (n == 1) return x[0];
+  x[0] += x[1];
+  if (n == 2) return x[0];
+  x[2] += x[3];
+  x[0] += x[2];
+  if (n == 4) return x[0];
+  x[4] += x[5];
+  x[6] += x[7];
+  x[4] += x[6];
+  return x[0] + x[4];
 }
 
-__global__ void arnoldi_normalize(int64_t n_real, const double* __restrict__ z,
-                                  const double* __restrict__ part, int G,
-                                  double* __restrict__ Hcol, int j, double* __restrict__ vnext,
-                                  int epb = KT) {
-  arnoldi_normalize_body(n_real, z, part, G, Hcol, Hcol, j, vnext, epb);
+// Block sums bp[2 i], bp[2 i + 1] of conj(V_i) z over the block's chunks, bp[2 j + 2] of
+// |z|^2 (the dot with z itself, i = j + 1).  SINGLE: every warp has one chunk, zv is this
+// lane's element; otherwise the warps loop over chunks and read a.z.
+template <bool SINGLE>
+__device__ void gs_dots(const GsArgs& a, const GsWarp& w, double zv, double* bp) {
+  __shared__ double red[8][GS_NV];
+  constexpr int U = 8;
+  const int nvec = a.j + 2;
+  for (int i0 = w.vg; i0 < nvec && w.wid < 8; i0 += U * w.VG) {
+    double v[2 * U];
+#pragma unroll
+    for (int u = 0; u < 2 * U; u++) v[u] = 0.0;
+    for (int64_t ch = w.first(a); ch < w.S; ch += w.step) {
+      int comp;
+      int64_t e;
+      bool in;
+      w.locate(a, ch, comp, e, in);
+      const double z = SINGLE ? zv : (in ? a.z[comp * a.n + e] : 0.0);
+      double vs[U], vo[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int i = i0 + u * w.VG;
+        const double* p = a.V + (int64_t)i * a.vstride;
+        vs[u] = in && i <= a.j ? p[comp * a.n + e] : (i == a.j + 1 ? z : 0.0);
+        vo[u] = in && i <= a.j && a.cplx ? p[(1 - comp) * a.n + e] : 0.0;
+      }
+      // Re: vr zr + vi zi; Im: vr zi - vi zr
+      const double zo = comp ? z : -z;
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        if (i0 + u * w.VG < nvec) {
+          v[2 * u] = fma(vs[u], z, v[2 * u]);
+          if (a.cplx) v[2 * u + 1] = fma(vo[u], zo, v[2 * u + 1]);
+        }
+      }
+    }
+    // few vectors: fewer values to sum
+    const int left = (nvec - i0 + w.VG - 1) / w.VG;
+    if (left > 4) {
+      warp_sum_many<16>(v);
+    } else if (left > 1) {
+      double v8[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) v8[u] = v[u];
+      warp_sum_many<8>(v8);
+      v[0] = v8[0];
+    } else {
+      double v2[2] = {v[0], v[1]};
+      warp_sum_many<2>(v2);
+      v[0] = v2[0];
+    }
+    const int sh = left > 4 ? 1 : (left > 1 ? 2 : 4);
+    const int q = w.lane >> sh;                // value index: 2 u + component
+    const int i = i0 + (q >> 1) * w.VG;
+    if ((w.lane & ((1 << sh) - 1)) == 0 && i < nvec) red[w.cs][2 * i + (q & 1)] = v[0];
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < 2 * nvec - 1) bp[threadIdx.x] = gs_tree(&red[0][threadIdx.x], GS_NV, a.cpb);
+  __syncthreads();
 }
 
-// ---- the whole orthogonalisation step of one Arnoldi vector as ONE cooperative launch:
-// pass 1 (partial dots, barrier, coefficients, z -= V c), pass 2 (the same), barrier,
-// normalisation.  Every block computes the coefficients itself in the summation order of
-// multidot_finalize (coef_group), so the results are bit-identical to the seven separate
-// launches.  The
-// grid barriers are bounded (2 s on %globaltimer): a timeout sets the abort flag and the
-// handle's status word and every block returns.
+template <int K>
+__device__ __forceinline__ void gs_total_k(const double* part, int G, int nv, double* c) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  double x[K][4];
+#pragma unroll
+  for (int u = 0; u < K; u++)
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int t = wid + 8 * u, g = lane + 32 * q;
+      x[u][q] = t < nv && g < G ? __ldcg(part + (int64_t)t * G + g) : 0.0;
+    }
+  double v[K];
+#pragma unroll
+  for (int u = 0; u < K; u++) v[u] = x[u][0];
+  if (G > 32) {
+#pragma unroll
+    for (int u = 0; u < K; u++) v[u] += x[u][1];
+  }
+  if (G > 64) {
+#pragma unroll
+    for (int u = 0; u < K; u++) x[u][2] += x[u][3];
+#pragma unroll
+    for (int u = 0; u < K; u++) v[u] += x[u][2];
+  }
+  warp_sum_many<K>(v);
+  constexpr int sh = K == 8 ? 2 : (K == 4 ? 3 : (K == 2 ? 4 : 5));
+  const int t = wid + 8 * (lane >> sh);
+  if ((lane & ((1 << sh) - 1)) == 0 && t < nv) c[t] = v[0];
+}
+
+// sums over the G <= 128 blocks: c[t] for t < nv; warp w < 8 takes t = w + 8 u
+__device__ __forceinline__ void gs_total(const double* part, int G, int nv, double* c) {
+  const int wid = threadIdx.x >> 5;
+  const int mine = wid < 8 ? (nv - wid + 7) / 8 : 0;
+  if (mine > 4) gs_total_k<8>(part, G, nv, c);
+  else if (mine > 2) gs_total_k<4>(part, G, nv, c);
+  else if (mine > 1) gs_total_k<2>(part, G, nv, c);
+  else if (mine == 1) gs_total_k<1>(part, G, nv, c);
+}
+
+// sum over the vectors of this warp of -c_i V_i at its element of one component
+__device__ __forceinline__ double gs_correction(const GsArgs& a, const GsWarp& w, const double* c,
+                                                int comp, int64_t e, bool in) {
+  constexpr int U = 8;
+  const int jj = a.j + 1;
+  double p[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int i0 = w.vg; i0 < jj; i0 += U * w.VG) {
+    double vs[U], vo[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int i = i0 + u * w.VG;
+      const double* q = a.V + (int64_t)i * a.vstride;
+      vs[u] = in && i < jj ? q[comp * a.n + e] : 0.0;
+      vo[u] = in && i < jj && a.cplx ? q[(1 - comp) * a.n + e] : 0.0;
+    }
+    // Re: - (cr vr - ci vi); Im: - (cr vi + ci vr)
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int i = i0 + u * w.VG;
+      if (i < jj) {
+        p[u & 1] = fma(-c[2 * i], vs[u], p[u & 1]);
+        if (a.cplx) p[2 + (u & 1)] = fma(comp ? -c[2 * i + 1] : c[2 * i + 1], vo[u], p[2 + (u & 1)]);
+      }
+    }
+  }
+  if (!a.cplx) return p[0] + p[1];
+  return (p[0] + p[1]) + (p[2] + p[3]);
+}
+
+// The step's closure by one warp: hc = c1 + c2 into H's column, s from the second pass's
+// |z|^2.  If s is below 1e-12 of the norm before the step the Krylov space is exhausted
+// (happy breakdown) and V_{j+1}, H[j+1][j] are zero.  Returns 1 / s or 0.
+__device__ double gs_close(const GsArgs& a, const double* c1, const double* c2, bool write) {
+  const int lane = threadIdx.x & 31, jj = a.j + 1;
+  double q2 = 0.0;
+  for (int t = lane; t < 2 * jj; t += 32) {
+    q2 = fma(c2[t], c2[t], q2);
+    if (write) a.Hcol[t] = c1[t] + c2[t];
+  }
+  q2 = warp_sum(q2);
+  const double d = c2[2 * jj] - q2;
+  const double s2 = d < 0.0 ? 0.0 : d;                         // NaN stays
+  const bool breakdown = s2 <= 1e-24 * c1[2 * jj];
+  const double s = sqrt(s2);
+  if (write && lane == 0) {
+    a.Hcol[2 * jj] = breakdown ? 0.0 : s;
+    a.Hcol[2 * jj + 1] = 0.0;
+  }
+  return breakdown ? 0.0 : 1.0 / s;
+}
+
+// z - sum c_i V_i: SINGLE returns this lane's new element (the same in all warps of a
+// chunk), otherwise z is updated in place.  After the second pass (last) the result is
+// scaled by 1 / s and goes to V_{j+1}; close() runs on the ninth warp meanwhile and returns
+// 1 / s.
+template <bool SINGLE, class Close>
+__device__ double gs_axpy(const GsArgs& a, const GsWarp& w, const double* c, double zv, bool last,
+                          Close close) {
+  __shared__ double ps[8][32], s_inv;
+  int comp = 0;
+  int64_t e = 0;
+  bool in = false;
+  if (w.wid == 8) {
+    if (last) {
+      const double inv = close();
+      if (w.lane == 0) s_inv = inv;
+    }
+  } else if (SINGLE) {
+    w.locate(a, w.first(a), comp, e, in);
+    ps[w.wid][w.lane] = gs_correction(a, w, c, comp, e, in);
+  }
+  __syncthreads();
+  const double inv = last ? s_inv : 1.0;
+  if (w.wid == 8) return 0.0;
+  if constexpr (SINGLE) {
+    zv += gs_tree(&ps[w.cs][w.lane], 32 * a.cpb, w.VG);
+    if (last) zv *= inv;
+    if (last && w.vg == 0 && in) a.vnext[comp * a.n + e] = zv;
+    return zv;
+  } else {
+    for (int64_t ch = w.first(a); ch < w.S; ch += w.step) {    // cpb = 8: VG = 1
+      w.locate(a, ch, comp, e, in);
+      const double p = gs_correction(a, w, c, comp, e, in);
+      if (in) {
+        const double z = a.z[comp * a.n + e] + p;
+        if (last) a.vnext[comp * a.n + e] = z * inv;
+        else a.z[comp * a.n + e] = z;
+      }
+    }
+    return 0.0;
+  }
+}
+
+// this lane's element when every warp has one chunk
+__device__ __forceinline__ double gs_load(const GsArgs& a, const GsWarp& w) {
+  int comp;
+  int64_t e;
+  bool in;
+  w.locate(a, w.first(a), comp, e, in);
+  return in && w.wid < 8 ? a.z[comp * a.n + e] : 0.0;
+}
+
+// ---- the step as ONE cooperative launch.  Its grid-wide waits are bounded (2 s on
+// %globaltimer): a timeout sets the abort flag and the handle's status word and every block
+// returns.  The arrival counter runs on from step to step (target; zeroed once per basis).
 struct CoopBar {
-  int* count;        // arrivals (zeroed before each launch, in stream order)
+  int* count;        // arrivals
   int* abort_flag;
   int* status;       // handle status word
   uint64_t wait_ns;
@@ -388,12 +610,14 @@ __device__ __forceinline__ uint64_t now_ns() {
   return t;
 }
 
-__device__ bool coop_barrier(const CoopBar& b, int target) {
+// Every block has written its sums.  False: given up.  The block barriers order the block's
+// writes before its release and its reads after the acquire (cumulativity); the readers go
+// to L2 (__ldcg).
+__device__ bool gs_grid_wait(const CoopBar& b, int target) {
   __shared__ int ok_s;
   __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(b.count, 1);
+    asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(b.count) : "memory");
     int ok = 1;
     const uint64_t t0 = now_ns();
     // the count alone is polled; every 32nd poll also looks at the abort flag, the status
@@ -409,54 +633,75 @@ __device__ bool coop_barrier(const CoopBar& b, int target) {
         break;
       }
     }
-    __threadfence();
     ok_s = ok;
   }
   __syncthreads();
   return ok_s != 0;
 }
 
-template <int QMAX>
-__global__ void __launch_bounds__(KT) arnoldi_gs_fused(int cplx, int64_t n, int j,
-                                                       const double* __restrict__ V,
-                                                       int64_t vstride, double* __restrict__ z,
-                                                       double* __restrict__ partA,
-                                                       double* __restrict__ partB,
-                                                       double* __restrict__ partN,
-                                                       double* __restrict__ Hcol,
-                                                       double* __restrict__ vnext, CoopBar bar,
-                                                       int epb) {
-  __shared__ double c1[64], c2[64], hc[64];
-  const int G = gridDim.x, jj = j + 1;
-  // pass 1
-  multidot_body<16>(cplx, n, jj, V, vstride, z, partA, epb);
-  if (!coop_barrier(bar, G)) return;
-  coef_group<QMAX>(jj, G, partA, 0, c1, nullptr);     // 2 jj <= 62 values: one group
-  __syncthreads();
-  multi_axpy_body(cplx, n, jj, V, vstride, c1, z, partN, epb);
-  // pass 2 (each thread reads back only the elements it has just written)
-  multidot_body<16>(cplx, n, jj, V, vstride, z, partB, epb);
-  if (!coop_barrier(bar, 2 * G)) return;
-  coef_group<QMAX>(jj, G, partB, 0, c2, nullptr);
-  __syncthreads();
-  for (int t = threadIdx.x; t < 2 * jj; t += KT) {
-    hc[t] = (0.0 + c1[t]) + c2[t];    // the accumulation order of Hcol in the separate form
-    if (blockIdx.x == 0) Hcol[t] = hc[t];
+template <bool SINGLE>
+__global__ void __launch_bounds__(GS_T) arnoldi_gs_fused(GsArgs a, CoopBar bar) {
+  __shared__ double bp[GS_NV], c[2][GS_NV];
+  const GsWarp w(a);
+  const int G = gridDim.x, nv = 2 * a.j + 3;
+  double zv = SINGLE ? gs_load(a, w) : 0.0;
+  for (int pass = 0; pass < 2; pass++) {
+    double* part = a.part + (int64_t)pass * GS_NV * G;
+    if (G == 1) {
+      gs_dots<SINGLE>(a, w, zv, c[pass]);
+    } else {
+      gs_dots<SINGLE>(a, w, zv, bp);
+      if ((int)threadIdx.x < nv) part[(int64_t)threadIdx.x * G + blockIdx.x] = bp[threadIdx.x];
+      if (!gs_grid_wait(bar, (2 * a.j + pass + 1) * G)) return;
+      gs_total(part, G, nv, c[pass]);
+      __syncthreads();
+    }
+    zv = gs_axpy<SINGLE>(a, w, c[pass], zv, pass == 1,
+                         [&]() { return gs_close(a, c[0], c[1], blockIdx.x == 0); });
   }
-  __syncthreads();
-  multi_axpy_body(cplx, n, jj, V, vstride, c2, z, partN, epb);
-  if (!coop_barrier(bar, 3 * G)) return;
-  arnoldi_normalize_body(n * (cplx ? 2 : 1), z, partN, G, hc, Hcol, j, vnext, epb);
 }
 
-// the kernel instance for a grid of G blocks (partials per lane: G / 32 rounded up)
-using GsKernel = void (*)(int, int64_t, int, const double*, int64_t, double*, double*, double*,
-                          double*, double*, double*, CoopBar, int);
-GsKernel gs_kernel_for(int G) {
-  if (G <= 64) return arnoldi_gs_fused<2>;
-  if (G <= 160) return arnoldi_gs_fused<5>;
-  if (G <= 320) return arnoldi_gs_fused<10>;
-  return arnoldi_gs_fused<19>;                 // G <= 608 = 4 blocks x 152 SMs
+// ---- the same step as six launches (fmpt_set_fused_krylov off): the same device functions
+// on the same grid, so the same sums
+template <bool SINGLE>
+__global__ void __launch_bounds__(GS_T) arnoldi_gs_dots(GsArgs a, int pass) {
+  __shared__ double bp[GS_NV];
+  const GsWarp w(a);
+  gs_dots<SINGLE>(a, w, SINGLE ? gs_load(a, w) : 0.0, bp);
+  double* part = a.part + (int64_t)pass * GS_NV * gridDim.x;
+  if ((int)threadIdx.x < 2 * a.j + 3)
+    part[(int64_t)threadIdx.x * gridDim.x + blockIdx.x] = bp[threadIdx.x];
+}
+
+// one block: totals c[pass], after the second pass also H's column and 1 / s
+__global__ void __launch_bounds__(GS_T) arnoldi_gs_sums(GsArgs a, int pass, int G, double* coef) {
+  __shared__ double c[2][GS_NV];
+  const int nv = 2 * a.j + 3;
+  gs_total(a.part + (int64_t)pass * GS_NV * G, G, nv, c[1]);
+  __syncthreads();
+  for (int t = threadIdx.x; t < nv; t += GS_T) {
+    coef[pass * GS_NV + t] = c[1][t];
+    c[0][t] = coef[t];
+  }
+  __syncthreads();
+  if (pass == 1 && threadIdx.x < 32) {
+    const double inv = gs_close(a, c[0], c[1], true);
+    if (threadIdx.x == 0) coef[2 * GS_NV] = inv;
+  }
+}
+
+template <bool SINGLE>
+__global__ void __launch_bounds__(GS_T) arnoldi_gs_axpy(GsArgs a, int pass, const double* coef) {
+  const GsWarp w(a);
+  const double zv = gs_axpy<SINGLE>(a, w, coef + pass * GS_NV, SINGLE ? gs_load(a, w) : 0.0,
+                                    pass == 1, [&]() { return coef[2 * GS_NV]; });
+  if (SINGLE && pass == 0 && w.wid < 8 && w.vg == 0) {
+    int comp;
+    int64_t e;
+    bool in;
+    w.locate(a, w.first(a), comp, e, in);
+    if (in) a.z[comp * a.n + e] = zv;
+  }
 }
 
 // acc *= v (device scalars)
@@ -1096,63 +1341,119 @@ int op_project(fmpt_op* op, double* y, const int* gate) {
   return FMPT_OK;
 }
 
-// Grid of the Arnoldi orthogonalisation kernels: EPB_A vector elements (complex elements
-// for complex data) per block and pass.  A D = 64 vector (8192 elements) runs on 64 blocks
-// whose four element-holding warps spread over the SM's four FP64 sub-partitions (one
-// exponential of 20 vectors: 1.92 ms, against 1.97 ms with 64 elements per block on 128
-// SMs and 2.18 ms with 32); at most two blocks per SM.
-constexpr int EPB_A = 128;
-int arnoldi_grid(fmpt_handle* h, int64_t n) {
-  const int64_t g = (n + EPB_A - 1) / EPB_A;
-  const int64_t cap = 2LL * std::max(1, h->sm_count);
-  return (int)std::max<int64_t>(1, std::min(g, cap));
-}
-
-// Workspace of the fused orthogonalisation step (arnoldi_gs_fused): the pass-2 partials
-// (pass 1 uses the caller's partM), the barrier words and the status word.
+// Workspace and launch shape of the Arnoldi orthogonalisation step.
 struct GsWork {
-  double* partB;
+  int G, cpb;
+  bool single;        // every warp has one chunk
+  bool fused;         // one cooperative launch per step
+  double* part;       // [2][GS_NV][G]
+  double* coef;       // [2 GS_NV + 1] (separate launches)
   int* bar;
   int* status;
   uint64_t wait_ns;
   int hold;
 };
 
-// Whether G blocks of arnoldi_gs_fused are co-resident on this device (the cooperative
-// launch needs it); measured once per device.
+// Blocks of the step and chunks per block for S chunks: one block, without grid-wide waits,
+// up to 4 chunks; then as few chunks per block as keep it within 128 blocks (n = 8192
+// complex: 4 chunks, one per SM sub-partition); beyond 1024 chunks the warps loop.
+void gs_geometry(int64_t S, int& G, int& cpb, bool& single) {
+  single = true;
+  if (S <= 4) {
+    G = 1;
+    cpb = S <= 1 ? 1 : (S <= 2 ? 2 : 4);
+    return;
+  }
+  for (cpb = 1; cpb <= 8; cpb *= 2)
+    if ((S + cpb - 1) / cpb <= 128) {
+      G = (int)((S + cpb - 1) / cpb);
+      return;
+    }
+  cpb = 8;
+  G = 128;
+  single = false;
+}
+
+// Whether G blocks of the fused step are co-resident on this device (the cooperative launch
+// needs it); measured once per device.
 bool gs_fused_fits(fmpt_handle* h, int G) {
+  static std::mutex mu;
   static int occ[64] = {};
   static bool done[64] = {};
   const int dev = h->device;
   if (dev < 0 || dev >= 64) return false;
+  std::lock_guard<std::mutex> lock(mu);
   if (!done[dev]) {
-    int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, arnoldi_gs_fused<19>, KT, 0) !=
-        cudaSuccess) {
+    int a = 0, b = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, arnoldi_gs_fused<true>, GS_T, 0) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, arnoldi_gs_fused<false>, GS_T, 0) !=
+            cudaSuccess) {
       cudaGetLastError();
-      b = 0;
+      a = b = 0;
     }
-    occ[dev] = b;
+    occ[dev] = std::min(a, b);
     done[dev] = true;
   }
   return (int64_t)occ[dev] * h->sm_count >= G;
 }
 
-// Set up the fused step's workspace in `buf` (allocated here) when it applies: enabled on
-// the handle (fmpt_set_fused_krylov), a co-resident grid and a Krylov space of at most 31
-// vectors.  gs stays null otherwise (the separate launches run).
-int gs_setup(fmpt_op* op, int G, int M, DevBuf& buf, GsWork& w, const GsWork** gs) {
-  fmpt_handle* h = op->h;
-  *gs = nullptr;
-  if (!h->fused_gs || M > 31 || !gs_fused_fits(h, G)) return FMPT_OK;
-  const size_t nb = (size_t)G * (M + 1) * 2 * sizeof(double);
-  FMPT_TRY(buf.alloc(h, nb + 16 * sizeof(int)));
-  w.partB = buf.d();
-  w.bar = reinterpret_cast<int*>(static_cast<char*>(buf.p) + nb);
+int gs_setup(fmpt_handle* h, int cp, int64_t n, int M, DevBuf& buf, GsWork& w) {
+  const int64_t nch = (n + 31) / 32;
+  gs_geometry(cp ? 2 * nch : nch, w.G, w.cpb, w.single);
+  w.fused = h->fused_gs && gs_fused_fits(h, w.G);
+  const size_t parts = (size_t)2 * GS_NV * w.G;
+  FMPT_TRY(buf.alloc(h, (parts + 2 * GS_NV + 2 + 2) * sizeof(double)));
+  w.part = buf.d();
+  w.coef = w.part + parts;
+  w.bar = reinterpret_cast<int*>(w.coef + 2 * GS_NV + 2);
   FMPT_TRY(gp_status_word(h, &w.status));
   w.wait_ns = h->wait_test_ns > 0 ? (uint64_t)h->wait_test_ns : 2000000000ull;
   w.hold = h->wait_test_hold;
-  *gs = &w;
+  return FMPT_OK;
+}
+
+// V_{j+1} and H's column j from z = op(V_j)
+int gs_step(fmpt_handle* h, const GsWork& w, int cp, int64_t n, int64_t nr, int j, double* V,
+            double* z, double* Hcol) {
+  cudaStream_t st = h->stream;
+  GsArgs a{};
+  a.cplx = cp;
+  a.j = j;
+  a.n = n;
+  a.cpb = w.cpb;
+  a.V = V;
+  a.vstride = nr;
+  a.z = z;
+  a.part = w.part;
+  a.Hcol = Hcol;
+  a.vnext = V + (int64_t)(j + 1) * nr;
+  if (w.fused) {
+    const CoopBar bar{w.bar, w.bar + 1, w.status, w.wait_ns, w.hold};
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(w.G);
+    cfg.blockDim = dim3(GS_T);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    FMPT_CUDA(h, w.single ? cudaLaunchKernelEx(&cfg, arnoldi_gs_fused<true>, a, bar)
+                          : cudaLaunchKernelEx(&cfg, arnoldi_gs_fused<false>, a, bar));
+    FMPT_LAUNCHED(h);
+    return FMPT_OK;
+  }
+  for (int pass = 0; pass < 2; pass++) {
+    if (w.single) arnoldi_gs_dots<true><<<w.G, GS_T, 0, st>>>(a, pass);
+    else arnoldi_gs_dots<false><<<w.G, GS_T, 0, st>>>(a, pass);
+    FMPT_LAUNCHED(h);
+    arnoldi_gs_sums<<<1, GS_T, 0, st>>>(a, pass, w.G, w.coef);
+    FMPT_LAUNCHED(h);
+    if (w.single) arnoldi_gs_axpy<true><<<w.G, GS_T, 0, st>>>(a, pass, w.coef);
+    else arnoldi_gs_axpy<false><<<w.G, GS_T, 0, st>>>(a, pass, w.coef);
+    FMPT_LAUNCHED(h);
+  }
   return FMPT_OK;
 }
 
@@ -1164,44 +1465,16 @@ int gs_setup(fmpt_op* op, int G, int M, DevBuf& buf, GsWork& w, const GsWork** g
 // vector.  Any capture, instantiation, update or launch failure -- the first call on a
 // fresh operator among them, whose scratch is sized outside capture -- runs the same
 // launches directly.
-int arnoldi_basis(fmpt_op* op, int cp, int64_t n, int64_t nr, int G, int M, int ldh, double* V,
-                  double* z, double* part, double* partM, double* coef, DevBuf& Hdev,
-                  const GsWork* gs) {
+int arnoldi_basis(fmpt_op* op, int cp, int64_t n, int64_t nr, int M, int ldh, double* V,
+                  double* z, DevBuf& Hdev, const GsWork& gs) {
   fmpt_handle* h = op->h;
   cudaStream_t st = h->stream;
   auto record = [&]() -> int {
     FMPT_CUDA(h, cudaMemsetAsync(Hdev.p, 0, Hdev.bytes, st));
+    if (gs.fused) FMPT_CUDA(h, cudaMemsetAsync(gs.bar, 0, 2 * sizeof(int), st));
     for (int j = 0; j < M; j++) {
-      double* Hcol = Hdev.d() + (size_t)2 * ldh * j;
-      double* vj = V + (int64_t)j * nr;
-      FMPT_TRY(fmpt_op_apply(op, vj, z));
-      if (gs) {
-        FMPT_CUDA(h, cudaMemsetAsync(gs->bar, 0, 2 * sizeof(int), st));
-        CoopBar bar{gs->bar, gs->bar + 1, gs->status, gs->wait_ns, gs->hold};
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(G);
-        cfg.blockDim = dim3(KT);
-        cfg.stream = st;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeCooperative;
-        attr[0].val.cooperative = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        FMPT_CUDA(h, cudaLaunchKernelEx(&cfg, gs_kernel_for(G), cp, n, j, (const double*)V, nr,
-                                        z, partM, gs->partB, part, Hcol, vj + nr, bar, EPB_A));
-        FMPT_LAUNCHED(h);
-        continue;
-      }
-      for (int pass = 0; pass < 2; pass++) {
-        multidot_partial<<<G, KT, 0, st>>>(cp, n, j + 1, V, nr, z, partM, nullptr, EPB_A);
-        FMPT_LAUNCHED(h);
-        multidot_finalize<<<1, KT, 0, st>>>(j + 1, G, partM, coef, Hcol);
-        FMPT_LAUNCHED(h);
-        multi_axpy_sub<<<G, KT, 0, st>>>(cp, n, j + 1, V, nr, coef, z, part, nullptr, EPB_A);
-        FMPT_LAUNCHED(h);
-      }
-      arnoldi_normalize<<<G, KT, 0, st>>>(nr, z, part, G, Hcol, j, vj + nr, EPB_A);
-      FMPT_LAUNCHED(h);
+      FMPT_TRY(fmpt_op_apply(op, V + (int64_t)j * nr, z));
+      FMPT_TRY(gs_step(h, gs, cp, n, nr, j, V, z, Hdev.d() + (size_t)2 * ldh * j));
     }
     return FMPT_OK;
   };
@@ -1225,7 +1498,7 @@ int arnoldi_basis(fmpt_op* op, int cp, int64_t n, int64_t nr, int G, int M, int 
   }
   char key[96];
   std::snprintf(key, sizeof(key), "k%d p%d c%d u%d q%zu M%d g%d", op->kind, op->precision, cp,
-                op->u1 ? 1 : 0, op->proj.size(), M, gs ? 1 : 0);
+                op->u1 ? 1 : 0, op->proj.size(), M, gs.fused ? 1 : 0);
   cudaGraphExec_t& ex = h->arnoldi_exec[key];
   bool ready = false;
   if (ex) {
@@ -1410,16 +1683,13 @@ int fmpt_exponentiate(fmpt_op* op, double t_re, double t_im, const double* x, do
   const int64_t n = op->n;                     // elements (complex for C128)
   const int64_t nr = n * (cp ? 2 : 1);         // real view
   const int G = grid_for(h, nr);
-  const int Ga = arnoldi_grid(h, n);           // grid of the orthogonalisation kernels
   // the Krylov space cannot be larger than the vector space
   const int M = (int)std::min<int64_t>(krylovdim, n);
   const int ldh = M + 1;
-  DevBuf Vb, zb, part, partM, coef, Hdev, Ed, nrm, acc;
+  DevBuf Vb, zb, part, Hdev, Ed, nrm, acc;
   FMPT_TRY(Vb.alloc(h, (size_t)(M + 1) * nr * sizeof(double)));
   FMPT_TRY(zb.alloc(h, (size_t)nr * sizeof(double)));
-  FMPT_TRY(part.alloc(h, (size_t)std::max(G, Ga) * sizeof(double)));
-  FMPT_TRY(partM.alloc(h, (size_t)Ga * (M + 1) * 2 * sizeof(double)));
-  FMPT_TRY(coef.alloc(h, (size_t)(M + 1) * 2 * sizeof(double)));
+  FMPT_TRY(part.alloc(h, (size_t)G * sizeof(double)));
   FMPT_TRY(Hdev.alloc(h, (size_t)ldh * M * 2 * sizeof(double)));
   FMPT_TRY(Ed.alloc(h, (size_t)M * 2 * sizeof(double)));
   std::vector<double> colbuf((size_t)2 * M);
@@ -1427,9 +1697,8 @@ int fmpt_exponentiate(fmpt_op* op, double t_re, double t_im, const double* x, do
   FMPT_TRY(acc.alloc(h, 2 * sizeof(double)));
   FMPT_TRY(ensure_pinned(h, (size_t)ldh * M * 2 + 8));
   DevBuf gsbuf;
-  GsWork gsw{};
-  const GsWork* gs = nullptr;
-  FMPT_TRY(gs_setup(op, Ga, M, gsbuf, gsw, &gs));
+  GsWork gs{};
+  FMPT_TRY(gs_setup(h, cp, n, M, gsbuf, gs));
   double* V = Vb.d();
   auto V_ = [&](int i) { return V + (int64_t)i * nr; };
   const double tabs = std::hypot(t_re, t_im);
@@ -1452,12 +1721,11 @@ int fmpt_exponentiate(fmpt_op* op, double t_re, double t_im, const double* x, do
   while (tau_done < tabs * (1.0 - 1e-15)) {
     if (++steps > 1000) return set_error(h, FMPT_ERR_NOCONV, "exponentiate: too many steps");
     // ---- Arnoldi (two-pass classical Gram-Schmidt) entirely on the device
-    FMPT_TRY(arnoldi_basis(op, cp, n, nr, Ga, M, ldh, V, zb.d(), part.d(), partM.d(), coef.d(),
-                           Hdev, gs));
+    FMPT_TRY(arnoldi_basis(op, cp, n, nr, M, ldh, V, zb.d(), Hdev, gs));
     FMPT_CUDA(h, cudaMemcpyAsync(h->pinned, Hdev.p, Hdev.bytes, cudaMemcpyDeviceToHost,
                                  h->stream));
     FMPT_CUDA(h, cudaStreamSynchronize(h->stream));
-    if (gs) FMPT_TRY(gp_check_status(h));     // a fused step that gave up left H invalid
+    if (gs.fused) FMPT_TRY(gp_check_status(h));     // a fused step that gave up left H invalid
     std::copy(h->pinned, h->pinned + Hh.size(), Hh.begin());
     for (double v : Hh)
       if (!std::isfinite(v)) return set_error(h, FMPT_ERR_NONFINITE, "exponentiate: NaN");
@@ -1493,7 +1761,7 @@ int fmpt_exponentiate(fmpt_op* op, double t_re, double t_im, const double* x, do
     FMPT_CUDA(h, cudaMemcpyAsync(Ed.d(), colbuf.data(), (size_t)2 * m * sizeof(double),
                                  cudaMemcpyHostToDevice, h->stream));
     // w = sum_i E[i, 0] V_i, renormalised into V_0; acc *= ||w||
-    combine_basis<<<G, KT, 0, h->stream>>>(cp, n, m, V, nr, Ed.d(), 2, 1.0, zb.d());
+    combine_basis<<<G, KT, 0, h->stream>>>(cp, n, m, V, nr, Ed.d(), 0, nullptr, zb.d(), 0);
     FMPT_LAUNCHED(h);
     rdot_partial<<<G, KT, 0, h->stream>>>(nr, zb.d(), zb.d(), part.d());
     FMPT_LAUNCHED(h);
@@ -1510,7 +1778,7 @@ int fmpt_exponentiate(fmpt_op* op, double t_re, double t_im, const double* x, do
   scale_by<<<G, KT, 0, h->stream>>>(nr, xout, acc.d());
   FMPT_LAUNCHED(h);
   if (!prec_is_f64(op->precision)) FMPT_TRY(op_tc_check(op));
-  if (op->u1 || gs) FMPT_TRY(gp_check_status(op->h));
+  if (op->u1 || gs.fused) FMPT_TRY(gp_check_status(op->h));
   if (info) *info = steps;
   return FMPT_OK;
 }
@@ -1533,35 +1801,30 @@ int fmpt_expm_nodes(fmpt_op* op, double t_re, double t_im, const double* x, int 
   const int64_t n = op->n;
   const int64_t nr = n * (cp ? 2 : 1);
   const int G = grid_for(h, nr);
-  const int Ga = arnoldi_grid(h, n);           // grid of the orthogonalisation kernels
   const int M = (int)std::min<int64_t>(krylovdim, n);
   const int ldh = M + 1;
-  DevBuf Vb, zb, part, partM, coef, Hdev, Ed, acc;
+  DevBuf Vb, zb, part, Hdev, Ed, acc;
   FMPT_TRY(Vb.alloc(h, (size_t)(M + 1) * nr * sizeof(double)));
   FMPT_TRY(zb.alloc(h, (size_t)nr * sizeof(double)));
-  FMPT_TRY(part.alloc(h, (size_t)std::max(G, Ga) * sizeof(double)));
-  FMPT_TRY(partM.alloc(h, (size_t)Ga * (M + 1) * 2 * sizeof(double)));
-  FMPT_TRY(coef.alloc(h, (size_t)(M + 1) * 2 * sizeof(double)));
+  FMPT_TRY(part.alloc(h, (size_t)G * sizeof(double)));
   FMPT_TRY(Hdev.alloc(h, (size_t)ldh * M * 2 * sizeof(double)));
   FMPT_TRY(Ed.alloc(h, (size_t)nnodes * M * 2 * sizeof(double)));
   FMPT_TRY(acc.alloc(h, 2 * sizeof(double)));
   FMPT_TRY(ensure_pinned(h, (size_t)ldh * M * 2 + 8));
   DevBuf gsbuf;
-  GsWork gsw{};
-  const GsWork* gs = nullptr;
-  FMPT_TRY(gs_setup(op, Ga, M, gsbuf, gsw, &gs));
+  GsWork gs{};
+  FMPT_TRY(gs_setup(h, cp, n, M, gsbuf, gs));
   double* V = Vb.d();
   auto V_ = [&](int i) { return V + (int64_t)i * nr; };
   rdot_partial<<<G, KT, 0, h->stream>>>(nr, x, x, part.d());
   FMPT_LAUNCHED(h);
   normalize_from_parts<<<G, KT, 0, h->stream>>>(nr, x, V_(0), part.d(), G, acc.d());
   FMPT_LAUNCHED(h);
-  FMPT_TRY(arnoldi_basis(op, cp, n, nr, Ga, M, ldh, V, zb.d(), part.d(), partM.d(), coef.d(),
-                         Hdev, gs));
+  FMPT_TRY(arnoldi_basis(op, cp, n, nr, M, ldh, V, zb.d(), Hdev, gs));
   std::vector<double> Hh((size_t)ldh * M * 2);
   FMPT_CUDA(h, cudaMemcpyAsync(h->pinned, Hdev.p, Hdev.bytes, cudaMemcpyDeviceToHost, h->stream));
   FMPT_CUDA(h, cudaStreamSynchronize(h->stream));
-  if (gs) FMPT_TRY(gp_check_status(h));       // a fused step that gave up left H invalid
+  if (gs.fused) FMPT_TRY(gp_check_status(h));       // a fused step that gave up left H invalid
   std::copy(h->pinned, h->pinned + Hh.size(), Hh.begin());
   for (double v : Hh)
     if (!std::isfinite(v)) return set_error(h, FMPT_ERR_NONFINITE, "expm_nodes: NaN");
@@ -1592,17 +1855,12 @@ int fmpt_expm_nodes(fmpt_op* op, double t_re, double t_im, const double* x, int 
   }
   FMPT_CUDA(h, cudaMemcpyAsync(Ed.d(), cols.data(), cols.size() * sizeof(double),
                                cudaMemcpyHostToDevice, h->stream));
-  for (int q = 0; q < nnodes; q++) {
-    double* oq = out + (int64_t)q * nr;
-    combine_basis<<<G, KT, 0, h->stream>>>(cp, n, m, V, nr, Ed.d() + (size_t)2 * m * q, 2, 1.0,
-                                             oq);
-    FMPT_LAUNCHED(h);
-    scale_by<<<G, KT, 0, h->stream>>>(nr, oq, acc.d());
-    FMPT_LAUNCHED(h);
-  }
+  combine_basis<<<dim3(G, nnodes), KT, 0, h->stream>>>(cp, n, m, V, nr, Ed.d(), 2 * m, acc.d(), out,
+                                                       nr);
+  FMPT_LAUNCHED(h);
   if (err_est) *err_est = e;
   if (!prec_is_f64(op->precision)) FMPT_TRY(op_tc_check(op));
-  if (op->u1 || gs) FMPT_TRY(gp_check_status(op->h));
+  if (op->u1 || gs.fused) FMPT_TRY(gp_check_status(op->h));
   return FMPT_OK;
 }
 

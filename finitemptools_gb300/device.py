@@ -64,7 +64,7 @@ class Handle:
 
     def set_fused_krylov(self, on=True):
         """One cooperative launch per Arnoldi orthogonalisation step of the Krylov
-        exponentials (default on); off: seven launches, bit-identical results."""
+        exponentials (default on); off: six launches, bit-identical results."""
         self.check(lib().fmpt_set_fused_krylov(self.ptr, 1 if on else 0))
 
     def set_cluster_qr(self, on=True):

@@ -98,8 +98,8 @@ int fmpt_set_graphs(fmpt_handle* h, int on);
 uint64_t fmpt_graph_launch_count(fmpt_handle* h);
 /* Krylov exponentials (fmpt_exponentiate, fmpt_expm_nodes): on (default), each
  * Arnoldi vector's two-pass Gram-Schmidt orthogonalisation and normalisation
- * run as ONE cooperative launch with bounded grid barriers instead of seven
- * launches; off, the seven launches.  Both give bit-identical results.  No
+ * run as ONE cooperative launch with bounded grid barriers instead of six
+ * launches; off, the six launches.  Both give bit-identical results.  No
  * counterpart in the reference. */
 int fmpt_set_fused_krylov(fmpt_handle* h, int on);
 /* Thin QR (fmpt_qr, fmpt_lq, leftorth!/rightorth) of small tall panels: on
