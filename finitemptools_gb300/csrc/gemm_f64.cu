@@ -1,12 +1,13 @@
 // Plain FP64 (and split-plane complex FP64) GEMM on the CUDA cores.
 //
-// GB300's FP64 rate is small (about 2 DFMA per clock per SM), so this kernel
-// is FP64-pipe bound for every shape that matters, and what decides its speed
-// is how evenly it spreads the multiply-adds over the SMs.  Large problems use a
-// 64x64 tile with a 4x4 register block per thread.  Small ones (the D <= 128
-// contractions of TDVP and of the first DMRG bonds) use 32x32 or 16x16 tiles
-// and may split K over the grid; a cost model picks the tile and the split that
-// put the fewest multiply-adds on the busiest SM.  Every split writes its
+// GB300's FP64 rate is small: a warp's FMA occupies its SM sub-partition for 64 to
+// 77 cycles, dependent or not, so these kernels are FP64-pipe bound for every shape
+// that matters, and what decides their speed is how evenly they spread the
+// multiply-adds over the 608 sub-partitions.  Large problems use a 64x64 tile with a
+// 4x4 register block per thread (gemm_kernel).  Small ones (the D <= 128
+// contractions of TDVP and of the first DMRG bonds) give every warp an 8x4 tile
+// straight from L1/L2 (gemm_warp) and may split K over the grid; a cost model picks
+// the split.  Every split writes its
 // partial product to a workspace; the last split of a tile to finish (an atomic
 // count per tile) sums the tile's partials in split order, so the result does
 // not depend on scheduling, applies alpha/beta and resets the count.  Where no
@@ -227,6 +228,160 @@ __global__ void __launch_bounds__(NT) gemm_kernel(GemmArgs g, int splits, int kc
   }
 }
 
+// Small problems: one warp per 8 x 4 tile of C (complex: one for the real and one for the
+// imaginary part), one output per lane, two warps per block: the small unit of work fills
+// the 608 sub-partitions evenly.  A 16x16 tile per block of eight warps left a D = 64
+// contraction (320 x 256 x 64) on 3 blocks or 2 per SM, with two barriers and a load latency
+// per 8-deep slab.  Here the operands stream through a ring of WST slabs of WK by cp.async
+// (the whole K of a small contraction is in flight at once: one latency, not one per slab).
+// Each output is the same chain of FMAs over k as in gemm_kernel.  Per contraction, D = 64:
+// real 16.1 and 20.4 -> 14.6 and 17.8 us (FP64 pipe 80% busy), complex 24.2 and 22.8 ->
+// 17.7 and 18.2 us.
+constexpr int WM = 8, WN = 4, WWARPS = 2, WK = 32, WST = 4;
+
+// 8 bytes, zeros if !in
+__device__ __forceinline__ void cp_async8z(double* dst, const double* src, bool in) {
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src),
+               "r"(in ? 8 : 0)
+               : "memory");
+}
+
+template <bool CPLX>
+__global__ void __launch_bounds__(32 * WWARPS) gemm_warp(GemmArgs g, int splits, int kchunk,
+                                                         double* __restrict__ ws,
+                                                         int* __restrict__ tile_cnt) {
+  constexpr int NP = CPLX ? 2 : 1;                       // planes
+  // the ring belongs to a warp (real) or to the two warps of a tile (complex): T threads
+  constexpr int T = CPLX ? 64 : 32, RINGS = CPLX ? 1 : WWARPS;
+  __shared__ double As[RINGS][WST][NP][WK][WM], Bs[RINGS][WST][NP][WK][WN];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int t = threadIdx.x % T, ring = CPLX ? 0 : wid;
+  const int comp = CPLX ? wid : 0;                       // the part of C this warp forms
+  const int mt = CPLX ? blockIdx.x : blockIdx.x * WWARPS + wid;
+  const int m0 = mt * WM, n0 = blockIdx.y * WN;
+  const int lm = lane & 7, ln = lane >> 3;
+  const int gm = m0 + lm, gn = n0 + ln;
+  const int zb = blockIdx.z / splits, sp = blockIdx.z % splits;
+  const int k_lo = sp * kchunk, k_hi = min(g.k, k_lo + kchunk);
+  const int K = max(0, k_hi - k_lo), nslab = (K + WK - 1) / WK;
+  const bool live = gm < g.m && gn < g.n;
+  // This thread's elements of a slab: (mm, kk) of A, (kk, nn) of B, the first ones here and
+  // the next ones a fixed step on, so that lanes run along the contiguous index.
+  const bool a_mfast = g.ta == 0 || g.ta == 3, b_kfast = g.tb == 0 || g.tb == 3;
+  const int amm = a_mfast ? t % WM : t / WK, akk = a_mfast ? t / WM : t % WK;
+  const int adm = a_mfast ? 0 : T / WK, adk = a_mfast ? T / WM : 0;
+  const int bnn = b_kfast ? t / WK : t % WN, bkk = b_kfast ? t % WK : t / WN;
+  const int bdn = b_kfast ? T / WK : 0, bdk = b_kfast ? 0 : T / WN;
+  const int64_t sam = a_mfast ? 1 : g.lda, sak = a_mfast ? g.lda : 1;
+  const int64_t sbk = b_kfast ? 1 : g.ldb, sbn = b_kfast ? g.ldb : 1;
+  const double* A = g.A + zb * g.strideA + (m0 + amm) * sam + (k_lo + akk) * sak;
+  const double* B = g.B + zb * g.strideB + (n0 + bnn) * sbn + (k_lo + bkk) * sbk;
+  const int64_t ai_step = adm * sam + adk * sak, bi_step = bdn * sbn + bdk * sbk;
+  auto issue = [&](int j) {
+    if (j < nslab) {
+      const int st = j % WST, k0 = j * WK;
+      const double* pa = A + k0 * sak;
+      const double* pb = B + k0 * sbk;
+#pragma unroll
+      for (int e = 0; e < WM * WK / T; e++) {
+        const int mm = amm + e * adm, kk = akk + e * adk;
+        const bool in = m0 + mm < g.m && k0 + kk < K;
+        const double* q = in ? pa + e * ai_step : g.A;
+#pragma unroll
+        for (int c = 0; c < NP; c++) cp_async8z(&As[ring][st][c][kk][mm], q + (in ? c * g.planeA : 0), in);
+      }
+#pragma unroll
+      for (int e = 0; e < WN * WK / T; e++) {
+        const int nn = bnn + e * bdn, kk = bkk + e * bdk;
+        const bool in = n0 + nn < g.n && k0 + kk < K;
+        const double* q = in ? pb + e * bi_step : g.B;
+#pragma unroll
+        for (int c = 0; c < NP; c++) cp_async8z(&Bs[ring][st][c][kk][nn], q + (in ? c * g.planeB : 0), in);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");   // one group per slab slot
+  };
+  auto ring_sync = [&]() {
+    if (CPLX) __syncthreads(); else __syncwarp();
+  };
+  // real part: a b - ai bi; imaginary part: a bi + ai b; conj(op) flips the sign of ai, bi
+  const bool conj_a = g.ta == 2 || g.ta == 3, conj_b = g.tb == 2 || g.tb == 3;
+  const uint64_t kSign = 1ull << 63;
+  const uint64_t na = (conj_a != (comp == 0)) ? kSign : 0ull;    // sign of ai as used
+  const uint64_t nb = conj_b ? kSign : 0ull;
+  auto flip = [](double x, uint64_t m) {
+    return __longlong_as_double(__double_as_longlong(x) ^ (long long)m);
+  };
+  double acc = 0.0;
+#pragma unroll
+  for (int j = 0; j < WST - 1; j++) issue(j);
+  for (int j = 0; j < nslab; j++) {
+    issue(j + WST - 1);
+    asm volatile("cp.async.wait_group %0;" ::"n"(WST - 1) : "memory");
+    ring_sync();
+    const int st = j % WST, kn = min(WK, K - j * WK);
+#pragma unroll 8
+    for (int kk = 0; kk < kn; kk++) {
+      const double a = As[ring][st][0][kk][lm], b = Bs[ring][st][0][kk][ln];
+      if (CPLX) {
+        const double ai = flip(As[ring][st][NP - 1][kk][lm], na);
+        const double bi = flip(Bs[ring][st][NP - 1][kk][ln], nb);
+        acc = fma(a, comp ? bi : b, acc);
+        acc = fma(ai, comp ? b : bi, acc);
+      } else {
+        acc = fma(a, b, acc);
+      }
+    }
+    if (j + WST < nslab) ring_sync();                    // stage j % WST is refilled next
+  }
+  double* C = g.C + zb * g.strideC;
+  const int64_t idx = (int64_t)gm + (int64_t)gn * g.ldc;
+  const bool has_beta = g.beta[0] != 0.0 || g.beta[1] != 0.0;
+  __shared__ double part[32 * WWARPS];                   // complex: the other part's value
+  if (splits > 1) {
+    const int64_t mn = (int64_t)g.m * g.n, t = (int64_t)gm + (int64_t)gn * g.m;
+    if (live) ws[(int64_t)sp * mn * (CPLX ? 2 : 1) + comp * mn + t] = acc;
+    if (!tile_cnt) return;                               // the reduction kernel sums the splits
+    // the last split of this tile to arrive sums the partials in split order
+    __shared__ int s_last[WWARPS];
+    const int tiles_x = CPLX ? gridDim.x : gridDim.x * WWARPS;
+    if (CPLX) __syncthreads(); else __syncwarp();        // both parts are written
+    if (CPLX ? threadIdx.x == 0 : lane == 0) {
+      __threadfence();
+      int* cnt = tile_cnt + ((int64_t)zb * gridDim.y + blockIdx.y) * tiles_x + mt;
+      const bool last = atomicAdd(cnt, 1) == splits - 1;
+      if (last) *cnt = 0;                                // ready for the next launch
+      __threadfence();
+      s_last[wid] = last;
+    }
+    if (CPLX) __syncthreads(); else __syncwarp();
+    if (!s_last[CPLX ? 0 : wid]) return;
+    acc = 0.0;
+    if (live)
+      for (int q = 0; q < splits; q++) acc += __ldcg(ws + (int64_t)q * mn * (CPLX ? 2 : 1) + comp * mn + t);
+  }
+  if (CPLX) {
+    if (g.alpha[0] != 1.0 || g.alpha[1] != 0.0 || has_beta) {
+      part[threadIdx.x] = acc;
+      __syncthreads();
+      const double sr = part[lane], si = part[32 + lane];
+      double r = comp ? g.alpha[0] * si + g.alpha[1] * sr : g.alpha[0] * sr - g.alpha[1] * si;
+      if (has_beta && live) {
+        const double cr = C[idx], ci = C[g.planeC + idx];
+        r += comp ? g.beta[0] * ci + g.beta[1] * cr : g.beta[0] * cr - g.beta[1] * ci;
+      }
+      __syncthreads();                                   // both have read the old C
+      acc = r;
+    }
+    if (live) C[comp * g.planeC + idx] = acc;
+  } else if (live) {
+    double r = g.alpha[0] * acc;
+    if (has_beta) r += g.beta[0] * C[idx];
+    C[idx] = r;
+  }
+}
+
 // C = alpha * sum_{s < splits} W_s + beta * C, summed in split order
 template <bool CPLX>
 __global__ void split_reduce(GemmArgs g, int splits, const double* __restrict__ ws) {
@@ -267,10 +422,10 @@ constexpr int kMaxSplitTiles = 1 << 14;
 template <bool CPLX>
 int launch(fmpt_handle* h, const GemmArgs& g) {
   const int sms = h->sm_count > 0 ? h->sm_count : 1;
-  // (tile edge, splits) with the fewest multiply-adds on the busiest SM; a split adds the
-  // partials' round trip, priced as that many multiply-adds
+  // the K split that, with its best tile edge, puts the fewest multiply-adds on the busiest
+  // SM; a split adds the partials' round trip, priced as that many multiply-adds
   const double cm = CPLX ? 4.0 : 1.0;
-  int bmn = 64, splits = 1;
+  int splits = 1;
   double best = 1e300;
   for (int e : {64, 32, 16}) {
     const int64_t t = (int64_t)((g.m + e - 1) / e) * ((g.n + e - 1) / e) * g.batch;
@@ -284,14 +439,26 @@ int launch(fmpt_handle* h, const GemmArgs& g) {
       if (e == 16) cost *= 1.15;               // one output per thread: more loads per FMA
       if (cost < best * 0.98) {
         best = cost;
-        bmn = e;
         splits = s;
       }
     }
   }
   const int kchunk = splits > 1 ? ((g.k + splits - 1) / splits + BK - 1) / BK * BK : g.k;
   if (splits > 1) splits = (g.k + kchunk - 1) / kchunk;
-  dim3 grid((g.m + bmn - 1) / bmn, (g.n + bmn - 1) / bmn, g.batch * splits);
+  // The kernel: 8x4 tiles per warp where they put fewer multiply-adds on the busiest
+  // sub-partition than 64x64 tiles do on the busiest SM, those otherwise.  The split stays
+  // as it is, so the sums do not depend on this choice; the warps' operand reads come to
+  // 1.5 TB/s whatever the shape.
+  const int64_t wx = (g.m + WM - 1) / WM, wy = (g.n + WN - 1) / WN;
+  const int64_t warps = wx * wy * g.batch * splits * (CPLX ? 2 : 1);
+  const double cost_warp = (double)((warps + 4 * sms - 1) / (4 * sms)) * 4.0 * WM * WN * kchunk *
+                           (CPLX ? 2.0 : 1.0);
+  const int64_t tiles64 = (int64_t)((g.m + 63) / 64) * ((g.n + 63) / 64) * g.batch * splits;
+  const double cost64 = (double)((tiles64 + sms - 1) / sms) * 4096.0 * kchunk * cm;
+  const bool warp_tiles = wy <= 65535 && cost_warp < 0.95 * cost64;
+  dim3 grid((g.m + 63) / 64, (g.n + 63) / 64, g.batch * splits);
+  if (warp_tiles)
+    grid = dim3((unsigned)(CPLX ? wx : (wx + WWARPS - 1) / WWARPS), (unsigned)wy, g.batch * splits);
   if (grid.y > 65535 || grid.z > 65535)
     return set_error(h, FMPT_ERR_SHAPE, "gemm: grid too large (%d x %d x %d)", grid.x, grid.y,
                      grid.z);
@@ -302,7 +469,8 @@ int launch(fmpt_handle* h, const GemmArgs& g) {
     FMPT_TRY(grow_buffer(h, &h->gemm_ws, &h->gemm_ws_bytes,
                          (size_t)splits * g.m * g.n * sizeof(double) * (CPLX ? 2 : 1)));
     ws = static_cast<double*>(h->gemm_ws);
-    if ((int64_t)grid.x * grid.y * g.batch <= kMaxSplitTiles) {
+    const int64_t tiles = (int64_t)grid.x * (warp_tiles && !CPLX ? WWARPS : 1) * grid.y * g.batch;
+    if (tiles <= kMaxSplitTiles) {
       cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
       if (!h->gemm_cnt && cudaStreamIsCapturing(h->stream, &cs) == cudaSuccess &&
           cs == cudaStreamCaptureStatusNone) {
@@ -315,12 +483,10 @@ int launch(fmpt_handle* h, const GemmArgs& g) {
     }
   }
   ProfScope prof(h, FMPT_K_F64_GEMM);
-  if (bmn == 64)
-    gemm_kernel<CPLX, 64><<<grid, NT, 0, h->stream>>>(g, splits, kchunk, ws, cnt);
-  else if (bmn == 32)
-    gemm_kernel<CPLX, 32><<<grid, NT, 0, h->stream>>>(g, splits, kchunk, ws, cnt);
+  if (warp_tiles)
+    gemm_warp<CPLX><<<grid, 32 * WWARPS, 0, h->stream>>>(g, splits, kchunk, ws, cnt);
   else
-    gemm_kernel<CPLX, 16><<<grid, NT, 0, h->stream>>>(g, splits, kchunk, ws, cnt);
+    gemm_kernel<CPLX, 64><<<grid, NT, 0, h->stream>>>(g, splits, kchunk, ws, cnt);
   FMPT_LAUNCHED(h);
   if (splits > 1 && !cnt) {
     const int64_t mn = (int64_t)g.m * g.n;
