@@ -567,6 +567,208 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   }
 }
 
+// ------------------------------------------------- small GEMMs: K pieces in a cluster
+// GEMMs of at most half a round of pair tiles (a D = 256 bond: 20 and 4 tiles of 256 x 256 for
+// 76 clusters) run here: one CTA per 128 x BN tile and K piece, the S <= 4 pieces of a tile in
+// one cluster.  The pieces are those of the pair kernel's split tiles and are added in the
+// same order in FP32, so the results are the same bits; but the partial tiles meet in
+// distributed shared memory (CTA p adds columns [p BN / S, (p + 1) BN / S) of all pieces)
+// instead of a round trip through L2 behind a counter, and four to eight times as many SMs
+// work.  3xTF32, D = 256: GEMM 2 (1024 x 256, K = 1280) 37.9 -> 13.4 us, GEMM 1 (1280 x 1024,
+// K = 256) 18.2 us either way; see small_tile for whole steps and the choice of BN.
+template <int MODE, int BN, int STAGES>
+struct SmallCfg {
+  static constexpr int KELEMS = MODE == BF16 ? 64 : 32;
+  static constexpr int A_BYTES = BM * 128, B_BYTES = BN * 128;
+  static constexpr int SPLIT = MODE == TF32X3 ? 2 : 1;
+  static constexpr int STAGE_BYTES = (A_BYTES + B_BYTES) * SPLIT;
+  static constexpr int PART_BYTES = BM * BN * 4;       // FP32 partial tile, over the stages
+  static constexpr int RING = STAGES * STAGE_BYTES > PART_BYTES ? STAGES * STAGE_BYTES : PART_BYTES;
+  static constexpr int SMEM = RING + 1024 + 256;
+  static_assert(SMEM <= 227 * 1024, "shared memory");
+  static_assert((2 * STAGES + 2) * 8 + 8 <= 256, "barrier area");
+};
+
+template <int OUT>
+__device__ __forceinline__ void store_one(void* C, int64_t idx, float v) {
+  if (OUT == 1)
+    static_cast<double*>(C)[idx] = (double)v;
+  else if (OUT == 2)
+    static_cast<__nv_bfloat16*>(C)[idx] = __float2bfloat16_rn(v);
+  else
+    static_cast<float*>(C)[idx] = v;
+}
+
+template <int MODE, int BN, int STAGES, int OUT>
+__global__ void __launch_bounds__(NTHREADS, 1)
+    gemm_small_kernel(const __grid_constant__ CUtensorMap mapA,
+                      const __grid_constant__ CUtensorMap mapB,
+                      const __grid_constant__ CUtensorMap mapA2,
+                      const __grid_constant__ CUtensorMap mapB2, int K, int tiles_m, int tiles_n,
+                      int S, EpiArgs ep) {
+  using C_ = SmallCfg<MODE, BN, STAGES>;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C_::RING);
+  uint64_t* acc_full = bars + 2 * STAGES;              // [2 S] accumulator full, [2 S + 1] drain
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int p = S > 1 ? (int)cluster_rank() : 0;       // K piece
+  int mt, nt, z;
+  tile_coords(blockIdx.x / S, tiles_m, tiles_n, ep.nfast, mt, nt, z);
+  const int m0 = mt * BM, n0 = nt * BN;
+  const int nk = (K + C_::KELEMS - 1) / C_::KELEMS;
+  const int kb0 = (int)((int64_t)p * nk / S), kb1 = (int)((int64_t)(p + 1) * nk / S);
+  auto stageA = [&](int s, int part) {
+    return smem + s * C_::STAGE_BYTES + part * (C_::A_BYTES + C_::B_BYTES);
+  };
+  auto stageB = [&](int s, int part) { return stageA(s, part) + C_::A_BYTES; };
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < 2 * STAGES; s++) mbar_init(smem_u32(&bars[s]), 1);
+    mbar_init(smem_u32(acc_full), 1);
+    mbar_init(smem_u32(acc_full + 1), 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(tmem_slot)),
+                 "r"(BN)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  bool got = false;                                    // epilogue warps: the piece is complete
+  if (warp == 0) {
+    if (lane == 0) {
+      int it = 0;
+      for (int kb = kb0; kb < kb1; kb++, it++) {
+        const int s = it % STAGES;
+        if (!mbar_wait(smem_u32(&bars[STAGES + s]), ((it / STAGES) & 1) ^ 1, abort_flag, ep.err))
+          break;
+        const uint32_t full = smem_u32(&bars[s]);
+        mbar_expect_tx(full, C_::STAGE_BYTES);
+        const int kc = kb * C_::KELEMS;
+        tma_load_3d(smem_u32(stageA(s, 0)), &mapA, full, kc, m0, z);
+        tma_load_3d(smem_u32(stageB(s, 0)), &mapB, full, kc, n0, z);
+        if (MODE == TF32X3) {
+          tma_load_3d(smem_u32(stageA(s, 1)), &mapA2, full, kc, m0, z);
+          tma_load_3d(smem_u32(stageB(s, 1)), &mapB2, full, kc, n0, z);
+        }
+      }
+      // on an abort every load issued must land before the CTA goes on
+      if (*abort_flag) {
+        const unsigned long long t0 = globaltimer();
+        for (int j = max(0, it - STAGES); j < it; j++)
+          while (!mbar_try(smem_u32(&bars[j % STAGES]), (j / STAGES) & 1) &&
+                 globaltimer() - t0 < WAIT_NS) {
+          }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc(MODE, BM, BN);
+      int it = 0;
+      for (int kb = kb0; kb < kb1; kb++, it++) {
+        const int s = it % STAGES;
+        if (!mbar_wait(smem_u32(&bars[s]), (it / STAGES) & 1, abort_flag, ep.err)) break;
+        tc_fence_after();
+        const uint32_t a0 = smem_u32(stageA(s, 0)), b0 = smem_u32(stageB(s, 0));
+#pragma unroll
+        for (int ks = 0; ks < 4; ks++) {
+          const uint32_t acc = (kb > kb0 || ks > 0) ? 1u : 0u;
+          const uint64_t ad = smem_desc(a0 + ks * 32), bd = smem_desc(b0 + ks * 32);
+          mma<MODE>(tmem, ad, bd, idesc, acc);
+          if (MODE == TF32X3) {                        // hi*hi + hi*lo + lo*hi
+            const uint32_t a1 = smem_u32(stageA(s, 1)), b1 = smem_u32(stageB(s, 1));
+            mma<MODE>(tmem, ad, smem_desc(b1 + ks * 32), idesc, 1u);
+            mma<MODE>(tmem, smem_desc(a1 + ks * 32), bd, idesc, 1u);
+          }
+        }
+        mma_commit(smem_u32(&bars[STAGES + s]));
+      }
+      mma_commit(smem_u32(acc_full));
+    }
+  } else {
+    got = mbar_wait(smem_u32(acc_full), 0, abort_flag, ep.err) && !*abort_flag;
+    tc_fence_after();
+    const int q = warp & 3, rloc = 32 * q + lane;
+    const uint32_t tbase = tmem + ((uint32_t)(32 * q) << 16);
+    if (got && S == 1) {
+      store_acc<BN, OUT>(tbase, m0 + rloc, n0, z, ep);
+    } else if (got) {
+      // the partial tile over the stages (every MMA that reads them has retired)
+      float* part = reinterpret_cast<float*>(smem);
+#pragma unroll 1
+      for (int c0 = 0; c0 < BN; c0 += 32) {
+        uint32_t r[32];
+        tmem_ld32_async(tbase + c0, r);
+        tmem_wait_ld(r);
+#pragma unroll
+        for (int j = 0; j < 32; j++) part[(c0 + j) * BM + rloc] = __uint_as_float(r[j]);
+      }
+    }
+  }
+  if (S > 1) {
+    // Every CTA of the cluster comes here after bounded work.  A piece that was given up is
+    // summed as it stands: the error flag is set and the caller discards the result.
+    cluster_sync();
+    if (warp >= 2 && got) {
+      const int row = 32 * (warp & 3) + lane;
+      const uint32_t own = smem_u32(smem) + row * 4;
+      const int c1 = (p + 1) * BN / S;
+      // 16 columns' loads of every piece before the first add: a remote load takes about a
+      // microsecond
+#pragma unroll 1
+      for (int c0 = p * BN / S; c0 < c1; c0 += 16) {
+        float v[4][16];
+#pragma unroll
+        for (int pc = 0; pc < 4; pc++) {
+          if (pc < S) {
+            const uint32_t a = cluster_addr(own + c0 * (BM * 4), pc);
+#pragma unroll
+            for (int j = 0; j < 16; j++)
+              asm volatile("ld.shared::cluster.f32 %0, [%1];"
+                           : "=f"(v[pc][j])
+                           : "r"(a + min(j, c1 - 1 - c0) * (BM * 4)));
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+          float a = v[0][j];
+#pragma unroll
+          for (int pc = 1; pc < 4; pc++)
+            if (pc < S) a += v[pc][j];
+          const int c = c0 + j;
+          if (c < c1 && m0 + row < ep.M && n0 + c < ep.N)
+            store_one<OUT>(ep.C, (int64_t)m0 + row + ep.strideC * z + ep.ldc * (n0 + c), a);
+        }
+      }
+    }
+    cluster_sync();                                    // no CTA leaves while it may be read
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    if (lane == 0) {
+      mma_commit(smem_u32(acc_full + 1));
+      const unsigned long long t0 = globaltimer();
+      while (!mbar_try(smem_u32(acc_full + 1), 0) && globaltimer() - t0 < WAIT_NS) {
+      }
+    }
+    __syncwarp();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN)
+                 : "memory");
+  }
+}
+
 // ---------------------------------------------------------- tensor maps
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -607,6 +809,99 @@ int make_map(fmpt_handle* h, CUtensorMap* map, const void* base, int mode, int64
 }
 
 }  // namespace tc
+
+// ----------------------------------------------------- small-GEMM launch
+// Launch of the small kernel with BN columns per tile and S K pieces per tile (a cluster);
+// FMPT_ERR_UNSUPPORTED (nothing launched) when such a cluster does not fit.
+template <int MODE, int BN, int ST>
+static int tc_gemm_small(fmpt_handle* h, int M, int N, int K, int batch, int S, const TcOperand& A,
+                         const TcOperand& B, const tc::EpiArgs& ep, int out_f64) {
+  using namespace tc;
+  using C_ = SmallCfg<MODE, BN, ST>;
+  CUtensorMap ma, mb, ma2, mb2;
+  FMPT_TRY(make_map(h, &ma, A.hi, MODE, K, M, A.ld, batch, A.bstride, BM));
+  FMPT_TRY(make_map(h, &mb, B.hi, MODE, K, N, B.ld, batch, B.bstride, BN));
+  ma2 = ma;
+  mb2 = mb;
+  if (MODE == TF32X3) {
+    if (!A.lo || !B.lo) return set_error(h, FMPT_ERR_ARG, "3xTF32 needs lo planes");
+    FMPT_TRY(make_map(h, &ma2, A.lo, MODE, K, M, A.ld, batch, A.bstride, BM));
+    FMPT_TRY(make_map(h, &mb2, B.lo, MODE, K, N, B.ld, batch, B.bstride, BN));
+  }
+  const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + BN - 1) / BN;
+  void (*kfn)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, int, int, int, int, EpiArgs) =
+      out_f64 == 1   ? gemm_small_kernel<MODE, BN, ST, 1>
+      : out_f64 == 2 ? gemm_small_kernel<MODE, BN, ST, MODE == BF16 ? 2 : 0>
+                     : gemm_small_kernel<MODE, BN, ST, 0>;
+  const int vi = out_f64 == 1 ? 1 : out_f64 == 2 ? 2 : 0;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(tiles_m * tiles_n * batch * S));
+  cfg.blockDim = dim3(NTHREADS);
+  cfg.dynamicSmemBytes = C_::SMEM;
+  cfg.stream = h->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = S;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = S > 1 ? 1 : 0;
+  static int fits[3][5] = {};                          // 1 / -1: clusters of S (do not) fit
+  if (fits[vi][S] == 0) {
+    FMPT_CUDA(h, cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, C_::SMEM));
+    int n = 1;
+    if (S > 1 && cudaOccupancyMaxActiveClusters(&n, kfn, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      n = 0;
+    }
+    fits[vi][S] = n > 0 ? 1 : -1;
+  }
+  if (fits[vi][S] < 0) return FMPT_ERR_UNSUPPORTED;
+  ProfScope prof(h, FMPT_K_TC_GEMM);
+  FMPT_CUDA(h, cudaLaunchKernelEx(&cfg, kfn, ma, mb, ma2, mb2, K, tiles_m, tiles_n, S, ep));
+  FMPT_LAUNCHED(h);
+  return FMPT_OK;
+}
+
+// The tile width of a small GEMM, or 0 where pair tiles (one round of them, cut into S pieces
+// each) are expected to be no slower.  Cycles on the busiest SM: rounds of CTAs times
+// - 5000 to fill and drain,
+// - the K slices, by the slower of the L2 -> shared-memory copies at 64 B per clock and the
+//   MMAs, which one CTA alone runs at 1 / 1.3 of the pair's rate,
+// - the epilogue: about 1300 per 16 columns added over a cluster, 24000 for a pair tile's
+//   pieces through L2.
+// With pair tiles everywhere a D = 256 H_eff*x took 72 / 62 / 53 us in 3xTF32 / TF32 / BF16, now
+// 45 / 38 / 28; at D = 700 in 3xTF32, MMA-bound, both take 180.
+static int small_tile(int mode, int M, int N, int K, int batch, int S, int sms) {
+  const int kel = mode == tc::BF16 ? 64 : 32;
+  const double x = mode == tc::TF32X3 ? 2.0 : 1.0, mmas = mode == tc::TF32X3 ? 12.0 : 4.0;
+  const double slices = ((K + kel - 1) / kel + S - 1) / S;
+  double t = 5000.0 + slices * std::max(256 * 128.0 * x / 64.0, mmas * 156.0) +
+             (S > 1 ? 24000.0 : 3000.0);
+  t *= 0.95;
+  int best = 0;
+  for (int bn : {64, 128, 256}) {
+    const int64_t ctas = (int64_t)((M + 127) / 128) * ((N + bn - 1) / bn) * batch * S;
+    const int64_t rounds = (ctas + sms - 1) / sms;
+    const double slice = std::max((128 + bn) * 128.0 * x / 64.0, mmas * 39.0 * 1.3 * (bn / 64));
+    const double c = (double)rounds * (5000.0 + slices * slice +
+                                       (S > 1 ? 1300.0 * ((bn / S + 15) / 16) : 6.0 * bn));
+    if (c < t) {
+      t = c;
+      best = bn;
+    }
+  }
+  return best;
+}
+
+template <int MODE>
+static int tc_gemm_small_bn(fmpt_handle* h, int bn, int M, int N, int K, int batch, int S,
+                            const TcOperand& A, const TcOperand& B, const tc::EpiArgs& ep,
+                            int out_f64) {
+  constexpr int X = MODE == tc::TF32X3 ? 1 : 2;        // stages that fit: twice as many unsplit
+  if (bn == 64) return tc_gemm_small<MODE, 64, 4 * X>(h, M, N, K, batch, S, A, B, ep, out_f64);
+  if (bn == 128) return tc_gemm_small<MODE, 128, 3 * X>(h, M, N, K, batch, S, A, B, ep, out_f64);
+  return tc_gemm_small<MODE, 256, 2 * X>(h, M, N, K, batch, S, A, B, ep, out_f64);
+}
 
 // ----------------------------------------------------- CTA-pair launch
 // FMPT_ERR_UNSUPPORTED (nothing launched) when no cluster of two fits on the device.
@@ -666,6 +961,14 @@ static int tc_gemm_pair_st(fmpt_handle* h, int M, int N, int K, int batch, const
   PairSched sp{(int)units, 0, 1, nullptr, nullptr};
   const int rem = (int)(units % cl);
   const int S = rem > 0 ? std::min(std::min(4, cl / rem), nk / 4) : 1;
+  // at most half a round of tiles: 128-row tiles with the same K pieces on more SMs
+  if (2 * units <= cl) {
+    const int Ss = std::max(1, S), sms = std::max(1, h->sm_count);
+    const int bn = small_tile(MODE, M, N, K, batch, Ss, sms);
+    const int st = bn ? tc_gemm_small_bn<MODE>(h, bn, M, N, K, batch, Ss, A, B, ep, out_f64)
+                      : FMPT_ERR_UNSUPPORTED;
+    if (st != FMPT_ERR_UNSUPPORTED) return st;
+  }
   if (S >= 2) {
     const size_t part = (size_t)rem * S * 65536 * sizeof(float);
     const size_t need = part + (size_t)rem * 8 * sizeof(int);
