@@ -53,31 +53,80 @@ __device__ __forceinline__ void warp_sum_many(double (&a)[K]) {
   for (; o > 0; o >>= 1) a[0] += __shfl_xor_sync(0xffffffffu, a[0], o);
 }
 
-// Warps at or above nw hold exact zeros (the threads of a block past its elements) and skip
-// their shuffle sums: the result is the same, and their FP64 adds no longer queue on the
-// SM's FP64 pipe in front of the warps with data.
-__device__ double block_sum(double v, int nw = KT / 32) {
-  __shared__ double red[KT / 32];
+// Sum over the lanes and over the first nw <= 8 of 8 rows a[w] (rows past nw are exact zeros),
+// by one warp: the rows' warp sums, then their sum in the order of a warp sum over lanes 0..7.
+// The adds of rows that do not exist are left out (x + 0 = x).  All lanes get the result.
+__device__ __forceinline__ double rows_sum(double (&a)[8], int nw) {
+  if (nw <= 1) return warp_sum(a[0]);
+  if (nw <= 2) {
+    double b[2] = {a[0], a[1]};
+    warp_sum_many<2>(b);
+    return b[0] + __shfl_xor_sync(0xffffffffu, b[0], 16);
+  }
+  if (nw <= 4) {
+    double b[4] = {a[0], a[1], a[2], a[3]};
+    warp_sum_many<4>(b);
+    b[0] += __shfl_xor_sync(0xffffffffu, b[0], 16);
+    return b[0] + __shfl_xor_sync(0xffffffffu, b[0], 8);
+  }
+  warp_sum_many<8>(a);
+  a[0] += __shfl_xor_sync(0xffffffffu, a[0], 16);
+  a[0] += __shfl_xor_sync(0xffffffffu, a[0], 8);
+  return a[0] + __shfl_xor_sync(0xffffffffu, a[0], 4);
+}
+
+// Sum over the block, in warp order.  One warp adds all of it: the adds of eight warp sums
+// (45 FP64 warp instructions of 64 to 77 cycles each) become 12, and with four blocks on an
+// SM that is most of what the short vector kernels below do.
+__device__ double block_sum(double v) {
+  __shared__ double red[KT];
   __shared__ double total;
-  if ((threadIdx.x >> 5) < nw) v = warp_sum(v);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = (threadIdx.x >> 5) < nw ? v : 0.0;
+  red[threadIdx.x] = v;
   __syncthreads();
   if (threadIdx.x < 32) {
-    double w = threadIdx.x < KT / 32 ? red[threadIdx.x] : 0.0;
-    w = warp_sum(w);
-    if (threadIdx.x == 0) total = w;
+    double a[8];
+#pragma unroll
+    for (int w = 0; w < 8; w++) a[w] = red[32 * w + threadIdx.x];
+    const double t = rows_sum(a, 8);
+    if (threadIdx.x == 0) total = t;
   }
   __syncthreads();
-  double r = total;
+  const double r = total;
   __syncthreads();
   return r;
 }
 
-// fixed-order sum of G partials (every block computes the same value)
-__device__ double sum_parts(const double* part, int G) {
-  double s = 0.0;
-  for (int i = threadIdx.x; i < G; i += KT) s += part[i];
-  return block_sum(s, G >= KT ? KT / 32 : (G + 31) / 32);
+// Fixed-order sum of G partials, or its square root (every block computes the same value): by
+// one warp, with the sums of 256 threads striding over the partials.
+__device__ double sum_parts(const double* part, int G, bool root = false) {
+  __shared__ double total;
+  if (threadIdx.x < 32) {
+    const int nw = G >= KT ? 8 : (G + 31) / 32;
+    double a[8];
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+      const int i = 32 * w + (int)threadIdx.x;
+      a[w] = i < G ? part[i] : 0.0;
+    }
+    for (int k = KT; k < G; k += KT) {
+      double b[8];
+#pragma unroll
+      for (int w = 0; w < 8; w++) {
+        const int i = k + 32 * w + (int)threadIdx.x;
+        b[w] = i < G ? part[i] : 0.0;
+      }
+#pragma unroll
+      for (int w = 0; w < 8; w++)
+        if (k + 32 * w < G) a[w] += b[w];
+    }
+    double t = rows_sum(a, nw);
+    if (root) t = sqrt(t);
+    if (threadIdx.x == 0) total = t;
+  }
+  __syncthreads();
+  const double r = total;
+  __syncthreads();
+  return r;
 }
 
 // part[b] = sum x*y over a grid-stride slice (real view of length n)
@@ -94,7 +143,7 @@ __global__ void rdot_partial(int64_t n, const double* __restrict__ x, const doub
 // x = v / ||v|| with ||v||^2 = sum(part); stores the norm in *nrm
 __global__ void normalize_from_parts(int64_t n, const double* __restrict__ v, double* __restrict__ x,
                                      const double* __restrict__ part, int G, double* nrm) {
-  double s = sqrt(sum_parts(part, G));
+  const double s = sum_parts(part, G, true);
   if (blockIdx.x == 0 && threadIdx.x == 0) *nrm = s;
   double inv = s > 0.0 ? 1.0 / s : 0.0;
   for (int64_t i = (int64_t)blockIdx.x * KT + threadIdx.x; i < n; i += (int64_t)gridDim.x * KT)
@@ -127,7 +176,7 @@ __global__ void lanczos_axpy(int64_t n, double* __restrict__ y, const double* __
 __global__ void lanczos_scale(int64_t n, const double* __restrict__ y,
                               const double* __restrict__ part_b, int G, const double* alpha,
                               double* beta_out, double* __restrict__ vnext, double* ab) {
-  const double b = sqrt(sum_parts(part_b, G));
+  const double b = sum_parts(part_b, G, true);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *beta_out = b;
     ab[0] = *alpha;
@@ -140,7 +189,7 @@ __global__ void lanczos_scale(int64_t n, const double* __restrict__ y,
 
 // ---- multi-vector kernels over the Krylov basis V (j vectors of length n,
 // complex split planes when cplx: V_i re at V + i*2n, im at V + i*2n + n)
-// partial dots h_i = <V_i, z> ; part layout [G][j][2].  Chunks of MD_CH vectors per pass
+// partial dots h_i = <V_i, z> ; part layout [j][2][G].  Chunks of MD_CH vectors per pass
 // over z: every thread keeps MD_CH running sums (re, im), reduced by warp shuffles and one
 // shared-memory pass per chunk -- instead of one full block reduction per vector.  Fixed
 // summation order throughout (deterministic).
@@ -181,53 +230,56 @@ __global__ void multidot_partial(int cplx, int64_t n, int j, const double* __res
       v[2 * c] = sr[c];
       v[2 * c + 1] = si[c];
     }
-    warp_sum_many<2 * MD_CH>(v);
-    if ((lane & 1) == 0) red[wid][lane >> 1] = v[0];        // 2 MD_CH = 16 values
+    if (cplx) {
+      warp_sum_many<2 * MD_CH>(v);
+      if ((lane & 1) == 0) red[wid][lane >> 1] = v[0];      // 2 MD_CH = 16 values
+    } else {
+      warp_sum_many<MD_CH>(sr);                             // no imaginary parts to add
+      if ((lane & 3) == 0) {
+        red[wid][2 * (lane >> 2)] = sr[0];
+        red[wid][2 * (lane >> 2) + 1] = 0.0;
+      }
+    }
     __syncthreads();
     if (threadIdx.x < 2 * MD_CH) {
       const int c = threadIdx.x >> 1;
       double t = 0.0;
       for (int w = 0; w < KT / 32; w++) t += red[w][threadIdx.x];
-      if (i0 + c < j) part[((int64_t)blockIdx.x * j + i0 + c) * 2 + (threadIdx.x & 1)] = t;
+      if (i0 + c < j) part[(int64_t)(2 * i0 + threadIdx.x) * gridDim.x + blockIdx.x] = t;
     }
     __syncthreads();
   }
 }
 
-// coef[i] (re, im) = sum over the G partials, one warp per value (lanes stride over the
-// partials in a fixed order, then a shuffle sum); launched with one block of KT threads
-// Coefficients t0 .. t0 + 63 (t = 2 i + re/im) of the sums over the G partials [G][j][2]:
-// warp w takes t = t0 + w + 8 u (u < 8); a lane adds its partials g = lane, lane + 32, ...
-// in g order, then the warp sums its 8 values with warp_sum_many.  out[t] = the sum
-// (accum[t] += it when given).
-__device__ __forceinline__ void coef_group(int j, int G, const double* __restrict__ part, int t0,
-                                           double* out, double* accum) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  double acc[8];
-#pragma unroll
-  for (int u = 0; u < 8; u++) {
-    const int t = t0 + wid + 8 * u;
-    double sum = 0.0;
-    if (t < 2 * j) {
-      const int i = t >> 1, comp = t & 1;
-      for (int g = lane; g < G; g += 32) sum += part[((int64_t)g * j + i) * 2 + comp];
-    }
-    acc[u] = sum;
-  }
-  warp_sum_many<8>(acc);
-  const int t = t0 + wid + 8 * (lane >> 2);
-  if ((lane & 3) == 0 && t < 2 * j) {
-    out[t] = acc[0];
-    if (accum) accum[t] += acc[0];
-  }
-}
-
-// coef[t] = the sums (accum[t] += them when given); launched with one block of KT threads
-__global__ void multidot_finalize(int j, int G, const double* __restrict__ part,
+// coef[t] (t = 2 i + re/im) = the sum over the G partials [2 j][G] (accum[t] += it when
+// given): one warp per value, a lane adds its partials g = lane, lane + 32, .. in order, then
+// the warp sums; real data has no odd values.  Launched with (2 j + 7) / 8 blocks: one block
+// for all values took 12 us at G = 608, 20 partials per lane one after the other on one SM.
+__global__ void multidot_finalize(int cplx, int j, int G, const double* __restrict__ part,
                                   double* __restrict__ coef, double* __restrict__ accum,
                                   const int* gate = nullptr) {
   if (gate && *gate) return;
-  for (int t0 = 0; t0 < 2 * j; t0 += 64) coef_group(j, G, part, t0, coef, accum);
+  const int t = blockIdx.x * (KT / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= 2 * j) return;
+  double s = 0.0;
+  if (cplx || !(t & 1)) {
+    for (int g0 = 0; g0 < G; g0 += 32 * 8) {
+      double v[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const int g = g0 + 32 * q + lane;
+        v[q] = g < G ? part[(int64_t)t * G + g] : 0.0;
+      }
+#pragma unroll
+      for (int q = 0; q < 8; q++)
+        if (g0 + 32 * q < G) s += v[q];
+    }
+    s = warp_sum(s);
+  }
+  if (lane == 0) {
+    coef[t] = s;
+    if (accum) accum[t] += s;
+  }
 }
 
 __global__ void multi_axpy_sub(int cplx, int64_t n, int j, const double* __restrict__ V,
@@ -824,7 +876,7 @@ __global__ void lanczos_close(int64_t n, const double* __restrict__ y,
                               const double* __restrict__ part_b, int G, double* beta_out,
                               int* ctl, double btol, int j, double* __restrict__ vnext) {
   if (ctl[0]) return;
-  const double b = sqrt(sum_parts(part_b, G));
+  const double b = sum_parts(part_b, G, true);
   const bool bad = !isfinite(b);
   const bool conv = !bad && b < btol;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1006,7 +1058,8 @@ int lanczos_graph(fmpt_op* op, const double* x0, int kmax, double btol, int reor
       if (reorth) {
         multidot_partial<<<G, KT, 0, st>>>(0, n, j + 1, V, n, y, partM.d(), ctl);
         FMPT_LAUNCHED(h);
-        multidot_finalize<<<1, KT, 0, st>>>(j + 1, G, partM.d(), coef.d(), nullptr, ctl);
+        multidot_finalize<<<(2 * (j + 1) + 7) / 8, KT, 0, st>>>(0, j + 1, G, partM.d(), coef.d(),
+                                                                nullptr, ctl);
         FMPT_LAUNCHED(h);
         multi_axpy_sub<<<G, KT, 0, st>>>(0, n, j + 1, V, n, coef.d(), y, partB.d(), ctl);
         FMPT_LAUNCHED(h);
@@ -1242,7 +1295,8 @@ int eigsolve_impl(fmpt_op* op, const double* x0, int num, int kdim, int maxiter,
       for (int pass = 0; pass < 2; pass++) {
         multidot_partial<<<G, KT, 0, st>>>(cp, n, j + 1, V, nr, z, partM.d());
         FMPT_LAUNCHED(h);
-        multidot_finalize<<<1, KT, 0, st>>>(j + 1, G, partM.d(), coef.d(), acc.d());
+        multidot_finalize<<<(2 * (j + 1) + 7) / 8, KT, 0, st>>>(cp, j + 1, G, partM.d(), coef.d(),
+                                                                acc.d());
         FMPT_LAUNCHED(h);
         multi_axpy_sub<<<G, KT, 0, st>>>(cp, n, j + 1, V, nr, coef.d(), z, partA.d());
         FMPT_LAUNCHED(h);
@@ -1606,7 +1660,7 @@ int fmpt_lanczos_ground(fmpt_op* op, const double* x0, int kmax, double btol, in
   auto reorthogonalise = [&](int j) -> int {
     multidot_partial<<<G, KT, 0, h->stream>>>(0, n, j, V, n, y, partM.d());
     FMPT_LAUNCHED(h);
-    multidot_finalize<<<1, KT, 0, h->stream>>>(j, G, partM.d(), coef.d(), nullptr);
+    multidot_finalize<<<(2 * j + 7) / 8, KT, 0, h->stream>>>(0, j, G, partM.d(), coef.d(), nullptr);
     FMPT_LAUNCHED(h);
     multi_axpy_sub<<<G, KT, 0, h->stream>>>(0, n, j, V, n, coef.d(), y, partB.d());
     FMPT_LAUNCHED(h);
