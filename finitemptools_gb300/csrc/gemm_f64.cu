@@ -32,6 +32,7 @@ template <bool CPLX, int BMN>
 __global__ void __launch_bounds__(NT) gemm_kernel(GemmArgs g, int splits, int kchunk,
                                                   double* __restrict__ ws,
                                                   int* __restrict__ tile_cnt) {
+  chain_begin();
   constexpr int TPR = BMN / 16;                // outputs per thread along each dimension
   __shared__ double As[2][BK][BMN + 1];
   __shared__ double Bs[2][BK][BMN + 1];
@@ -251,6 +252,7 @@ template <bool CPLX>
 __global__ void __launch_bounds__(32 * WWARPS) gemm_warp(GemmArgs g, int splits, int kchunk,
                                                          double* __restrict__ ws,
                                                          int* __restrict__ tile_cnt) {
+  chain_begin();
   constexpr int NP = CPLX ? 2 : 1;                       // planes
   // the ring belongs to a warp (real) or to the two warps of a tile (complex): T threads
   constexpr int T = CPLX ? 64 : 32, RINGS = CPLX ? 1 : WWARPS;
@@ -484,9 +486,11 @@ int launch(fmpt_handle* h, const GemmArgs& g) {
   }
   ProfScope prof(h, FMPT_K_F64_GEMM);
   if (warp_tiles)
-    gemm_warp<CPLX><<<grid, 32 * WWARPS, 0, h->stream>>>(g, splits, kchunk, ws, cnt);
+    FMPT_CUDA(h, launch_chain(gemm_warp<CPLX>, grid, 32 * WWARPS, 0, h->stream, g, splits, kchunk,
+                              ws, cnt));
   else
-    gemm_kernel<CPLX, 64><<<grid, NT, 0, h->stream>>>(g, splits, kchunk, ws, cnt);
+    FMPT_CUDA(h, launch_chain(gemm_kernel<CPLX, 64>, grid, NT, 0, h->stream, g, splits, kchunk, ws,
+                              cnt));
   FMPT_LAUNCHED(h);
   if (splits > 1 && !cnt) {
     const int64_t mn = (int64_t)g.m * g.n;

@@ -97,6 +97,7 @@ __global__ void __launch_bounds__(128)
     mid_sparse_kernel(const double* __restrict__ in, int64_t plane_in, MidStrides si,
                       double* __restrict__ out, int64_t plane_out, MidStrides so, int n1, int n2,
                       int p_out, const __grid_constant__ MidSparse<OUT, TERMS> ms) {
+  chain_begin();
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)n1 * n2) return;
   const int o1 = (int)(t % n1), o2 = (int)(t / n1);
@@ -297,8 +298,8 @@ static int mid_sparse_launch(fmpt_handle* h, const MidSchedule& s, const double*
   // below a few blocks per SM the outputs are spread over threads of their own (see the
   // kernel); above, the input is read once
   const int gy = blocks < 8LL * std::max(1, h->sm_count) ? ms.n_out : 1;
-  mid_sparse_kernel<CPLX, OUT, TERMS><<<dim3((unsigned)blocks, gy), 128, 0, h->stream>>>(
-      in, plane_in, si, out, plane_out, so, n1, n2, s.p_out, ms);
+  FMPT_CUDA(h, launch_chain(mid_sparse_kernel<CPLX, OUT, TERMS>, dim3((unsigned)blocks, gy), 128, 0,
+                            h->stream, in, plane_in, si, out, plane_out, so, n1, n2, s.p_out, ms));
   FMPT_LAUNCHED(h);
   return FMPT_OK;
 }

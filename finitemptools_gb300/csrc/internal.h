@@ -113,6 +113,36 @@ int set_error(fmpt_handle* h, int status, const char* fmt, ...);
                                __LINE__, cudaGetErrorString(_e));                       \
   } while (0)
 
+// Kernels that follow one another in a stream overlap their launches (programmatic dependent
+// launch): launch_chain lets the kernel be launched while its predecessor still runs, and
+// chain_begin, before its first access to global memory, waits until every earlier kernel
+// has completed with its writes visible (a plain launch of the same kernel waits for nothing
+// there).  The predecessors do not release their successors early: blocks that wait beside a
+// running grid start unevenly spread over the SMs, and a D = 64 Krylov exponential took 1.42 ms
+// instead of 1.30 (1.42 with plain launches too).  An H_eff*x at D = 32, three kernels, 18.4 us
+// with plain launches and 11.3 with these.
+#ifdef __CUDACC__
+__device__ __forceinline__ void chain_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+inline void chain_attr(cudaLaunchAttribute& a) {
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+}
+template <class... P, class... A>
+cudaError_t launch_chain(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                         cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  chain_attr(attr[0]);
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+#endif
+
 // Stream-ordered device scratch owned by a C++ scope.
 struct DevBuf {
   fmpt_handle* h = nullptr;

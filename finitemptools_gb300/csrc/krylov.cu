@@ -21,6 +21,10 @@ namespace {
 
 constexpr int KT = 256;
 
+// a kernel of KT threads per block, overlapping its launch with the kernel before it
+#define CHAIN(kernel, grid, stream, ...) \
+  FMPT_CUDA(h, launch_chain(kernel, grid, KT, 0, stream, __VA_ARGS__))
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -132,6 +136,7 @@ __device__ double sum_parts(const double* part, int G, bool root = false) {
 // part[b] = sum x*y over a grid-stride slice (real view of length n)
 __global__ void rdot_partial(int64_t n, const double* __restrict__ x, const double* __restrict__ y,
                              double* __restrict__ part, const int* gate = nullptr) {
+  chain_begin();
   if (gate && *gate) return;
   double s = 0.0;
   for (int64_t i = (int64_t)blockIdx.x * KT + threadIdx.x; i < n; i += (int64_t)gridDim.x * KT)
@@ -143,6 +148,7 @@ __global__ void rdot_partial(int64_t n, const double* __restrict__ x, const doub
 // x = v / ||v|| with ||v||^2 = sum(part); stores the norm in *nrm
 __global__ void normalize_from_parts(int64_t n, const double* __restrict__ v, double* __restrict__ x,
                                      const double* __restrict__ part, int G, double* nrm) {
+  chain_begin();
   const double s = sum_parts(part, G, true);
   if (blockIdx.x == 0 && threadIdx.x == 0) *nrm = s;
   double inv = s > 0.0 ? 1.0 / s : 0.0;
@@ -155,6 +161,7 @@ __global__ void lanczos_axpy(int64_t n, double* __restrict__ y, const double* __
                              const double* __restrict__ qm1, const double* __restrict__ part_a,
                              int G, const double* b_old, double* alpha_out,
                              double* __restrict__ part_b, const int* gate = nullptr) {
+  chain_begin();
   if (gate && *gate) return;
   const double a = sum_parts(part_a, G);
   const double b = (qm1 != nullptr) ? *b_old : 0.0;
@@ -176,6 +183,7 @@ __global__ void lanczos_axpy(int64_t n, double* __restrict__ y, const double* __
 __global__ void lanczos_scale(int64_t n, const double* __restrict__ y,
                               const double* __restrict__ part_b, int G, const double* alpha,
                               double* beta_out, double* __restrict__ vnext, double* ab) {
+  chain_begin();
   const double b = sum_parts(part_b, G, true);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *beta_out = b;
@@ -197,6 +205,7 @@ constexpr int MD_CH = 8;
 __global__ void multidot_partial(int cplx, int64_t n, int j, const double* __restrict__ V,
                                  int64_t vstride, const double* __restrict__ z,
                                  double* __restrict__ part, const int* gate = nullptr) {
+  chain_begin();
   if (gate && *gate) return;
   __shared__ double red[KT / 32][2 * MD_CH];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -258,6 +267,7 @@ __global__ void multidot_partial(int cplx, int64_t n, int j, const double* __res
 __global__ void multidot_finalize(int cplx, int j, int G, const double* __restrict__ part,
                                   double* __restrict__ coef, double* __restrict__ accum,
                                   const int* gate = nullptr) {
+  chain_begin();
   if (gate && *gate) return;
   const int t = blockIdx.x * (KT / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (t >= 2 * j) return;
@@ -286,6 +296,7 @@ __global__ void multi_axpy_sub(int cplx, int64_t n, int j, const double* __restr
                                int64_t vstride, const double* __restrict__ coef,
                                double* __restrict__ z, double* __restrict__ part,
                                const int* gate = nullptr) {
+  chain_begin();
   if (gate && *gate) return;
   double s = 0.0;
   for (int64_t e = (int64_t)blockIdx.x * KT + threadIdx.x; e < n; e += (int64_t)gridDim.x * KT) {
@@ -332,6 +343,7 @@ __global__ void multi_axpy_sub(int cplx, int64_t n, int j, const double* __restr
 __global__ void combine_basis(int cplx, int64_t n, int j, const double* __restrict__ V,
                               int64_t vstride, const double* __restrict__ c, int64_t cq,
                               const double* scale, double* __restrict__ out, int64_t oq) {
+  chain_begin();
   constexpr int U = 8;
   c += blockIdx.y * cq;
   out += blockIdx.y * oq;
@@ -693,6 +705,7 @@ __device__ bool gs_grid_wait(const CoopBar& b, int target) {
 
 template <bool SINGLE>
 __global__ void __launch_bounds__(GS_T) arnoldi_gs_fused(GsArgs a, CoopBar bar) {
+  chain_begin();
   __shared__ double bp[GS_NV], c[2][GS_NV];
   const GsWarp w(a);
   const int G = gridDim.x, nv = 2 * a.j + 3;
@@ -761,6 +774,7 @@ __global__ void mul_scalar(double* acc, const double* v) { *acc *= *v; }
 
 // x *= *a (device scalar)
 __global__ void scale_by(int64_t n, double* __restrict__ x, const double* a) {
+  chain_begin();
   const double f = *a;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n;
        e += (int64_t)gridDim.x * blockDim.x)
@@ -860,6 +874,7 @@ struct RitzCoef {
 // (simple_lanczos.jl:70-78), which adds the last basis vector first
 __global__ void combine_ritz(int64_t n, int k, const double* __restrict__ V, int64_t vstride,
                              const __grid_constant__ RitzCoef c, double* __restrict__ out) {
+  chain_begin();
   for (int64_t e = (int64_t)blockIdx.x * KT + threadIdx.x; e < n; e += (int64_t)gridDim.x * KT) {
     double r = c.c[k - 1] * V[(int64_t)(k - 1) * vstride + e];
     for (int i = 0; i < k - 1; i++) r = fma(c.c[i], V[(int64_t)i * vstride + e], r);
@@ -875,6 +890,7 @@ __global__ void combine_ritz(int64_t n, int k, const double* __restrict__ V, int
 __global__ void lanczos_close(int64_t n, const double* __restrict__ y,
                               const double* __restrict__ part_b, int G, double* beta_out,
                               int* ctl, double btol, int j, double* __restrict__ vnext) {
+  chain_begin();
   if (ctl[0]) return;
   const double b = sum_parts(part_b, G, true);
   const bool bad = !isfinite(b);
@@ -1043,28 +1059,28 @@ int lanczos_graph(fmpt_op* op, const double* x0, int kmax, double btol, int reor
   cudaStream_t st = h->stream;
   auto record = [&]() -> int {
     FMPT_CUDA(h, cudaMemsetAsync(ctl, 0, 4 * sizeof(int), st));
-    rdot_partial<<<G, KT, 0, st>>>(n, x0, x0, partA.d());
+    CHAIN(rdot_partial, G, st, n, x0, x0, partA.d(), nullptr);
     FMPT_LAUNCHED(h);
-    normalize_from_parts<<<G, KT, 0, st>>>(n, x0, V_(0), partA.d(), G, s_vm);
+    CHAIN(normalize_from_parts, G, st, n, x0, V_(0), partA.d(), G, s_vm);
     FMPT_LAUNCHED(h);
     for (int j = 0; j < kmax; j++) {
       FMPT_TRY(op_u1_apply(op, V_(j), y, ctl));
       FMPT_TRY(op_project(op, y, ctl));
-      rdot_partial<<<G, KT, 0, st>>>(n, V_(j), y, partA.d(), ctl);
+      CHAIN(rdot_partial, G, st, n, V_(j), y, partA.d(), ctl);
       FMPT_LAUNCHED(h);
-      lanczos_axpy<<<G, KT, 0, st>>>(n, y, V_(j), j ? V_(j - 1) : nullptr, partA.d(), G,
+      CHAIN(lanczos_axpy, G, st, n, y, V_(j), j ? V_(j - 1) : nullptr, partA.d(), G,
                                      j ? s_beta + (j - 1) : nullptr, s_alpha + j, partB.d(), ctl);
       FMPT_LAUNCHED(h);
       if (reorth) {
-        multidot_partial<<<G, KT, 0, st>>>(0, n, j + 1, V, n, y, partM.d(), ctl);
+        CHAIN(multidot_partial, G, st, 0, n, j + 1, V, n, y, partM.d(), ctl);
         FMPT_LAUNCHED(h);
-        multidot_finalize<<<(2 * (j + 1) + 7) / 8, KT, 0, st>>>(0, j + 1, G, partM.d(), coef.d(),
+        CHAIN(multidot_finalize, (2 * (j + 1) + 7) / 8, st, 0, j + 1, G, partM.d(), coef.d(),
                                                                 nullptr, ctl);
         FMPT_LAUNCHED(h);
-        multi_axpy_sub<<<G, KT, 0, st>>>(0, n, j + 1, V, n, coef.d(), y, partB.d(), ctl);
+        CHAIN(multi_axpy_sub, G, st, 0, n, j + 1, V, n, coef.d(), y, partB.d(), ctl);
         FMPT_LAUNCHED(h);
       }
-      lanczos_close<<<G, KT, 0, st>>>(n, y, partB.d(), G, s_beta + j, ctl, btol, j, V_(j + 1));
+      CHAIN(lanczos_close, G, st, n, y, partB.d(), G, s_beta + j, ctl, btol, j, V_(j + 1));
       FMPT_LAUNCHED(h);
     }
     // alpha and beta are adjacent
@@ -1116,7 +1132,7 @@ int lanczos_graph(fmpt_op* op, const double* x0, int kmax, double btol, int reor
   if (!bad && k > 0) tridiag_lowest(k, h->pinned, h->pinned + kmax, &ev, rc.c);
   FMPT_TRY(gp_check_status(h));
   if (bad) return set_error(h, FMPT_ERR_NONFINITE, "lanczos: beta is not finite");
-  combine_ritz<<<G, KT, 0, st>>>(n, k, V, n, rc, xout);
+  CHAIN(combine_ritz, G, st, n, k, V, n, rc, xout);
   FMPT_LAUNCHED(h);
   *eigval = ev;
   if (info) *info = conv ? 0 : -1;
@@ -1273,9 +1289,9 @@ int eigsolve_impl(fmpt_op* op, const double* x0, int num, int kdim, int maxiter,
   double* z = zb.d();
   auto V_ = [&](int i) { return V + (int64_t)i * nr; };
   cudaStream_t st = h->stream;
-  rdot_partial<<<G, KT, 0, st>>>(nr, x0, x0, partA.d());
+  CHAIN(rdot_partial, G, st, nr, x0, x0, partA.d(), nullptr);
   FMPT_LAUNCHED(h);
-  normalize_from_parts<<<G, KT, 0, st>>>(nr, x0, V_(0), partA.d(), G, snrm.d());
+  CHAIN(normalize_from_parts, G, st, nr, x0, V_(0), partA.d(), G, snrm.d());
   FMPT_LAUNCHED(h);
   FMPT_CUDA(h, cudaMemcpyAsync(h->pinned, snrm.d(), sizeof(double), cudaMemcpyDeviceToHost, st));
   FMPT_CUDA(h, cudaStreamSynchronize(st));
@@ -1293,12 +1309,12 @@ int eigsolve_impl(fmpt_op* op, const double* x0, int num, int kdim, int maxiter,
       applies++;
       FMPT_CUDA(h, cudaMemsetAsync(acc.d(), 0, (size_t)2 * (j + 1) * sizeof(double), st));
       for (int pass = 0; pass < 2; pass++) {
-        multidot_partial<<<G, KT, 0, st>>>(cp, n, j + 1, V, nr, z, partM.d());
+        CHAIN(multidot_partial, G, st, cp, n, j + 1, V, nr, z, partM.d(), nullptr);
         FMPT_LAUNCHED(h);
-        multidot_finalize<<<(2 * (j + 1) + 7) / 8, KT, 0, st>>>(cp, j + 1, G, partM.d(), coef.d(),
-                                                                acc.d());
+        CHAIN(multidot_finalize, (2 * (j + 1) + 7) / 8, st, cp, j + 1, G, partM.d(), coef.d(),
+                                                                acc.d(), nullptr);
         FMPT_LAUNCHED(h);
-        multi_axpy_sub<<<G, KT, 0, st>>>(cp, n, j + 1, V, nr, coef.d(), z, partA.d());
+        CHAIN(multi_axpy_sub, G, st, cp, n, j + 1, V, nr, coef.d(), z, partA.d(), nullptr);
         FMPT_LAUNCHED(h);
       }
       double* hp = h->pinned;
@@ -1321,7 +1337,7 @@ int eigsolve_impl(fmpt_op* op, const double* x0, int num, int kdim, int maxiter,
         j++;
         break;
       }
-      normalize_from_parts<<<G, KT, 0, st>>>(nr, z, V_(j + 1), partA.d(), G, snrm.d());
+      CHAIN(normalize_from_parts, G, st, nr, z, V_(j + 1), partA.d(), G, snrm.d());
       FMPT_LAUNCHED(h);
       Hx(j + 1, j) = Hx(j, j + 1) = beta;
     }
@@ -1658,11 +1674,12 @@ int fmpt_lanczos_ground(fmpt_op* op, const double* x0, int kmax, double btol, in
 
   // reorthogonalise y against V_0..V_{j-1} (classical Gram-Schmidt, one pass)
   auto reorthogonalise = [&](int j) -> int {
-    multidot_partial<<<G, KT, 0, h->stream>>>(0, n, j, V, n, y, partM.d());
+    CHAIN(multidot_partial, G, h->stream, 0, n, j, V, n, y, partM.d(), nullptr);
     FMPT_LAUNCHED(h);
-    multidot_finalize<<<(2 * j + 7) / 8, KT, 0, h->stream>>>(0, j, G, partM.d(), coef.d(), nullptr);
+    CHAIN(multidot_finalize, (2 * j + 7) / 8, h->stream, 0, j, G, partM.d(), coef.d(), nullptr,
+          nullptr);
     FMPT_LAUNCHED(h);
-    multi_axpy_sub<<<G, KT, 0, h->stream>>>(0, n, j, V, n, coef.d(), y, partB.d());
+    CHAIN(multi_axpy_sub, G, h->stream, 0, n, j, V, n, coef.d(), y, partB.d(), nullptr);
     FMPT_LAUNCHED(h);
     return FMPT_OK;
   };
@@ -1673,21 +1690,21 @@ int fmpt_lanczos_ground(fmpt_op* op, const double* x0, int kmax, double btol, in
   double* ab = h->step_host;
   auto launch_step = [&](int j) -> int {
     FMPT_TRY(fmpt_op_apply(op, V_(j), y));
-    rdot_partial<<<G, KT, 0, h->stream>>>(n, V_(j), y, partA.d());
+    CHAIN(rdot_partial, G, h->stream, n, V_(j), y, partA.d(), nullptr);
     FMPT_LAUNCHED(h);
-    lanczos_axpy<<<G, KT, 0, h->stream>>>(n, y, V_(j), j ? V_(j - 1) : nullptr, partA.d(), G,
-                                          j ? s_beta + (j - 1) : nullptr, s_alpha + j, partB.d());
+    CHAIN(lanczos_axpy, G, h->stream, n, y, V_(j), j ? V_(j - 1) : nullptr, partA.d(), G,
+                                          j ? s_beta + (j - 1) : nullptr, s_alpha + j, partB.d(), nullptr);
     FMPT_LAUNCHED(h);
     if (reorth) FMPT_TRY(reorthogonalise(j + 1));
-    lanczos_scale<<<G, KT, 0, h->stream>>>(n, y, partB.d(), G, s_alpha + j, s_beta + j, V_(j + 1),
+    CHAIN(lanczos_scale, G, h->stream, n, y, partB.d(), G, s_alpha + j, s_beta + j, V_(j + 1),
                                            ab + 2 * j);
     FMPT_LAUNCHED(h);
     FMPT_CUDA(h, cudaEventRecord(h->step_event[j & 1], h->stream));
     return FMPT_OK;
   };
-  rdot_partial<<<G, KT, 0, h->stream>>>(n, x0, x0, partA.d());
+  CHAIN(rdot_partial, G, h->stream, n, x0, x0, partA.d(), nullptr);
   FMPT_LAUNCHED(h);
-  normalize_from_parts<<<G, KT, 0, h->stream>>>(n, x0, V_(0), partA.d(), G, s_vm);
+  CHAIN(normalize_from_parts, G, h->stream, n, x0, V_(0), partA.d(), G, s_vm);
   FMPT_LAUNCHED(h);
   // Step j + 1 is queued before beta_j is looked at, so the device does not wait for the
   // host's test (25 us per step at D = 64); one step past convergence is thrown away.
@@ -1714,7 +1731,7 @@ int fmpt_lanczos_ground(fmpt_op* op, const double* x0, int kmax, double btol, in
     // eigen(Symmetric(T[1:k,1:k])), lowest pair (find_lanczos "SR")
     RitzCoef rc;
     tridiag_lowest(k, al, be, eigval, rc.c);
-    combine_ritz<<<G, KT, 0, h->stream>>>(n, k, V, n, rc, xout);
+    CHAIN(combine_ritz, G, h->stream, n, k, V, n, rc, xout);
     FMPT_LAUNCHED(h);
   }
   if (!prec_is_f64(op->precision)) FMPT_TRY(op_tc_check(op));
@@ -1764,9 +1781,9 @@ int fmpt_exponentiate(fmpt_op* op, double t_re, double t_im, const double* x, do
   }
   const double sg_r = t_re / tabs, sg_i = t_im / tabs;
   // w = x / ||x||, acc = ||x|| (the running norm stays on the device)
-  rdot_partial<<<G, KT, 0, h->stream>>>(nr, x, x, part.d());
+  CHAIN(rdot_partial, G, h->stream, nr, x, x, part.d(), nullptr);
   FMPT_LAUNCHED(h);
-  normalize_from_parts<<<G, KT, 0, h->stream>>>(nr, x, V_(0), part.d(), G, acc.d());
+  CHAIN(normalize_from_parts, G, h->stream, nr, x, V_(0), part.d(), G, acc.d());
   FMPT_LAUNCHED(h);
   double tau_done = 0.0, dtau = tabs;
   int steps = 0;
@@ -1815,11 +1832,11 @@ int fmpt_exponentiate(fmpt_op* op, double t_re, double t_im, const double* x, do
     FMPT_CUDA(h, cudaMemcpyAsync(Ed.d(), colbuf.data(), (size_t)2 * m * sizeof(double),
                                  cudaMemcpyHostToDevice, h->stream));
     // w = sum_i E[i, 0] V_i, renormalised into V_0; acc *= ||w||
-    combine_basis<<<G, KT, 0, h->stream>>>(cp, n, m, V, nr, Ed.d(), 0, nullptr, zb.d(), 0);
+    CHAIN(combine_basis, G, h->stream, cp, n, m, V, nr, Ed.d(), 0, nullptr, zb.d(), 0);
     FMPT_LAUNCHED(h);
-    rdot_partial<<<G, KT, 0, h->stream>>>(nr, zb.d(), zb.d(), part.d());
+    CHAIN(rdot_partial, G, h->stream, nr, zb.d(), zb.d(), part.d(), nullptr);
     FMPT_LAUNCHED(h);
-    normalize_from_parts<<<G, KT, 0, h->stream>>>(nr, zb.d(), V_(0), part.d(), G, nrm.d());
+    CHAIN(normalize_from_parts, G, h->stream, nr, zb.d(), V_(0), part.d(), G, nrm.d());
     FMPT_LAUNCHED(h);
     mul_scalar<<<1, 1, 0, h->stream>>>(acc.d(), nrm.d());
     FMPT_LAUNCHED(h);
@@ -1829,7 +1846,7 @@ int fmpt_exponentiate(fmpt_op* op, double t_re, double t_im, const double* x, do
   // xout = acc * V_0
   FMPT_CUDA(h, cudaMemcpyAsync(xout, V_(0), nr * sizeof(double), cudaMemcpyDeviceToDevice,
                                h->stream));
-  scale_by<<<G, KT, 0, h->stream>>>(nr, xout, acc.d());
+  CHAIN(scale_by, G, h->stream, nr, xout, acc.d());
   FMPT_LAUNCHED(h);
   if (!prec_is_f64(op->precision)) FMPT_TRY(op_tc_check(op));
   if (op->u1 || gs.fused) FMPT_TRY(gp_check_status(op->h));
@@ -1870,9 +1887,9 @@ int fmpt_expm_nodes(fmpt_op* op, double t_re, double t_im, const double* x, int 
   FMPT_TRY(gs_setup(h, cp, n, M, gsbuf, gs));
   double* V = Vb.d();
   auto V_ = [&](int i) { return V + (int64_t)i * nr; };
-  rdot_partial<<<G, KT, 0, h->stream>>>(nr, x, x, part.d());
+  CHAIN(rdot_partial, G, h->stream, nr, x, x, part.d(), nullptr);
   FMPT_LAUNCHED(h);
-  normalize_from_parts<<<G, KT, 0, h->stream>>>(nr, x, V_(0), part.d(), G, acc.d());
+  CHAIN(normalize_from_parts, G, h->stream, nr, x, V_(0), part.d(), G, acc.d());
   FMPT_LAUNCHED(h);
   FMPT_TRY(arnoldi_basis(op, cp, n, nr, M, ldh, V, zb.d(), Hdev, gs));
   std::vector<double> Hh((size_t)ldh * M * 2);
@@ -1909,7 +1926,7 @@ int fmpt_expm_nodes(fmpt_op* op, double t_re, double t_im, const double* x, int 
   }
   FMPT_CUDA(h, cudaMemcpyAsync(Ed.d(), cols.data(), cols.size() * sizeof(double),
                                cudaMemcpyHostToDevice, h->stream));
-  combine_basis<<<dim3(G, nnodes), KT, 0, h->stream>>>(cp, n, m, V, nr, Ed.d(), 2 * m, acc.d(), out,
+  CHAIN(combine_basis, dim3(G, nnodes), h->stream, cp, n, m, V, nr, Ed.d(), 2 * m, acc.d(), out,
                                                        nr);
   FMPT_LAUNCHED(h);
   if (err_est) *err_est = e;

@@ -72,6 +72,7 @@ __device__ __forceinline__ void fetch_tile(const SliceSrc& src, int z, int r0, i
 // atomic max (mx zeroed beforehand).
 __global__ void __launch_bounds__(256, 4) oz_rowmax(SliceSrc src, int rows_out, int k_out,
                                                  unsigned long long* __restrict__ mx) {
+  chain_begin();
   __shared__ unsigned long long smax[SL_ROWS];
   const int r0 = blockIdx.x * SL_ROWS, kc0 = blockIdx.y * SL_KCH, z = blockIdx.z;
   const int t = threadIdx.x;
@@ -126,6 +127,7 @@ constexpr int RK_KCH = 1024;          // K columns per block, K-contiguous row m
 __global__ void __launch_bounds__(128) oz_rowmax_rowfast(const double* __restrict__ p, int64_t ld,
                                                          int64_t bstride, int rows, int k, int kch,
                                                          unsigned long long* __restrict__ mx) {
+  chain_begin();
   const int z = blockIdx.z;
   const int r = (blockIdx.x * 128 + threadIdx.x) * 2;
   const int c0 = blockIdx.y * kch, c1 = min(c0 + kch, k);
@@ -154,6 +156,7 @@ __global__ void __launch_bounds__(128) oz_rowmax_rowfast(const double* __restric
 __global__ void __launch_bounds__(256) oz_rowmax_kfast(const double* __restrict__ p, int64_t ld,
                                                        int64_t bstride, int rows, int k,
                                                        unsigned long long* __restrict__ mx) {
+  chain_begin();
   const int z = blockIdx.z, lane = threadIdx.x & 31;
   const int r = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (r >= rows) return;                                   // uniform over the warp
@@ -219,15 +222,15 @@ inline int oz_row_maxima(fmpt_handle* h, const SliceSrc& x, int rows, int k, int
     const int64_t want = (int64_t)k * gx * batch / (16LL * std::max(1, h->sm_count));
     const int kc = (int)std::max<int64_t>(8, std::min<int64_t>(128, want) / 8 * 8);
     const dim3 g1((unsigned)gx, (unsigned)((k + kc - 1) / kc), (unsigned)batch);
-    oz_rowmax_rowfast<<<g1, 128, 0, h->stream>>>(x.p, x.sc, x.bstride, rows, k, kc, mx);
+    FMPT_CUDA(h, launch_chain(oz_rowmax_rowfast, g1, 128, 0, h->stream, x.p, x.sc, x.bstride, rows, k, kc, mx));
   } else if (oz_kfast(x, k)) {
     const dim3 g1((unsigned)((rows + 7) / 8), (unsigned)((k + RK_KCH - 1) / RK_KCH),
                   (unsigned)batch);
-    oz_rowmax_kfast<<<g1, 256, 0, h->stream>>>(x.p, x.sr, x.bstride, rows, k, mx);
+    FMPT_CUDA(h, launch_chain(oz_rowmax_kfast, g1, 256, 0, h->stream, x.p, x.sr, x.bstride, rows, k, mx));
   } else {
     const dim3 g1((unsigned)((rows + SL_ROWS - 1) / SL_ROWS),
                   (unsigned)((k + SL_KCH - 1) / SL_KCH), (unsigned)batch);
-    oz_rowmax<<<g1, 256, 0, h->stream>>>(x, rows, k, mx);
+    FMPT_CUDA(h, launch_chain(oz_rowmax, g1, 256, 0, h->stream, x, rows, k, mx));
   }
   FMPT_LAUNCHED(h);
   return FMPT_OK;

@@ -175,6 +175,7 @@ __global__ void __launch_bounds__(256, 2) oz_residues(SliceSrc src, int rows_out
                                                    int kch, int tbits,
                                                    const unsigned long long* __restrict__ mxa,
                                                    uint16_t* __restrict__ S, int* __restrict__ E) {
+  chain_begin();
   __shared__ uint64_t tile[2][SL_ROWS][65];
   const int r0 = blockIdx.x * SL_ROWS, kc0 = blockIdx.y * kch, z = blockIdx.z;
   const int t = threadIdx.x, rr = t >> 3, part = t & 7;
@@ -217,6 +218,7 @@ __global__ void __launch_bounds__(256, 2) oz_residues_kfast(const double* __rest
                                                        const unsigned long long* __restrict__ mxa,
                                                        uint16_t* __restrict__ S,
                                                        int* __restrict__ E) {
+  chain_begin();
   const int r0 = blockIdx.x * SL_ROWS, kc0 = blockIdx.y * kch, z = blockIdx.z;
   const int t = threadIdx.x, rr = t >> 3, part = t & 7;
   const int r = r0 + rr;
@@ -253,6 +255,7 @@ __global__ void __launch_bounds__(256, 2) oz_residues_rowfast(const double* __re
                                                          const unsigned long long* __restrict__ mxa,
                                                          uint16_t* __restrict__ S,
                                                          int* __restrict__ E) {
+  chain_begin();
   extern __shared__ __align__(16) uint64_t dr_smem[];
   auto tile = [&](int st, int lr, int lc) -> uint64_t& {
     return dr_smem[((size_t)st * SL_ROWS + lr) * 65 + lc];
@@ -396,6 +399,7 @@ __global__ void __launch_bounds__(NTHR, 1)
   cluster_sync();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  chain_begin();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -629,6 +633,7 @@ __device__ __forceinline__ double crt_value(const uint32_t (&c)[NMOD], int E) {
 // applies alpha / beta in FP64.
 template <int NMOD, bool GENERAL>
 __global__ void __launch_bounds__(256) oz_crt(CrtArgs a) {
+  chain_begin();
   const int u = blockIdx.x >> 6, cg = blockIdx.x & 63;
   int mt2, nt, z;
   oz_tile(u, a.tiles_m2, a.tiles_n, mt2, nt, z);
@@ -667,6 +672,7 @@ __global__ void __launch_bounds__(256) oz_crt(CrtArgs a) {
 // C = alpha T + beta C of a complex product T (split planes, ld m) with general alpha, beta
 __global__ void oz_axpby_cplx(int m, int64_t n, const double* __restrict__ T, int64_t planeT,
                               CrtArgs a, int batch) {
+  chain_begin();
   const int64_t mn = (int64_t)m * n, total = mn * batch;
   const bool has_beta = a.beta[0] != 0.0 || a.beta[1] != 0.0;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
@@ -790,7 +796,7 @@ int gemm_f64_ozaki(fmpt_handle* h, const GemmArgs& g) {
   cfg.blockDim = dim3(NTHR);
   cfg.dynamicSmemBytes = SMEM;
   cfg.stream = h->stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
@@ -859,14 +865,12 @@ int gemm_f64_ozaki(fmpt_handle* h, const GemmArgs& g) {
       const dim3 grid(strips, (ldk + kch - 1) / kch, batch);
       FMPT_TRY(oz_row_maxima(h, x, rows, K2, batch, mx));
       if (oz_kfast(x, K2))
-        residues_kfast_kernel(nmod)<<<grid, 256, 0, h->stream>>>(
-            x.p, x.sr, x.bstride, rows, K2, ldk, kch, plan.tbits, mx, planes, ex);
+        FMPT_CUDA(h, launch_chain(residues_kfast_kernel(nmod), grid, 256, 0, h->stream, x.p, x.sr, x.bstride, rows, K2, ldk, kch, plan.tbits, mx, planes, ex));
       else if (x.sr == 1 && !x.cplx)
-        residues_rowfast_kernel(nmod)<<<grid, 256, DR_SMEM, h->stream>>>(
-            x.p, x.sc, x.bstride, rows, K2, ldk, kch, plan.tbits, mx, planes, ex);
+        FMPT_CUDA(h, launch_chain(residues_rowfast_kernel(nmod), grid, 256, DR_SMEM, h->stream, x.p, x.sc, x.bstride, rows, K2, ldk, kch, plan.tbits, mx, planes, ex));
       else
-        residues_kernel(nmod)<<<grid, 256, 0, h->stream>>>(x, rows, K2, ldk, kch, plan.tbits, mx,
-                                                           planes, ex);
+        FMPT_CUDA(h, launch_chain(residues_kernel(nmod), grid, 256, 0, h->stream, x, rows, K2, ldk, kch, plan.tbits, mx,
+                                                           planes, ex));
       FMPT_LAUNCHED(h);
       return FMPT_OK;
     };
@@ -892,6 +896,8 @@ int gemm_f64_ozaki(fmpt_handle* h, const GemmArgs& g) {
   cfg.gridDim = dim3((unsigned)(2 * std::min<int64_t>(units * nmod, clusters)));
   {
     ProfScope prof(h, FMPT_K_TC_GEMM);
+    chain_attr(attr[1]);
+    cfg.numAttrs = 2;
     FMPT_CUDA(h, cudaLaunchKernelEx(&cfg, oz_gemm_pair, ma, mb, K2, tiles_m2, tiles_n, batch, nmod,
                                     ep));
     FMPT_LAUNCHED(h);
@@ -925,11 +931,11 @@ int gemm_f64_ozaki(fmpt_handle* h, const GemmArgs& g) {
   ProfScope prof(h, FMPT_K_CONVERT);
   const unsigned blocks = (unsigned)(units * 64);
   if (nmod == 15) {
-    if (general) oz_crt<15, true><<<blocks, 256, 0, h->stream>>>(ca);
-    else oz_crt<15, false><<<blocks, 256, 0, h->stream>>>(ca);
+    if (general) FMPT_CUDA(h, launch_chain(oz_crt<15, true>, blocks, 256, 0, h->stream, ca));
+    else FMPT_CUDA(h, launch_chain(oz_crt<15, false>, blocks, 256, 0, h->stream, ca));
   } else {
-    if (general) oz_crt<16, true><<<blocks, 256, 0, h->stream>>>(ca);
-    else oz_crt<16, false><<<blocks, 256, 0, h->stream>>>(ca);
+    if (general) FMPT_CUDA(h, launch_chain(oz_crt<16, true>, blocks, 256, 0, h->stream, ca));
+    else FMPT_CUDA(h, launch_chain(oz_crt<16, false>, blocks, 256, 0, h->stream, ca));
   }
   FMPT_LAUNCHED(h);
   if (via_copy) {
@@ -944,7 +950,7 @@ int gemm_f64_ozaki(fmpt_handle* h, const GemmArgs& g) {
     }
     const int64_t total = (int64_t)g.m * N * batch;
     const int nb = (int)std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, 8LL * h->sm_count));
-    oz_axpby_cplx<<<nb, 256, 0, h->stream>>>(g.m, N, COPY, ca.planeC, cc, batch);
+    FMPT_CUDA(h, launch_chain(oz_axpby_cplx, nb, 256, 0, h->stream, g.m, N, COPY, ca.planeC, cc, batch));
     FMPT_LAUNCHED(h);
   }
   return FMPT_OK;

@@ -153,6 +153,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  chain_begin();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -411,6 +412,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   cluster_sync();                 // both CTAs' barriers exist before either signals the other
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  chain_begin();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -643,6 +645,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  chain_begin();
 
   bool got = false;                                    // epilogue warps: the piece is complete
   if (warp == 0) {
@@ -839,7 +842,7 @@ static int tc_gemm_small(fmpt_handle* h, int M, int N, int K, int batch, int S, 
   cfg.blockDim = dim3(NTHREADS);
   cfg.dynamicSmemBytes = C_::SMEM;
   cfg.stream = h->stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = S;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
@@ -856,6 +859,7 @@ static int tc_gemm_small(fmpt_handle* h, int M, int N, int K, int batch, int S, 
     fits[vi][S] = n > 0 ? 1 : -1;
   }
   if (fits[vi][S] < 0) return FMPT_ERR_UNSUPPORTED;
+  chain_attr(attr[cfg.numAttrs++]);
   ProfScope prof(h, FMPT_K_TC_GEMM);
   FMPT_CUDA(h, cudaLaunchKernelEx(&cfg, kfn, ma, mb, ma2, mb2, K, tiles_m, tiles_n, S, ep));
   FMPT_LAUNCHED(h);
@@ -935,7 +939,7 @@ static int tc_gemm_pair_st(fmpt_handle* h, int M, int N, int K, int batch, const
   cfg.blockDim = dim3(NTHREADS);
   cfg.dynamicSmemBytes = C_::SMEM;
   cfg.stream = h->stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
@@ -992,6 +996,7 @@ static int tc_gemm_pair_st(fmpt_handle* h, int M, int N, int K, int batch, const
   }
   const int64_t items = (int64_t)sp.full + (int64_t)sp.tail * sp.S;
   cfg.gridDim = dim3((unsigned)(2 * std::min<int64_t>(items, cl)));
+  chain_attr(attr[cfg.numAttrs++]);
   ProfScope prof(h, FMPT_K_TC_GEMM);
   FMPT_CUDA(h, cudaLaunchKernelEx(&cfg, kfn, ma, mb, ma2, mb2, K, tiles_m2, tiles_n, batch, ep, sp));
   FMPT_LAUNCHED(h);
@@ -1055,7 +1060,8 @@ int tc_gemm(fmpt_handle* h, int mode, int M, int N, int K, int batch, const TcOp
       FMPT_CUDA(h, cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_)); \
       attr_done = true;                                                                       \
     }                                                                                         \
-    kfn<<<grid, NTHREADS, SM_, h->stream>>>(ma, mb, ma2, mb2, K, tiles_m, tiles_n, batch, ep); \
+    FMPT_CUDA(h, launch_chain(kfn, grid, NTHREADS, SM_, h->stream, ma, mb, ma2, mb2, K, tiles_m,  \
+                              tiles_n, batch, ep));                                         \
   } while (0)
   if (mode == TF32) {
     if (out_f64) LAUNCH(TF32, 256, 4, 1); else LAUNCH(TF32, 256, 4, 0);

@@ -54,6 +54,7 @@ __device__ __forceinline__ void put(void* hi, void* lo, int64_t i, double v) {
 template <int MODE>
 __global__ void conv_state(const double* __restrict__ x, int Dl, int Kp, int64_t M, void* hi,
                            void* lo, int64_t dld) {
+  chain_begin();
   const int64_t tot = (int64_t)Kp * M;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < tot;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -68,6 +69,7 @@ __global__ void conv_state(const double* __restrict__ x, int Dl, int Kp, int64_t
 // n4 = Kp*M/4 (Kp is a multiple of 8).  Same rounding per element as put().
 template <int MODE>
 __global__ void conv_state_vec(const double* __restrict__ x, int64_t n4, void* hi, void* lo) {
+  chain_begin();
   const double2* x2 = reinterpret_cast<const double2*>(x);
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n4;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -97,6 +99,7 @@ template <int MODE>
 __global__ void conv_transpose(const double* __restrict__ src, int64_t sld, int64_t sz, int R,
                                int C, int Cp, void* hi, void* lo, int64_t dld, int64_t dz,
                                double scale) {
+  chain_begin();
   __shared__ double tile[32][33];
   const int z = blockIdx.z;
   const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
@@ -119,6 +122,7 @@ template <int MODE, int MAXP>
 __global__ void mid_tc(const float* __restrict__ T1, int P, int Dl, int Dr, int Drp, int64_t K2,
                        int nw_out, const int* __restrict__ win, const int* __restrict__ wstart,
                        const double* __restrict__ coef, void* hi, void* lo) {
+  chain_begin();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)Dl * Dr) return;
   const int b = (int)(t % Dr), ap = (int)(t / Dr);
@@ -177,6 +181,7 @@ __global__ void __launch_bounds__(256) mid_tc_p4(const V4* __restrict__ T1, int 
                                                  int Drp, int64_t K2, int nw_in, int nw_out,
                                                  uint64_t mask, const __grid_constant__ MidCoef cp,
                                                  void* hi, void* lo) {
+  chain_begin();
   const auto& c = cp.c;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)Dl * Dr) return;
@@ -225,6 +230,7 @@ __global__ void __launch_bounds__(256) mid_bf16_x2(const uint4* __restrict__ T1,
                                                    uint64_t mask,
                                                    const __grid_constant__ MidCoef cp,
                                                    __nv_bfloat16* __restrict__ out) {
+  chain_begin();
   const auto& c = cp.c;
   const int hr = Dr >> 1;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -278,6 +284,7 @@ __global__ void __launch_bounds__(256) mid_tc_mask(const float* __restrict__ T, 
                                                    const __grid_constant__ MidCoef cp, void* hi,
                                                    void* lo, int64_t o1s, int64_t o2s,
                                                    int64_t ows, int64_t oqs) {
+  chain_begin();
   const auto& c = cp.c;                           // [wi*8 + wo][q*P + s], constant bank
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (int64_t)n1 * n2) return;
@@ -334,8 +341,8 @@ int launch_transpose(fmpt_handle* h, const double* src, int64_t sld, int64_t sz,
                      int Cp, int Z, void* hi, void* lo, int64_t dld, int64_t dz, double scale) {
   dim3 grid((R + 31) / 32, (Cp + 31) / 32, Z);
   ProfScope prof(h, FMPT_K_CONVERT);
-  conv_transpose<MODE><<<grid, dim3(32, 8), 0, h->stream>>>(src, sld, sz, R, C, Cp, hi, lo, dld, dz,
-                                                           scale);
+  FMPT_CUDA(h, launch_chain(conv_transpose<MODE>, grid, dim3(32, 8), 0, h->stream, src, sld, sz, R, C, Cp, hi, lo, dld, dz,
+                                                           scale));
   FMPT_LAUNCHED(h);
   return FMPT_OK;
 }
@@ -519,17 +526,17 @@ int op_tc_apply_head(fmpt_op* op, const double* x) {
   if (ident) {
     const int64_t n4 = nx / 4;
     if (st->mode == M_TF32)
-      conv_state_vec<M_TF32><<<grid1(h, n4), 256, 0, h->stream>>>(x, n4, st->xg[0].p, xlo);
+      FMPT_CUDA(h, launch_chain(conv_state_vec<M_TF32>, grid1(h, n4), 256, 0, h->stream, x, n4, st->xg[0].p, xlo));
     else if (st->mode == M_TF32X3)
-      conv_state_vec<M_TF32X3><<<grid1(h, n4), 256, 0, h->stream>>>(x, n4, st->xg[0].p, xlo);
+      FMPT_CUDA(h, launch_chain(conv_state_vec<M_TF32X3>, grid1(h, n4), 256, 0, h->stream, x, n4, st->xg[0].p, xlo));
     else
-      conv_state_vec<M_BF16><<<grid1(h, n4), 256, 0, h->stream>>>(x, n4, st->xg[0].p, xlo);
+      FMPT_CUDA(h, launch_chain(conv_state_vec<M_BF16>, grid1(h, n4), 256, 0, h->stream, x, n4, st->xg[0].p, xlo));
   } else if (st->mode == M_TF32)
-    conv_state<M_TF32><<<grid1(h, nx), 256, 0, h->stream>>>(x, Dl, st->Kp, (int64_t)P * Dr, st->xg[0].p, xlo, st->Kp);
+    FMPT_CUDA(h, launch_chain(conv_state<M_TF32>, grid1(h, nx), 256, 0, h->stream, x, Dl, st->Kp, (int64_t)P * Dr, st->xg[0].p, xlo, st->Kp));
   else if (st->mode == M_TF32X3)
-    conv_state<M_TF32X3><<<grid1(h, nx), 256, 0, h->stream>>>(x, Dl, st->Kp, (int64_t)P * Dr, st->xg[0].p, xlo, st->Kp);
+    FMPT_CUDA(h, launch_chain(conv_state<M_TF32X3>, grid1(h, nx), 256, 0, h->stream, x, Dl, st->Kp, (int64_t)P * Dr, st->xg[0].p, xlo, st->Kp));
   else
-    conv_state<M_BF16><<<grid1(h, nx), 256, 0, h->stream>>>(x, Dl, st->Kp, (int64_t)P * Dr, st->xg[0].p, xlo, st->Kp);
+    FMPT_CUDA(h, launch_chain(conv_state<M_BF16>, grid1(h, nx), 256, 0, h->stream, x, Dl, st->Kp, (int64_t)P * Dr, st->xg[0].p, xlo, st->Kp));
   FMPT_LAUNCHED(h);
   }
   // GEMM 1: T1[(s b), (a' w)] = sum_a xg[a, (s b)] Lg[a, (a' w)]
@@ -550,27 +557,23 @@ int op_tc_apply_head(fmpt_op* op, const double* x) {
 #define MIDP4(NW_)                                                                                \
   do {                                                                                            \
     if (st->mode == M_TF32)                                                                       \
-      mid_tc_p4<M_TF32, float4, NW_><<<blocks, 256, 0, h->stream>>>(                              \
-          t1, Dl, Dr, st->Drp, st->K2, s.nw_in, s.nw_out, st->mask, st->cpar, st->T3[0].p, tlo); \
+      FMPT_CUDA(h, launch_chain(mid_tc_p4<M_TF32, float4, NW_>, blocks, 256, 0, h->stream, t1, Dl, Dr, st->Drp, st->K2, s.nw_in, s.nw_out, st->mask, st->cpar, st->T3[0].p, tlo)); \
     else if (st->mode == M_TF32X3)                                                                \
-      mid_tc_p4<M_TF32X3, float4, NW_><<<blocks, 256, 0, h->stream>>>(                            \
-          t1, Dl, Dr, st->Drp, st->K2, s.nw_in, s.nw_out, st->mask, st->cpar, st->T3[0].p, tlo); \
+      FMPT_CUDA(h, launch_chain(mid_tc_p4<M_TF32X3, float4, NW_>, blocks, 256, 0, h->stream, t1, Dl, Dr, st->Drp, st->K2, s.nw_in, s.nw_out, st->mask, st->cpar, st->T3[0].p, tlo)); \
     else if (Dr % 2 == 0)                                                                         \
-      mid_bf16_x2<NW_><<<(unsigned)((nt / 2 + 255) / 256), 256, 0, h->stream>>>(                  \
-          (const uint4*)st->T1.p, Dl, Dr, st->Drp, st->K2, s.nw_in, s.nw_out, st->mask, st->cpar, \
-          (__nv_bfloat16*)st->T3[0].p);                                                           \
+      FMPT_CUDA(h, launch_chain(mid_bf16_x2<NW_>, (unsigned)((nt / 2 + 255) / 256), 256, 0, h->stream, (const uint4*)st->T1.p, Dl, Dr, st->Drp, st->K2, s.nw_in, s.nw_out, st->mask, st->cpar, \
+          (__nv_bfloat16*)st->T3[0].p));                                                           \
     else                                                                                          \
-      mid_tc_p4<M_BF16, uint2, NW_><<<blocks, 256, 0, h->stream>>>(                               \
-          (const uint2*)st->T1.p, Dl, Dr, st->Drp, st->K2, s.nw_in, s.nw_out, st->mask, st->cpar, \
-          st->T3[0].p, tlo);                                                                      \
+      FMPT_CUDA(h, launch_chain(mid_tc_p4<M_BF16, uint2, NW_>, blocks, 256, 0, h->stream, (const uint2*)st->T1.p, Dl, Dr, st->Drp, st->K2, s.nw_in, s.nw_out, st->mask, st->cpar, \
+          st->T3[0].p, tlo));                                                                      \
   } while (0)
       if (nw <= 4) MIDP4(4); else if (nw <= 6) MIDP4(6); else MIDP4(8);
 #undef MIDP4
     } else
 #define MIDTC(MODE_, MP_)                                                                    \
-  mid_tc<MODE_, MP_><<<blocks, 256, 0, h->stream>>>((const float*)st->T1.p,                \
+  FMPT_CUDA(h, launch_chain(mid_tc<MODE_, MP_>, blocks, 256, 0, h->stream, (const float*)st->T1.p,                \
                                                     P, Dl, Dr, st->Drp, st->K2, s.nw_out,      \
-                                                    s.d_win, s.d_wstart, s.d_coef, st->T3[0].p, tlo)
+                                                    s.d_win, s.d_wstart, s.d_coef, st->T3[0].p, tlo))
     if (P <= 4) {
       if (st->mode == M_TF32) MIDTC(M_TF32, 4); else if (st->mode == M_TF32X3) MIDTC(M_TF32X3, 4); else MIDTC(M_BF16, 4);
     } else {
@@ -629,11 +632,11 @@ int op_tc_apply_complex(fmpt_op* op, TcState* st, const double* x, double* y) {
       void* hi = offset(st->xg[0].p, part * st->Kp, es);
       void* lo = offset(xlo, part * st->Kp, es);
       if (st->mode == M_TF32)
-        conv_state<M_TF32><<<grid1(h, nx), 256, 0, h->stream>>>(src, Dl, st->Kp, (int64_t)P * Dr, hi, lo, 2LL * st->Kp);
+        FMPT_CUDA(h, launch_chain(conv_state<M_TF32>, grid1(h, nx), 256, 0, h->stream, src, Dl, st->Kp, (int64_t)P * Dr, hi, lo, 2LL * st->Kp));
       else if (st->mode == M_TF32X3)
-        conv_state<M_TF32X3><<<grid1(h, nx), 256, 0, h->stream>>>(src, Dl, st->Kp, (int64_t)P * Dr, hi, lo, 2LL * st->Kp);
+        FMPT_CUDA(h, launch_chain(conv_state<M_TF32X3>, grid1(h, nx), 256, 0, h->stream, src, Dl, st->Kp, (int64_t)P * Dr, hi, lo, 2LL * st->Kp));
       else
-        conv_state<M_BF16><<<grid1(h, nx), 256, 0, h->stream>>>(src, Dl, st->Kp, (int64_t)P * Dr, hi, lo, 2LL * st->Kp);
+        FMPT_CUDA(h, launch_chain(conv_state<M_BF16>, grid1(h, nx), 256, 0, h->stream, src, Dl, st->Kp, (int64_t)P * Dr, hi, lo, 2LL * st->Kp));
       FMPT_LAUNCHED(h);
     }
   }
@@ -654,15 +657,15 @@ int op_tc_apply_complex(fmpt_op* op, TcState* st, const double* x, double* y) {
       void* lo = offset(tlo, part * st->K2, es);
       if (st->fast_mid) {
           if (st->mode == M_TF32)
-          mid_tc_p4<M_TF32, float4, 8><<<blocks, 256, 0, h->stream>>>((const float4*)t1, Dl, Dr, st->Drp, K2c, s.nw_in, s.nw_out, st->mask, st->cpar, hi, lo);
+          FMPT_CUDA(h, launch_chain(mid_tc_p4<M_TF32, float4, 8>, blocks, 256, 0, h->stream, (const float4*)t1, Dl, Dr, st->Drp, K2c, s.nw_in, s.nw_out, st->mask, st->cpar, hi, lo));
         else if (st->mode == M_TF32X3)
-          mid_tc_p4<M_TF32X3, float4, 8><<<blocks, 256, 0, h->stream>>>((const float4*)t1, Dl, Dr, st->Drp, K2c, s.nw_in, s.nw_out, st->mask, st->cpar, hi, lo);
+          FMPT_CUDA(h, launch_chain(mid_tc_p4<M_TF32X3, float4, 8>, blocks, 256, 0, h->stream, (const float4*)t1, Dl, Dr, st->Drp, K2c, s.nw_in, s.nw_out, st->mask, st->cpar, hi, lo));
         else
-          mid_tc_p4<M_BF16, float4, 8><<<blocks, 256, 0, h->stream>>>((const float4*)t1, Dl, Dr, st->Drp, K2c, s.nw_in, s.nw_out, st->mask, st->cpar, hi, lo);
+          FMPT_CUDA(h, launch_chain(mid_tc_p4<M_BF16, float4, 8>, blocks, 256, 0, h->stream, (const float4*)t1, Dl, Dr, st->Drp, K2c, s.nw_in, s.nw_out, st->mask, st->cpar, hi, lo));
       } else {
 #define MIDTCC(MODE_, MP_)                                                                   \
-  mid_tc<MODE_, MP_><<<blocks, 256, 0, h->stream>>>(t1, P, Dl, Dr, st->Drp, K2c, s.nw_out,    \
-                                                    s.d_win, s.d_wstart, s.d_coef, hi, lo)
+  FMPT_CUDA(h, launch_chain(mid_tc<MODE_, MP_>, blocks, 256, 0, h->stream, t1, P, Dl, Dr, st->Drp, K2c, s.nw_out,    \
+                                                    s.d_win, s.d_wstart, s.d_coef, hi, lo))
         if (P <= 4) {
           if (st->mode == M_TF32) MIDTCC(M_TF32, 4); else if (st->mode == M_TF32X3) MIDTCC(M_TF32X3, 4); else MIDTCC(M_BF16, 4);
         } else {
@@ -717,11 +720,11 @@ int launch_mask(fmpt_handle* h, int P, const float* T, int64_t i1, int64_t i2, i
   const unsigned blocks = (unsigned)((nt + 255) / 256);
   ProfScope prof(h, FMPT_K_MPO_STEP);
   if (P <= 2)
-    mid_tc_mask<MODE, 2><<<blocks, 256, 0, h->stream>>>(T, i1, i2, iw, is, n1, n2, nw_in, nw_out,
-                                                         mask, c, hi, lo, o1, o2, ow, oq);
+    FMPT_CUDA(h, launch_chain(mid_tc_mask<MODE, 2>, blocks, 256, 0, h->stream, T, i1, i2, iw, is, n1, n2, nw_in, nw_out,
+                                                         mask, c, hi, lo, o1, o2, ow, oq));
   else
-    mid_tc_mask<MODE, 4><<<blocks, 256, 0, h->stream>>>(T, i1, i2, iw, is, n1, n2, nw_in, nw_out,
-                                                         mask, c, hi, lo, o1, o2, ow, oq);
+    FMPT_CUDA(h, launch_chain(mid_tc_mask<MODE, 4>, blocks, 256, 0, h->stream, T, i1, i2, iw, is, n1, n2, nw_in, nw_out,
+                                                         mask, c, hi, lo, o1, o2, ow, oq));
   FMPT_LAUNCHED(h);
   return FMPT_OK;
 }
@@ -731,11 +734,11 @@ int conv_state_any(fmpt_handle* h, int mode, const double* x, int K, int Kp, int
   const int64_t n = (int64_t)Kp * M;
   ProfScope prof(h, FMPT_K_CONVERT);
   if (mode == M_TF32)
-    conv_state<M_TF32><<<grid1(h, n), 256, 0, h->stream>>>(x, K, Kp, M, hi, lo, Kp);
+    FMPT_CUDA(h, launch_chain(conv_state<M_TF32>, grid1(h, n), 256, 0, h->stream, x, K, Kp, M, hi, lo, Kp));
   else if (mode == M_TF32X3)
-    conv_state<M_TF32X3><<<grid1(h, n), 256, 0, h->stream>>>(x, K, Kp, M, hi, lo, Kp);
+    FMPT_CUDA(h, launch_chain(conv_state<M_TF32X3>, grid1(h, n), 256, 0, h->stream, x, K, Kp, M, hi, lo, Kp));
   else
-    conv_state<M_BF16><<<grid1(h, n), 256, 0, h->stream>>>(x, K, Kp, M, hi, lo, Kp);
+    FMPT_CUDA(h, launch_chain(conv_state<M_BF16>, grid1(h, n), 256, 0, h->stream, x, K, Kp, M, hi, lo, Kp));
   FMPT_LAUNCHED(h);
   return FMPT_OK;
 }
