@@ -7,16 +7,18 @@
 //   SUM  phase:  C_p = sum_{j in segs(p)} coef_j * op(A_j)             (overwrite)
 // where every operand is a strided sub-matrix (offset + leading dimension) of
 // one of a few operand slots (device base pointers given at run time).  The
-// whole program runs as ONE cooperative launch: CTAs pull 32x32 output tiles
-// of the current phase from a device work counter (atomicAdd, largest blocks
-// first) and meet at a grid barrier between phases.  The barrier spin is
+// whole program runs as ONE cooperative launch: warps pull 8x4 output tiles (or,
+// in the other variants, CTAs pull 32x32 or 64x64 tiles) of the current phase
+// from a device work counter (atomicAdd, largest blocks first) and meet at a
+// grid barrier between phases.  The barrier spin is
 // bounded (2 s on %globaltimer); on timeout a CTA sets the launch's abort
 // flag and the handle's status word, and every CTA returns.
 //
 // Each output tile sums its segments in the order they were added, so the
-// result does not depend on scheduling.  FP64 is FMA-pipe bound on GB300
-// (about 2 DFMA per clock per SM), so the kernel's job is to keep every SM's
-// FP64 pipe fed across thousands of 1..400-wide blocks.
+// result does not depend on scheduling.  FP64 is FMA-pipe bound on GB300: a
+// warp's FMA occupies its SM sub-partition for 64 to 77 cycles, so the kernel's
+// job is to spread the FMAs of thousands of 1..400-wide blocks evenly over the
+// 608 sub-partitions.
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -46,7 +48,9 @@ struct GKArgs {
   const GSegment* segs;
   const int* tile_prob;
   const int* tile_mn;
-  int* ctl;        // [0, GP_MAX_PHASES) tile counters, then barrier count, then abort flag
+  const GWarpProb* wprob;   // GP_WARP: [tile0, tile1) of a phase index these (tile1 - 1: the end)
+  int* ctl;        // [0, GP_MAX_PHASES) tile counters, barrier count, abort flag, exit count:
+                   // zero before a launch and left zero by it
   int* status;     // handle status word (1 = a bounded wait gave up)
   const int* gate; // nonzero at launch: return at once (nullptr: always run)
   uint64_t wait_ns;   // bound of every barrier wait
@@ -97,6 +101,16 @@ __device__ bool grid_barrier(const GKArgs& a, int target, int* s_flag) {
   }
   __syncthreads();
   return *s_flag != 0;
+}
+
+// Every thread of every CTA, last of all: the last CTA to leave zeroes the control words for
+// the next launch (no CTA polls the abort flag any more by then).
+__device__ __forceinline__ void leave(const GKArgs& a) {
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  __threadfence();
+  if (atomicAdd(a.ctl + GP_MAX_PHASES + 2, 1) != (int)gridDim.x - 1) return;
+  for (int i = 0; i < GP_MAX_PHASES + 3; i++) a.ctl[i] = 0;
 }
 
 // Tile word: origin in 16-row / 16-column units and extent in 16-wide groups,
@@ -230,7 +244,7 @@ __global__ void __launch_bounds__(GNT) grouped_kernel(const GKArgs a) {
   __shared__ int s_tile, s_flag;
   if (a.gate && *a.gate) return;   // uniform for the whole grid: set before the launch
   for (int p = 0; p < a.nphase; p++) {
-    if (p > 0 && !grid_barrier(a, p * (int)gridDim.x, &s_flag)) return;
+    if (p > 0 && !grid_barrier(a, p * (int)gridDim.x, &s_flag)) break;
     const GPhaseDesc ph = a.ph[p];
     const int ntiles = ph.tile1 - ph.tile0;
     while (true) {
@@ -247,21 +261,244 @@ __global__ void __launch_bounds__(GNT) grouped_kernel(const GKArgs a) {
         sum_tile<GT>(a, ph, ph.tile0 + t);
     }
   }
+  leave(a);
 }
 
-int g_occupancy[2] = {0, 0};
+// Variant GP_WARP: every warp pulls 8x4 tiles of its own (one output per lane), the unit of
+// work that fills the sub-partitions evenly and pads blocks least.  At a centre bond of 64
+// sites and D = 512 the last contraction has 258 tiles of 32x32, up to 93 us each on an SM of
+// their own, for 152 SMs, and 16-wide groups pad its blocks (10 to 71 wide) by a third; its
+// 3604 tiles of 8x4 pad by 8%.  Re-reading the operands per small tile costs nothing beside
+// an FMA's 64 cycles.  H_eff*x, us, best block tile -> warp tile: D = 32 (16 sites) 18.7 ->
+// 16.9, D = 64 24.8 -> 18.8, D = 128 84 -> 26, D = 256 200 -> 52, D = 512 366 -> 121,
+// D = 1024 1006 -> 764, D = 1500 2498 -> 2316 (FP64 pipe bound).  Four blocks of four warps
+// per SM: with two, a warp's start on a tile (descriptors, first slab) shows, 140 us at
+// D = 512; slabs in flight per warp: 2 (4 or 6 stages were no faster).
+constexpr int QM = 8, QN = 4, QK = 16, QST = 3, QWARPS = 4, QBLOCKS = 4;
+constexpr int QSM = 32, QSN = 4;           // tile of a SUM phase
+
+// 8 bytes, zeros if !in
+__device__ __forceinline__ void cp_async8z(double* dst, const double* src, bool in) {
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src),
+               "r"(in ? 8 : 0)
+               : "memory");
+}
+
+// The segments of a tile: each lane holds one of the 32 around the last one asked for, so that
+// a tile waits for one load of its descriptors, not for one per segment.
+struct SegWindow {
+  const GSegment* segs;
+  GSegment mine{};
+  int base = 0, end = 0;
+  __device__ __forceinline__ void open(int seg0, int seg1) {
+    base = seg0;
+    end = seg1;
+    load();
+  }
+  __device__ __forceinline__ void load() {
+    const int i = base + (int)(threadIdx.x & 31);
+    if (i < end) mine = segs[i];
+  }
+  // whole warp, ascending i < end
+  __device__ __forceinline__ GSegment get(int i) {
+    if (i >= base + 32) { base = i; load(); }
+    const int l = i - base;
+    GSegment s{};
+    s.a_off = __shfl_sync(~0u, mine.a_off, l); s.lda = __shfl_sync(~0u, mine.lda, l);
+    s.b_off = __shfl_sync(~0u, mine.b_off, l); s.ldb = __shfl_sync(~0u, mine.ldb, l);
+    s.coef = __shfl_sync(~0u, mine.coef, l); s.k = __shfl_sync(~0u, mine.k, l);
+    return s;
+  }
+};
+
+// One 8x4 tile at (m0, n0) of a GEMM problem by one warp.  The K slabs of all its segments
+// stream through the warp's ring by cp.async, QST - 1 slabs ahead.  Each output is the same
+// chain of FMAs over segments and k as in gemm_tile.
+__device__ __forceinline__ void gemm_warp_tile(const GKArgs& a, const GPhaseDesc& ph,
+                                               const GProblem& P, int m0, int n0, SegWindow& win,
+                                               double (*As)[QK][QM], double (*Bs)[QK][QN]) {
+  const int lane = threadIdx.x & 31, lm = lane & 7, ln = lane >> 3;
+  const bool a_mfast = (ph.ta == FMPT_N || ph.ta == FMPT_R);
+  const bool b_kfast = (ph.tb == FMPT_N || ph.tb == FMPT_R);
+  // this lane's elements of a slab: the first one here, the next ones a fixed step on, so
+  // that lanes run along the contiguous index
+  const int amm = a_mfast ? lane % QM : lane / QK, akk = a_mfast ? lane / QM : lane % QK;
+  const int adm = a_mfast ? 0 : 32 / QK, adk = a_mfast ? 32 / QM : 0;
+  const int bnn = b_kfast ? lane / QK : lane % QN, bkk = b_kfast ? lane % QK : lane / QN;
+  const int bdn = b_kfast ? 32 / QK : 0, bdk = b_kfast ? 0 : 32 / QN;
+  const double* Ab = a.slot[ph.a_slot];
+  const double* Bb = a.slot[ph.b_slot];
+  int isg = P.seg0, ik = 0, iK = 0, ist = 0;         // the slab issued next
+  int64_t sam = 0, sak = 0, sbk = 0, sbn = 0;
+  double icoef = 1.0;
+  const double *pa = Ab, *pb = Bb;
+  // issues the next slab; its depth in k (0: none is left) and coefficient go to kn, coef
+  auto issue = [&](int& kn, double& coef) {
+    while (ik >= iK && isg < P.seg1) {               // the next segment that has a k
+      const GSegment S = win.get(isg++);
+      ik = 0;
+      iK = S.k;
+      icoef = S.coef;
+      sam = a_mfast ? 1 : S.lda; sak = a_mfast ? S.lda : 1;
+      sbk = b_kfast ? 1 : S.ldb; sbn = b_kfast ? S.ldb : 1;
+      pa = Ab + S.a_off + (m0 + amm) * sam + akk * sak;
+      pb = Bb + S.b_off + (n0 + bnn) * sbn + bkk * sbk;
+    }
+    kn = max(0, min(QK, iK - ik));
+    coef = icoef;
+    if (kn > 0) {
+#pragma unroll
+      for (int e = 0; e < QM * QK / 32; e++) {
+        const int mm = amm + e * adm, kk = akk + e * adk;
+        const bool in = m0 + mm < P.m && kk < kn;
+        cp_async8z(&As[ist][kk][mm], in ? pa + e * (adm * sam + adk * sak) : Ab, in);
+      }
+#pragma unroll
+      for (int e = 0; e < QN * QK / 32; e++) {
+        const int nn = bnn + e * bdn, kk = bkk + e * bdk;
+        const bool in = n0 + nn < P.n && kk < kn;
+        cp_async8z(&Bs[ist][kk][nn], in ? pb + e * (bdn * sbn + bdk * sbk) : Bb, in);
+      }
+      pa += QK * sak;
+      pb += QK * sbk;
+      ik += QK;
+      ist = (ist + 1) % QST;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");   // one group per slab slot
+  };
+  double acc = 0.0;
+  int st = 0, kn[QST];                               // depths and coefficients of the slabs
+  double coef[QST];                                  // in flight, oldest first
+#pragma unroll
+  for (int j = 0; j < QST - 1; j++) issue(kn[j], coef[j]);
+  while (kn[0] > 0) {
+    issue(kn[QST - 1], coef[QST - 1]);
+    asm volatile("cp.async.wait_group %0;" ::"n"(QST - 1) : "memory");
+    __syncwarp();
+    if (coef[0] != 1.0) {
+#pragma unroll
+      for (int e = 0; e < QM * QK / 32; e++) As[st][ln + e * (32 / QM)][lm] *= coef[0];
+      __syncwarp();
+    }
+    if (kn[0] == QK) {
+#pragma unroll
+      for (int kk = 0; kk < QK; kk++) acc = fma(As[st][kk][lm], Bs[st][kk][ln], acc);
+    } else {
+      for (int kk = 0; kk < kn[0]; kk++) acc = fma(As[st][kk][lm], Bs[st][kk][ln], acc);
+    }
+    __syncwarp();                                    // the stage is refilled by the next issue
+    st = (st + 1) % QST;
+#pragma unroll
+    for (int j = 0; j < QST - 1; j++) { kn[j] = kn[j + 1]; coef[j] = coef[j + 1]; }
+  }
+  const int r = m0 + lm, c = n0 + ln;
+  if (r < P.m && c < P.n) a.slot[ph.c_slot][P.c_off + r + (int64_t)c * P.ldc] = acc;
+}
+
+// A QSM x QSN tile of a SUM problem by one warp: a row per lane.
+__device__ __forceinline__ void sum_warp_tile(const GKArgs& a, const GPhaseDesc& ph,
+                                              const GProblem& P, int m0, int n0,
+                                              SegWindow& win) {
+  const int r = m0 + (int)(threadIdx.x & 31);
+  const double* Ab = a.slot[ph.a_slot];
+  double* C = a.slot[ph.c_slot] + P.c_off;
+  const int nc = r < P.m ? min(P.n - n0, QSN) : 0;    // this lane's columns
+  double s[QSN] = {};
+  // four summands' loads are in flight at a time; each output adds them in their order
+  constexpr int Q = 4;
+  for (int sg = P.seg0; sg < P.seg1; sg += Q) {
+    double v[Q][QSN], coef[Q];
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      if (sg + q >= P.seg1) break;
+      const GSegment S = win.get(sg + q);
+      coef[q] = S.coef;
+#pragma unroll
+      for (int j = 0; j < QSN; j++)
+        v[q][j] = j < nc ? __ldg(Ab + S.a_off + op_index(ph.ta, r, n0 + j, S.lda)) : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      if (sg + q >= P.seg1) break;
+#pragma unroll
+      for (int j = 0; j < QSN; j++)
+        if (j < nc) s[j] = fma(coef[q], v[q][j], s[j]);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < QSN; j++)
+    if (j < nc) C[r + (int64_t)(n0 + j) * P.ldc] = s[j];
+}
+
+// The block that holds tile t of a phase: the last entry i of w[0, n) with w[i].tile0 <= t,
+// by a search of the whole warp (32 probes per round).
+__device__ __forceinline__ int find_block(const GWarpProb* w, int n, int t) {
+  int lo = 0, len = n;
+  while (len > 1) {
+    const int step = (len + 31) / 32, i = (int)(threadIdx.x & 31) * step;
+    const unsigned le = __ballot_sync(~0u, i < len && w[lo + i].tile0 <= t);
+    const int q = 31 - __clz(le);                    // lane 0 is always in
+    lo += q * step;
+    len = min(step, len - q * step);
+  }
+  return lo;
+}
+
+__global__ void __launch_bounds__(32 * QWARPS, QBLOCKS) grouped_warp(const GKArgs a) {
+  __shared__ double As[QWARPS][QST][QK][QM], Bs[QWARPS][QST][QK][QN];
+  __shared__ int s_flag;
+  if (a.gate && *a.gate) return;   // uniform for the whole grid: set before the launch
+  const int wid = threadIdx.x >> 5, nw = (int)gridDim.x * QWARPS;
+  SegWindow win{a.segs};
+  for (int p = 0; p < a.nphase; p++) {
+    const GPhaseDesc ph = a.ph[p];
+    const GWarpProb* w = a.wprob + ph.tile0;
+    const int nb = ph.tile1 - ph.tile0 - 1;
+    const int ntiles = nb > 0 ? w[nb].tile0 : 0;
+    // The first tile of a warp is its number, the next ones come from the counter; the first
+    // one's descriptors are read before the barrier.
+    int next = wid * (int)gridDim.x + (int)blockIdx.x;
+    GWarpProb b{};
+    auto find = [&]() {
+      if (next >= ntiles) return;
+      b = w[find_block(w, nb, next)];
+      win.open(b.p.seg0, b.p.seg1);
+    };
+    find();
+    if (p > 0 && !grid_barrier(a, p * (int)gridDim.x, &s_flag)) break;
+    while (next < ntiles) {
+      const int t = next - b.tile0;
+      if (ph.type == GP_GEMM) {
+        const int tm = (b.p.m + QM - 1) / QM;
+        gemm_warp_tile(a, ph, b.p, t % tm * QM, t / tm * QN, win, As[wid], Bs[wid]);
+      } else {
+        const int tm = (b.p.m + QSM - 1) / QSM;
+        sum_warp_tile(a, ph, b.p, t % tm * QSM, t / tm * QSN, win);
+      }
+      if ((threadIdx.x & 31) == 0) next = nw + atomicAdd(a.ctl + p, 1);
+      next = __shfl_sync(~0u, next, 0);
+      find();
+    }
+  }
+  leave(a);
+}
+
+int g_occupancy[3] = {0, 0, 0};
 std::mutex g_occ_mu;
 
 int kernel_occupancy(fmpt_handle* h, int variant) {
-  const int v = variant & 1;
+  const int v = variant == GP_WARP ? 2 : variant & 1;
   std::lock_guard<std::mutex> lock(g_occ_mu);
   if (g_occupancy[v] == 0) {
     int occ = 0;
-    if (v == 0)
+    if (v == 2)
+      FMPT_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, grouped_warp, 32 * QWARPS, 0));
+    else if (v == 0)
       FMPT_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, grouped_kernel<32>, GNT, 0));
     else
       FMPT_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, grouped_kernel<64>, GNT, 0));
-    g_occupancy[v] = std::max(1, std::min(occ, 8));
+    g_occupancy[v] = std::max(1, std::min(occ, v == 2 ? QBLOCKS : 8));
   }
   return g_occupancy[v];
 }
@@ -356,7 +593,8 @@ int gp_finalize(fmpt_handle* h, GroupedProgram& g) {
   FMPT_TRY(validate(h, g));
   g.tile_prob.clear();
   g.tile_mn.clear();
-  int max_tiles[GP_VARIANTS] = {0, 0, 0, 0};
+  int max_tiles[GP_VARIANTS] = {0, 0, 0, 0, 0};
+  std::vector<GWarpProb> wprob;
   for (int v = 0; v < GP_VARIANTS; v++) {
     const int GT = kTile[v & 1], sched = v >> 1;
     g.vtile0[v].assign(g.phases.size(), 0);
@@ -374,6 +612,24 @@ int gp_finalize(fmpt_handle* h, GroupedProgram& g) {
       std::iota(order.begin(), order.end(), p0);
       std::stable_sort(order.begin(), order.end(),
                        [&](int x, int y) { return cost[x - p0] > cost[y - p0]; });
+      if (v == GP_WARP) {
+        const bool gemm = g.phases[ph].type == GP_GEMM;
+        const int tm = gemm ? QM : QSM, tn = gemm ? QN : QSN;
+        g.vtile0[v][ph] = (int)wprob.size();
+        int64_t tiles = 0;
+        for (int i : order) {
+          const GProblem& p = g.probs[i];
+          if (p.m <= 0 || p.n <= 0) continue;
+          wprob.push_back({p, (int)tiles, 0});
+          tiles += (int64_t)((p.m + tm - 1) / tm) * ((p.n + tn - 1) / tn);
+          if (tiles > (int64_t)1 << 30)
+            return set_error(h, FMPT_ERR_SHAPE, "grouped: too many tiles in phase %d", (int)ph);
+        }
+        if ((int)wprob.size() > g.vtile0[v][ph]) wprob.push_back({GProblem{}, (int)tiles, 0});
+        g.vtile1[v][ph] = (int)wprob.size();
+        max_tiles[v] = std::max(max_tiles[v], (int)((tiles + QWARPS - 1) / QWARPS));
+        continue;
+      }
       g.vtile0[v][ph] = (int)g.tile_prob.size();
       const size_t first = g.tile_prob.size();
       std::vector<int64_t> tcost;            // schedule 1: work of each emitted tile
@@ -422,14 +678,17 @@ int gp_finalize(fmpt_handle* h, GroupedProgram& g) {
   const size_t bp = up256(g.probs.size() * sizeof(GProblem));
   const size_t bs = up256(g.segs.size() * sizeof(GSegment));
   const size_t bt = up256(g.tile_prob.size() * sizeof(int));
+  const size_t bw = up256(wprob.size() * sizeof(GWarpProb));
   const size_t ctl_bytes = 256;
-  FMPT_TRY(g.dev.alloc(h, bp + bs + 2 * bt + ctl_bytes));
+  FMPT_TRY(g.dev.alloc(h, bp + bs + 2 * bt + bw + ctl_bytes));
   char* base = static_cast<char*>(g.dev.p);
   g.d_probs = reinterpret_cast<GProblem*>(base);
   g.d_segs = reinterpret_cast<GSegment*>(base + bp);
   g.d_tile_prob = reinterpret_cast<int*>(base + bp + bs);
   g.d_tile_mn = reinterpret_cast<int*>(base + bp + bs + bt);
-  g.d_ctl = reinterpret_cast<int*>(base + bp + bs + 2 * bt);
+  g.d_wprob = reinterpret_cast<GWarpProb*>(base + bp + bs + 2 * bt);
+  g.d_ctl = reinterpret_cast<int*>(base + bp + bs + 2 * bt + bw);
+  FMPT_CUDA(h, cudaMemsetAsync(g.d_ctl, 0, ctl_bytes, h->stream));
   // pageable-source copies return once the source is staged
   if (!g.probs.empty())
     FMPT_CUDA(h, cudaMemcpyAsync(g.d_probs, g.probs.data(), g.probs.size() * sizeof(GProblem),
@@ -444,6 +703,9 @@ int gp_finalize(fmpt_handle* h, GroupedProgram& g) {
     FMPT_CUDA(h, cudaMemcpyAsync(g.d_tile_mn, g.tile_mn.data(), g.tile_mn.size() * sizeof(int),
                                  cudaMemcpyHostToDevice, h->stream));
   }
+  if (!wprob.empty())
+    FMPT_CUDA(h, cudaMemcpyAsync(g.d_wprob, wprob.data(), wprob.size() * sizeof(GWarpProb),
+                                 cudaMemcpyHostToDevice, h->stream));
   const int sms = h->sm_count > 0 ? h->sm_count : 1;
   for (int v = 0; v < GP_VARIANTS; v++) {
     const int occ = kernel_occupancy(h, v);
@@ -459,8 +721,8 @@ int gp_autotune(fmpt_handle* h, GroupedProgram& g, double* const* slots, int nsl
     g.variant = h->tune_mode - 1;
     return FMPT_OK;
   }
-  g.variant = 0;
-  // small programs: the 32x32 tile balances better and timing costs more than it saves
+  g.variant = GP_WARP;
+  // small programs: the warp tiles balance best and timing costs more than it saves
   if (g.flops < 2.0e7 || g.tile_prob.empty()) return FMPT_OK;
   const int key = kind * 1000 + (int)std::floor(std::log2(g.flops) * 2.0);
   auto it = h->tune_cache.find(key);
@@ -479,7 +741,7 @@ int gp_autotune(fmpt_handle* h, GroupedProgram& g, double* const* slots, int nsl
     cudaEventDestroy(e0);
     return set_error(h, FMPT_ERR_CUDA, "autotune: event creation failed");
   }
-  int best = 0, st = FMPT_OK;
+  int best = GP_WARP, st = FMPT_OK;
   float best_ms = 0.f;
   for (int v = 0; v < GP_VARIANTS && st == FMPT_OK; v++) {
     st = gp_run(h, g, slots, nslots, nullptr, v);          // warm-up
@@ -556,16 +818,16 @@ int gp_run(fmpt_handle* h, const GroupedProgram& g, double* const* slots, int ns
   }
   a.probs = g.d_probs; a.segs = g.d_segs;
   a.tile_prob = g.d_tile_prob; a.tile_mn = g.d_tile_mn;
+  a.wprob = g.d_wprob;
   a.ctl = g.d_ctl;
   a.gate = gate;
   a.wait_ns = h->wait_test_ns > 0 ? (uint64_t)h->wait_test_ns : kBarrierTimeoutNs;
   a.hold = h->wait_test_hold;
   FMPT_TRY(gp_status_word(h, &a.status));
-  FMPT_CUDA(h, cudaMemsetAsync(g.d_ctl, 0, (GP_MAX_PHASES + 2) * sizeof(int), h->stream));
   ProfScope prof(h, FMPT_K_GROUPED);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(g.vgrid[v]);
-  cfg.blockDim = dim3(GNT);
+  cfg.blockDim = dim3(v == GP_WARP ? 32 * QWARPS : GNT);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = h->stream;
   cudaLaunchAttribute attr[1];
@@ -573,7 +835,9 @@ int gp_run(fmpt_handle* h, const GroupedProgram& g, double* const* slots, int ns
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if ((v & 1) == 0)
+  if (v == GP_WARP)
+    FMPT_CUDA(h, cudaLaunchKernelEx(&cfg, grouped_warp, a));
+  else if ((v & 1) == 0)
     FMPT_CUDA(h, cudaLaunchKernelEx(&cfg, grouped_kernel<32>, a));
   else
     FMPT_CUDA(h, cudaLaunchKernelEx(&cfg, grouped_kernel<64>, a));

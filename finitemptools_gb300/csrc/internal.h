@@ -265,7 +265,9 @@ int schedule_env(fmpt_handle* h, int cplx, const double* W, int d, int wl, int w
 
 // -------- grouped persistent block-sparse engine (grouped.cu)
 constexpr int GP_MAX_PHASES = 4, GP_SLOTS = 8;
-constexpr int GP_VARIANTS = 4;   // (tile, schedule): v & 1 -> 32x32 / 64x64 tiles, v >> 1 -> schedule
+// variants 0-3: (tile, schedule), v & 1 -> 32x32 / 64x64 tiles of a block, v >> 1 -> schedule;
+// GP_WARP: 8x4 tiles of a warp
+constexpr int GP_VARIANTS = 5, GP_WARP = 4;
 enum { GP_GEMM = 0, GP_SUM = 1 };
 // One output block: C (m x n, column-major with ldc) at c_off in the phase's C slot.
 struct GProblem {
@@ -278,6 +280,11 @@ struct GSegment {
   double coef;
   int k, pad;
 };
+// GP_WARP: a block in its phase's order with the number of tiles before it
+struct GWarpProb {
+  GProblem p;
+  int tile0, pad;
+};
 struct GPhaseDesc {
   int type, ta, tb, a_slot, b_slot, c_slot, tile0, tile1;
 };
@@ -286,10 +293,10 @@ struct GroupedProgram {
   std::vector<int> phase_prob0;
   std::vector<GProblem> probs;
   std::vector<GSegment> segs;
-  std::vector<int> tile_prob, tile_mn;           // the tiles of every variant, one after another
+  std::vector<int> tile_prob, tile_mn;           // the tiles of variants 0-3, one after another
   std::vector<int> vtile0[GP_VARIANTS], vtile1[GP_VARIANTS];   // per variant and phase
-  int vgrid[GP_VARIANTS] = {0, 0, 0, 0};
-  int variant = 0;                                // the one gp_run launches by default
+  int vgrid[GP_VARIANTS] = {0, 0, 0, 0, 0};
+  int variant = GP_WARP;                          // the one gp_run launches by default
   double flops = 0.0;       // 2 m n k over the GEMM segments
   double sum_elems = 0.0;   // output elements x terms of the SUM phases
   int64_t slot_elems[GP_SLOTS] = {-1, -1, -1, -1, -1, -1, -1, -1};  // operand extents
@@ -298,6 +305,7 @@ struct GroupedProgram {
   GSegment* d_segs = nullptr;
   int* d_tile_prob = nullptr;
   int* d_tile_mn = nullptr;
+  GWarpProb* d_wprob = nullptr;                   // GP_WARP: blocks by descending work
   int* d_ctl = nullptr;
   bool ready = false;
 };

@@ -572,7 +572,8 @@ int fmpt_u1_op_ac2(fmpt_handle* h, int dtype, const double* W1, const double* W2
 
 int fmpt_op_tile(fmpt_op* op) {
   if (!op || !op->u1) return 0;
-  return (static_cast<U1OpState*>(op->u1)->prog.variant & 1) == 0 ? 32 : 64;
+  const int v = static_cast<U1OpState*>(op->u1)->prog.variant;
+  return v == GP_WARP ? 8 : (v & 1) == 0 ? 32 : 64;
 }
 
 int fmpt_op_flops(fmpt_op* op, double* flops) {

@@ -76,9 +76,9 @@ class Handle:
         return int(lib().fmpt_graph_launch_count(self.ptr))
 
     def set_tuning(self, mode=0):
-        """Grouped-kernel variant choice: 0 autotune over tiles and block schedules (default),
-        1 / 2 force 32x32 / 64x64 tiles with the blocks-by-work schedule, 3 / 4 the same tiles
-        with the tiles-by-work schedule."""
+        """Grouped-kernel variant choice: 0 autotune over tiles and block schedules (default;
+        small programs run the 8x4 warp tiles untimed), 1 / 2 force 32x32 / 64x64 tiles with
+        the blocks-by-work schedule, 3 / 4 the same tiles with the tiles-by-work schedule."""
         self.check(lib().fmpt_set_tuning(self.ptr, int(mode)))
 
     def tuning_info(self):

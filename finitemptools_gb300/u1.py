@@ -382,7 +382,7 @@ class U1HeffOp:
         self.shape = (self.n,)
 
     def tile(self):
-        """Output tile edge the grouped kernel runs this operator with (autotuned)."""
+        """Output tile edge (8: warp tiles, 32 or 64) the grouped kernel runs this operator with (autotuned)."""
         return int(lib().fmpt_op_tile(self.ptr))
 
     def flops(self):

@@ -113,9 +113,10 @@ int fmpt_set_cluster_qr(fmpt_handle* h, int on);
  * time a block-sparse operator or environment update of a new work size (kind,
  * half-octave of FLOPs) is built, every kernel variant -- 32x32 or 64x64 output
  * tiles, each with two block schedules (blocks by descending work, or tiles by
- * descending work of their own) -- is timed on it and the fastest is cached in
- * the handle; mode 1 / 2 force the 32x32 / 64x64 tile with the first schedule,
- * mode 3 / 4 the same tiles with the second.
+ * descending work of their own), or 8x4 tiles of a warp -- is timed on it and the
+ * fastest is cached in the handle (small programs run the 8x4 tiles untimed);
+ * mode 1 / 2 force the 32x32 / 64x64 tile with the first schedule, mode 3 / 4 the
+ * same tiles with the second.
  * All variants sum every output in the same order: the choice never changes
  * results.  No counterpart in the reference. */
 int fmpt_set_tuning(fmpt_handle* h, int mode);
@@ -143,7 +144,7 @@ int fmpt_set_f64_engine(fmpt_handle* h, int mode);
 int fmpt_set_wait_test(fmpt_handle* h, int64_t timeout_ns, int hold);
 /* Number of cached tuning decisions and of timed tunings so far. */
 int fmpt_tuning_info(fmpt_handle* h, int* entries, int64_t* timed);
-/* Output tile edge (32 or 64) a block-sparse operator runs with (0: dense op). */
+/* Output tile edge (8, 32 or 64; 8: the 8x4 tiles of a warp) a block-sparse operator runs with (0: dense op). */
 int fmpt_op_tile(fmpt_op* op);
 /* Run subsequent work of this handle on an external cudaStream_t (NULL: the
  * handle's own stream). */
@@ -402,8 +403,8 @@ int fmpt_lq(fmpt_handle* h, int dtype, const double* M, int m, int n, double* Lo
  * two-site vector x[a, s1, s2, b] is PACKED: only its allowed blocks
  * (ia, s, ib), s = s1 + d1*s2, each column-major dim(ia) x dim(ib), in the
  * order ia fastest, then s, then ib.  All of these run FP64 (real only) on the
- * grouped persistent engine: one cooperative launch per contraction, CTAs
- * pulling 32x32 tiles of the uneven blocks from a device work counter, a
+ * grouped persistent engine: one cooperative launch per contraction, warps
+ * or CTAs pulling tiles of the uneven blocks from a device work counter, a
  * bounded grid barrier between the three steps (L*x, MPO step, *R). */
 typedef struct fmpt_u1_space {
   int nsect;            /* number of sectors                     */
