@@ -92,6 +92,7 @@ static_assert(NS == 9 && SB == 6, "the digit extraction below is written for 9 d
 __global__ void __launch_bounds__(256, 3) ozd_digits(SliceSrc src, int rows_out, int k_out, int ldk,
                                                  const unsigned long long* __restrict__ mxa,
                                                  uint16_t* __restrict__ S, int* __restrict__ E) {
+  chain_begin();
   __shared__ uint64_t tile[2][SL_ROWS][65];
   const int r0 = blockIdx.x * SL_ROWS, kc0 = blockIdx.y * SL_KCH, z = blockIdx.z;
   const int t = threadIdx.x, rr = t >> 3, part = t & 7;
@@ -213,6 +214,7 @@ __global__ void __launch_bounds__(256) ozd_digits_kfast(const double* __restrict
                                                        const unsigned long long* __restrict__ mxa,
                                                        uint16_t* __restrict__ S,
                                                        int* __restrict__ E) {
+  chain_begin();
   const int r0 = blockIdx.x * SL_ROWS, kc0 = blockIdx.y * SL_KCH, z = blockIdx.z;
   const int t = threadIdx.x, rr = t >> 3, part = t & 7;
   const int r = r0 + rr;
@@ -259,6 +261,7 @@ __global__ void __launch_bounds__(256) ozd_digits_rowfast(const double* __restri
                                                          const unsigned long long* __restrict__ mxa,
                                                          uint16_t* __restrict__ S,
                                                          int* __restrict__ E) {
+  chain_begin();
   extern __shared__ __align__(16) uint64_t dr_smem[];
   auto tile = [&](int st, int lr, int lc) -> uint64_t& {
     return dr_smem[((size_t)st * SL_ROWS + lr) * 65 + lc];
@@ -526,6 +529,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   cluster_sync();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  chain_begin();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -707,6 +711,7 @@ __device__ __forceinline__ double ws_sum(const RedArgs& a, int z, int r, int c) 
 }
 
 __global__ void ozd_reduce(RedArgs a) {
+  chain_begin();
   const int64_t mn = (int64_t)a.m * a.n;
   const int64_t total = mn * a.batch;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
@@ -809,7 +814,7 @@ int gemm_f64_digits(fmpt_handle* h, const GemmArgs& g) {
   cfg.blockDim = dim3(NTHREADS);
   cfg.dynamicSmemBytes = SMEM;
   cfg.stream = h->stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
@@ -871,13 +876,13 @@ int gemm_f64_digits(fmpt_handle* h, const GemmArgs& g) {
                      uint16_t* planes, int* ex) -> int {
       FMPT_TRY(oz_row_maxima(h, x, rows, K2, batch, mx));
       if (oz_kfast(x, K2))
-        ozd_digits_kfast<<<grid, 256, 0, h->stream>>>(x.p, x.sr, x.bstride, rows, K2, ldk, mx,
-                                                      planes, ex);
+        FMPT_CUDA(h, launch_chain(ozd_digits_kfast, grid, 256, 0, h->stream, x.p, x.sr, x.bstride, rows, K2, ldk, mx,
+                                                      planes, ex));
       else if (x.sr == 1 && !x.cplx)
-        ozd_digits_rowfast<<<grid, 256, DR_SMEM, h->stream>>>(x.p, x.sc, x.bstride, rows, K2,
-                                                              ldk, mx, planes, ex);
+        FMPT_CUDA(h, launch_chain(ozd_digits_rowfast, grid, 256, DR_SMEM, h->stream, x.p, x.sc, x.bstride, rows, K2,
+                                                              ldk, mx, planes, ex));
       else
-        ozd_digits<<<grid, 256, 0, h->stream>>>(x, rows, K2, ldk, mx, planes, ex);
+        FMPT_CUDA(h, launch_chain(ozd_digits, grid, 256, 0, h->stream, x, rows, K2, ldk, mx, planes, ex));
       FMPT_LAUNCHED(h);
       return FMPT_OK;
     };
@@ -922,6 +927,8 @@ int gemm_f64_digits(fmpt_handle* h, const GemmArgs& g) {
   cfg.gridDim = dim3((unsigned)(2 * std::min<int64_t>(items, clusters)));
   {
     ProfScope prof(h, FMPT_K_TC_GEMM);
+    chain_attr(attr[1]);
+    cfg.numAttrs = 2;
     FMPT_CUDA(h, cudaLaunchKernelEx(&cfg, ozd_gemm_pair, ma, mb, K2, tiles_m2, tiles_n, batch, ep));
     FMPT_LAUNCHED(h);
   }
@@ -947,7 +954,7 @@ int gemm_f64_digits(fmpt_handle* h, const GemmArgs& g) {
     ra.beta[1] = g.beta[1];
     const int64_t total = (int64_t)g.m * g.n * batch;
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, 8LL * h->sm_count));
-    ozd_reduce<<<blocks, 256, 0, h->stream>>>(ra);
+    FMPT_CUDA(h, launch_chain(ozd_reduce, blocks, 256, 0, h->stream, ra));
     FMPT_LAUNCHED(h);
   }
   return FMPT_OK;
