@@ -80,6 +80,10 @@ struct Crt {
   uint32_t w[NMOD][3];        // round(2^96 frac(y_i / p_i)), low word first
   uint64_t phat;              // top 64 bits of P, P = phat 2^pexp
   int pexp;
+  // k-th 16-bit limb of weight i, 0 beyond the moduli
+  __host__ __device__ constexpr uint32_t limb(int i, int k) const {
+    return i < NMOD ? (w[i < NMOD ? i : 0][k >> 1] >> (16 * (k & 1))) & 0xffffu : 0u;
+  }
 };
 
 template <int NMOD>
@@ -324,6 +328,11 @@ __host__ __device__ inline void oz_tile(int u, int tiles_m2, int tiles_n, int& m
   const int idx = r - g * GH * tiles_n;
   mt2 = g * GH + idx % rows;
   nt = idx / rows;
+}
+// the place u of tile (mt2, nt, z) in that order
+__device__ __forceinline__ int oz_tile_index(int mt2, int nt, int z, int tiles_m2, int tiles_n) {
+  const int g = mt2 / GH, rows = min(GH, tiles_m2 - g * GH);
+  return (z * tiles_m2 + g * GH) * tiles_n + nt * rows + (mt2 - g * GH);
 }
 
 // chunk ch of nch equal chunks of the nk K slices (nch = ceil(nk / KCHUNK), so every chunk
@@ -572,95 +581,121 @@ struct CrtArgs {
   int m, cplx;
 };
 
-// x 2^E of a 53-bit integer outside the range of normal results
-__device__ __noinline__ double scaled_slow(uint64_t mant, int E, uint32_t sgn) {
-  const double v = ldexp((double)mant, E);
+// The sums of the residues times the six 16-bit limbs of the weights, two moduli per instruction
+// (dp2a): 48 instructions per value where 32-bit words take 16 multiply-adds and 32 wide ones
+// at half their rate.  The integer pipes bound this kernel (151 instructions per value, 194
+// before; D = 1024, 15 moduli: 158 -> 119 us, 74 at the copy bandwidth).  Four columns at a time, so that a weight is put into a register
+// once for four values.  c[j][q]: residues of moduli 4 q .. 4 q + 3 in column j.
+template <int NMOD>
+__device__ __forceinline__ void crt_limbs(const uint32_t (&c)[4][4], uint32_t (&L)[4][6]) {
+  constexpr Crt<NMOD> T = make_crt<NMOD>();
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+#pragma unroll
+    for (int k = 0; k < 6; k++) L[j][k] = 0u;     // below 16 * 255 * 2^16 in the end
+#pragma unroll
+  for (int i = 0; i < MAXMOD; i += 2)
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+      const uint32_t w = T.limb(i, k) | (T.limb(i + 1, k) << 16);
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        L[j][k] = (i & 2) ? __dp2a_hi(w, c[j][i / 4], L[j][k]) : __dp2a_lo(w, c[j][i / 4], L[j][k]);
+    }
+}
+
+// The cases that crt_value leaves out: X = 0 or below 2^-33 P, results outside the range of
+// normal numbers, rows or columns that hold Inf / NaN (exponents from E_BAD on).  |S| in words.
+__device__ __noinline__ double crt_rare(uint32_t s0, uint32_t s1, uint32_t s2, uint32_t sgn, int E,
+                                        uint64_t phat, int pexp) {
+  if (E >= E_BAD / 2) return __longlong_as_double(0x7ff8000000000000ll);
+  int n = 0;
+  for (int k = 0; k < 2 && s2 == 0u; k++) { s2 = s1; s1 = s0; s0 = 0u; n += 32; }
+  if (s2 == 0u) return 0.0;
+  const int lz = __clz(s2);
+  const uint64_t hi =
+      ((uint64_t)__funnelshift_l(s1, s2, lz) << 32) | __funnelshift_l(s0, s1, lz);
+  const uint64_t m = __umul64hi(hi, phat);
+  const int top = (int)(m >> 63);
+  const double v = ldexp((double)(((m >> (9 + top)) + 1) >> 1), E + pexp - n - lz + top + 10);
   return sgn ? -v : v;
 }
 
-// The FP64 value of the residues c[i] (i-th byte of a column over the moduli), scaled by
-// 2^E: S = sum c_i w_i mod 2^96 is X / P as a signed 96-bit fraction (error below 2^-85, and
-// exactly 0 for X = 0), and X 2^E is rounded once, to 53 bits.
+// The FP64 value of the limb sums L, scaled by 2^E.  S = sum c_i w_i mod 2^96 is X / P as a
+// signed 96-bit fraction (error below 2^-85, and exactly 0 for X = 0), and X 2^E is rounded
+// once, to 53 bits.  One branch: what is rare is left to crt_rare.
 template <int NMOD>
-__device__ __forceinline__ double crt_value(const uint32_t (&c)[NMOD], int E) {
+__device__ __forceinline__ double crt_value(const uint32_t (&L)[6], int E) {
   constexpr Crt<NMOD> T = make_crt<NMOD>();
-  uint64_t a0 = 0, a1 = 0;
-  uint32_t s2 = 0;
-#pragma unroll
-  for (int i = 0; i < NMOD; i++) {
-    a0 += (uint64_t)c[i] * T.w[i][0];
-    a1 += (uint64_t)c[i] * T.w[i][1];
-    s2 += c[i] * T.w[i][2];
-  }
-  a1 += a0 >> 32;
-  s2 += (uint32_t)(a1 >> 32);
-  uint32_t s0 = (uint32_t)a0, s1 = (uint32_t)a1;
-  const uint32_t sgn = s2 & 0x80000000u;
-  if (sgn) {
-    // two's complement
-    s0 = ~s0 + 1u;
-    s1 = ~s1 + (s0 == 0u);
-    s2 = ~s2 + (s0 == 0u && s1 == 0u);
-  }
-  // the top 64 bits, normalised: S = hi 2^(32 - n) (n leading zeros)
-  int n = 0;
-  if (s2 == 0u) {
-    s2 = s1; s1 = s0; s0 = 0u; n = 32;
-    if (s2 == 0u) { s2 = s1; s1 = 0u; n = 64; }
-  }
+  const uint64_t a = ((uint64_t)L[1] << 16) + L[0], b = ((uint64_t)L[3] << 16) + L[2];
+  const uint64_t a1 = (a >> 32) + (uint32_t)b;
+  uint32_t s0 = (uint32_t)a, s1 = (uint32_t)a1;
+  uint32_t s2 = (L[5] << 16) + L[4] + (uint32_t)(b >> 32) + (uint32_t)(a1 >> 32);
+  const uint32_t sgn = s2 & 0x80000000u, neg = (uint32_t)((int32_t)s2 >> 31);
+  // |S|: the complement plus one if negative
+  asm("{\n\t"
+      "xor.b32 %0, %0, %3;\n\txor.b32 %1, %1, %3;\n\txor.b32 %2, %2, %3;\n\t"
+      "sub.cc.u32 %0, %0, %3;\n\tsubc.cc.u32 %1, %1, %3;\n\tsubc.u32 %2, %2, %3;\n\t}"
+      : "+r"(s0), "+r"(s1), "+r"(s2)
+      : "r"(neg));
+  // the top 64 bits, normalised: |S| = hi 2^(32 - lz)
   const int lz = __clz(s2);
-  n += lz;
-  const uint32_t h1 = __funnelshift_l(s1, s2, lz), h0 = __funnelshift_l(s0, s1, lz);
-  const uint64_t hi = ((uint64_t)h1 << 32) | h0;
-  if (hi == 0) return 0.0;
-  // X = hi 2^(32 - n) 2^-96 phat 2^pexp = m 2^(64 - 64 - n + pexp), m = high half of hi phat
-  uint64_t m = __umul64hi(hi, T.phat);
-  int ex = E + T.pexp - n;
-  if (!(m >> 63)) { m <<= 1; ex -= 1; }
-  const uint64_t r = m + 1024u;
-  if (r < m) { m = 1ull << 63; ex += 1; } else { m = r; }
-  const uint64_t mant = m >> 11;                  // 53 bits; the value is mant 2^(ex + 11)
-  const int be = ex + 11 + 52 + 1023;             // biased exponent
-  if (be < 1 || be > 2046) return scaled_slow(mant, ex + 11, sgn);
-  const uint64_t bits = ((uint64_t)(be - 1) << 52) + mant;
-  return __hiloint2double((int)((uint32_t)(bits >> 32) | sgn), (int)(uint32_t)bits);
+  const uint64_t hi =
+      ((uint64_t)__funnelshift_l(s1, s2, lz) << 32) | __funnelshift_l(s0, s1, lz);
+  // |X| = hi 2^(32 - lz) 2^-96 phat 2^pexp = m 2^(pexp - lz), m = high half of hi phat, whose
+  // top bit is bit 63 or 62
+  const uint64_t m = __umul64hi(hi, T.phat);
+  const int top = (int)(m >> 63);
+  // 53 bits and the rounding carry, which may run on into the exponent
+  const uint64_t mant = ((m >> (9 + top)) + 1) >> 1;
+  const int be1 = E + (T.pexp + 10 + 52 + 1022) - lz + top;      // biased exponent less 1
+  if (s2 == 0u || (uint32_t)be1 > 2045u) return crt_rare(s0, s1, s2, sgn, E, T.phat, T.pexp);
+  return __hiloint2double((int)(((uint32_t)(mant >> 32) + ((uint32_t)be1 << 20)) | sgn),
+                          (int)(uint32_t)mant);
 }
 
 // Thread = one tile row of a 4-column group: one 4-byte load per modulus (a warp reads 128
-// contiguous bytes), 4 outputs (a warp writes 256 contiguous bytes per column).  Four
-// columns rather than sixteen keep the loaded residues in 16 registers, so that enough
-// warps are resident to hide the loads behind the integer work of the others; GENERAL
-// applies alpha / beta in FP64.
+// contiguous bytes), 4 outputs (a warp writes 256 contiguous bytes per column).  Four columns
+// rather than sixteen keep the loaded residues in 16 registers, so that enough warps are
+// resident to hide the loads behind the integer work of the others; the grid's axes are the
+// tile's coordinates, so that a thread needs no division.  GENERAL applies alpha / beta in FP64.
 template <int NMOD, bool GENERAL>
-__global__ void __launch_bounds__(256) oz_crt(CrtArgs a) {
+__global__ void __launch_bounds__(256, 5) oz_crt(CrtArgs a) {
   chain_begin();
-  const int u = blockIdx.x >> 6, cg = blockIdx.x & 63;
-  int mt2, nt, z;
-  oz_tile(u, a.tiles_m2, a.tiles_n, mt2, nt, z);
-  const int row = mt2 * TILE + threadIdx.x, col0 = nt * TILE + cg * 4;
-  if (row >= a.M || col0 >= a.N) return;
-  const uint8_t* base = a.res + ((int64_t)blockIdx.x * TILE + threadIdx.x) * 4;
-  uint32_t v[NMOD];
+  const int mt2 = blockIdx.y, z = blockIdx.z;
+  const int row = mt2 * TILE + threadIdx.x, col0 = blockIdx.x * 4;
+  if (row >= a.M) return;
+  // 4-column groups of all tiles in the tile order, 1 KB per modulus each
+  const int64_t grp = (int64_t)oz_tile_index(mt2, blockIdx.x >> 6, z, a.tiles_m2, a.tiles_n) * 64 +
+                      (blockIdx.x & 63);
+  const uint8_t* base = a.res + (grp * TILE + threadIdx.x) * 4;
+  const int64_t mstep = (int64_t)a.units * (TILE * TILE);
+  uint32_t v[MAXMOD];
 #pragma unroll
-  for (int i = 0; i < NMOD; i++)
-    v[i] = __ldcs(reinterpret_cast<const uint32_t*>(base + (int64_t)i * a.units * (TILE * TILE)));
-  const int er = __ldg(a.ea + (int64_t)z * a.M + row);
+  for (int i = 0; i < MAXMOD; i++)
+    v[i] = i < NMOD ? __ldcs(reinterpret_cast<const uint32_t*>(base + i * mstep)) : 0u;
+  const int e0 = __ldg(a.ea + (int64_t)z * a.M + row) - 2 * a.tbits;
   const int* eb = a.eb + (int64_t)z * a.N + col0;
   const bool im = row >= a.mh;
   double* p = a.C + (int64_t)z * a.strideC + (im ? a.planeC + row - a.mh : (int64_t)row) +
               (int64_t)col0 * a.ldc;
+  // bytes by column: c[j][q] holds the residues of moduli 4 q .. 4 q + 3 in column j
+  uint32_t c[4][4], L[4][6];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const uint32_t* x = v + 4 * q;
+    const uint32_t a0 = __byte_perm(x[0], x[1], 0x5140), a1 = __byte_perm(x[0], x[1], 0x7362);
+    const uint32_t b0 = __byte_perm(x[2], x[3], 0x5140), b1 = __byte_perm(x[2], x[3], 0x7362);
+    c[0][q] = __byte_perm(a0, b0, 0x5410);
+    c[1][q] = __byte_perm(a0, b0, 0x7632);
+    c[2][q] = __byte_perm(a1, b1, 0x5410);
+    c[3][q] = __byte_perm(a1, b1, 0x7632);
+  }
+  crt_limbs<NMOD>(c, L);
 #pragma unroll
   for (int j = 0; j < 4; j++, p += a.ldc) {
     if (col0 + j >= a.N) break;
-    uint32_t c[NMOD];
-#pragma unroll
-    for (int i = 0; i < NMOD; i++) c[i] = (v[i] >> (8 * j)) & 0xffu;
-    const int ec = __ldg(eb + j);
-    double x;
-    if (er >= E_BAD || ec >= E_BAD)
-      x = __longlong_as_double(0x7ff8000000000000ll);
-    else
-      x = crt_value<NMOD>(c, er + ec - 2 * a.tbits);
+    double x = crt_value<NMOD>(L[j], e0 + __ldg(eb + j));
     if (GENERAL) {
       x *= a.alpha[0];
       if (a.beta[0] != 0.0) x += a.beta[0] * *p;
@@ -929,7 +964,7 @@ int gemm_f64_ozaki(fmpt_handle* h, const GemmArgs& g) {
   }
   const bool general = ca.alpha[0] != 1.0 || ca.beta[0] != 0.0;
   ProfScope prof(h, FMPT_K_CONVERT);
-  const unsigned blocks = (unsigned)(units * 64);
+  const dim3 blocks((unsigned)((N + 3) / 4), (unsigned)tiles_m2, (unsigned)batch);
   if (nmod == 15) {
     if (general) FMPT_CUDA(h, launch_chain(oz_crt<15, true>, blocks, 256, 0, h->stream, ca));
     else FMPT_CUDA(h, launch_chain(oz_crt<15, false>, blocks, 256, 0, h->stream, ca));
