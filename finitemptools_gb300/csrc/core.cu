@@ -350,6 +350,7 @@ int fmpt_destroy(fmpt_handle* h) {
   if (h->gemm_cnt) cudaFree(h->gemm_cnt);
   if (h->tc_ws) cudaFree(h->tc_ws);
   if (h->oz_ws) cudaFree(h->oz_ws);
+  if (h->oz_mx) cudaFree(h->oz_mx);
   if (h->gstatus) cudaFree(h->gstatus);
   for (cudaEvent_t e : h->step_event)
     if (e) cudaEventDestroy(e);

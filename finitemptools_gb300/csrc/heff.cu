@@ -88,6 +88,37 @@ struct MidSparse {
 };
 constexpr int MS_SMALL_OUT = 32, MS_SMALL_T = 96;
 
+// bits of |x|.  Not through __double_as_longlong: the compiler turns its masked form into an
+// FP64 instruction, 64 cycles of the pipe that bounds these kernels.
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+  uint32_t lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(x));
+  return ((unsigned long long)(hi & 0x7fffffffu) << 32) | lo;
+}
+
+// one output of the sparse form at the input position ib
+template <bool CPLX, int OUT, int TERMS>
+__device__ __forceinline__ void mid_sparse_sum(const MidSparse<OUT, TERMS>& ms, int o,
+                                               const double* ib, int64_t plane_in,
+                                               const MidStrides& si, double& ar, double& ai) {
+  ar = ai = 0.0;
+  for (int e = ms.start[o]; e < ms.start[o + 1]; e++) {
+    const int ix = ms.idx[e];
+    const int64_t off = (ix >> 4) * si.w + (ix & 15) * si.s;
+    const double vr = ib[off];
+    if (CPLX) {
+      const double vi = ib[plane_in + off];
+      const double cr = ms.c[2 * e], ci = ms.c[2 * e + 1];
+      ar = fma(cr, vr, ar);
+      ar = fma(-ci, vi, ar);
+      ai = fma(cr, vi, ai);
+      ai = fma(ci, vr, ai);
+    } else {
+      ar = fma(ms.c[e], vr, ar);
+    }
+  }
+}
+
 // Thread = one (o1, o2), outputs blockIdx.y, blockIdx.y + gridDim.y, ..  A large problem
 // runs gridDim.y = 1 (one pass over the input, L1 serves the repeated reads; 4.6 TB/s at
 // D = 2048).  A small one gives every output its own threads: with all 20 outputs in one
@@ -105,24 +136,62 @@ __global__ void __launch_bounds__(128)
   double* ob = out + o1 * so.o1 + o2 * so.o2;
   for (int o = blockIdx.y; o < ms.n_out; o += gridDim.y) {
     const int wo = o / p_out, q = o - wo * p_out;
-    double ar = 0.0, ai = 0.0;
-    for (int e = ms.start[o]; e < ms.start[o + 1]; e++) {
-      const int ix = ms.idx[e];
-      const int64_t off = (ix >> 4) * si.w + (ix & 15) * si.s;
-      const double vr = ib[off];
-      if (CPLX) {
-        const double vi = ib[plane_in + off];
-        const double cr = ms.c[2 * e], ci = ms.c[2 * e + 1];
-        ar = fma(cr, vr, ar);
-        ar = fma(-ci, vi, ar);
-        ai = fma(cr, vi, ai);
-        ai = fma(ci, vr, ai);
-      } else {
-        ar = fma(ms.c[e], vr, ar);
-      }
-    }
+    double ar, ai;
+    mid_sparse_sum<CPLX>(ms, o, ib, plane_in, si, ar, ai);
     ob[wo * so.w + q * so.s] = ar;
     if (CPLX) ob[plane_out + wo * so.w + q * so.s] = ai;
+  }
+}
+
+// The same with the row maxima that the next GEMM's conversion needs (rows o1 + n1 so over wo and
+// o2; mx zeroed beforehand, dup: where a complex product's row appears again) instead of a pass
+// over the output of its own.  Block = 32 o1 x 8 o2, QN values of so per thread from
+// QN * blockIdx.z on: the maxima of the eight o2 meet in shared memory, and only one above the
+// current maximum goes to the atomic.  D = 2048: 283 us, where the step alone took 289 and the
+// pass 168; D = 256: 9.3 instead of 11.1 + 8.2.
+template <bool CPLX, int OUT, int TERMS, int QN>
+__global__ void __launch_bounds__(256)
+    mid_sparse_max(const double* __restrict__ in, int64_t plane_in, MidStrides si,
+                   double* __restrict__ out, int64_t plane_out, MidStrides so, int n1, int n2,
+                   int p_out, unsigned long long* __restrict__ mx, int64_t dup,
+                   const __grid_constant__ MidSparse<OUT, TERMS> ms) {
+  chain_begin();
+  __shared__ unsigned long long tops[QN][8][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int o1 = blockIdx.x * 32 + lane;
+  const int64_t o2 = (int64_t)blockIdx.y * 8 + wid;
+  const int q0 = blockIdx.z * QN, nw = ms.n_out / p_out;
+  const bool live = o1 < n1 && o2 < n2;
+  const double* ib = in + (live ? o1 * si.o1 + o2 * si.o2 : 0);
+  double* ob = out + (live ? o1 * so.o1 + o2 * so.o2 : 0);
+  unsigned long long top[QN] = {};
+  if (live) {
+    for (int wo = 0; wo < nw; wo++)
+#pragma unroll
+      for (int i = 0; i < QN; i++) {
+        if (q0 + i >= p_out) break;
+        double ar, ai;
+        mid_sparse_sum<CPLX>(ms, wo * p_out + q0 + i, ib, plane_in, si, ar, ai);
+        ob[wo * so.w + (q0 + i) * so.s] = ar;
+        top[i] = max(top[i], abs_bits(ar));
+        if (CPLX) {
+          ob[plane_out + wo * so.w + (q0 + i) * so.s] = ai;
+          top[i] = max(top[i], abs_bits(ai));
+        }
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < QN; i++) tops[i][wid][lane] = top[i];
+  __syncthreads();
+  if (wid < QN && o1 < n1 && q0 + wid < p_out) {
+    unsigned long long v = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) v = max(v, tops[wid][k][lane]);
+    unsigned long long* m = mx + (int64_t)(q0 + wid) * n1 + o1;
+    if (v > __ldcg(m)) {
+      atomicMax(m, v);
+      if (CPLX) atomicMax(m + dup, v);
+    }
   }
 }
 
@@ -288,7 +357,7 @@ void mid_free(fmpt_handle* h, MidSchedule& s) {
 template <bool CPLX, int OUT, int TERMS>
 static int mid_sparse_launch(fmpt_handle* h, const MidSchedule& s, const double* in,
                              int64_t plane_in, MidStrides si, double* out, int64_t plane_out,
-                             MidStrides so, int n1, int n2) {
+                             MidStrides so, int n1, int n2, unsigned long long* mx) {
   MidSparse<OUT, TERMS> ms;
   ms.n_out = (int)s.sp_start.size() - 1;
   for (size_t i = 0; i < s.sp_start.size(); i++) ms.start[i] = (short)s.sp_start[i];
@@ -298,6 +367,22 @@ static int mid_sparse_launch(fmpt_handle* h, const MidSchedule& s, const double*
   // below a few blocks per SM the outputs are spread over threads of their own (see the
   // kernel); above, the input is read once
   const int gy = blocks < 8LL * std::max(1, h->sm_count) ? ms.n_out : 1;
+  if (mx) {
+    // four values of so per thread read the input once (L1 serves the repeats); small problems
+    // take one, for four times the threads
+    const dim3 g((unsigned)((n1 + 31) / 32), (unsigned)((n2 + 7) / 8));
+    const int64_t dup = (int64_t)n1 * s.p_out;
+    if (blocks < 16LL * std::max(1, h->sm_count))
+      FMPT_CUDA(h, launch_chain(mid_sparse_max<CPLX, OUT, TERMS, 1>,
+                                dim3(g.x, g.y, (unsigned)s.p_out), 256, 0, h->stream, in, plane_in,
+                                si, out, plane_out, so, n1, n2, s.p_out, mx, dup, ms));
+    else
+      FMPT_CUDA(h, launch_chain(mid_sparse_max<CPLX, OUT, TERMS, 4>,
+                                dim3(g.x, g.y, (unsigned)((s.p_out + 3) / 4)), 256, 0, h->stream,
+                                in, plane_in, si, out, plane_out, so, n1, n2, s.p_out, mx, dup, ms));
+    FMPT_LAUNCHED(h);
+    return FMPT_OK;
+  }
   FMPT_CUDA(h, launch_chain(mid_sparse_kernel<CPLX, OUT, TERMS>, dim3((unsigned)blocks, gy), 128, 0,
                             h->stream, in, plane_in, si, out, plane_out, so, n1, n2, s.p_out, ms));
   FMPT_LAUNCHED(h);
@@ -305,7 +390,8 @@ static int mid_sparse_launch(fmpt_handle* h, const MidSchedule& s, const double*
 }
 
 int mid_apply(fmpt_handle* h, const MidSchedule& s, const double* in, int64_t plane_in,
-              MidStrides si, double* out, int64_t plane_out, MidStrides so, int n1, int n2) {
+              MidStrides si, double* out, int64_t plane_out, MidStrides so, int n1, int n2,
+              unsigned long long* mx) {
   int64_t nt = (int64_t)n1 * n2;
   if (nt == 0) return FMPT_OK;
   const int threads = 256;
@@ -319,9 +405,9 @@ int mid_apply(fmpt_handle* h, const MidSchedule& s, const double* in, int64_t pl
     const bool small = n_out <= MS_SMALL_OUT && (int)s.sp_coef.size() <= MS_SMALL_T;
 #define MIDS(CP)                                                                              \
   (small ? mid_sparse_launch<CP, MS_SMALL_OUT, MS_SMALL_T>(h, s, in, plane_in, si, out,       \
-                                                           plane_out, so, n1, n2)             \
+                                                           plane_out, so, n1, n2, mx)         \
          : mid_sparse_launch<CP, MS_MAX_OUT, MS_MAX_T>(h, s, in, plane_in, si, out, plane_out, \
-                                                       so, n1, n2))
+                                                       so, n1, n2, mx))
     return s.cplx ? MIDS(true) : MIDS(false);
 #undef MIDS
   }
@@ -390,6 +476,32 @@ int op_apply_fp64(fmpt_op* op, const double* x, double* y) {
   return op_fp64_tail(op, y);
 }
 
+static int64_t t1_elems(const fmpt_op* op) {
+  return (int64_t)op->Dl * op->wl * (op->kind == 0 ? op->d1 * op->d2 : op->d1) * op->Dr;
+}
+static int64_t t3_elems(const fmpt_op* op) {
+  return (int64_t)op->Dl * op->wr * (op->kind == 0 ? op->d1 * op->d2 : op->d1) * op->Dr;
+}
+// the row maxima of T3 lie behind it
+static unsigned long long* tail_maxima(const fmpt_op* op) {
+  return reinterpret_cast<unsigned long long*>(op->scratch + (t1_elems(op) + t3_elems(op)) *
+                                                                 (op->dtype == FMPT_C128 ? 2 : 1));
+}
+
+// GEMM 2: y[(a' s'), b'] = T3[(a' s'), (w2 b)] R[b', (w2 b)]^T
+static GemmArgs tail_gemm(fmpt_op* op, double* y) {
+  const int cp = op->dtype == FMPT_C128;
+  const int Dl = op->Dl, Dr = op->Dr, wr = op->wr;
+  const int P = op->kind == 0 ? op->d1 * op->d2 : op->d1;
+  const double* T3 = op->scratch ? op->scratch + t1_elems(op) * (cp ? 2 : 1) : nullptr;
+  GemmArgs g = gemm_args(cp, FMPT_N, FMPT_T, Dl * P, Dr, wr * Dr, T3, (int64_t)Dl * P,
+                         t3_elems(op), op->hright, Dr, (int64_t)Dr * wr * Dr, y, (int64_t)Dl * P,
+                         (int64_t)Dl * P * Dr);
+  g.engine = op->precision == FMPT_PREC_FP64_TC ? 1 : 0;
+  if (g.engine) g.cacheB = right_cache(op);
+  return g;
+}
+
 // One- and two-site FP64 application in two halves, so that a caller can overlap the
 // upload of the right environment with the first half: head = GEMM 1 and the MPO step
 // (reads x and the left environment, writes T1 and T3 in the operator's scratch), tail =
@@ -405,10 +517,30 @@ int op_fp64_head(fmpt_op* op, const double* x) {
   const int64_t nx = (int64_t)Dl * P * Dr;
   const int64_t n1 = (int64_t)Dl * wl * P * Dr, n3 = (int64_t)Dl * P * wr * Dr;
   // T1 and T3 in the operator's scratch (one buffer, T3 after T1)
+  // and, where GEMM 2 takes them, the row maxima of T3
+  const bool maxima = !op->sched.sp_start.empty() &&
+                      gemm_f64_ozaki_takes_maxima(h, tail_gemm(op, nullptr));
+  const size_t mxb = maxima ? (size_t)Dl * P * (cp ? 2 : 1) * sizeof(uint64_t) : 0;
+  const size_t held = op->scratch_bytes;
   FMPT_TRY(grow_buffer(h, reinterpret_cast<void**>(&op->scratch), &op->scratch_bytes,
-                       (size_t)(n1 + n3) * es));
+                       (size_t)(n1 + n3) * es + mxb));
+  if (op->scratch_bytes != held) op->mx_clean = false;
   double* T1 = op->scratch;
   double* T3 = op->scratch + n1 * (cp ? 2 : 1);
+  unsigned long long* mx = nullptr;
+  op->mx_ready = false;
+  if (maxima) {
+    mx = tail_maxima(op);
+    op->mx_keep = true;
+    if (!op->mx_clean) {
+      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+      op->mx_keep =
+          cudaStreamIsCapturing(h->stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+      FMPT_CUDA(h, cudaMemsetAsync(mx, 0, mxb, h->stream));
+    }
+    op->mx_clean = false;
+    op->mx_ready = true;
+  }
   // 1. T1[(a' w), (s b)] = L[(a' w), a] x[a, (s b)]
   GemmArgs g1 = gemm_args(cp, FMPT_N, FMPT_N, Dl * wl, P * Dr, Dl, op->hleft, (int64_t)Dl * wl,
                           (int64_t)Dl * wl * Dl, x, Dl, nx, T1, (int64_t)Dl * wl, n1);
@@ -418,25 +550,17 @@ int op_fp64_head(fmpt_op* op, const double* x) {
   // 2. T3[a', s', w2, b] = sum_blocks O[s', s] T1[a', w, s, b]
   MidStrides si{1, (int64_t)Dl * wl * P, Dl, (int64_t)Dl * wl};
   MidStrides so{1, (int64_t)Dl * P * wr, (int64_t)Dl * P, Dl};
-  return mid_apply(h, op->sched, T1, n1, si, T3, n3, so, Dl, Dr);
+  return mid_apply(h, op->sched, T1, n1, si, T3, n3, so, Dl, Dr, mx);
 }
 
 int op_fp64_tail(fmpt_op* op, double* y) {
-  fmpt_handle* h = op->h;
-  const int eng = op->precision == FMPT_PREC_FP64_TC ? 1 : 0;
-  const int cp = op->dtype == FMPT_C128;
-  const int Dl = op->Dl, Dr = op->Dr;
-  const int P = op->kind == 0 ? op->d1 * op->d2 : op->d1;
-  const int wl = op->wl, wr = op->wr;
-  const int64_t nx = (int64_t)Dl * P * Dr;
-  const int64_t n1 = (int64_t)Dl * wl * P * Dr, n3 = (int64_t)Dl * P * wr * Dr;
-  const double* T3 = op->scratch + n1 * (cp ? 2 : 1);
-  // 3. y[(a' s'), b'] = T3[(a' s'), (w2 b)] R[b', (w2 b)]^T
-  GemmArgs g2 = gemm_args(cp, FMPT_N, FMPT_T, Dl * P, Dr, wr * Dr, T3, (int64_t)Dl * P, n3,
-                          op->hright, Dr, (int64_t)Dr * wr * Dr, y, (int64_t)Dl * P, nx);
-  g2.engine = eng;
-  if (eng) g2.cacheB = right_cache(op);
-  return gemm_f64(h, g2);
+  GemmArgs g2 = tail_gemm(op, y);
+  if (op->mx_ready) {
+    g2.maxA = tail_maxima(op);
+    if (op->mx_keep) g2.maxA_clean = &op->mx_clean;
+    op->mx_ready = false;
+  }
+  return gemm_f64(op->h, g2);
 }
 
 }  // namespace fmpt

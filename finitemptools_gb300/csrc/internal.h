@@ -73,6 +73,11 @@ struct fmpt_handle {
   int wait_test_hold = 0;
   void* oz_ws = nullptr;
   size_t oz_ws_bytes = 0;
+  // row maxima of the residue GEMM's operands: zero between calls (its last kernel zeroes what
+  // the call used) unless a call failed half-way (oz_mx_dirty)
+  void* oz_mx = nullptr;
+  size_t oz_mx_bytes = 0;
+  bool oz_mx_dirty = true;
   // executable graphs of the captured Arnoldi basis, one per operator structure
   std::map<std::string, cudaGraphExec_t> arnoldi_exec;
   cudaGraphExec_t lanczos_exec = nullptr;   // reused through cudaGraphExecUpdate
@@ -212,11 +217,16 @@ struct GemmArgs {
   int engine;               // 0: the handle's FP64 engine, 1: tensor cores where faster
   OzCache* cacheA;          // optional residue-plane caches of A / B (tensor-core engine)
   OzCache* cacheB;
+  // optional row maxima of op(A) (bit patterns of |.|, one per row of the real embedding), formed
+  // by the kernel that wrote A; the residue GEMM zeroes them after use and then sets *maxA_clean
+  unsigned long long* maxA;
+  bool* maxA_clean;
 };
 int gemm_f64(fmpt_handle* h, const GemmArgs& g);
 // the Ozaki-scheme FP64 GEMM on the BF16 tensor cores (ozaki.cu): whether it applies to g
 // (engine requested, shape large enough to win), and the call itself
 int gemm_f64_ozaki_possible(fmpt_handle* h, const GemmArgs& g);
+bool gemm_f64_ozaki_takes_maxima(fmpt_handle* h, const GemmArgs& g);   // would use g.maxA
 int gemm_f64_ozaki(fmpt_handle* h, const GemmArgs& g);
 // the same by digit products (ozaki_digits.cu), inside the Lanczos solve
 int gemm_f64_digits_possible(fmpt_handle* h, const GemmArgs& g);
@@ -249,8 +259,11 @@ struct MidSchedule {
 int mid_upload(fmpt_handle* h, MidSchedule& s);
 void mid_free(fmpt_handle* h, MidSchedule& s);
 struct MidStrides { int64_t o1, o2, w, s; };
+// mx: optionally the maxima over (wo, o2) of |out| per row o1 + n1 so of the real embedding (a
+// complex product's rows appear twice); only with a by-value table (sp_start not empty)
 int mid_apply(fmpt_handle* h, const MidSchedule& s, const double* in, int64_t plane_in,
-              MidStrides si, double* out, int64_t plane_out, MidStrides so, int n1, int n2);
+              MidStrides si, double* out, int64_t plane_out, MidStrides so, int n1, int n2,
+              unsigned long long* mx = nullptr);
 
 // Schedules from dense host MPO tensors (W[wl, s_out, wr, s_in]).
 int schedule_ac2(fmpt_handle* h, int cplx, const double* W1, const double* W2, int d1, int d2,
@@ -363,6 +376,9 @@ struct fmpt_op {
   fmpt::OzCache oz_left, oz_right;
   fmpt::OzCache ozd_left, ozd_right;   // digit planes (the Lanczos solve's engine)
   size_t scratch_bytes = 0;
+  // row maxima of T3 behind it in the scratch: formed by the last head; zero (which they are
+  // again after a tail unless the zeros were only recorded, mx_keep)
+  bool mx_ready = false, mx_clean = false, mx_keep = false;
   // projectors of the excited-state sweeps: after every application
   // y -= dot(y, p) p for each p in order (device vectors of n elements, not owned)
   std::vector<const double*> proj;

@@ -579,6 +579,9 @@ struct CrtArgs {
   int tbits;
   double alpha[2], beta[2];
   int m, cplx;
+  int mt0;              // first row of tiles of this launch
+  unsigned long long* zero[2];   // row maxima that the call has used, to be zeroed
+  int64_t nzero[2];
 };
 
 // The sums of the residues times the six 16-bit limbs of the weights, two moduli per instruction
@@ -662,7 +665,12 @@ __device__ __forceinline__ double crt_value(const uint32_t (&L)[6], int E) {
 template <int NMOD, bool GENERAL>
 __global__ void __launch_bounds__(256, 5) oz_crt(CrtArgs a) {
   chain_begin();
-  const int mt2 = blockIdx.y, z = blockIdx.z;
+  const int mt2 = a.mt0 + blockIdx.y, z = blockIdx.z;
+  for (int q = 0; q < 2; q++) {
+    const int64_t t = ((int64_t)z * a.tiles_m2 + mt2) * (gridDim.x * 256LL) + blockIdx.x * 256 +
+                      threadIdx.x;
+    if (t < a.nzero[q]) a.zero[q][t] = 0ull;
+  }
   const int row = mt2 * TILE + threadIdx.x, col0 = blockIdx.x * 4;
   if (row >= a.M) return;
   // 4-column groups of all tiles in the tile order, 1 KB per modulus each
@@ -779,6 +787,11 @@ int gemm_f64_ozaki_possible(fmpt_handle* h, const GemmArgs& g) {
              : 0;
 }
 
+bool gemm_f64_ozaki_takes_maxima(fmpt_handle* h, const GemmArgs& g) {
+  return !h->oz_digits && g.batch == 1 && (int64_t)g.k * (g.cplx ? 2 : 1) <= oz::KMAX &&
+         gemm_f64_ozaki_possible(h, g);
+}
+
 namespace oz {
 // kernels by modulus count
 typedef void (*ResGeneric)(SliceSrc, int, int, int, int, int, const unsigned long long*, uint16_t*, int*);
@@ -809,6 +822,7 @@ int gemm_f64_ozaki(fmpt_handle* h, const GemmArgs& g) {
     hi.beta[0] = 1.0;
     hi.beta[1] = 0.0;
     lo.cacheA = lo.cacheB = hi.cacheA = hi.cacheB = nullptr;
+    lo.maxA = hi.maxA = nullptr;           // they are those of the whole K
     FMPT_TRY(gemm_f64_ozaki(h, lo));
     return gemm_f64_ozaki(h, hi);
   }
@@ -863,8 +877,17 @@ int gemm_f64_ozaki(fmpt_handle* h, const GemmArgs& g) {
   const bool hitA = oz_cache_hit(g.cacheA, g.A, keyA), hitB = oz_cache_hit(g.cacheB, g.B, keyB);
   const bool inA = g.cacheA != nullptr, inB = g.cacheB != nullptr;
   const size_t need = (inA ? 0 : al(planesA) + al(expA)) + (inB ? 0 : al(planesB) + al(expB)) +
-                      al(mxb) + al(resb) + copyb;
+                      al(resb) + copyb;
   FMPT_TRY(grow_buffer(h, &h->oz_ws, &h->oz_ws_bytes, need));
+  if (h->oz_mx_bytes < mxb) h->oz_mx_dirty = true;
+  FMPT_TRY(grow_buffer(h, &h->oz_mx, &h->oz_mx_bytes, al(mxb)));
+  bool clean = true;                       // zero again once this call's kernels have run
+  if (h->oz_mx_dirty) {
+    FMPT_CUDA(h, cudaMemsetAsync(h->oz_mx, 0, h->oz_mx_bytes, h->stream));
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    clean = cudaStreamIsCapturing(h->stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+  }
+  h->oz_mx_dirty = true;
   for (int side = 0; side < 2; side++) {
     OzCache* c = side == 0 ? g.cacheA : g.cacheB;
     if (!c || (side == 0 ? hitA : hitB)) continue;
@@ -881,14 +904,13 @@ int gemm_f64_ozaki(fmpt_handle* h, const GemmArgs& g) {
   int* EA = reinterpret_cast<int*>(pa + al(planesA));
   uint16_t* SBp = reinterpret_cast<uint16_t*>(pb);
   int* EB = reinterpret_cast<int*>(pb + al(planesB));
-  unsigned long long* MX = reinterpret_cast<unsigned long long*>(base);
-  uint8_t* RES = reinterpret_cast<uint8_t*>(base + al(mxb));
-  double* COPY = reinterpret_cast<double*>(base + al(mxb) + al(resb));
+  unsigned long long* MX = static_cast<unsigned long long*>(h->oz_mx);
+  uint8_t* RES = reinterpret_cast<uint8_t*>(base);
+  double* COPY = reinterpret_cast<double*>(base + al(resb));
 
   const SliceSrc sa = oz_side_a(g), sb = oz_side_b(g);
   if (!hitA || !hitB) {
     ProfScope prof(h, FMPT_K_CONVERT);
-    FMPT_CUDA(h, cudaMemsetAsync(MX, 0, (size_t)batch * (M2 + N) * sizeof(uint64_t), h->stream));
     auto convert = [&](const SliceSrc& x, int rows, unsigned long long* mx, uint16_t* planes,
                        int* ex) -> int {
       // K columns per block: 512 where that leaves four blocks per SM, else down to one
@@ -898,7 +920,7 @@ int gemm_f64_ozaki(fmpt_handle* h, const GemmArgs& g) {
       while (kch > 64 && (int64_t)strips * ((ldk + kch - 1) / kch) * batch < 4LL * h->sm_count)
         kch /= 2;
       const dim3 grid(strips, (ldk + kch - 1) / kch, batch);
-      FMPT_TRY(oz_row_maxima(h, x, rows, K2, batch, mx));
+      if (mx != g.maxA) FMPT_TRY(oz_row_maxima(h, x, rows, K2, batch, mx));
       if (oz_kfast(x, K2))
         FMPT_CUDA(h, launch_chain(residues_kfast_kernel(nmod), grid, 256, 0, h->stream, x.p, x.sr, x.bstride, rows, K2, ldk, kch, plan.tbits, mx, planes, ex));
       else if (x.sr == 1 && !x.cplx)
@@ -909,7 +931,7 @@ int gemm_f64_ozaki(fmpt_handle* h, const GemmArgs& g) {
       FMPT_LAUNCHED(h);
       return FMPT_OK;
     };
-    if (!hitA) FMPT_TRY(convert(sa, M2, MX, SA, EA));
+    if (!hitA) FMPT_TRY(convert(sa, M2, g.maxA ? g.maxA : MX, SA, EA));
     if (!hitB) FMPT_TRY(convert(sb, N, MX + (size_t)batch * M2, SBp, EB));
   }
   for (int side = 0; side < 2; side++) {
@@ -964,15 +986,24 @@ int gemm_f64_ozaki(fmpt_handle* h, const GemmArgs& g) {
   }
   const bool general = ca.alpha[0] != 1.0 || ca.beta[0] != 0.0;
   ProfScope prof(h, FMPT_K_CONVERT);
-  const dim3 blocks((unsigned)((N + 3) / 4), (unsigned)tiles_m2, (unsigned)batch);
-  if (nmod == 15) {
-    if (general) FMPT_CUDA(h, launch_chain(oz_crt<15, true>, blocks, 256, 0, h->stream, ca));
-    else FMPT_CUDA(h, launch_chain(oz_crt<15, false>, blocks, 256, 0, h->stream, ca));
-  } else {
-    if (general) FMPT_CUDA(h, launch_chain(oz_crt<16, true>, blocks, 256, 0, h->stream, ca));
-    else FMPT_CUDA(h, launch_chain(oz_crt<16, false>, blocks, 256, 0, h->stream, ca));
+  ca.zero[0] = MX;
+  ca.nzero[0] = (int64_t)batch * (M2 + N);
+  ca.zero[1] = g.maxA;
+  ca.nzero[1] = g.maxA ? M2 : 0;
+  for (ca.mt0 = 0; ca.mt0 < tiles_m2; ca.mt0 += 65535) {
+    const dim3 blocks((unsigned)((N + 3) / 4), (unsigned)std::min(65535, tiles_m2 - ca.mt0),
+                      (unsigned)batch);
+    if (nmod == 15) {
+      if (general) FMPT_CUDA(h, launch_chain(oz_crt<15, true>, blocks, 256, 0, h->stream, ca));
+      else FMPT_CUDA(h, launch_chain(oz_crt<15, false>, blocks, 256, 0, h->stream, ca));
+    } else {
+      if (general) FMPT_CUDA(h, launch_chain(oz_crt<16, true>, blocks, 256, 0, h->stream, ca));
+      else FMPT_CUDA(h, launch_chain(oz_crt<16, false>, blocks, 256, 0, h->stream, ca));
+    }
+    FMPT_LAUNCHED(h);
   }
-  FMPT_LAUNCHED(h);
+  if (clean) h->oz_mx_dirty = false;
+  if (g.maxA && g.maxA_clean) *g.maxA_clean = true;
   if (via_copy) {
     CrtArgs cc = ca;
     cc.C = g.C;
