@@ -116,44 +116,64 @@ __global__ void __launch_bounds__(256, 4) oz_rowmax(SliceSrc src, int rows_out, 
 }
 
 // ------------------------------------------------------------ fast conversion of real operands
-// Real operands whose row or K index has unit stride (with 16-byte aligned rows or columns)
-// take these kernels instead of the generic ones above: 16-byte loads, eight independent
-// loads in flight per thread and no shared-memory staging for the row maxima, the residues
-// of a K-contiguous operand straight from registers.  The generic kernels are bound by
-// memory latency (long-scoreboard stalls, 22-37% of DRAM bandwidth).
+// Real operands whose row or K index has unit stride take these kernels instead of the generic
+// ones above: eight independent loads in flight per thread and no shared-memory staging for the
+// row maxima, the residues of a K-contiguous operand straight from registers.  The generic
+// kernels are bound by memory latency (long-scoreboard stalls, 22-37% of DRAM bandwidth).
+// V = 2: 16-byte loads, for 16-byte aligned rows or columns and an even extent along the
+// unit-stride index; V = 1: 8-byte loads, for the rest.  Loaded as integers: from doubles, the
+// compiler turns the masking of the sign into an FP64 instruction per element (kfast 37 -> 23 us
+// at 2048 x 8192).
 constexpr int RK_KCH = 1024;          // K columns per block, K-contiguous row maxima
 
-// Loaded as integers: from doubles, the compiler turns the masking of the sign into an FP64
-// instruction per element (kfast 37 -> 23 us at 2048 x 8192).
-// rows r, r + 1 of a row-contiguous operand (element (r, c) at p[r + c ld])
+template <int V>
+struct OzBits {
+  uint64_t x[V];
+};
+// V doubles' bits without their signs; zeros if !in
+template <int V>
+__device__ __forceinline__ OzBits<V> oz_load_abs(const double* p, bool in) {
+  constexpr uint64_t kAbs = 0x7fffffffffffffffull;
+  OzBits<V> r{};
+  if constexpr (V == 2) {
+    const ulonglong2 v =
+        in ? __ldg(reinterpret_cast<const ulonglong2*>(p)) : make_ulonglong2(0, 0);
+    r.x[0] = v.x & kAbs;
+    r.x[1] = v.y & kAbs;
+  } else {
+    r.x[0] = in ? __ldg(reinterpret_cast<const unsigned long long*>(p)) & kAbs : 0ull;
+  }
+  return r;
+}
+
+// rows r .. r + V - 1 of a row-contiguous operand (element (r, c) at p[r + c ld])
+template <int V>
 __global__ void __launch_bounds__(128) oz_rowmax_rowfast(const double* __restrict__ p, int64_t ld,
                                                          int64_t bstride, int rows, int k, int kch,
                                                          unsigned long long* __restrict__ mx) {
   chain_begin();
   const int z = blockIdx.z;
-  const int r = (blockIdx.x * 128 + threadIdx.x) * 2;
+  const int r = (blockIdx.x * 128 + threadIdx.x) * V;
   const int c0 = blockIdx.y * kch, c1 = min(c0 + kch, k);
   if (r >= rows) return;
   const double* b = p + (int64_t)z * bstride + r;
-  uint64_t m0 = 0, m1 = 0;
+  uint64_t m[V] = {};
   for (int c = c0; c < c1; c += 8) {
-    ulonglong2 v[8];
+    OzBits<V> v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) v[u] = oz_load_abs<V>(b + (int64_t)(c + u) * ld, c + u < c1);
 #pragma unroll
     for (int u = 0; u < 8; u++)
-      v[u] = c + u < c1 ? __ldg(reinterpret_cast<const ulonglong2*>(b + (int64_t)(c + u) * ld))
-                        : make_ulonglong2(0, 0);
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const uint64_t a0 = v[u].x & 0x7fffffffffffffffull, a1 = v[u].y & 0x7fffffffffffffffull;
-      m0 = a0 > m0 ? a0 : m0;
-      m1 = a1 > m1 ? a1 : m1;
-    }
+      for (int q = 0; q < V; q++) m[q] = v[u].x[q] > m[q] ? v[u].x[q] : m[q];
   }
-  if (m0) atomicMax(mx + (int64_t)z * rows + r, (unsigned long long)m0);
-  if (m1) atomicMax(mx + (int64_t)z * rows + r + 1, (unsigned long long)m1);
+#pragma unroll
+  for (int q = 0; q < V; q++)
+    if (m[q]) atomicMax(mx + (int64_t)z * rows + r + q, (unsigned long long)m[q]);
 }
 
 // one warp per row of a K-contiguous operand (element (r, c) at p[r ld + c])
+template <int V>
 __global__ void __launch_bounds__(256) oz_rowmax_kfast(const double* __restrict__ p, int64_t ld,
                                                        int64_t bstride, int rows, int k,
                                                        unsigned long long* __restrict__ mx) {
@@ -164,18 +184,14 @@ __global__ void __launch_bounds__(256) oz_rowmax_kfast(const double* __restrict_
   const int c0 = blockIdx.y * RK_KCH, c1 = min(c0 + RK_KCH, k);
   const double* b = p + (int64_t)z * bstride + (int64_t)r * ld;
   uint64_t m = 0;
-  for (int c = c0 + 2 * lane; c < c1; c += 64 * 8) {
-    ulonglong2 v[8];
+  for (int c = c0 + V * lane; c < c1; c += 32 * V * 8) {
+    OzBits<V> v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) v[u] = oz_load_abs<V>(b + c + 32 * V * u, c + 32 * V * u < c1);
 #pragma unroll
     for (int u = 0; u < 8; u++)
-      v[u] = c + 64 * u < c1 ? __ldg(reinterpret_cast<const ulonglong2*>(b + c + 64 * u))
-                             : make_ulonglong2(0, 0);
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const uint64_t a0 = v[u].x & 0x7fffffffffffffffull, a1 = v[u].y & 0x7fffffffffffffffull;
-      m = a0 > m ? a0 : m;
-      m = a1 > m ? a1 : m;
-    }
+      for (int q = 0; q < V; q++) m = v[u].x[q] > m ? v[u].x[q] : m;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -202,31 +218,40 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 
-// Row maxima of |op(X)| (bit patterns) into mx, zeroed by the caller.  The fast kernels need
-// a real operand with a unit-stride index, 16-byte aligned rows or columns and an even
-// extent along the unit-stride index.
-inline bool oz_aligned(const SliceSrc& x, int64_t ld) {
-  return !x.cplx && (reinterpret_cast<uintptr_t>(x.p) & 15) == 0 && (ld & 1) == 0 &&
-         (x.bstride & 1) == 0;
+// 16-byte loads along the unit-stride index (extent n, other stride ld)
+inline bool oz_aligned(const SliceSrc& x, int64_t ld, int n) {
+  return (reinterpret_cast<uintptr_t>(x.p) & 15) == 0 && (ld & 1) == 0 && (x.bstride & 1) == 0 &&
+         (n & 1) == 0;
 }
-inline bool oz_kfast(const SliceSrc& x, int k) {
-  return x.sc == 1 && oz_aligned(x, x.sr) && (k & 1) == 0;
-}
+inline bool oz_kfast(const SliceSrc& x) { return !x.cplx && x.sc == 1; }
+
+// Row maxima of |op(X)| (bit patterns) into mx, zeroed by the caller.
 inline int oz_row_maxima(fmpt_handle* h, const SliceSrc& x, int rows, int k, int batch,
                          unsigned long long* mx) {
-  if (x.sr == 1 && oz_aligned(x, x.sc) && (rows & 1) == 0) {
+  if (!x.cplx && x.sr == 1) {
+    const bool two = oz_aligned(x, x.sc, rows);
     // K columns per block (a multiple of the eight loads in flight): short enough for about
     // 16 blocks per SM, so that a small operand is spread out (1024 x 1280: 35 us on 20
     // blocks) and a large one ends evenly, at most 128
-    const int gx = (rows / 2 + 127) / 128;
+    const int gx = (rows / (two ? 2 : 1) + 127) / 128;
     const int64_t want = (int64_t)k * gx * batch / (16LL * std::max(1, h->sm_count));
     const int kc = (int)std::max<int64_t>(8, std::min<int64_t>(128, want) / 8 * 8);
     const dim3 g1((unsigned)gx, (unsigned)((k + kc - 1) / kc), (unsigned)batch);
-    FMPT_CUDA(h, launch_chain(oz_rowmax_rowfast, g1, 128, 0, h->stream, x.p, x.sc, x.bstride, rows, k, kc, mx));
-  } else if (oz_kfast(x, k)) {
+    if (two)
+      FMPT_CUDA(h, launch_chain(oz_rowmax_rowfast<2>, g1, 128, 0, h->stream, x.p, x.sc, x.bstride,
+                                rows, k, kc, mx));
+    else
+      FMPT_CUDA(h, launch_chain(oz_rowmax_rowfast<1>, g1, 128, 0, h->stream, x.p, x.sc, x.bstride,
+                                rows, k, kc, mx));
+  } else if (oz_kfast(x)) {
     const dim3 g1((unsigned)((rows + 7) / 8), (unsigned)((k + RK_KCH - 1) / RK_KCH),
                   (unsigned)batch);
-    FMPT_CUDA(h, launch_chain(oz_rowmax_kfast, g1, 256, 0, h->stream, x.p, x.sr, x.bstride, rows, k, mx));
+    if (oz_aligned(x, x.sr, k))
+      FMPT_CUDA(h, launch_chain(oz_rowmax_kfast<2>, g1, 256, 0, h->stream, x.p, x.sr, x.bstride,
+                                rows, k, mx));
+    else
+      FMPT_CUDA(h, launch_chain(oz_rowmax_kfast<1>, g1, 256, 0, h->stream, x.p, x.sr, x.bstride,
+                                rows, k, mx));
   } else {
     const dim3 g1((unsigned)((rows + SL_ROWS - 1) / SL_ROWS),
                   (unsigned)((k + SL_KCH - 1) / SL_KCH), (unsigned)batch);

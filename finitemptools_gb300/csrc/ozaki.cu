@@ -214,8 +214,8 @@ __global__ void __launch_bounds__(256, 2) oz_residues(SliceSrc src, int rows_out
 }
 
 // Residues of a K-contiguous operand: thread (rr, part) of a block owns row r0 + rr and, per
-// 64-column tile, the 8 entries from part * 8.
-template <int NMOD>
+// 64-column tile, the 8 entries from part * 8, by 16-byte (V = 2) or 8-byte loads.
+template <int NMOD, int V>
 __global__ void __launch_bounds__(256, 2) oz_residues_kfast(const double* __restrict__ p, int64_t ld,
                                                        int64_t bstride, int rows_out, int k_out,
                                                        int ldk, int kch, int tbits,
@@ -237,12 +237,16 @@ __global__ void __launch_bounds__(256, 2) oz_residues_kfast(const double* __rest
   for (int cb = kc0 + part * 8; cb < c1; cb += 64) {
     uint64_t bits8[8];
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const int cc = cb + 2 * u;
-      const double2 v = cc < k_out ? __ldg(reinterpret_cast<const double2*>(b + cc))
-                                   : make_double2(0.0, 0.0);
-      bits8[2 * u] = (uint64_t)__double_as_longlong(v.x);
-      bits8[2 * u + 1] = (uint64_t)__double_as_longlong(v.y);
+    for (int u = 0; u < 8; u += V) {
+      const int cc = cb + u;
+      if constexpr (V == 2) {
+        const ulonglong2 v = cc < k_out ? __ldg(reinterpret_cast<const ulonglong2*>(b + cc))
+                                        : make_ulonglong2(0, 0);
+        bits8[u] = v.x;
+        bits8[u + 1] = v.y;
+      } else {
+        bits8[u] = cc < k_out ? __ldg(reinterpret_cast<const unsigned long long*>(b + cc)) : 0ull;
+      }
     }
     residues8_store<NMOD>(bits8, tbits - e, bad, out, plane_stride, cb);
   }
@@ -803,8 +807,9 @@ static ResGeneric residues_kernel(int nmod) {
 static ResFast residues_rowfast_kernel(int nmod) {
   return nmod == 15 ? oz_residues_rowfast<15> : oz_residues_rowfast<16>;
 }
-static ResFast residues_kfast_kernel(int nmod) {
-  return nmod == 15 ? oz_residues_kfast<15> : oz_residues_kfast<16>;
+static ResFast residues_kfast_kernel(int nmod, bool two) {
+  if (two) return nmod == 15 ? oz_residues_kfast<15, 2> : oz_residues_kfast<16, 2>;
+  return nmod == 15 ? oz_residues_kfast<15, 1> : oz_residues_kfast<16, 1>;
 }
 }  // namespace oz
 
@@ -921,8 +926,10 @@ int gemm_f64_ozaki(fmpt_handle* h, const GemmArgs& g) {
         kch /= 2;
       const dim3 grid(strips, (ldk + kch - 1) / kch, batch);
       if (mx != g.maxA) FMPT_TRY(oz_row_maxima(h, x, rows, K2, batch, mx));
-      if (oz_kfast(x, K2))
-        FMPT_CUDA(h, launch_chain(residues_kfast_kernel(nmod), grid, 256, 0, h->stream, x.p, x.sr, x.bstride, rows, K2, ldk, kch, plan.tbits, mx, planes, ex));
+      if (oz_kfast(x))
+        FMPT_CUDA(h, launch_chain(residues_kfast_kernel(nmod, oz_aligned(x, x.sr, K2)), grid, 256, 0,
+                                  h->stream, x.p, x.sr, x.bstride, rows, K2, ldk, kch, plan.tbits,
+                                  mx, planes, ex));
       else if (x.sr == 1 && !x.cplx)
         FMPT_CUDA(h, launch_chain(residues_rowfast_kernel(nmod), grid, 256, DR_SMEM, h->stream, x.p, x.sc, x.bstride, rows, K2, ldk, kch, plan.tbits, mx, planes, ex));
       else

@@ -875,7 +875,7 @@ int gemm_f64_digits(fmpt_handle* h, const GemmArgs& g) {
     auto slice = [&](const SliceSrc& x, int rows, const dim3& grid, unsigned long long* mx,
                      uint16_t* planes, int* ex) -> int {
       FMPT_TRY(oz_row_maxima(h, x, rows, K2, batch, mx));
-      if (oz_kfast(x, K2))
+      if (oz_kfast(x) && oz_aligned(x, x.sr, K2))
         FMPT_CUDA(h, launch_chain(ozd_digits_kfast, grid, 256, 0, h->stream, x.p, x.sr, x.bstride, rows, K2, ldk, mx,
                                                       planes, ex));
       else if (x.sr == 1 && !x.cplx)
