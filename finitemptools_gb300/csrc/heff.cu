@@ -83,10 +83,14 @@ template <int OUT, int TERMS>
 struct MidSparse {
   int n_out;                          // nw_out * p_out
   short start[OUT + 1];
-  short idx[TERMS];                   // wi * 16 + s
+  short idx[TERMS];                   // wi * 16 + s, MS_COPY / MS_NEG: coefficient +1 / -1
   double c[TERMS];                    // real coefficients; complex: re, im pairs
 };
 constexpr int MS_SMALL_OUT = 32, MS_SMALL_T = 96;
+// An output's first term with coefficient +-1 is a copy: a multiply-add less, where the step is
+// bound by them (30 per element of a Heisenberg bond, 11 of them copies; D = 2048: 283 -> 272
+// us).  Flags of real tables in idx, above wi < MS_MAX_WI.
+constexpr int MS_COPY = 0x2000, MS_NEG = 0x4000, MS_IDX = 0x1fff, MS_MAX_WI = 512;
 
 // bits of |x|.  Not through __double_as_longlong: the compiler turns its masked form into an
 // FP64 instruction, 64 cycles of the pipe that bounds these kernels.
@@ -102,8 +106,23 @@ __device__ __forceinline__ void mid_sparse_sum(const MidSparse<OUT, TERMS>& ms, 
                                                const double* ib, int64_t plane_in,
                                                const MidStrides& si, double& ar, double& ai) {
   ar = ai = 0.0;
-  for (int e = ms.start[o]; e < ms.start[o + 1]; e++) {
+  int e = ms.start[o];
+  const int e1 = ms.start[o + 1];
+  if (!CPLX && e < e1) {
     const int ix = ms.idx[e];
+    if (ix & (MS_COPY | MS_NEG)) {
+      // fma(+-1, v, 0): v with its sign, zeros as +0, on the words (as doubles, the sign change
+      // would become an FP64 instruction)
+      const int off16 = ix & MS_IDX;
+      uint2 v = *reinterpret_cast<const uint2*>(ib + (off16 >> 4) * si.w + (off16 & 15) * si.s);
+      if (ix & MS_NEG) v.y ^= 0x80000000u;
+      if (((v.y << 1) | v.x) == 0u) v.y = 0u;
+      asm("mov.b64 %0, {%1, %2};" : "=d"(ar) : "r"(v.x), "r"(v.y));
+      e++;
+    }
+  }
+  for (; e < e1; e++) {
+    const int ix = ms.idx[e] & MS_IDX;
     const int64_t off = (ix >> 4) * si.w + (ix & 15) * si.s;
     const double vr = ib[off];
     if (CPLX) {
@@ -239,6 +258,7 @@ void build_schedule(int cplx, int nw_in, int nw_out, int p_in, int p_out,
         for (int si = 0; si < p_in; si++) {
           const double cr = cb[q * p_in + si], ci = cplx ? cb[csz + q * p_in + si] : 0.0;
           if (cr == 0.0 && ci == 0.0) continue;
+          if (s.blk_win[b] >= MS_MAX_WI) fits = false;
           ix.push_back(s.blk_win[b] * 16 + si);
           cf.push_back(cr);
           if (cplx) cf.push_back(ci);
@@ -363,6 +383,10 @@ static int mid_sparse_launch(fmpt_handle* h, const MidSchedule& s, const double*
   for (size_t i = 0; i < s.sp_start.size(); i++) ms.start[i] = (short)s.sp_start[i];
   for (size_t i = 0; i < s.sp_idx.size(); i++) ms.idx[i] = (short)s.sp_idx[i];
   for (size_t i = 0; i < s.sp_coef.size(); i++) ms.c[i] = s.sp_coef[i];
+  for (int o = 0; !CPLX && o < ms.n_out; o++) {
+    const int e = ms.start[o];
+    if (e < ms.start[o + 1] && std::fabs(ms.c[e]) == 1.0) ms.idx[e] |= ms.c[e] > 0.0 ? MS_COPY : MS_NEG;
+  }
   const int64_t blocks = ((int64_t)n1 * n2 + 127) / 128;
   // below a few blocks per SM the outputs are spread over threads of their own (see the
   // kernel); above, the input is read once
