@@ -128,6 +128,44 @@ int set_error(fmpt_handle* h, int status, const char* fmt, ...);
 // with plain launches and 11.3 with these.
 #ifdef __CUDACC__
 __device__ __forceinline__ void chain_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Conversions between FP32 and FP64 on the integer pipe: a conversion instruction runs on the
+// FP64 pipe of GB300, 64 cycles of its SM sub-partition, and the epilogues and layout kernels
+// that widen or narrow every element were bound by it.  Zeros and normal numbers here; the rest
+// (rare) through the instruction.
+__device__ __forceinline__ bool widen_rare(uint32_t b) {     // denormal, Inf, NaN
+  const uint32_t mag = b & 0x7fffffffu;
+  return mag - 1u < 0x007fffffu || mag >= 0x7f800000u;
+}
+__device__ __forceinline__ double widen_common(uint32_t b) {
+  const uint32_t mag = b & 0x7fffffffu;
+  const uint32_t hi = (b & 0x80000000u) | (mag ? (mag >> 3) + 0x38000000u : 0u);
+  double r;
+  asm("mov.b64 %0, {%1, %2};" : "=d"(r) : "r"(b << 29), "r"(hi));
+  return r;
+}
+__device__ __forceinline__ double widen(float v) {
+  const uint32_t b = __float_as_uint(v);
+  return widen_rare(b) ? (double)v : widen_common(b);
+}
+__device__ __forceinline__ double xor_high(double v, uint32_t mask) {
+  uint32_t lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(v));
+  asm("mov.b64 %0, {%1, %2};" : "=d"(v) : "r"(lo), "r"(hi ^ mask));
+  return v;
+}
+// round to nearest even
+__device__ __forceinline__ float narrow(double v) {
+  uint32_t lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(v));
+  const uint32_t mag = hi & 0x7fffffffu;
+  const uint32_t hm = mag - 0x38000000u;                     // exponent rebased
+  if ((mag | lo) == 0u) return __uint_as_float(hi);
+  if (hm - 0x00100000u >= 0x0fe00000u) return (float)v;      // below the normal range, above it
+  uint32_t f = __funnelshift_l(lo, hm, 3);
+  f += ((lo & 0x1fffffffu) + 0x0fffffffu + (f & 1u)) >> 29;
+  return __uint_as_float(f | (hi & 0x80000000u));
+}
 inline void chain_attr(cudaLaunchAttribute& a) {
   a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   a.val.programmaticStreamSerializationAllowed = 1;

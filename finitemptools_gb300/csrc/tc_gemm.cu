@@ -32,12 +32,17 @@ template <int OUT>
 __device__ __forceinline__ void store_cols(void* base, int64_t ldc, int n_base, int n_lim,
                                            const uint32_t (&r)[32]) {
   // base points at C[row, n_base]; columns n_base + j for j < 32, those >= n_lim skipped
-  if (n_base + 32 <= n_lim) {
+  bool rare = false;                               // OUT == 1: some value needs the instruction
+  if (OUT == 1) {
+#pragma unroll
+    for (int j = 0; j < 32; j++) rare |= widen_rare(r[j]);
+  }
+  if (n_base + 32 <= n_lim && !rare) {
 #pragma unroll
     for (int j = 0; j < 32; j++) {
       const float v = __uint_as_float(r[j]);
       if (OUT == 1)
-        static_cast<double*>(base)[ldc * j] = (double)v;
+        static_cast<double*>(base)[ldc * j] = widen_common(r[j]);
       else if (OUT == 2)
         static_cast<__nv_bfloat16*>(base)[ldc * j] = __float2bfloat16_rn(v);
       else
@@ -594,7 +599,7 @@ struct SmallCfg {
 template <int OUT>
 __device__ __forceinline__ void store_one(void* C, int64_t idx, float v) {
   if (OUT == 1)
-    static_cast<double*>(C)[idx] = (double)v;
+    static_cast<double*>(C)[idx] = widen(v);
   else if (OUT == 2)
     static_cast<__nv_bfloat16*>(C)[idx] = __float2bfloat16_rn(v);
   else

@@ -41,11 +41,23 @@ __device__ __forceinline__ float tf32_rna(float x) {
 template <int MODE>
 __device__ __forceinline__ void put(void* hi, void* lo, int64_t i, double v) {
   if (MODE == M_BF16) {
-    static_cast<__nv_bfloat16*>(hi)[i] = __float2bfloat16_rn((float)v);
+    static_cast<__nv_bfloat16*>(hi)[i] = __float2bfloat16_rn(narrow(v));
   } else {
-    const float h = tf32_rna((float)v);
+    const float h = tf32_rna(narrow(v));
     static_cast<float*>(hi)[i] = h;
-    if (MODE == M_TF32X3) static_cast<float*>(lo)[i] = tf32_rna((float)(v - (double)h));
+    if (MODE == M_TF32X3) static_cast<float*>(lo)[i] = tf32_rna(narrow(v - widen(h)));
+  }
+}
+// the same of an FP32 value: v - h is exact in FP32 (a multiple of v's last place, below 2^13 of
+// them), so no FP64 is needed
+template <int MODE>
+__device__ __forceinline__ void put(void* hi, void* lo, int64_t i, float v) {
+  if (MODE == M_BF16) {
+    static_cast<__nv_bfloat16*>(hi)[i] = __float2bfloat16_rn(v);
+  } else {
+    const float h = tf32_rna(v);
+    static_cast<float*>(hi)[i] = h;
+    if (MODE == M_TF32X3) static_cast<float*>(lo)[i] = tf32_rna(v - h);
   }
 }
 
@@ -75,30 +87,31 @@ __global__ void conv_state_vec(const double* __restrict__ x, int64_t n4, void* h
        t += (int64_t)gridDim.x * blockDim.x) {
     const double2 p = x2[2 * t], q = x2[2 * t + 1];
     if (MODE == M_BF16) {
-      const __nv_bfloat162 u = __floats2bfloat162_rn((float)p.x, (float)p.y);
-      const __nv_bfloat162 w = __floats2bfloat162_rn((float)q.x, (float)q.y);
+      const __nv_bfloat162 u = __floats2bfloat162_rn(narrow(p.x), narrow(p.y));
+      const __nv_bfloat162 w = __floats2bfloat162_rn(narrow(q.x), narrow(q.y));
       uint2 o;
       o.x = *reinterpret_cast<const uint32_t*>(&u);
       o.y = *reinterpret_cast<const uint32_t*>(&w);
       reinterpret_cast<uint2*>(hi)[t] = o;
     } else {
-      const float4 hv = make_float4(tf32_rna((float)p.x), tf32_rna((float)p.y),
-                                    tf32_rna((float)q.x), tf32_rna((float)q.y));
+      const float4 hv = make_float4(tf32_rna(narrow(p.x)), tf32_rna(narrow(p.y)),
+                                    tf32_rna(narrow(q.x)), tf32_rna(narrow(q.y)));
       reinterpret_cast<float4*>(hi)[t] = hv;
       if (MODE == M_TF32X3)
         reinterpret_cast<float4*>(lo)[t] =
-            make_float4(tf32_rna((float)(p.x - (double)hv.x)), tf32_rna((float)(p.y - (double)hv.y)),
-                        tf32_rna((float)(q.x - (double)hv.z)), tf32_rna((float)(q.y - (double)hv.w)));
+            make_float4(tf32_rna(narrow(p.x - widen(hv.x))), tf32_rna(narrow(p.y - widen(hv.y))),
+                        tf32_rna(narrow(q.x - widen(hv.z))), tf32_rna(narrow(q.y - widen(hv.w))));
     }
   }
 }
 
 // batched transpose with conversion:
-//   dst[c + dld*r + dz*z] = scale * src[r + sld*c + sz*z]   for r < R, c < Cp (zero for c >= C)
+//   dst[c + dld*r + dz*z] = src[r + sld*c + sz*z]   for r < R, c < Cp (zero for c >= C)
+// with the sign bits in flip changed (0 or 2^31 of the high word)
 template <int MODE>
 __global__ void conv_transpose(const double* __restrict__ src, int64_t sld, int64_t sz, int R,
                                int C, int Cp, void* hi, void* lo, int64_t dld, int64_t dz,
-                               double scale) {
+                               uint32_t flip) {
   chain_begin();
   __shared__ double tile[32][33];
   const int z = blockIdx.z;
@@ -111,7 +124,7 @@ __global__ void conv_transpose(const double* __restrict__ src, int64_t sld, int6
   __syncthreads();
   for (int j = ty; j < 32; j += 8) {
     const int c = c0 + tx, r = r0 + j;
-    if (r < R && c < Cp) put<MODE>(hi, lo, (int64_t)c + dld * r + dz * z, scale * tile[tx][j]);
+    if (r < R && c < Cp) put<MODE>(hi, lo, (int64_t)c + dld * r + dz * z, xor_high(tile[tx][j], flip));
   }
 }
 
@@ -152,7 +165,7 @@ __global__ void mid_tc(const float* __restrict__ T1, int P, int Dl, int Dr, int 
 #pragma unroll
     for (int q = 0; q < MAXP; q++) {
       if (q >= P) break;
-      put<MODE>(hi, lo, (int64_t)b + (int64_t)Drp * wo + K2 * (ap + (int64_t)Dl * q), (double)acc[q]);
+      put<MODE>(hi, lo, (int64_t)b + (int64_t)Drp * wo + K2 * (ap + (int64_t)Dl * q), acc[q]);
     }
   }
 }
@@ -209,10 +222,10 @@ __global__ void __launch_bounds__(256) mid_tc_p4(const V4* __restrict__ T1, int 
     }
     const int64_t o = (int64_t)b + (int64_t)Drp * wo + K2 * ap;
     const int64_t qs = K2 * Dl;
-    put<MODE>(hi, lo, o, (double)a0);
-    put<MODE>(hi, lo, o + qs, (double)a1);
-    put<MODE>(hi, lo, o + 2 * qs, (double)a2);
-    put<MODE>(hi, lo, o + 3 * qs, (double)a3);
+    put<MODE>(hi, lo, o, a0);
+    put<MODE>(hi, lo, o + qs, a1);
+    put<MODE>(hi, lo, o + 2 * qs, a2);
+    put<MODE>(hi, lo, o + 3 * qs, a3);
   }
 }
 
@@ -311,7 +324,7 @@ __global__ void __launch_bounds__(256) mid_tc_mask(const float* __restrict__ T, 
         for (int s2 = 0; s2 < P; s2++) acc[q] = fmaf(c[wi * 8 + wo][q * P + s2], v[wi][s2], acc[q]);
     }
 #pragma unroll
-    for (int q = 0; q < P; q++) put<MODE>(hi, lo, ob + wo * ows + q * oqs, (double)acc[q]);
+    for (int q = 0; q < P; q++) put<MODE>(hi, lo, ob + wo * ows + q * oqs, acc[q]);
   }
 }
 
@@ -338,23 +351,23 @@ int grid1(fmpt_handle* h, int64_t n) {
 
 template <int MODE>
 int launch_transpose(fmpt_handle* h, const double* src, int64_t sld, int64_t sz, int R, int C,
-                     int Cp, int Z, void* hi, void* lo, int64_t dld, int64_t dz, double scale) {
+                     int Cp, int Z, void* hi, void* lo, int64_t dld, int64_t dz, bool negate) {
   dim3 grid((R + 31) / 32, (Cp + 31) / 32, Z);
   ProfScope prof(h, FMPT_K_CONVERT);
   FMPT_CUDA(h, launch_chain(conv_transpose<MODE>, grid, dim3(32, 8), 0, h->stream, src, sld, sz, R, C, Cp, hi, lo, dld, dz,
-                                                           scale));
+                            negate ? 0x80000000u : 0u));
   FMPT_LAUNCHED(h);
   return FMPT_OK;
 }
 
 int transpose_any(fmpt_handle* h, int mode, const double* src, int64_t sld, int64_t sz, int R,
                   int C, int Cp, int Z, void* hi, void* lo, int64_t dld, int64_t dz,
-                  double scale = 1.0) {
+                  bool negate = false) {
   if (mode == M_TF32)
-    return launch_transpose<M_TF32>(h, src, sld, sz, R, C, Cp, Z, hi, lo, dld, dz, scale);
+    return launch_transpose<M_TF32>(h, src, sld, sz, R, C, Cp, Z, hi, lo, dld, dz, negate);
   if (mode == M_TF32X3)
-    return launch_transpose<M_TF32X3>(h, src, sld, sz, R, C, Cp, Z, hi, lo, dld, dz, scale);
-  return launch_transpose<M_BF16>(h, src, sld, sz, R, C, Cp, Z, hi, lo, dld, dz, scale);
+    return launch_transpose<M_TF32X3>(h, src, sld, sz, R, C, Cp, Z, hi, lo, dld, dz, negate);
+  return launch_transpose<M_BF16>(h, src, sld, sz, R, C, Cp, Z, hi, lo, dld, dz, negate);
 }
 
 inline void* offset(void* p, int64_t elems, int es) {
@@ -371,13 +384,13 @@ int embed_complex(fmpt_handle* h, int mode, const double* src, int64_t plane, in
   const int64_t dld = 2LL * Kc;
   const double* re = src;
   const double* im = src + plane;
-  FMPT_TRY(transpose_any(h, mode, re, sld, sz, R, C, Cp, Z, hi, lo, dld, dz, 1.0));
+  FMPT_TRY(transpose_any(h, mode, re, sld, sz, R, C, Cp, Z, hi, lo, dld, dz));
   FMPT_TRY(transpose_any(h, mode, im, sld, sz, R, C, Cp, Z, offset(hi, Kc, es), offset(lo, Kc, es),
-                         dld, dz, -1.0));
+                         dld, dz, true));
   FMPT_TRY(transpose_any(h, mode, im, sld, sz, R, C, Cp, Z, offset(hi, N * dld, es),
-                         offset(lo, N * dld, es), dld, dz, 1.0));
+                         offset(lo, N * dld, es), dld, dz));
   return transpose_any(h, mode, re, sld, sz, R, C, Cp, Z, offset(hi, N * dld + Kc, es),
-                       offset(lo, N * dld + Kc, es), dld, dz, 1.0);
+                       offset(lo, N * dld + Kc, es), dld, dz);
 }
 
 }  // namespace
