@@ -349,6 +349,7 @@ int fmpt_destroy(fmpt_handle* h) {
   if (h->gemm_ws) cudaFree(h->gemm_ws);
   if (h->gemm_cnt) cudaFree(h->gemm_cnt);
   if (h->tc_ws) cudaFree(h->tc_ws);
+  if (h->tc_cnt) cudaFree(h->tc_cnt);
   if (h->oz_ws) cudaFree(h->oz_ws);
   if (h->oz_mx) cudaFree(h->oz_mx);
   if (h->gstatus) cudaFree(h->gstatus);
