@@ -270,8 +270,9 @@ __global__ void __launch_bounds__(GNT) grouped_kernel(const GKArgs a) {
 // their own, for 152 SMs, and 16-wide groups pad its blocks (10 to 71 wide) by a third; its
 // 3604 tiles of 8x4 pad by 8%.  Re-reading the operands per small tile costs nothing beside
 // an FMA's 64 cycles.  H_eff*x, us, best block tile -> warp tile: D = 32 (16 sites) 18.7 ->
-// 16.9, D = 64 24.8 -> 18.8, D = 128 84 -> 26, D = 256 200 -> 52, D = 512 366 -> 121,
-// D = 1024 1006 -> 764, D = 1500 2498 -> 2316 (FP64 pipe bound).  Four blocks of four warps
+// 16.9, D = 64 24.8 -> 18.8, D = 128 84 -> 25, D = 256 200 -> 50, D = 512 366 -> 114,
+// D = 1024 1006 -> 705, D = 1500 2498 -> 2122 (FP64 pipe bound; the test of a coefficient for one
+// is on its words, since an FP64 comparison per 16-deep slab cost 8%).  Four blocks of four warps
 // per SM: with two, a warp's start on a tile (descriptors, first slab) shows, 140 us at
 // D = 512; slabs in flight per warp: 2 (4 or 6 stages were no faster).
 constexpr int QM = 8, QN = 4, QK = 16, QST = 3, QWARPS = 4, QBLOCKS = 4;
@@ -376,7 +377,7 @@ __device__ __forceinline__ void gemm_warp_tile(const GKArgs& a, const GPhaseDesc
     issue(kn[QST - 1], coef[QST - 1]);
     asm volatile("cp.async.wait_group %0;" ::"n"(QST - 1) : "memory");
     __syncwarp();
-    if (coef[0] != 1.0) {
+    if (!is_one(coef[0])) {
 #pragma unroll
       for (int e = 0; e < QM * QK / 32; e++) As[st][ln + e * (32 / QM)][lm] *= coef[0];
       __syncwarp();

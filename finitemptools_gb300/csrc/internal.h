@@ -153,6 +153,11 @@ __device__ __forceinline__ double widen(float v) {
   const uint32_t b = __float_as_uint(v);
   return widen_rare(b) ? (double)v : widen_common(b);
 }
+__device__ __forceinline__ bool is_one(double v) {           // an FP64 comparison takes the pipe too
+  uint32_t lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(v));
+  return lo == 0u && hi == 0x3ff00000u;
+}
 __device__ __forceinline__ double xor_high(double v, uint32_t mask) {
   uint32_t lo, hi;
   asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(v));
