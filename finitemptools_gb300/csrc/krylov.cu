@@ -742,6 +742,31 @@ __global__ void __launch_bounds__(GS_T) arnoldi_gs_fused(GsArgs a, CoopBar bar) 
   }
 }
 
+// The step of a short vector (gs_geometry) as one block or one cluster: the blocks meet at the
+// cluster's hardware barrier, and as the launch is not a cooperative one it overlaps the kernel
+// before it.  The same device functions on the same grid, so the same sums.
+__global__ void __launch_bounds__(GS_T) arnoldi_gs_cluster(GsArgs a) {
+  chain_begin();
+  __shared__ double bp[GS_NV], c[2][GS_NV];
+  const GsWarp w(a);
+  const int G = gridDim.x, nv = 2 * a.j + 3;
+  double zv = gs_load(a, w);
+  for (int pass = 0; pass < 2; pass++) {
+    double* part = a.part + (int64_t)pass * GS_NV * G;
+    if (G == 1) {
+      gs_dots<true>(a, w, zv, c[pass]);
+    } else {
+      gs_dots<true>(a, w, zv, bp);
+      if ((int)threadIdx.x < nv) part[(int64_t)threadIdx.x * G + blockIdx.x] = bp[threadIdx.x];
+      asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+      gs_total(part, G, nv, c[pass]);
+      __syncthreads();
+    }
+    zv = gs_axpy<true>(a, w, c[pass], zv, pass == 1,
+                       [&]() { return gs_close(a, c[0], c[1], blockIdx.x == 0); });
+  }
+}
+
 // ---- the same step as six launches (fmpt_set_fused_krylov off): the same device functions
 // on the same grid, so the same sums
 template <bool SINGLE>
@@ -1432,7 +1457,8 @@ int op_project(fmpt_op* op, double* y, const int* gate) {
 struct GsWork {
   int G, cpb;
   bool single;        // every warp has one chunk
-  bool fused;         // one cooperative launch per step
+  bool fused;         // one launch per step
+  bool cluster;       // .. of one block or one cluster, otherwise cooperative
   double* part;       // [2][GS_NV][G]
   double* coef;       // [2 GS_NV + 1] (separate launches)
   int* bar;
@@ -1442,13 +1468,24 @@ struct GsWork {
 };
 
 // Blocks of the step and chunks per block for S chunks: one block, without grid-wide waits,
-// up to 4 chunks; then as few chunks per block as keep it within 128 blocks (n = 8192
-// complex: 4 chunks, one per SM sub-partition); beyond 1024 chunks the warps loop.
+// up to 4 chunks; one cluster of 4, 8 or 16 blocks up to GS_CLUSTER_S chunks (complex exponential
+// of 20 vectors, cooperative -> cluster: D = 8 649 -> 592 us, D = 16 754 -> 706, D = 22, the
+// last one, 832 -> 810; D = 27 would take 978 instead of 904: 16 SMs are too few for it); then as few chunks
+// per block as keep it within 128 blocks (n = 8192 complex: 4 chunks, one per SM sub-partition);
+// beyond 1024 chunks the warps loop.
+constexpr int GS_CLUSTER_S = 64;
 void gs_geometry(int64_t S, int& G, int& cpb, bool& single) {
   single = true;
   if (S <= 4) {
     G = 1;
     cpb = S <= 1 ? 1 : (S <= 2 ? 2 : 4);
+    return;
+  }
+  if (S <= GS_CLUSTER_S) {
+    cpb = 1;
+    while ((S + cpb - 1) / cpb > 16) cpb *= 2;
+    G = 4;
+    while ((int64_t)G * cpb < S) G *= 2;
     return;
   }
   for (cpb = 1; cpb <= 8; cpb *= 2)
@@ -1485,10 +1522,54 @@ bool gs_fused_fits(fmpt_handle* h, int G) {
   return (int64_t)occ[dev] * h->sm_count >= G;
 }
 
+void gs_cluster_config(fmpt_handle* h, int G, cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr) {
+  cfg = cudaLaunchConfig_t{};
+  cfg.gridDim = dim3(G);
+  cfg.blockDim = dim3(GS_T);
+  cfg.stream = h->stream;
+  cfg.attrs = attr;
+  chain_attr(attr[0]);
+  cfg.numAttrs = 1;
+  if (G > 1) {
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = G;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+  }
+}
+// Whether a cluster of G blocks (up to 16: beyond the portable 8) fits this device.
+bool gs_cluster_fits(fmpt_handle* h, int G) {
+  if (G == 1) return true;
+  static std::mutex mu;
+  static signed char fits[64][5] = {};                      // 0 unknown, 1 yes, -1 no; by log2 G
+  const int dev = h->device, l = G == 4 ? 2 : (G == 8 ? 3 : 4);
+  if (dev < 0 || dev >= 64) return false;
+  std::lock_guard<std::mutex> lock(mu);
+  if (!fits[dev][l]) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[2];
+    gs_cluster_config(h, G, cfg, attr);
+    std::swap(attr[0], attr[1]);                            // the cluster attribute alone
+    cfg.numAttrs = 1;
+    int n = 0;
+    const bool ok = cudaFuncSetAttribute(arnoldi_gs_cluster,
+                                         cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                        cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&n, arnoldi_gs_cluster, &cfg) == cudaSuccess &&
+                    n > 0;
+    if (!ok) cudaGetLastError();
+    fits[dev][l] = ok ? 1 : -1;
+  }
+  return fits[dev][l] > 0;
+}
+
 int gs_setup(fmpt_handle* h, int cp, int64_t n, int M, DevBuf& buf, GsWork& w) {
   const int64_t nch = (n + 31) / 32;
   gs_geometry(cp ? 2 * nch : nch, w.G, w.cpb, w.single);
   w.fused = h->fused_gs && gs_fused_fits(h, w.G);
+  // (the test of the bounded grid waits needs the launch that has them)
+  w.cluster = w.fused && (cp ? 2 * nch : nch) <= GS_CLUSTER_S && h->wait_test_hold == 0 &&
+              gs_cluster_fits(h, w.G);
   const size_t parts = (size_t)2 * GS_NV * w.G;
   FMPT_TRY(buf.alloc(h, (parts + 2 * GS_NV + 2 + 2) * sizeof(double)));
   w.part = buf.d();
@@ -1515,6 +1596,15 @@ int gs_step(fmpt_handle* h, const GsWork& w, int cp, int64_t n, int64_t nr, int 
   a.part = w.part;
   a.Hcol = Hcol;
   a.vnext = V + (int64_t)(j + 1) * nr;
+  if (w.cluster) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[2];
+    gs_cluster_config(h, w.G, cfg, attr);
+    h->cluster_sig = h->cluster_sig * 31 + w.G;
+    FMPT_CUDA(h, cudaLaunchKernelEx(&cfg, arnoldi_gs_cluster, a));
+    FMPT_LAUNCHED(h);
+    return FMPT_OK;
+  }
   if (w.fused) {
     const CoopBar bar{w.bar, w.bar + 1, w.status, w.wait_ns, w.hold};
     cudaLaunchConfig_t cfg{};
@@ -1557,8 +1647,9 @@ int arnoldi_basis(fmpt_op* op, int cp, int64_t n, int64_t nr, int M, int ldh, do
   fmpt_handle* h = op->h;
   cudaStream_t st = h->stream;
   auto record = [&]() -> int {
+    h->cluster_sig = 0;
     FMPT_CUDA(h, cudaMemsetAsync(Hdev.p, 0, Hdev.bytes, st));
-    if (gs.fused) FMPT_CUDA(h, cudaMemsetAsync(gs.bar, 0, 2 * sizeof(int), st));
+    if (gs.fused && !gs.cluster) FMPT_CUDA(h, cudaMemsetAsync(gs.bar, 0, 2 * sizeof(int), st));
     for (int j = 0; j < M; j++) {
       FMPT_TRY(fmpt_op_apply(op, V + (int64_t)j * nr, z));
       FMPT_TRY(gs_step(h, gs, cp, n, nr, j, V, z, Hdev.d() + (size_t)2 * ldh * j));
@@ -1583,9 +1674,10 @@ int arnoldi_basis(fmpt_op* op, int cp, int64_t n, int64_t nr, int M, int ldh, do
     cudaGetLastError();
     return record();
   }
-  char key[96];
-  std::snprintf(key, sizeof(key), "k%d p%d c%d u%d q%zu M%d g%d", op->kind, op->precision, cp,
-                op->u1 ? 1 : 0, op->proj.size(), M, gs.fused ? 1 : 0);
+  char key[112];
+  std::snprintf(key, sizeof(key), "k%d p%d c%d u%d q%zu M%d g%d s%x", op->kind, op->precision, cp,
+                op->u1 ? 1 : 0, op->proj.size(), M, gs.cluster ? 2 : (gs.fused ? 1 : 0),
+                (unsigned)h->cluster_sig);
   cudaGraphExec_t& ex = h->arnoldi_exec[key];
   bool ready = false;
   if (ex) {

@@ -19,6 +19,9 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("dl,dr,cplx", [
     (1, 2, True), (2, 4, True), (8, 4, True), (8, 4, False), (9, 4, True), (16, 16, True),
     (32, 65, True), (65, 64, False), (64, 64, True), (91, 94, True), (130, 130, False),
+    # one cluster of 4 (5 chunks), 8 (10, 16) and 16 blocks (18, 64), the first beyond it (66)
+    (9, 8, False), (8, 10, True), (8, 16, True), (12, 12, True), (32, 16, True), (32, 32, False),
+    (33, 16, True),
 ])
 def test_exponential_launch_shapes(dl, dr, cplx):
     rng = np.random.default_rng(dl * dr + cplx)
