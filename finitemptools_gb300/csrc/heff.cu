@@ -292,7 +292,7 @@ int schedule_ac2(fmpt_handle* h, int cplx, const double* W1, const double* W2, i
                  int wl, int wm, int wr, MidSchedule& s) {
   if (!W1 || !W2) return set_error(h, FMPT_ERR_ARG, "ac2: null MPO tensor");
   schedule_ac2_host(cplx, W1, W2, d1, d2, wl, wm, wr, s);
-  return mid_upload(h, s);
+  return s.sp_start.empty() ? mid_upload(h, s) : FMPT_OK;   // the kernel takes it by value
 }
 
 void schedule_ac2_host(int cplx, const double* W1, const double* W2, int d1, int d2, int wl,
@@ -343,7 +343,7 @@ int schedule_env(fmpt_handle* h, int cplx, const double* W, int d, int wl, int w
           O[(((size_t)wi * nw_out + wo) * d + so) * d + si] = v;
         }
   build_schedule(cplx, nw_in, nw_out, d, d, O, s);
-  return mid_upload(h, s);
+  return s.sp_start.empty() ? mid_upload(h, s) : FMPT_OK;   // the kernel takes it by value
 }
 
 int mid_upload(fmpt_handle* h, MidSchedule& s) {

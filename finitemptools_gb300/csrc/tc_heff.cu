@@ -420,7 +420,6 @@ int op_tc_prepare(fmpt_op* op) {
         rs.coef.push_back(cs.coef[e * 2 * pp + q]);
       }
     }
-    FMPT_TRY(mid_upload(h, rs));
   }
   const int Dl = op->Dl, Dr = op->Dr, wl = op->wl, wr = op->wr;
   if (op->kind == 2) {
@@ -431,7 +430,6 @@ int op_tc_prepare(fmpt_op* op) {
     s.blk_win.resize(wl); s.wout_start.resize(wl + 1); s.coef.assign(wl, 1.0);
     for (int w = 0; w < wl; w++) { s.blk_win[w] = w; s.wout_start[w] = w; }
     s.wout_start[wl] = wl;
-    FMPT_TRY(mid_upload(h, s));
   } else {
     st->P = op->kind == 0 ? op->d1 * op->d2 : op->d1;
   }
@@ -451,7 +449,7 @@ int op_tc_prepare(fmpt_op* op) {
     FMPT_CUDA(h, cudaMemsetAsync(st->T3[p].p, 0, st->T3[p].bytes, h->stream));  // K padding
   }
   {
-    const MidSchedule& ms = st->cplx && op->kind != 2 ? st->rsched : op->sched;
+    MidSchedule& ms = st->cplx && op->kind != 2 ? st->rsched : op->sched;
     if (P == 4 && ms.nw_in <= 8 && ms.nw_out <= 8) {
       std::vector<float> cf(64 * 16, 0.f);
       uint64_t mask = 0;
@@ -464,6 +462,8 @@ int op_tc_prepare(fmpt_op* op) {
       std::memcpy(st->cpar.c, cf.data(), sizeof(st->cpar.c));
       st->mask = mask;
       st->fast_mid = true;
+    } else if (!ms.d_win) {
+      FMPT_TRY(mid_upload(h, ms));               // mid_tc reads the table from memory
     }
   }
   // T1 is BF16 when the BF16 fast MPO step reads it (its values are rounded to BF16 for
@@ -924,6 +924,7 @@ void op_tc_free(fmpt_op* op) {
   TcState* st = static_cast<TcState*>(op->tc);
   if (!st) return;
   if (st->err) cudaFreeAsync(st->err, op->h->stream);
+  mid_free(op->h, st->rsched);
   delete st;
   op->tc = nullptr;
 }
