@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(NT) gemm_kernel(GemmArgs g, int splits, int kc
 // Each output is the same chain of FMAs over k as in gemm_kernel.  Per contraction, D = 64:
 // real 16.1 and 20.4 -> 14.6 and 17.8 us (FP64 pipe 80% busy), complex 24.2 and 22.8 ->
 // 17.7 and 18.2 us.
-constexpr int WM = 8, WN = 4, WWARPS = 2, WK = 32, WST = 4;
+constexpr int WM = 8, WN = 4, WWARPS = 2, WK1 = 32, WST1 = 4;
 
 // 8 bytes, zeros if !in
 __device__ __forceinline__ void cp_async8z(double* dst, const double* src, bool in) {
@@ -248,24 +248,36 @@ __device__ __forceinline__ void cp_async8z(double* dst, const double* src, bool 
                : "memory");
 }
 
-template <bool CPLX>
-__global__ void __launch_bounds__(32 * WWARPS) gemm_warp(GemmArgs g, int splits, int kchunk,
-                                                         double* __restrict__ ws,
-                                                         int* __restrict__ tile_cnt) {
+// KP > 1 (complex, Arnoldi only): KP pairs of warps take a K piece of the tile each, and the
+// pieces are added in order.  At D <= 32 a tile's chain of multiply-adds is longer than
+// everything else (K = 96: 192 of them, 64 cycles each) while most sub-partitions are idle.
+// The sum's order differs from the other forms', so the Lanczos solve (whose eigenvector's sign
+// hangs on a last bit) and the plain GEMM keep to KP = 1.  Exponential of 20 vectors: D = 16
+// 689 -> 615 us, D = 22 790 -> 708, D = 32 923 -> 800, D = 8 574 -> 553; from D = 40 on the
+// pieces do not fit the idle sub-partitions.
+template <bool CPLX, int KP>
+__global__ void __launch_bounds__(32 * WWARPS * KP) gemm_warp(GemmArgs g, int splits, int kchunk,
+                                                              double* __restrict__ ws,
+                                                              int* __restrict__ tile_cnt) {
+  static_assert(KP == 1 || CPLX, "K pieces of complex tiles");
   chain_begin();
   constexpr int NP = CPLX ? 2 : 1;                       // planes
-  // the ring belongs to a warp (real) or to the two warps of a tile (complex): T threads
-  constexpr int T = CPLX ? 64 : 32, RINGS = CPLX ? 1 : WWARPS;
+  constexpr int WK = KP > 1 ? 16 : WK1, WST = KP > 1 ? 3 : WST1;
+  // the ring belongs to a warp (real) or to the two warps of a tile and piece (complex)
+  constexpr int T = CPLX ? 64 : 32, RINGS = CPLX ? KP : WWARPS;
   __shared__ double As[RINGS][WST][NP][WK][WM], Bs[RINGS][WST][NP][WK][WN];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int t = threadIdx.x % T, ring = CPLX ? 0 : wid;
+  const int lane = threadIdx.x & 31, wid = CPLX ? (threadIdx.x >> 5) & 1 : threadIdx.x >> 5;
+  const int piece = CPLX ? threadIdx.x >> 6 : 0;
+  const int t = threadIdx.x % T, ring = CPLX ? piece : wid;
   const int comp = CPLX ? wid : 0;                       // the part of C this warp forms
   const int mt = CPLX ? blockIdx.x : blockIdx.x * WWARPS + wid;
   const int m0 = mt * WM, n0 = blockIdx.y * WN;
   const int lm = lane & 7, ln = lane >> 3;
   const int gm = m0 + lm, gn = n0 + ln;
   const int zb = blockIdx.z / splits, sp = blockIdx.z % splits;
-  const int k_lo = sp * kchunk, k_hi = min(g.k, k_lo + kchunk);
+  const int kp = KP > 1 ? (g.k + KP - 1) / KP : 0;       // KP > 1: splits is 1
+  const int k_lo = KP > 1 ? min(g.k, piece * kp) : sp * kchunk;
+  const int k_hi = min(g.k, k_lo + (KP > 1 ? kp : kchunk));
   const int K = max(0, k_hi - k_lo), nslab = (K + WK - 1) / WK;
   const bool live = gm < g.m && gn < g.n;
   // This thread's elements of a slab: (mm, kk) of A, (kk, nn) of B, the first ones here and
@@ -305,7 +317,9 @@ __global__ void __launch_bounds__(32 * WWARPS) gemm_warp(GemmArgs g, int splits,
     asm volatile("cp.async.commit_group;" ::: "memory");   // one group per slab slot
   };
   auto ring_sync = [&]() {
-    if (CPLX) __syncthreads(); else __syncwarp();
+    if (KP > 1) asm volatile("bar.sync %0, 64;" ::"r"(1 + piece) : "memory");
+    else if (CPLX) __syncthreads();
+    else __syncwarp();
   };
   // real part: a b - ai bi; imaginary part: a bi + ai b; conj(op) flips the sign of ai, bi
   const bool conj_a = g.ta == 2 || g.ta == 3, conj_b = g.tb == 2 || g.tb == 3;
@@ -340,8 +354,20 @@ __global__ void __launch_bounds__(32 * WWARPS) gemm_warp(GemmArgs g, int splits,
   double* C = g.C + zb * g.strideC;
   const int64_t idx = (int64_t)gm + (int64_t)gn * g.ldc;
   const bool has_beta = g.beta[0] != 0.0 || g.beta[1] != 0.0;
-  __shared__ double part[32 * WWARPS];                   // complex: the other part's value
-  if (splits > 1) {
+  __shared__ double part[32 * WWARPS * KP];              // complex: the other part's value
+  if constexpr (KP > 1) {                                // the pieces' sums, in order
+    part[threadIdx.x] = acc;
+    __syncthreads();
+    if (piece > 0) return;
+#pragma unroll
+    for (int q = 1; q < KP; q++) acc += part[64 * q + threadIdx.x];
+    if (g.alpha[0] == 1.0 && g.alpha[1] == 0.0 && !has_beta) {
+      if (live) C[comp * g.planeC + idx] = acc;
+      return;
+    }
+    asm volatile("bar.sync 1, 64;" ::: "memory");        // part is written again
+  }
+  if (KP == 1 && splits > 1) {
     const int64_t mn = (int64_t)g.m * g.n, t = (int64_t)gm + (int64_t)gn * g.m;
     if (live) ws[(int64_t)sp * mn * (CPLX ? 2 : 1) + comp * mn + t] = acc;
     if (!tile_cnt) return;                               // the reduction kernel sums the splits
@@ -366,14 +392,14 @@ __global__ void __launch_bounds__(32 * WWARPS) gemm_warp(GemmArgs g, int splits,
   if (CPLX) {
     if (g.alpha[0] != 1.0 || g.alpha[1] != 0.0 || has_beta) {
       part[threadIdx.x] = acc;
-      __syncthreads();
+      if (KP > 1) asm volatile("bar.sync 1, 64;" ::: "memory"); else __syncthreads();
       const double sr = part[lane], si = part[32 + lane];
       double r = comp ? g.alpha[0] * si + g.alpha[1] * sr : g.alpha[0] * sr - g.alpha[1] * si;
       if (has_beta && live) {
         const double cr = C[idx], ci = C[g.planeC + idx];
         r += comp ? g.beta[0] * ci + g.beta[1] * cr : g.beta[0] * cr - g.beta[1] * ci;
       }
-      __syncthreads();                                   // both have read the old C
+      if (KP > 1) asm volatile("bar.sync 1, 64;" ::: "memory"); else __syncthreads();   // both have read the old C
       acc = r;
     }
     if (live) C[comp * g.planeC + idx] = acc;
@@ -485,8 +511,13 @@ int launch(fmpt_handle* h, const GemmArgs& g) {
     }
   }
   ProfScope prof(h, FMPT_K_F64_GEMM);
-  if (warp_tiles)
-    FMPT_CUDA(h, launch_chain(gemm_warp<CPLX>, grid, 32 * WWARPS, 0, h->stream, g, splits, kchunk,
+  // four K pieces per tile while the sub-partitions (four per SM) have room for them all
+  constexpr int KP = CPLX ? 4 : 1;
+  if (CPLX && warp_tiles && h->k_pieces && splits == 1 && g.k >= 16 && warps * KP <= 4LL * sms)
+    FMPT_CUDA(h, launch_chain(gemm_warp<CPLX, KP>, grid, 32 * WWARPS * KP, 0, h->stream, g, splits,
+                              kchunk, ws, cnt));
+  else if (warp_tiles)
+    FMPT_CUDA(h, launch_chain(gemm_warp<CPLX, 1>, grid, 32 * WWARPS, 0, h->stream, g, splits, kchunk,
                               ws, cnt));
   else
     FMPT_CUDA(h, launch_chain(gemm_kernel<CPLX, 64>, grid, NT, 0, h->stream, g, splits, kchunk, ws,

@@ -72,6 +72,8 @@ struct fmpt_handle {
   // set while fmpt_lanczos_ground runs: its tensor-core FP64 GEMMs are the digit products of
   // ozaki_digits.cu (see there), not the residue products of ozaki.cu
   int oz_digits = 0;
+  // 1 while an Arnoldi basis is built: small complex FP64 GEMMs may add K pieces (gemm_f64.cu)
+  int k_pieces = 0;
   // failure-detection test hook (fmpt_set_wait_test): bound of the grouped kernel's barrier
   // waits (0: 2 s) and extra arrivals they wait for (0 in normal use)
   int64_t wait_test_ns = 0;

@@ -1646,7 +1646,13 @@ int arnoldi_basis(fmpt_op* op, int cp, int64_t n, int64_t nr, int M, int ldh, do
                   double* z, DevBuf& Hdev, const GsWork& gs) {
   fmpt_handle* h = op->h;
   cudaStream_t st = h->stream;
+  struct KPieces {
+    fmpt_handle* h;
+    explicit KPieces(fmpt_handle* hh) : h(hh) { h->k_pieces = 1; }
+    ~KPieces() { h->k_pieces = 0; }
+  };
   auto record = [&]() -> int {
+    const KPieces pieces(h);
     h->cluster_sig = 0;
     FMPT_CUDA(h, cudaMemsetAsync(Hdev.p, 0, Hdev.bytes, st));
     if (gs.fused && !gs.cluster) FMPT_CUDA(h, cudaMemsetAsync(gs.bar, 0, 2 * sizeof(int), st));
