@@ -345,7 +345,6 @@ int fmpt_destroy(fmpt_handle* h) {
   for (auto st : h->aux_stream) cudaStreamDestroy(st);
   for (auto ev : h->aux_event) cudaEventDestroy(ev);
   if (h->lanczos_exec) cudaGraphExecDestroy(h->lanczos_exec);
-  for (auto& kv : h->arnoldi_exec) cudaGraphExecDestroy(kv.second);
   if (h->gemm_ws) cudaFree(h->gemm_ws);
   if (h->gemm_cnt) cudaFree(h->gemm_cnt);
   if (h->tc_ws) cudaFree(h->tc_ws);

@@ -85,11 +85,6 @@ struct fmpt_handle {
   void* oz_mx = nullptr;
   size_t oz_mx_bytes = 0;
   bool oz_mx_dirty = true;
-  // hash of the cluster sizes launched since it was last set to 0: part of the key below, since
-  // an executable graph's update may keep the old cluster size of a kernel node
-  uint32_t cluster_sig = 0;
-  // executable graphs of the captured Arnoldi basis, one per operator structure
-  std::map<std::string, cudaGraphExec_t> arnoldi_exec;
   cudaGraphExec_t lanczos_exec = nullptr;   // reused through cudaGraphExecUpdate
   uint64_t graph_launches = 0;
   // grouped-kernel tile autotuner (fmpt_set_tuning): 0 measure, 1 force the

@@ -1600,7 +1600,6 @@ int gs_step(fmpt_handle* h, const GsWork& w, int cp, int64_t n, int64_t nr, int 
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
     gs_cluster_config(h, w.G, cfg, attr);
-    h->cluster_sig = h->cluster_sig * 31 + w.G;
     FMPT_CUDA(h, cudaLaunchKernelEx(&cfg, arnoldi_gs_cluster, a));
     FMPT_LAUNCHED(h);
     return FMPT_OK;
@@ -1635,77 +1634,25 @@ int gs_step(fmpt_handle* h, const GsWork& w, int cp, int64_t n, int64_t nr, int 
 }
 
 // The Arnoldi basis V_1..V_M of fmpt_exponentiate / fmpt_expm_nodes (two-pass classical
-// Gram-Schmidt; the columns of H into Hdev), device launches only.  With graphs enabled the
-// launches are captured into one CUDA graph per operator structure and replayed: the
-// executable graph is updated in place (cudaGraphExecUpdate) for the next operator of the
-// same structure, so the host issues one launch per basis instead of about a dozen per
-// vector.  Any capture, instantiation, update or launch failure -- the first call on a
-// fresh operator among them, whose scratch is sized outside capture -- runs the same
-// launches directly.
+// Gram-Schmidt; the columns of H into Hdev), device launches only.  Launched one by one: a
+// vector's four or five kernels take the device 25 us and the host 10, while recording them into
+// a graph and updating its executable kept the device waiting (TDVP1 gradient of 8 sites, 116
+// bases: 109 ms recorded, 104 launched).
 int arnoldi_basis(fmpt_op* op, int cp, int64_t n, int64_t nr, int M, int ldh, double* V,
                   double* z, DevBuf& Hdev, const GsWork& gs) {
   fmpt_handle* h = op->h;
-  cudaStream_t st = h->stream;
   struct KPieces {
     fmpt_handle* h;
     explicit KPieces(fmpt_handle* hh) : h(hh) { h->k_pieces = 1; }
     ~KPieces() { h->k_pieces = 0; }
-  };
-  auto record = [&]() -> int {
-    const KPieces pieces(h);
-    h->cluster_sig = 0;
-    FMPT_CUDA(h, cudaMemsetAsync(Hdev.p, 0, Hdev.bytes, st));
-    if (gs.fused && !gs.cluster) FMPT_CUDA(h, cudaMemsetAsync(gs.bar, 0, 2 * sizeof(int), st));
-    for (int j = 0; j < M; j++) {
-      FMPT_TRY(fmpt_op_apply(op, V + (int64_t)j * nr, z));
-      FMPT_TRY(gs_step(h, gs, cp, n, nr, j, V, z, Hdev.d() + (size_t)2 * ldh * j));
-    }
-    return FMPT_OK;
-  };
-  cudaStreamCaptureStatus cap0 = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cap0) != cudaSuccess) {
-    cudaGetLastError();
-    return record();
+  } pieces(h);
+  FMPT_CUDA(h, cudaMemsetAsync(Hdev.p, 0, Hdev.bytes, h->stream));
+  if (gs.fused && !gs.cluster)
+    FMPT_CUDA(h, cudaMemsetAsync(gs.bar, 0, 2 * sizeof(int), h->stream));
+  for (int j = 0; j < M; j++) {
+    FMPT_TRY(fmpt_op_apply(op, V + (int64_t)j * nr, z));
+    FMPT_TRY(gs_step(h, gs, cp, n, nr, j, V, z, Hdev.d() + (size_t)2 * ldh * j));
   }
-  if (!h->graphs || cap0 != cudaStreamCaptureStatusNone) return record();
-  if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-    cudaGetLastError();
-    return record();
-  }
-  const int rs = record();
-  cudaGraph_t graph = nullptr;
-  const cudaError_t ce = cudaStreamEndCapture(st, &graph);
-  if (rs != FMPT_OK || ce != cudaSuccess || !graph) {
-    if (graph) cudaGraphDestroy(graph);
-    cudaGetLastError();
-    return record();
-  }
-  char key[112];
-  std::snprintf(key, sizeof(key), "k%d p%d c%d u%d q%zu M%d g%d s%x", op->kind, op->precision, cp,
-                op->u1 ? 1 : 0, op->proj.size(), M, gs.cluster ? 2 : (gs.fused ? 1 : 0),
-                (unsigned)h->cluster_sig);
-  cudaGraphExec_t& ex = h->arnoldi_exec[key];
-  bool ready = false;
-  if (ex) {
-    cudaGraphExecUpdateResultInfo ri;
-    if (cudaGraphExecUpdate(ex, graph, &ri) == cudaSuccess) {
-      ready = true;
-    } else {
-      cudaGetLastError();
-      cudaGraphExecDestroy(ex);
-      ex = nullptr;
-    }
-  }
-  if (!ready && cudaGraphInstantiate(&ex, graph, 0) != cudaSuccess) {
-    cudaGetLastError();
-    ex = nullptr;
-  }
-  cudaGraphDestroy(graph);
-  if (!ex || cudaGraphLaunch(ex, st) != cudaSuccess) {
-    cudaGetLastError();
-    return record();
-  }
-  h->graph_launches++;
   return FMPT_OK;
 }
 

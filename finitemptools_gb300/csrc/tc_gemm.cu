@@ -870,7 +870,6 @@ static int tc_gemm_small(fmpt_handle* h, int M, int N, int K, int batch, int S, 
   if (fits[vi][S] < 0) return FMPT_ERR_UNSUPPORTED;
   chain_attr(attr[cfg.numAttrs++]);
   ProfScope prof(h, FMPT_K_TC_GEMM);
-  h->cluster_sig = h->cluster_sig * 31 + S;
   FMPT_CUDA(h, cudaLaunchKernelEx(&cfg, kfn, ma, mb, ma2, mb2, K, tiles_m, tiles_n, S, ep));
   FMPT_LAUNCHED(h);
   return FMPT_OK;
@@ -1013,7 +1012,6 @@ static int tc_gemm_pair_st(fmpt_handle* h, int M, int N, int K, int batch, const
   cfg.gridDim = dim3((unsigned)(2 * std::min<int64_t>(items, cl)));
   chain_attr(attr[cfg.numAttrs++]);
   ProfScope prof(h, FMPT_K_TC_GEMM);
-  h->cluster_sig = h->cluster_sig * 31 + 2;
   FMPT_CUDA(h, cudaLaunchKernelEx(&cfg, kfn, ma, mb, ma2, mb2, K, tiles_m2, tiles_n, batch, ep, sp));
   FMPT_LAUNCHED(h);
   return FMPT_OK;

@@ -1,7 +1,8 @@
-"""Exponentials whose recorded launches differ only in their cluster sizes, on one handle: the
-executable graph of one operator must not be updated into that of another.  Orthogonalisation
-clusters of 1, 4, 8 and 16 blocks and tensor-core GEMMs with 1 to 4 K pieces per cluster take
-turns; with graphs every result is the one without, bit for bit (the same launches)."""
+"""Exponentials whose launches differ in their cluster sizes take turns on one handle:
+orthogonalisation clusters of 1, 4, 8 and 16 blocks and tensor-core GEMMs with 1 to 4 K pieces per
+cluster.  Whatever ran before, and with graphs allowed or not, every result is the first one, bit
+for bit (the same launches).  An executable graph that is updated from one operator to the next
+keeps the old cluster sizes, without an error."""
 
 import numpy as np
 import pytest
