@@ -53,7 +53,12 @@ NCU_TRAFFIC = {("bf16", 2048): {"bytes_per_launch": (88.77e6 + 134.09e6 + 334.29
                                 "algorithmic_operand_bytes": {"gemm1": 76.0e6, "gemm2": 210.0e6}}}
 UNIT = "TFLOP/s"
 W_MPO, D_PHYS = 5, 2
-OZ_PRODUCTS = 16          # BF16 residue products per FP64 multiply-add of the fp64_tc GEMM
+
+
+def oz_products(D, w=W_MPO):
+    """BF16 residue products per FP64 multiply-add of the fp64_tc H_eff*x: 15 moduli up to an inner
+    extent of 2048, 16 beyond; the mean over its two GEMMs (inner extents D and w D)."""
+    return sum(15 if k <= 2048 else 16 for k in (D, w * D)) / 2
 
 
 def flops_ac2(D, w=W_MPO, d=D_PHYS):
@@ -1063,10 +1068,10 @@ def main():
     if prec == "bf16":
         peak, peak_note = peaks.get("bf16_tflops", 1900.0), "bf16_tflops (burst) of measured"
     elif prec == "fp64_tc":
-        # the FP64-accurate GEMM forms 16 BF16 residue products per FP64 multiply-add (K > 1758):
-        # the FP64 rate it can reach is the measured BF16 peak / 16
-        peak = peaks.get("bf16_tflops", 1900.0) / OZ_PRODUCTS
-        peak_note = "bf16_tflops (burst) of measured / %d residue products" % OZ_PRODUCTS
+        # the FP64-accurate GEMMs form 15 or 16 BF16 residue products per FP64 multiply-add: the
+        # FP64 rate they can reach is the measured BF16 peak over that
+        peak = peaks.get("bf16_tflops", 1900.0) / oz_products(D)
+        peak_note = "bf16_tflops (burst) of measured / %.1f residue products" % oz_products(D)
     elif prec in ("tf32", "tf32x3"):
         peak = peaks.get("bf16_tflops", 1900.0) / 2
         peak_note = "half of measured bf16_tflops (dense TF32 rate is half of BF16)"
@@ -1089,7 +1094,7 @@ def main():
                 "other_kernels_ms_per_step": {"mpo_step": mid_ms / args.steps,
                                               "convert": cv_ms / args.steps}}
         if prec == "fp64_tc":
-            roof["bf16_mma_tflops"] = achieved * OZ_PRODUCTS
+            roof["bf16_mma_tflops"] = achieved * oz_products(D)
             roof["unit_note"] = ("achieved: algorithmic FP64 flops (2 w d^2 D^3 per launch) per "
                                  "second; bf16_mma_tflops: the residue-product MMA work per second")
         if prec == "bf16" and rank == 0:

@@ -24,13 +24,14 @@
 //
 // The products and sums are exact, so the error is that of step 1 (2^-54 of the row or
 // column maximum per entry, or less) and one rounding.  t follows from K: with 15 moduli
-// (P = 2^117.8) t >= 53 up to K = 1758, with 16 (2^125.4) t = 56 at K = 2048 and 55 at
+// (P = 2^118.0) t >= 53 up to K = 2048, with 16 (2^125.6) t = 56 up to K = 6295 and 55 at
 // K = 10240; more moduli are not needed, fewer do not hold two 53-bit factors.  That is 15
 // or 16 BF16 multiply-adds per FP64 one, against 45 of the digit products (ozaki_digits.cu):
-// a two-site H_eff*x at w = 5 takes 8.5 ms at D = 2048 (17.6 ms there), 0.16 ms at D = 256
-// (0.25), with error 2e-15 against 64-bit references (8e-14: the digit form drops the
-// products below 2^-60 of the row and column maxima).  The GEMM runs 1.75 PFLOP/s of BF16
-// work at D = 2048, 0.99 of the sustained cuBLAS rate.
+// a two-site H_eff*x at w = 5 takes 7.8 ms at D = 2048 (17.6 ms there), 0.076 ms at D = 256
+// (0.25).  Error of a product of random matrices relative to its norm, against 113-bit
+// references: 2.6e-16 at K = 2048 (15 moduli), 5e-17 at K = 5120 (16); of the digit form, which
+// drops the products below 2^-60 of the row and column maxima, 1.2e-15 and 1.9e-15.  The GEMM
+// runs 1.75 PFLOP/s of BF16 work at D = 2048, 0.99 of the sustained cuBLAS rate.
 // Complex operands use the real embedding [Re -Im; Im Re] x [Re; Im].
 //
 // Kernels: oz_rowmax* / oz_residues* (FP64 operand -> row exponents and NMOD K-major BF16
@@ -58,13 +59,14 @@ constexpr int EPI_WARPS = 8;
 constexpr int NTHR = 64 + 32 * EPI_WARPS;   // producer, MMA issuer, epilogue warps
 
 // ------------------------------------------------------------ moduli and their constants
+// the 15 and 16 pairwise coprime numbers up to 256 of the largest product (a search over all)
 __host__ __device__ constexpr int modulus(int i) {
-  constexpr int p[MAXMOD] = {256, 255, 253, 251, 247, 241, 239, 233,
-                             229, 227, 223, 217, 211, 199, 197, 193};
+  constexpr int p[MAXMOD] = {256, 253, 251, 249, 247, 241, 239, 235,
+                             233, 229, 227, 223, 217, 211, 199, 197};
   return p[i];
 }
 // log2 of the product of the first n moduli, rounded down to 1/100
-constexpr double log2_product(int n) { return n == 15 ? 117.78 : 125.37; }
+constexpr double log2_product(int n) { return n == 15 ? 118.00 : 125.62; }
 
 // 2^e mod p, balanced
 __host__ __device__ constexpr int pow2_mod(int e, int p) {
@@ -591,8 +593,9 @@ struct CrtArgs {
 // The sums of the residues times the six 16-bit limbs of the weights, two moduli per instruction
 // (dp2a): 48 instructions per value where 32-bit words take 16 multiply-adds and 32 wide ones
 // at half their rate.  The integer pipes bound this kernel (151 instructions per value, 194
-// before; D = 1024, 15 moduli: 158 -> 119 us, 74 at the copy bandwidth).  Four columns at a time, so that a weight is put into a register
-// once for four values.  c[j][q]: residues of moduli 4 q .. 4 q + 3 in column j.
+// before; D = 1024, 15 moduli: 158 -> 119 us, 74 at the copy bandwidth).  Four columns at a
+// time, so that a weight is put into a register once for four values.  c[j][q]: residues of
+// moduli 4 q .. 4 q + 3 in column j.
 template <int NMOD>
 __device__ __forceinline__ void crt_limbs(const uint32_t (&c)[4][4], uint32_t (&L)[4][6]) {
   constexpr Crt<NMOD> T = make_crt<NMOD>();
