@@ -1467,12 +1467,12 @@ struct GsWork {
   int hold;
 };
 
-// Blocks of the step and chunks per block for S chunks: one block, without grid-wide waits,
-// up to 4 chunks; one cluster of 4, 8 or 16 blocks up to GS_CLUSTER_S chunks (complex exponential
-// of 20 vectors, cooperative -> cluster: D = 8 649 -> 592 us, D = 16 754 -> 706, D = 22, the
-// last one, 832 -> 810; D = 27 would take 978 instead of 904: 16 SMs are too few for it); then as few chunks
-// per block as keep it within 128 blocks (n = 8192 complex: 4 chunks, one per SM sub-partition);
-// beyond 1024 chunks the warps loop.
+// Blocks of the step and chunks per block for S chunks: one block, without grid-wide waits, up
+// to 4 chunks; one cluster of 4, 8 or 16 blocks up to GS_CLUSTER_S chunks (complex exponential of
+// 20 vectors, cooperative -> cluster: D = 8 649 -> 592 us, D = 16 754 -> 706, D = 22, the last
+// one, 832 -> 810; D = 27 would take 978 instead of 904: 16 SMs are too few for it); then as few
+// chunks per block as keep it within 128 blocks (n = 8192 complex: 4 chunks, one per SM
+// sub-partition); beyond 1024 chunks the warps loop.
 constexpr int GS_CLUSTER_S = 64;
 void gs_geometry(int64_t S, int& G, int& cpb, bool& single) {
   single = true;

@@ -2,7 +2,7 @@
 // the operator applications inside fmpt_lanczos_ground.
 //
 // Everything else runs the residue form (ozaki.cu), which needs 16 BF16 products per FP64
-// one instead of 45 (D = 2048 two-site H_eff*x: 17.6 ms here, 8.5 ms there).  The Lanczos
+// one instead of 45 (D = 2048 two-site H_eff*x: 17.6 ms here, 7.8 ms there).  The Lanczos
 // solve keeps this one because its result's sign hangs on the last bit of the Ritz value:
 // the inverse iteration for the eigenvector runs at one of the two doubles that enclose the
 // eigenvalue, and which one is the parity of a mantissa.  Another rounding of the operator,

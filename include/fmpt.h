@@ -98,8 +98,9 @@ int fmpt_set_graphs(fmpt_handle* h, int on);
 uint64_t fmpt_graph_launch_count(fmpt_handle* h);
 /* Krylov exponentials (fmpt_exponentiate, fmpt_expm_nodes): on (default), each
  * Arnoldi vector's two-pass Gram-Schmidt orthogonalisation and normalisation
- * run as ONE cooperative launch with bounded grid barriers instead of six
- * launches; off, the six launches.  Both give bit-identical results.  No
+ * run as ONE launch instead of six: a cluster of up to 16 blocks for short
+ * vectors, a cooperative grid with bounded barriers otherwise; off, the six
+ * launches.  Both give bit-identical results.  No
  * counterpart in the reference. */
 int fmpt_set_fused_krylov(fmpt_handle* h, int on);
 /* Thin QR (fmpt_qr, fmpt_lq, leftorth!/rightorth) of small tall panels: on
