@@ -542,7 +542,7 @@ int op_fp64_head(fmpt_op* op, const double* x) {
   const int64_t n1 = (int64_t)Dl * wl * P * Dr, n3 = (int64_t)Dl * P * wr * Dr;
   // T1 and T3 in the operator's scratch (one buffer, T3 after T1)
   // and, where GEMM 2 takes them, the row maxima of T3
-  const bool maxima = !op->sched.sp_start.empty() &&
+  const bool maxima = !op->sched.sp_start.empty() && Dr <= 8 * 65535 &&
                       gemm_f64_ozaki_takes_maxima(h, tail_gemm(op, nullptr));
   const size_t mxb = maxima ? (size_t)Dl * P * (cp ? 2 : 1) * sizeof(uint64_t) : 0;
   const size_t held = op->scratch_bytes;
@@ -665,6 +665,14 @@ int fmpt_op_apply(fmpt_op* op, const double* x, double* y) {
   }
   return op_project(op, y);
 }
+
+}  // extern "C"
+int fmpt::op_apply_planes(fmpt_op* op, double* y) {
+  FMPT_TRY(op_tc_apply_head(op, nullptr));
+  FMPT_TRY(op_tc_apply_tail(op, y));
+  return op_project(op, y);
+}
+extern "C" {
 
 int64_t fmpt_op_size(fmpt_op* op) { return op ? op->n : -1; }
 

@@ -441,7 +441,13 @@ int op_tc_apply(fmpt_op* op, const double* x, double* y);
 // split application of a real tensor-core two-site operator (host-buffer pipeline):
 // head = x conversion, GEMM 1 and MPO step; tail = GEMM 2; prepare_right converts the
 // right environment of an operator created with defer_right
+// (x null: its operand planes, op_tc_planes, have been written already)
 int op_tc_apply_head(fmpt_op* op, const double* x);
+// where a real tensor-core operator keeps the operand planes of x: element i of x at element i of
+// hi (and, for 3xTF32, lo); mode < 0 where the layout is another one
+struct TcPlanes { int mode = -1; void* hi = nullptr; void* lo = nullptr; };
+TcPlanes op_tc_planes(fmpt_op* op);
+int op_apply_planes(fmpt_op* op, double* y);   // fmpt_op_apply on those planes
 int op_tc_apply_tail(fmpt_op* op, double* y);
 int op_tc_prepare_right(fmpt_op* op);
 // the same for the rows b' in [r0, r1) of the right environment / columns of y

@@ -19,46 +19,15 @@
 #include <algorithm>
 #include <cstring>
 
-#include "internal.h"
+#include "tc_planes.cuh"
 
 namespace fmpt {
 
 namespace {
 
-enum { M_TF32 = 0, M_TF32X3 = 1, M_BF16 = 2 };
 
 int tc_mode_of(int precision) {
   return precision == FMPT_PREC_TF32 ? M_TF32 : precision == FMPT_PREC_TF32X3 ? M_TF32X3 : M_BF16;
-}
-
-__device__ __forceinline__ float tf32_rna(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return __uint_as_float(r);
-}
-
-// write one converted value: TF32 (hi, optional lo) or BF16
-template <int MODE>
-__device__ __forceinline__ void put(void* hi, void* lo, int64_t i, double v) {
-  if (MODE == M_BF16) {
-    static_cast<__nv_bfloat16*>(hi)[i] = __float2bfloat16_rn(narrow(v));
-  } else {
-    const float h = tf32_rna(narrow(v));
-    static_cast<float*>(hi)[i] = h;
-    if (MODE == M_TF32X3) static_cast<float*>(lo)[i] = tf32_rna(narrow(v - widen(h)));
-  }
-}
-// the same of an FP32 value: v - h is exact in FP32 (a multiple of v's last place, below 2^13 of
-// them), so no FP64 is needed
-template <int MODE>
-__device__ __forceinline__ void put(void* hi, void* lo, int64_t i, float v) {
-  if (MODE == M_BF16) {
-    static_cast<__nv_bfloat16*>(hi)[i] = __float2bfloat16_rn(v);
-  } else {
-    const float h = tf32_rna(v);
-    static_cast<float*>(hi)[i] = h;
-    if (MODE == M_TF32X3) static_cast<float*>(lo)[i] = tf32_rna(v - h);
-  }
 }
 
 // xg[a + dld*m] = x[a + Dl*m] for a < Kp (zero for a >= Dl); dld >= Kp is the row
@@ -522,6 +491,12 @@ int op_tc_apply(fmpt_op* op, const double* x, double* y) {
   return op_tc_apply_tail(op, y);
 }
 
+TcPlanes op_tc_planes(fmpt_op* op) {
+  TcState* st = static_cast<TcState*>(op->tc);
+  if (!st || st->cplx || st->Kp != op->Dl) return TcPlanes{};
+  return TcPlanes{st->mode, st->xg[0].p, st->mode == M_TF32X3 ? st->xg[1].p : nullptr};
+}
+
 // The part of a real two-site application that needs x and the left environment
 // only: x conversion, GEMM 1 and the MPO step (T3 is left in the operator).
 int op_tc_apply_head(fmpt_op* op, const double* x) {
@@ -533,7 +508,7 @@ int op_tc_apply_head(fmpt_op* op, const double* x) {
   void* xlo = split > 1 ? st->xg[1].p : nullptr;
   void* tlo = split > 1 ? st->T3[1].p : nullptr;
   const int64_t nx = (int64_t)st->Kp * P * Dr;
-  {
+  if (x) {                                   // else op_tc_planes' owner has written the planes
   ProfScope prof(h, FMPT_K_CONVERT);
   const bool ident = st->Kp == Dl && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
   if (ident) {
