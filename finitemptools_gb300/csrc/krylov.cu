@@ -194,9 +194,11 @@ __global__ void lanczos_scale(int64_t n, const double* __restrict__ y,
     ab[0] = *alpha;
     ab[1] = b;
   }
-  // Julia's qi /= b divides element-wise; so does this (no reciprocal)
+  // Julia's qi /= b divides element-wise; so does this (no reciprocal).  b >= 0 or NaN; the test
+  // is on its words, an FP64 comparison otherwise.
+  const bool zero = (__double2hiint(b) | __double2loint(b)) == 0;
   for (int64_t i = (int64_t)blockIdx.x * KT + threadIdx.x; i < n; i += (int64_t)gridDim.x * KT) {
-    const double v = b == 0.0 ? y[i] : y[i] / b;
+    const double v = zero ? y[i] : y[i] / b;
     vnext[i] = v;
     if constexpr (MODE >= 0) put<MODE>(hi, lo, i, v);
   }
