@@ -63,8 +63,8 @@ class Handle:
         self.check(lib().fmpt_set_graphs(self.ptr, 1 if on else 0))
 
     def set_fused_krylov(self, on=True):
-        """One cooperative launch per Arnoldi orthogonalisation step of the Krylov
-        exponentials (default on); off: six launches, bit-identical results."""
+        """One launch per Arnoldi orthogonalisation step of the Krylov exponentials
+        (default on); off: six launches, bit-identical results."""
         self.check(lib().fmpt_set_fused_krylov(self.ptr, 1 if on else 0))
 
     def set_cluster_qr(self, on=True):
