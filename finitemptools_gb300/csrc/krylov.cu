@@ -1705,12 +1705,10 @@ int fmpt_op_set_projectors(fmpt_op* op, int nproj, const double* const* p) {
   return FMPT_OK;
 }
 
-int fmpt_lanczos_ground(fmpt_op* op, const double* x0, int kmax, double btol, int reorth,
-                        double* eigval, double* xout, int* info, int* niter) {
-  if (!op) return FMPT_ERR_ARG;
+// fmpt_lanczos_ground, its last launches (among them the one that writes xout) still queued
+static int lanczos_ground(fmpt_op* op, const double* x0, int kmax, double btol, int reorth,
+                          double* eigval, double* xout, int* info, int* niter) {
   fmpt_handle* h = op->h;
-  if (!x0 || !xout || !eigval) return set_error(h, FMPT_ERR_ARG, "lanczos: null pointer");
-  if (kmax < 1 || kmax > 128) return set_error(h, FMPT_ERR_ARG, "lanczos: kmax must be 1..128");
   // the solve's tensor-core FP64 GEMMs are the digit products (ozaki_digits.cu says why)
   struct DigitEngine {
     fmpt_handle* h;
@@ -1814,6 +1812,21 @@ int fmpt_lanczos_ground(fmpt_op* op, const double* x0, int kmax, double btol, in
   if (op->u1) FMPT_TRY(gp_check_status(op->h));
   if (info) *info = converged ? 0 : -1;
   if (niter) *niter = k;
+  return FMPT_OK;
+}
+
+int fmpt_lanczos_ground(fmpt_op* op, const double* x0, int kmax, double btol, int reorth,
+                        double* eigval, double* xout, int* info, int* niter) {
+  if (!op) return FMPT_ERR_ARG;
+  fmpt_handle* h = op->h;
+  if (!x0 || !xout || !eigval) return set_error(h, FMPT_ERR_ARG, "lanczos: null pointer");
+  if (kmax < 1 || kmax > 128) return set_error(h, FMPT_ERR_ARG, "lanczos: kmax must be 1..128");
+  const int st = lanczos_ground(op, x0, kmax, btol, reorth, eigval, xout, info, niter);
+  // A call that returns host scalars synchronises: xout may be read on any stream, and nothing
+  // that is still queued (a step thrown away, after an error too) reads the caller's data.
+  const cudaError_t e = cudaStreamSynchronize(h->stream);
+  if (st != FMPT_OK) return st;
+  FMPT_CUDA(h, e);
   return FMPT_OK;
 }
 
