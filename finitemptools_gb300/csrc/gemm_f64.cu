@@ -33,6 +33,7 @@ __global__ void __launch_bounds__(NT) gemm_kernel(GemmArgs g, int splits, int kc
                                                   double* __restrict__ ws,
                                                   int* __restrict__ tile_cnt) {
   chain_begin();
+  if (g.gate && *g.gate) return;
   constexpr int TPR = BMN / 16;                // outputs per thread along each dimension
   __shared__ double As[2][BK][BMN + 1];
   __shared__ double Bs[2][BK][BMN + 1];
@@ -261,6 +262,7 @@ __global__ void __launch_bounds__(32 * WWARPS * KP) gemm_warp(GemmArgs g, int sp
                                                               int* __restrict__ tile_cnt) {
   static_assert(KP == 1 || CPLX, "K pieces of complex tiles");
   chain_begin();
+  if (g.gate && *g.gate) return;
   constexpr int NP = CPLX ? 2 : 1;                       // planes
   constexpr int WK = KP > 1 ? 16 : WK1, WST = KP > 1 ? 3 : WST1;
   // the ring belongs to a warp (real) or to the two warps of a tile and piece (complex)
@@ -413,6 +415,7 @@ __global__ void __launch_bounds__(32 * WWARPS * KP) gemm_warp(GemmArgs g, int sp
 // C = alpha * sum_{s < splits} W_s + beta * C, summed in split order
 template <bool CPLX>
 __global__ void split_reduce(GemmArgs g, int splits, const double* __restrict__ ws) {
+  if (g.gate && *g.gate) return;
   const int64_t mn = (int64_t)g.m * g.n;
   const bool has_beta = (g.beta[0] != 0.0 || g.beta[1] != 0.0);
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < mn;
@@ -546,7 +549,9 @@ int gemm_f64(fmpt_handle* h, const GemmArgs& g) {
     // to grow inside a stream capture); the CUDA-core kernel runs instead
     if (st != FMPT_ERR_UNSUPPORTED) return st;
   }
-  return g.cplx ? launch<true>(h, g) : launch<false>(h, g);
+  GemmArgs gated = g;
+  gated.gate = h->gate;
+  return g.cplx ? launch<true>(h, gated) : launch<false>(h, gated);
 }
 
 }  // namespace fmpt

@@ -657,20 +657,20 @@ int fmpt_op_apply(fmpt_op* op, const double* x, double* y) {
   if (!op) return FMPT_ERR_ARG;
   if (!x || !y) return set_error(op->h, FMPT_ERR_ARG, "op_apply: null vector");
   if (op->u1) {
-    FMPT_TRY(op_u1_apply(op, x, y));
+    FMPT_TRY(op_u1_apply(op, x, y, op->h->gate));
   } else if (!prec_is_f64(op->precision)) {
     FMPT_TRY(op_tc_apply(op, x, y));
   } else {
     FMPT_TRY(op_apply_fp64(op, x, y));
   }
-  return op_project(op, y);
+  return op_project(op, y, op->h->gate);
 }
 
 }  // extern "C"
 int fmpt::op_apply_planes(fmpt_op* op, double* y) {
   FMPT_TRY(op_tc_apply_head(op, nullptr));
   FMPT_TRY(op_tc_apply_tail(op, y));
-  return op_project(op, y);
+  return op_project(op, y, op->h->gate);
 }
 extern "C" {
 

@@ -72,6 +72,9 @@ struct fmpt_handle {
   // set while fmpt_lanczos_ground runs: its tensor-core FP64 GEMMs are the digit products of
   // ozaki_digits.cu (see there), not the residue products of ozaki.cu
   int oz_digits = 0;
+  // device flag of the Lanczos solve that is running, set while it queues a step ahead of its
+  // stopping test: nonzero once the solve has stopped, and that step's GEMMs return at once
+  const int* gate = nullptr;
   // 1 while an Arnoldi basis is built: small complex FP64 GEMMs may add K pieces (gemm_f64.cu)
   int k_pieces = 0;
   // failure-detection test hook (fmpt_set_wait_test): bound of the grouped kernel's barrier
@@ -133,6 +136,13 @@ int set_error(fmpt_handle* h, int status, const char* fmt, ...);
 // with plain launches and 11.3 with these.
 #ifdef __CUDACC__
 __device__ __forceinline__ void chain_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The first statement of a kernel with a gate (fmpt_handle::gate): nothing is to be done.  Uniform
+// for the whole grid, since an earlier kernel sets the flag.
+__device__ __forceinline__ bool gate_closed(const int* gate) {
+  if (!gate) return false;
+  chain_begin();
+  return *gate != 0;
+}
 
 // Conversions between FP32 and FP64 on the integer pipe: a conversion instruction runs on the
 // FP64 pipe of GB300, 64 cycles of its SM sub-partition, and the epilogues and layout kernels
@@ -269,6 +279,7 @@ struct GemmArgs {
   // by the kernel that wrote A; the residue GEMM zeroes them after use and then sets *maxA_clean
   unsigned long long* maxA;
   bool* maxA_clean;
+  const int* gate;          // the handle's (filled in by gemm_f64)
 };
 int gemm_f64(fmpt_handle* h, const GemmArgs& g);
 // the Ozaki-scheme FP64 GEMM on the BF16 tensor cores (ozaki.cu): whether it applies to g

@@ -179,20 +179,22 @@ __global__ void lanczos_axpy(int64_t n, double* __restrict__ y, const double* __
 }
 
 // b = sqrt(sum(part_b)); beta_out = b; vnext = y / b (y itself if b is 0); alpha and b also
-// go to pinned host memory, ab[0] and ab[1].  MODE >= 0: vnext also goes, rounded, to the operand
+// go to pinned host memory, ab[0] and ab[1], and stop (if given) is raised where the host's test
+// of b ends the solve.  MODE >= 0: vnext also goes, rounded, to the operand
 // planes of the tensor-core operator that is applied to it next, which saves that operator's
 // conversion pass (5.7 us of a step at D = 256).
 template <int MODE>
 __global__ void lanczos_scale(int64_t n, const double* __restrict__ y,
                               const double* __restrict__ part_b, int G, const double* alpha,
-                              double* beta_out, double* __restrict__ vnext, double* ab, void* hi,
-                              void* lo) {
+                              double* beta_out, double* __restrict__ vnext, double* ab,
+                              double btol, int* stop, void* hi, void* lo) {
   chain_begin();
   const double b = sum_parts(part_b, G, true);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *beta_out = b;
     ab[0] = *alpha;
     ab[1] = b;
+    if (stop && (!(b >= btol) || isinf(b))) *stop = 1;
   }
   // Julia's qi /= b divides element-wise; so does this (no reciprocal).  b >= 0 or NaN; the test
   // is on its words, an FP64 comparison otherwise.
@@ -1726,7 +1728,7 @@ static int lanczos_ground(fmpt_op* op, const double* x0, int kmax, double btol, 
   DevBuf Vb, Yb, scal, partA, partB, partM, coef;
   FMPT_TRY(Vb.alloc(h, (size_t)(kmax + 1) * n * sizeof(double)));
   FMPT_TRY(Yb.alloc(h, (size_t)n * sizeof(double)));
-  FMPT_TRY(scal.alloc(h, (size_t)(2 * kmax + 1) * sizeof(double)));   // vm, alpha, beta
+  FMPT_TRY(scal.alloc(h, (size_t)(2 * kmax + 2) * sizeof(double)));   // vm, alpha, beta, stop
   FMPT_TRY(partA.alloc(h, (size_t)G * sizeof(double)));
   FMPT_TRY(partB.alloc(h, (size_t)G * sizeof(double)));
   FMPT_TRY(partM.alloc(h, (size_t)G * (kmax + 1) * 2 * sizeof(double)));
@@ -1753,13 +1755,34 @@ static int lanczos_ground(fmpt_op* op, const double* x0, int kmax, double btol, 
     return FMPT_OK;
   };
 
+  // Step j + 1 is queued before beta_j is looked at, so that the device does not wait for the
+  // host's test (10 us per step); one step past convergence is thrown away.  Where its GEMMs
+  // take more than about 50 us they look at a flag that the step before raises, and do nothing
+  // (a solve that ends with its first step: FP64 D = 256 195 -> 127 us, D = 512 1005 -> 551;
+  // the looks are 1% of a D = 128 step); below, the step is cheaper than the looks.
+  double flops = 0.0;
+  FMPT_TRY(fmpt_op_flops(op, &flops));
+  int* stop = nullptr;
+  if (flops > 50e-6 * (prec_is_f64(op->precision) ? 1.1e12 : 1e14)) {
+    stop = reinterpret_cast<int*>(s_beta + kmax);
+    FMPT_CUDA(h, cudaMemsetAsync(stop, 0, sizeof(int), h->stream));
+  }
+  struct Gate {
+    fmpt_handle* h;
+    Gate(fmpt_handle* hh, const int* g) : h(hh) { h->gate = g; }
+    ~Gate() { h->gate = nullptr; }
+  };
+
   // step j: lanczos_make_first_step / lanczos_make_step (simple_lanczos.jl:27-68), from V_j
   // to alpha_j, beta_j and V_{j+1}; alpha_j and beta_j are in step_host[2 j], [2 j + 1] once
   // step_event[j & 1] has passed
   double* ab = h->step_host;
   const TcPlanes px = op_tc_planes(op);        // V_1, V_2, .. are written there as well
   auto launch_step = [&](int j) -> int {
-    FMPT_TRY(j > 0 && px.mode >= 0 ? op_apply_planes(op, y) : fmpt_op_apply(op, V_(j), y));
+    {
+      Gate closed(h, j > 0 ? stop : nullptr);
+      FMPT_TRY(j > 0 && px.mode >= 0 ? op_apply_planes(op, y) : fmpt_op_apply(op, V_(j), y));
+    }
     CHAIN(rdot_partial, G, h->stream, n, V_(j), y, partA.d(), nullptr);
     FMPT_LAUNCHED(h);
     CHAIN(lanczos_axpy, G, h->stream, n, y, V_(j), j ? V_(j - 1) : nullptr, partA.d(), G,
@@ -1771,7 +1794,7 @@ static int lanczos_ground(fmpt_op* op, const double* x0, int kmax, double btol, 
                  : px.mode == M_BF16   ? lanczos_scale<M_BF16>
                                        : lanczos_scale<-1>;
     CHAIN(scale, G, h->stream, n, y, partB.d(), G, s_alpha + j, s_beta + j, V_(j + 1), ab + 2 * j,
-          px.hi, px.lo);
+          btol, stop, px.hi, px.lo);
     FMPT_LAUNCHED(h);
     FMPT_CUDA(h, cudaEventRecord(h->step_event[j & 1], h->stream));
     return FMPT_OK;
@@ -1780,8 +1803,6 @@ static int lanczos_ground(fmpt_op* op, const double* x0, int kmax, double btol, 
   FMPT_LAUNCHED(h);
   CHAIN(normalize_from_parts, G, h->stream, n, x0, V_(0), partA.d(), G, s_vm);
   FMPT_LAUNCHED(h);
-  // Step j + 1 is queued before beta_j is looked at, so the device does not wait for the
-  // host's test (25 us per step at D = 64); one step past convergence is thrown away.
   double al[128], be[128];
   int k = 0;
   bool converged = false;

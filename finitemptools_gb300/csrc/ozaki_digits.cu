@@ -322,6 +322,7 @@ struct OzEpi {
   int nfast;
   int split;            // pieces per tile: S level sets x Q chunk ranges (1: direct)
   int var, S, Q;        // level-set variant (kOrder / kSetStart), S = its piece count
+  const int* gate;      // fmpt_handle::gate
 };
 
 // K slices (of KELEMS) per exactness chunk of a level: the longest run of K over which the
@@ -465,6 +466,7 @@ __device__ __forceinline__ void drain(uint32_t tbase, int row, int rloc, int n0,
 __global__ void __launch_bounds__(NTHREADS, 1)
     ozd_gemm_pair(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                  int K, int tiles_m2, int tiles_n, int batch, OzEpi ep) {
+  if (gate_closed(ep.gate)) return;
   constexpr int A_BYTES = BM * 128, B_BYTES = 128 * 128;
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr int TMEM_COLS = 256;
@@ -691,6 +693,7 @@ struct RedArgs {
   int64_t ldc, strideC, planeC;
   int m, n, batch, cplx, split, S, tiles_m2, tiles_n, nfast;
   double alpha[2], beta[2];
+  const int* gate;
 };
 
 __device__ __forceinline__ double ws_sum(const RedArgs& a, int z, int r, int c) {
@@ -712,6 +715,7 @@ __device__ __forceinline__ double ws_sum(const RedArgs& a, int z, int r, int c) 
 
 __global__ void ozd_reduce(RedArgs a) {
   chain_begin();
+  if (a.gate && *a.gate) return;
   const int64_t mn = (int64_t)a.m * a.n;
   const int64_t total = mn * a.batch;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
@@ -911,6 +915,7 @@ int gemm_f64_digits(fmpt_handle* h, const GemmArgs& g) {
   ep.var = plan.var;
   ep.S = plan.S;
   ep.Q = plan.Q;
+  ep.gate = h->gate;
   if (direct) {
     ep.C = g.C;
     ep.ldc = g.ldc;
@@ -948,6 +953,7 @@ int gemm_f64_digits(fmpt_handle* h, const GemmArgs& g) {
     ra.tiles_m2 = tiles_m2;
     ra.tiles_n = tiles_n;
     ra.nfast = ep.nfast;
+    ra.gate = h->gate;
     ra.alpha[0] = g.alpha[0];
     ra.alpha[1] = g.alpha[1];
     ra.beta[0] = g.beta[0];

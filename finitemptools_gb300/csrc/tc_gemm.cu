@@ -108,6 +108,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                 const __grid_constant__ CUtensorMap mapA2, const __grid_constant__ CUtensorMap mapB2,
                 int K, int tiles_m, int tiles_n, int batch, EpiArgs ep) {
+  if (gate_closed(ep.gate)) return;
   // Persistent: CTA b processes tiles b, b + gridDim.x, ...  (M-tile index fastest, so
   // CTAs running at the same time share B tiles in L2).  The accumulator is double
   // buffered in TMEM: the epilogue of one tile drains buffer t&1 while the MMA warp
@@ -363,6 +364,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                      const __grid_constant__ CUtensorMap mapA2,
                      const __grid_constant__ CUtensorMap mapB2, int K, int tiles_m2, int tiles_n,
                      int batch, EpiArgs ep, PairSched sp) {
+  if (gate_closed(ep.gate)) return;
   // Persistent over work items: cluster c (CTAs 2c, 2c+1) takes items c, c + clusters, ...
   // Warp roles as in gemm_kernel; only the even CTA's warp 1 issues MMAs.
   using C_ = PairCfg<MODE, STAGES>;
@@ -617,6 +619,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                       const __grid_constant__ CUtensorMap mapA2,
                       const __grid_constant__ CUtensorMap mapB2, int K, int tiles_m, int tiles_n,
                       int S, EpiArgs ep) {
+  if (gate_closed(ep.gate)) return;
   using C_ = SmallCfg<MODE, BN, STAGES>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -1032,7 +1035,7 @@ int tc_gemm(fmpt_handle* h, int mode, int M, int N, int K, int batch, const TcOp
             const TcOperand& B, void* C, int out_f64, int64_t ldc, int64_t strideC, int* err_dev) {
   using namespace tc;
   if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return FMPT_OK;
-  EpiArgs ep{C, ldc, strideC, M, N, err_dev, M > N ? 1 : 0};   // A and B share K
+  EpiArgs ep{C, ldc, strideC, M, N, err_dev, M > N ? 1 : 0, h->gate};   // A and B share K
   // GEMMs of more than one 128-row tile run on the CTA-pair kernel (256 x 256 tiles; 6
   // stages of 32 KB, or 3 of 64 KB for the hi/lo planes of 3xTF32) unless the handle asks
   // for the one-CTA tile.  Average per

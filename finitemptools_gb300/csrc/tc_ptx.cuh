@@ -128,6 +128,7 @@ struct EpiArgs {
   int M, N;
   int* err;
   int nfast;          // tile order: 0 = M index fastest, 1 = N index fastest
+  const int* gate;    // fmpt_handle::gate
 };
 
 // tile -> (mt, nt, z).  M index fastest: the CTAs running together share B tiles; N
