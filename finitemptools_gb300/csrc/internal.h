@@ -59,11 +59,10 @@ struct fmpt_handle {
   // partial tiles and arrival counters of the BF16 pair GEMM's K-split last round
   void* tc_ws = nullptr;
   size_t tc_ws_bytes = 0;
-  // counters of the split tiles: zero between launches (the last piece of a tile resets its own)
-  // unless a launch gave up (tc_cnt_dirty)
+  // counters of the split tiles: zero between launches (the last piece of a tile resets its own,
+  // in a launch that gives up too)
   void* tc_cnt = nullptr;
   size_t tc_cnt_bytes = 0;
-  bool tc_cnt_dirty = false;
   // FP64 GEMMs on the BF16 tensor cores (Ozaki scheme: residue planes, exponents,
   // the product's residues):
   // f64_tc 1 routes every FP64 GEMM of this handle there when its cost model says it is

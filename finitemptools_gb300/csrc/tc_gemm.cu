@@ -23,6 +23,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "tc_pieces.h"
 #include "tc_ptx.cuh"
 
 namespace fmpt {
@@ -298,38 +299,6 @@ struct PairCfg {
   static_assert((2 * STAGES + 5) * 8 + 8 <= 256, "barrier area");
 };
 
-// Work items of the pair kernel: `full` whole tiles (units) and, when the last round of tiles
-// would leave clusters idle, the `tail` units after them, each cut into S pieces along K.  The
-// pieces are the first tail S items: their sums, a round trip through L2, then lie beside the
-// whole tiles' products instead of behind the last round (H_eff*x at D = 512: BF16 47.0 -> 42.2
-// us, TF32 57.0 -> 51.2, 3xTF32 90.8 -> 78.7; D = 1200: 149 -> 135, 230 -> 215, 517 -> 500; a
-// part of it because the counters no longer take a memset per GEMM).  Piece p sums K-slices
-// [p nk / S, (p+1) nk / S) and writes its FP32 partial tile to ws; the last piece of a
-// tile to finish (per CTA half and epilogue warp, counted in cnt) adds the S partials in
-// piece order and stores the tile, so the result does not depend on which piece ends last.
-struct PairSched {
-  int full, tail, S;
-  float* ws;          // [tail * S][256 columns][256 rows]
-  int* cnt;           // [tail][2 CTAs][4 warps], zero at launch, reset by the last piece
-};
-
-__device__ __forceinline__ void pair_item(const PairSched& sp, int item, int nk, int& u,
-                                          int& kb0, int& kb1, int& t) {
-  const int pieces = sp.tail * sp.S;
-  if (item >= pieces) {
-    u = item - pieces;
-    kb0 = 0;
-    kb1 = nk;
-    t = -1;
-  } else {
-    t = item;
-    const int p = t % sp.S;
-    u = sp.full + t / sp.S;
-    kb0 = (int)((int64_t)p * nk / sp.S);
-    kb1 = (int)((int64_t)(p + 1) * nk / sp.S);
-  }
-}
-
 // One row of a K-split tile: the S partial rows at w0 (pieces 65536 floats apart, columns
 // 256 apart) summed in piece order into C.  All 32 S loads of a 32-column chunk are issued
 // before the first add.
@@ -506,38 +475,43 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     }
   } else {
     const int q = warp & 3;
-    int local = 0;
-    for (int item = cl; item < num_items; item += ncl, local++) {
-      int u, kb0, kb1, t, mt2, nt, z;
-      pair_item(sp, item, nk, u, kb0, kb1, t);
-      const int buf = local & 1;
-      const uint32_t use = (uint32_t)(local >> 1);
-      const bool ok = mbar_wait(smem_u32(&acc_full[buf]), use & 1, abort_flag, ep.err);
-      if (!ok || *abort_flag) break;
-      tc_fence_after();
-      tile_coords(u, tiles_m2, tiles_n, ep.nfast, mt2, nt, z);
-      const int rloc = (int)rank * BM + 32 * q + lane;          // row within the 256-row tile
-      const int row = mt2 * 2 * BM + rloc;
-      const uint32_t tbase = tmem + buf * C_::TMEM_COLS + ((uint32_t)(32 * q) << 16);
-      if (t < 0) {
-        store_acc<C_::BN, OUT>(tbase, row, nt * C_::BN, z, ep);
-      } else {
-        EpiArgs pe{sp.ws + (int64_t)t * 65536, 256, 0, 256, 256, ep.err, 0};
-        store_acc<C_::BN, 0>(tbase, rloc, 0, 0, pe);
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(cluster_addr(smem_u32(&acc_empty[buf]), 0));
-      if (t >= 0) {
-        // publish this piece, then the last of the S pieces sums them in piece order
-        __threadfence();
-        __syncwarp();
-        const int ut = u - sp.full;
-        int* c = sp.cnt + (ut * 2 + (int)rank) * 4 + q;
-        int prev = 0;
-        if (lane == 0) prev = atomicAdd(c, 1);
-        prev = __shfl_sync(0xffffffffu, prev, 0);
-        if (prev == sp.S - 1) {
+    const int rloc = (int)rank * BM + 32 * q + lane;            // row within the 256-row tile
+    auto counter = [&](int ut) { return sp.cnt + (ut * 2 + (int)rank) * 4 + q; };
+    pair_epilogue(
+        sp, cl, ncl, nk,
+        [&](int local) {
+          const bool ok = mbar_wait(smem_u32(&acc_full[local & 1]), (uint32_t)(local >> 1) & 1,
+                                    abort_flag, ep.err);
+          return __all_sync(0xffffffffu, ok && !*abort_flag) != 0;
+        },
+        [&](int local, int u, int t) {
+          tc_fence_after();
+          const int buf = local & 1;
+          const uint32_t tbase = tmem + buf * C_::TMEM_COLS + ((uint32_t)(32 * q) << 16);
+          if (t < 0) {
+            int mt2, nt, z;
+            tile_coords(u, tiles_m2, tiles_n, ep.nfast, mt2, nt, z);
+            store_acc<C_::BN, OUT>(tbase, mt2 * 2 * BM + rloc, nt * C_::BN, z, ep);
+          } else {
+            EpiArgs pe{sp.ws + (int64_t)t * 65536, 256, 0, 256, 256, ep.err, 0, nullptr};
+            store_acc<C_::BN, 0>(tbase, rloc, 0, 0, pe);
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(cluster_addr(smem_u32(&acc_empty[buf]), 0));
+        },
+        [&](int ut) {
+          // publish this piece, then the last of the S pieces sums them in piece order
+          __threadfence();
+          __syncwarp();
+          int prev = 0;
+          if (lane == 0) prev = atomicAdd(counter(ut), 1);
+          return __shfl_sync(0xffffffffu, prev, 0) == sp.S - 1;
+        },
+        [&](int ut, int u) {
+          int mt2, nt, z;
+          tile_coords(u, tiles_m2, tiles_n, ep.nfast, mt2, nt, z);
+          const int row = mt2 * 2 * BM + rloc;
           __threadfence();
           const float* w0 = sp.ws + (int64_t)ut * sp.S * 65536 + rloc;
           if (row < ep.M) {
@@ -552,11 +526,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             else
               sum_pieces<4, OUT>(w0, base, ep.ldc, n0, ep.N);
           }
+        },
+        [&](int ut) {
           __syncwarp();
-          if (lane == 0) *c = 0;
-        }
-      }
-    }
+          if (lane == 0) *counter(ut) = 0;
+        });
   }
   tc_fence_before();
   __syncthreads();
@@ -997,11 +971,10 @@ static int tc_gemm_pair_st(fmpt_handle* h, int M, int N, int K, int batch, const
     // leaves the last round whole
     if (cs == cudaStreamCaptureStatusNone) {
       FMPT_TRY(grow_buffer(h, &h->tc_ws, &h->tc_ws_bytes, need));
-      if (h->tc_cnt_bytes < cnt) h->tc_cnt_dirty = true;
-      FMPT_TRY(grow_buffer(h, &h->tc_cnt, &h->tc_cnt_bytes, cnt));
-      if (h->tc_cnt_dirty)
+      if (h->tc_cnt_bytes < cnt) {
+        FMPT_TRY(grow_buffer(h, &h->tc_cnt, &h->tc_cnt_bytes, cnt));
         FMPT_CUDA(h, cudaMemsetAsync(h->tc_cnt, 0, h->tc_cnt_bytes, h->stream));
-      h->tc_cnt_dirty = false;
+      }
     }
     if (h->tc_ws_bytes >= need && h->tc_cnt_bytes >= cnt) {
       sp.full = (int)(units - rem);

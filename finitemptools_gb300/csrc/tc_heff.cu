@@ -802,10 +802,7 @@ int env_left_tc(fmpt_handle* h, int precision, const double* hold, const double*
   }
   cudaFreeAsync(err, h->stream);
   FMPT_TRY(st);
-  if (e) {
-    h->tc_cnt_dirty = true;
-    return set_error(h, FMPT_ERR_TIMEOUT, "tensor-core GEMM wait timed out");
-  }
+  if (e) return set_error(h, FMPT_ERR_TIMEOUT, "tensor-core GEMM wait timed out");
   return FMPT_OK;
 }
 
@@ -866,10 +863,7 @@ int env_right_tc(fmpt_handle* h, int precision, const double* hold, const double
   }
   cudaFreeAsync(err, h->stream);
   FMPT_TRY(st);
-  if (e) {
-    h->tc_cnt_dirty = true;
-    return set_error(h, FMPT_ERR_TIMEOUT, "tensor-core GEMM wait timed out");
-  }
+  if (e) return set_error(h, FMPT_ERR_TIMEOUT, "tensor-core GEMM wait timed out");
   return FMPT_OK;
 }
 
@@ -888,10 +882,7 @@ int op_tc_check(fmpt_op* op) {
   int e = 0;
   FMPT_CUDA(op->h, cudaMemcpyAsync(&e, st->err, sizeof(int), cudaMemcpyDeviceToHost, op->h->stream));
   FMPT_CUDA(op->h, cudaStreamSynchronize(op->h->stream));
-  if (e) {
-    op->h->tc_cnt_dirty = true;
-    return set_error(op->h, FMPT_ERR_TIMEOUT, "tensor-core GEMM wait timed out");
-  }
+  if (e) return set_error(op->h, FMPT_ERR_TIMEOUT, "tensor-core GEMM wait timed out");
   return FMPT_OK;
 }
 
