@@ -32,8 +32,8 @@ template <bool CPLX, int BMN>
 __global__ void __launch_bounds__(NT) gemm_kernel(GemmArgs g, int splits, int kchunk,
                                                   double* __restrict__ ws,
                                                   int* __restrict__ tile_cnt) {
+  if (gate_closed(g.gate)) return;
   chain_begin();
-  if (g.gate && *g.gate) return;
   constexpr int TPR = BMN / 16;                // outputs per thread along each dimension
   __shared__ double As[2][BK][BMN + 1];
   __shared__ double Bs[2][BK][BMN + 1];
@@ -261,8 +261,8 @@ __global__ void __launch_bounds__(32 * WWARPS * KP) gemm_warp(GemmArgs g, int sp
                                                               double* __restrict__ ws,
                                                               int* __restrict__ tile_cnt) {
   static_assert(KP == 1 || CPLX, "K pieces of complex tiles");
+  if (gate_closed(g.gate)) return;
   chain_begin();
-  if (g.gate && *g.gate) return;
   constexpr int NP = CPLX ? 2 : 1;                       // planes
   constexpr int WK = KP > 1 ? 16 : WK1, WST = KP > 1 ? 3 : WST1;
   // the ring belongs to a warp (real) or to the two warps of a tile and piece (complex)

@@ -136,7 +136,8 @@ int set_error(fmpt_handle* h, int status, const char* fmt, ...);
 #ifdef __CUDACC__
 __device__ __forceinline__ void chain_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // The first statement of a kernel with a gate (fmpt_handle::gate): nothing is to be done.  Uniform
-// for the whole grid, since an earlier kernel sets the flag.
+// for the whole grid, since an earlier kernel sets the flag.  Before the kernel's own chain_begin:
+// read after it, the parameter alone cost 0.05 us per launch.
 __device__ __forceinline__ bool gate_closed(const int* gate) {
   if (!gate) return false;
   chain_begin();

@@ -714,8 +714,8 @@ __device__ __forceinline__ double ws_sum(const RedArgs& a, int z, int r, int c) 
 }
 
 __global__ void ozd_reduce(RedArgs a) {
+  if (gate_closed(a.gate)) return;
   chain_begin();
-  if (a.gate && *a.gate) return;
   const int64_t mn = (int64_t)a.m * a.n;
   const int64_t total = mn * a.batch;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
