@@ -474,8 +474,18 @@ int launch(fmpt_handle* h, const GemmArgs& g) {
       }
     }
   }
-  const int kchunk = splits > 1 ? ((g.k + splits - 1) / splits + BK - 1) / BK * BK : g.k;
+  int kchunk = splits > 1 ? ((g.k + splits - 1) / splits + BK - 1) / BK * BK : g.k;
   if (splits > 1) splits = (g.k + kchunk - 1) / kchunk;
+  const size_t wsb = (size_t)splits * g.m * g.n * sizeof(double) * (CPLX ? 2 : 1);
+  if (splits > 1 && h->gemm_ws_bytes < wsb) {
+    // the workspace cannot grow inside a stream capture: K stays whole
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+      cudaGetLastError();
+      splits = 1;
+      kchunk = g.k;
+    }
+  }
   // The kernel: 8x4 tiles per warp where they put fewer multiply-adds on the busiest
   // sub-partition than 64x64 tiles do on the busiest SM, those otherwise.  The split stays
   // as it is, so the sums do not depend on this choice; the warps' operand reads come to
@@ -497,8 +507,7 @@ int launch(fmpt_handle* h, const GemmArgs& g) {
   double* ws = nullptr;
   int* cnt = nullptr;
   if (splits > 1) {
-    FMPT_TRY(grow_buffer(h, &h->gemm_ws, &h->gemm_ws_bytes,
-                         (size_t)splits * g.m * g.n * sizeof(double) * (CPLX ? 2 : 1)));
+    FMPT_TRY(grow_buffer(h, &h->gemm_ws, &h->gemm_ws_bytes, wsb));
     ws = static_cast<double*>(h->gemm_ws);
     const int64_t tiles = (int64_t)grid.x * (warp_tiles && !CPLX ? WWARPS : 1) * grid.y * g.batch;
     if (tiles <= kMaxSplitTiles) {

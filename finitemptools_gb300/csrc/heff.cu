@@ -540,11 +540,12 @@ int op_fp64_head(fmpt_op* op, const double* x) {
   const int wl = op->wl, wr = op->wr;
   const int64_t nx = (int64_t)Dl * P * Dr;
   const int64_t n1 = (int64_t)Dl * wl * P * Dr, n3 = (int64_t)Dl * P * wr * Dr;
-  // T1 and T3 in the operator's scratch (one buffer, T3 after T1)
-  // and, where GEMM 2 takes them, the row maxima of T3
+  // T1 and T3 in the operator's scratch (one buffer, T3 after T1) and the row maxima of T3, used
+  // where GEMM 2 takes them.  Their room does not depend on that: which engine GEMM 2 runs on
+  // differs between calls, and the scratch cannot grow inside a stream capture.
   const bool maxima = !op->sched.sp_start.empty() && Dr <= 8 * 65535 &&
                       gemm_f64_ozaki_takes_maxima(h, tail_gemm(op, nullptr));
-  const size_t mxb = maxima ? (size_t)Dl * P * (cp ? 2 : 1) * sizeof(uint64_t) : 0;
+  const size_t mxb = (size_t)Dl * P * (cp ? 2 : 1) * sizeof(uint64_t);
   const size_t held = op->scratch_bytes;
   FMPT_TRY(grow_buffer(h, reinterpret_cast<void**>(&op->scratch), &op->scratch_bytes,
                        (size_t)(n1 + n3) * es + mxb));
