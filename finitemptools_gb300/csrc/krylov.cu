@@ -2036,9 +2036,11 @@ int fmpt_expm_nodes(fmpt_op* op, double t_re, double t_im, const double* x, int 
   }
   FMPT_CUDA(h, cudaMemcpyAsync(Ed.d(), cols.data(), cols.size() * sizeof(double),
                                cudaMemcpyHostToDevice, h->stream));
-  CHAIN(combine_basis, dim3(G, nnodes), h->stream, cp, n, m, V, nr, Ed.d(), 2 * m, acc.d(), out,
-                                                       nr);
-  FMPT_LAUNCHED(h);
+  for (int q0 = 0; q0 < nnodes; q0 += 65535) {               // the nodes are the grid's y axis
+    CHAIN(combine_basis, dim3(G, std::min(65535, nnodes - q0)), h->stream, cp, n, m, V, nr,
+          Ed.d() + (int64_t)2 * m * q0, 2 * m, acc.d(), out + nr * q0, nr);
+    FMPT_LAUNCHED(h);
+  }
   if (err_est) *err_est = e;
   if (!prec_is_f64(op->precision)) FMPT_TRY(op_tc_check(op));
   if (op->u1 || gs.fused) FMPT_TRY(gp_check_status(op->h));
