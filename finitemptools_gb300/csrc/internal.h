@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -205,6 +206,30 @@ cudaError_t launch_chain(void (*kernel)(P...), dim3 grid, dim3 block, size_t sme
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 #endif
+
+// What a kernel needs to know or have set once per device (attributes, resident clusters), in N
+// slots.  Handles of several host threads may ask at the same time.
+template <int N = 1>
+class PerDevice {
+  static constexpr int kDevices = 64;
+  std::mutex mu_;
+  int value_[kDevices][N] = {};
+  bool done_[kDevices][N] = {};
+
+ public:
+  // value = what find(value) has found for h's device; an error of find is returned and not kept
+  template <class Find>
+  int get(fmpt_handle* h, int slot, int& value, Find find) {
+    if (h->device < 0 || h->device >= kDevices) return find(value);
+    std::lock_guard<std::mutex> lock(mu_);
+    if (!done_[h->device][slot]) {
+      FMPT_TRY(find(value_[h->device][slot]));
+      done_[h->device][slot] = true;
+    }
+    value = value_[h->device][slot];
+    return FMPT_OK;
+  }
+};
 
 // Stream-ordered device scratch owned by a C++ scope.
 struct DevBuf {

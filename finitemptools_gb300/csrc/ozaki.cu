@@ -848,7 +848,8 @@ int gemm_f64_ozaki(fmpt_handle* h, const GemmArgs& g) {
   const int64_t units = (int64_t)tiles_m2 * tiles_n * batch;
   if (units > INT32_MAX / 128) return set_error(h, FMPT_ERR_SHAPE, "ozaki: too many tiles");
   // resident clusters of the kernel
-  static int clusters = -1;
+  static PerDevice<> resident;
+  int clusters = 0;
   cudaLaunchConfig_t cfg{};
   cfg.blockDim = dim3(NTHR);
   cfg.dynamicSmemBytes = SMEM;
@@ -860,19 +861,18 @@ int gemm_f64_ozaki(fmpt_handle* h, const GemmArgs& g) {
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (clusters < 0) {
-    for (int n = 15; n <= 16; n++)
+  FMPT_TRY(resident.get(h, 0, clusters, [&](int& found) -> int {
+    for (int n : {15, 16})
       FMPT_CUDA(h, cudaFuncSetAttribute(residues_rowfast_kernel(n),
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DR_SMEM));
     FMPT_CUDA(h, cudaFuncSetAttribute(oz_gemm_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
     cfg.gridDim = dim3(2 * std::max(1, h->sm_count / 2));
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, oz_gemm_pair, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&found, oz_gemm_pair, &cfg) != cudaSuccess) {
       (void)cudaGetLastError();
-      n = 0;
+      found = 0;
     }
-    clusters = n;
-  }
+    return FMPT_OK;
+  }));
   if (clusters <= 0) return set_error(h, FMPT_ERR_UNSUPPORTED, "ozaki: no 2-CTA cluster fits");
   const size_t resb = (size_t)nmod * units * TILE * TILE;
   const size_t mxb = (size_t)batch * (M2 + N) * sizeof(uint64_t);

@@ -813,7 +813,8 @@ int gemm_f64_digits(fmpt_handle* h, const GemmArgs& g) {
   const int64_t units = (int64_t)tiles_m2 * tiles_n * batch;
   if (units > INT32_MAX / 64) return set_error(h, FMPT_ERR_SHAPE, "ozaki: too many tiles");
   // resident clusters of the kernel
-  static int clusters = -1;
+  static PerDevice<> resident;
+  int clusters = 0;
   cudaLaunchConfig_t cfg{};
   cfg.blockDim = dim3(NTHREADS);
   cfg.dynamicSmemBytes = SMEM;
@@ -825,18 +826,17 @@ int gemm_f64_digits(fmpt_handle* h, const GemmArgs& g) {
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (clusters < 0) {
+  FMPT_TRY(resident.get(h, 0, clusters, [&](int& found) -> int {
     FMPT_CUDA(h, cudaFuncSetAttribute(ozd_digits_rowfast,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DR_SMEM));
     FMPT_CUDA(h, cudaFuncSetAttribute(ozd_gemm_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
     cfg.gridDim = dim3(2 * std::max(1, h->sm_count / 2));
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, ozd_gemm_pair, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&found, ozd_gemm_pair, &cfg) != cudaSuccess) {
       (void)cudaGetLastError();
-      n = 0;
+      found = 0;
     }
-    clusters = n;
-  }
+    return FMPT_OK;
+  }));
   if (clusters <= 0) return set_error(h, FMPT_ERR_UNSUPPORTED, "ozaki: no 2-CTA cluster fits");
   const Plan plan = digits_plan(M2, N, K2, batch, clusters);
   const int split = plan.S * plan.Q;

@@ -834,17 +834,18 @@ static int tc_gemm_small(fmpt_handle* h, int M, int N, int K, int batch, int S, 
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = S > 1 ? 1 : 0;
-  static int fits[3][5] = {};                          // 1 / -1: clusters of S (do not) fit
-  if (fits[vi][S] == 0) {
+  static PerDevice<3 * 5> resident;                    // clusters of S, per variant
+  int clusters = 0;
+  FMPT_TRY(resident.get(h, 5 * vi + S, clusters, [&](int& n) -> int {
     FMPT_CUDA(h, cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, C_::SMEM));
-    int n = 1;
+    n = 1;
     if (S > 1 && cudaOccupancyMaxActiveClusters(&n, kfn, &cfg) != cudaSuccess) {
       (void)cudaGetLastError();
       n = 0;
     }
-    fits[vi][S] = n > 0 ? 1 : -1;
-  }
-  if (fits[vi][S] < 0) return FMPT_ERR_UNSUPPORTED;
+    return FMPT_OK;
+  }));
+  if (clusters <= 0) return FMPT_ERR_UNSUPPORTED;
   chain_attr(attr[cfg.numAttrs++]);
   ProfScope prof(h, FMPT_K_TC_GEMM);
   FMPT_CUDA(h, cudaLaunchKernelEx(&cfg, kfn, ma, mb, ma2, mb2, K, tiles_m, tiles_n, S, ep));
@@ -920,7 +921,7 @@ static int tc_gemm_pair_st(fmpt_handle* h, int M, int N, int K, int batch, const
       : out_f64 == 2 ? gemm_pair_kernel<MODE, ST, MODE == BF16 ? 2 : 0>
                      : gemm_pair_kernel<MODE, ST, 0>;
   const int vi = out_f64 == 1 ? 1 : out_f64 == 2 ? 2 : 0;
-  static int clusters[3] = {-1, -1, -1};           // resident 2-CTA clusters, per variant
+  static PerDevice<3> resident;                    // 2-CTA clusters, per variant
   cudaLaunchConfig_t cfg{};
   cfg.blockDim = dim3(NTHREADS);
   cfg.dynamicSmemBytes = C_::SMEM;
@@ -932,21 +933,20 @@ static int tc_gemm_pair_st(fmpt_handle* h, int M, int N, int K, int batch, const
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (clusters[vi] < 0) {
+  int cl = 0;
+  FMPT_TRY(resident.get(h, vi, cl, [&](int& n) -> int {
     FMPT_CUDA(h, cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, C_::SMEM));
     cfg.gridDim = dim3(2 * std::max(1, h->sm_count / 2));
-    int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, kfn, &cfg) != cudaSuccess) {
       (void)cudaGetLastError();
       n = 0;
     }
-    clusters[vi] = n;
-  }
-  if (clusters[vi] <= 0) return FMPT_ERR_UNSUPPORTED;
+    return FMPT_OK;
+  }));
+  if (cl <= 0) return FMPT_ERR_UNSUPPORTED;
   // Whole tiles fill rounds of `cl` clusters; when the last round holds R < cl / 2 tiles,
   // those are cut along K into S = min(4, cl / R) pieces (at least 4 K-slices each), so
   // the round ends after about 1/S of a tile instead of a whole one.
-  const int cl = clusters[vi];
   const int nk = (K + C_::KELEMS - 1) / C_::KELEMS;
   PairSched sp{(int)units, 0, 1, nullptr, nullptr};
   const int rem = (int)(units % cl);
@@ -1045,11 +1045,13 @@ int tc_gemm(fmpt_handle* h, int mode, int M, int N, int K, int batch, const TcOp
   do {                                                                                        \
     auto kfn = gemm_kernel<MODE_, BN_, ST_, OUT_>;                                            \
     constexpr int SM_ = Cfg<MODE_, BN_, ST_, OUT_>::SMEM;                                      \
-    static bool attr_done = false;                                                            \
-    if (!attr_done) {                                                                         \
+    static PerDevice<> attr;                                                                  \
+    int set = 0;                                                                              \
+    FMPT_TRY(attr.get(h, 0, set, [&](int& done) -> int {                                      \
       FMPT_CUDA(h, cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_)); \
-      attr_done = true;                                                                       \
-    }                                                                                         \
+      done = 1;                                                                               \
+      return FMPT_OK;                                                                         \
+    }));                                                                                      \
     FMPT_CUDA(h, launch_chain(kfn, grid, NTHREADS, SM_, h->stream, ma, mb, ma2, mb2, K, tiles_m,  \
                               tiles_n, batch, ep));                                         \
   } while (0)
