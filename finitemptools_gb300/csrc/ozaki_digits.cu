@@ -41,7 +41,7 @@
 // Kernels: oz_rowmax / ozd_digits (FP64 operand -> row exponents + 9 K-major BF16 digit
 // planes, gridded over 32-row strips and 512-column K chunks), ozd_gemm_pair (the CTA
 // pair tcgen05 kernel of tc_gemm.cu with the (chunk, level, product) sequence and the
-// FP64 epilogue), ozd_reduce (sums split pieces in a fixed order, applies alpha / beta).
+// FP64 epilogue), ozd_reduce (sums split pieces in a fixed order).
 #include <algorithm>
 #include <cmath>
 
@@ -317,7 +317,6 @@ struct OzEpi {
   int M, N, mh;         // rows >= mh of the real embedding go to the imaginary plane
   const int* ea;        // [batch][M] row exponents
   const int* eb;        // [batch][N] column exponents
-  double alpha;         // direct mode only
   int* err;
   int nfast;
   int split;            // pieces per tile: S level sets x Q chunk ranges (1: direct)
@@ -383,7 +382,7 @@ __device__ __noinline__ double scaled_slow(uint32_t u, int E) {
 // the general path.
 template <bool SPLIT>
 __device__ __forceinline__ void drain(uint32_t tbase, int row, int rloc, int n0, int z,
-                                      int level, bool first, bool last, const OzEpi& ep,
+                                      int level, bool first, const OzEpi& ep,
                                       double* wtile) {
   const bool live = row < ep.M;
   double* crow;
@@ -397,7 +396,6 @@ __device__ __forceinline__ void drain(uint32_t tbase, int row, int rloc, int n0,
   }
   const int er = live ? __ldg(ep.ea + (int64_t)z * ep.M + row) : 0;
   const int eb = er - SB * level;
-  const bool scale = !SPLIT && last && ep.alpha != 1.0;
   const int lane = threadIdx.x & 31;
 #pragma unroll 1
   for (int c0 = 0; c0 < TILE; c0 += 32) {
@@ -426,7 +424,6 @@ __device__ __forceinline__ void drain(uint32_t tbase, int row, int rloc, int n0,
                             ((u & 0x7fffffu) >> 3);
         double v = (u << 1) == 0 ? 0.0 : __hiloint2double((int)hi, (int)(u << 29));
         if (!first) v += old[j];
-        if (scale) v *= ep.alpha;
         p[j * ld] = v;
       }
     } else {
@@ -450,7 +447,6 @@ __device__ __forceinline__ void drain(uint32_t tbase, int row, int rloc, int n0,
           }
         }
         if (!first) v += old[j];
-        if (scale) v *= ep.alpha;
         p[j * ld] = v;
       }
     }
@@ -652,11 +648,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           tc_fence_after();
           const uint32_t tbase = tmem + buf * TMEM_COLS + ((uint32_t)(32 * q) << 16);
           const bool first = li == 0 && ch == 0;
-          const bool lastg = li == nl - 1 && ch == nch - 1;
           if (wtile)
-            drain<true>(tbase, row, rloc, nt * TILE, z, level, first, lastg, ep, wtile);
+            drain<true>(tbase, row, rloc, nt * TILE, z, level, first, ep, wtile);
           else
-            drain<false>(tbase, row, rloc, nt * TILE, z, level, first, lastg, ep, nullptr);
+            drain<false>(tbase, row, rloc, nt * TILE, z, level, first, ep, nullptr);
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(cluster_addr(smem_u32(&acc_empty[buf]), 0));
@@ -685,14 +680,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   }
 }
 
-// C = alpha (sum of the pieces, in piece order) + beta C.  ws holds the pieces of tile
+// C = the sum of the pieces, in piece order.  ws holds the pieces of tile
 // unit u at items u * split + p, each [256 columns][256 rows] of the real embedding.
 struct RedArgs {
   const double* ws;
   double* C;
   int64_t ldc, strideC, planeC;
   int m, n, batch, cplx, split, S, tiles_m2, tiles_n, nfast;
-  double alpha[2], beta[2];
   const int* gate;
 };
 
@@ -723,25 +717,9 @@ __global__ void ozd_reduce(RedArgs a) {
     const int z = (int)(t / mn);
     const int64_t rem = t - z * mn;
     const int r = (int)(rem % a.m), c = (int)(rem / a.m);
-    double* C = a.C + z * a.strideC;
-    const int64_t idx = (int64_t)r + (int64_t)c * a.ldc;
-    const bool has_beta = a.beta[0] != 0.0 || a.beta[1] != 0.0;
-    if (a.cplx) {
-      const double sr = ws_sum(a, z, r, c), si = ws_sum(a, z, r + a.m, c);
-      double re = a.alpha[0] * sr - a.alpha[1] * si;
-      double im = a.alpha[0] * si + a.alpha[1] * sr;
-      if (has_beta) {
-        const double cr = C[idx], ci = C[a.planeC + idx];
-        re += a.beta[0] * cr - a.beta[1] * ci;
-        im += a.beta[0] * ci + a.beta[1] * cr;
-      }
-      C[idx] = re;
-      C[a.planeC + idx] = im;
-    } else {
-      double v = a.alpha[0] * ws_sum(a, z, r, c);
-      if (has_beta) v += a.beta[0] * C[idx];
-      C[idx] = v;
-    }
+    double* C = a.C + z * a.strideC + (int64_t)r + (int64_t)c * a.ldc;
+    C[0] = ws_sum(a, z, r, c);
+    if (a.cplx) C[a.planeC] = ws_sum(a, z, r + a.m, c);
   }
 }
 
@@ -789,6 +767,8 @@ static ozd::Plan digits_plan(int64_t M2, int64_t N, int64_t K2, int batch, int c
 
 int gemm_f64_digits_possible(fmpt_handle* h, const GemmArgs& g) {
   if (!h->f64_tc && !g.engine) return 0;
+  // C = A B alone: what an operator's application needs
+  if (g.alpha[0] != 1.0 || g.alpha[1] != 0.0 || g.beta[0] != 0.0 || g.beta[1] != 0.0) return 0;
   if (g.m < 32 || g.n < 32 || g.k < 16) return 0;
   const int cp = g.cplx ? 2 : 1;
   const double flops = 2.0 * g.m * g.n * (double)g.k * g.batch * cp * cp;
@@ -840,7 +820,7 @@ int gemm_f64_digits(fmpt_handle* h, const GemmArgs& g) {
   if (clusters <= 0) return set_error(h, FMPT_ERR_UNSUPPORTED, "ozaki: no 2-CTA cluster fits");
   const Plan plan = digits_plan(M2, N, K2, batch, clusters);
   const int split = plan.S * plan.Q;
-  const bool direct = split == 1 && g.beta[0] == 0.0 && g.beta[1] == 0.0 && g.alpha[1] == 0.0;
+  const bool direct = split == 1;
   const size_t wsb = direct ? 0 : (size_t)units * split * TILE * TILE * sizeof(double);
   const size_t mxb = (size_t)batch * (M2 + N) * sizeof(uint64_t);
   // an operand with a cache keeps its planes there (built once while its key holds)
@@ -922,11 +902,9 @@ int gemm_f64_digits(fmpt_handle* h, const GemmArgs& g) {
     ep.strideC = g.strideC;
     ep.planeC = g.planeC;
     ep.mh = cp ? g.m : INT32_MAX;
-    ep.alpha = g.alpha[0];
   } else {
     ep.C = WS;
     ep.mh = -1;        // workspace tiles
-    ep.alpha = 1.0;
   }
   const int64_t items = units * split;
   cfg.gridDim = dim3((unsigned)(2 * std::min<int64_t>(items, clusters)));
@@ -954,10 +932,6 @@ int gemm_f64_digits(fmpt_handle* h, const GemmArgs& g) {
     ra.tiles_n = tiles_n;
     ra.nfast = ep.nfast;
     ra.gate = h->gate;
-    ra.alpha[0] = g.alpha[0];
-    ra.alpha[1] = g.alpha[1];
-    ra.beta[0] = g.beta[0];
-    ra.beta[1] = g.beta[1];
     const int64_t total = (int64_t)g.m * g.n * batch;
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, 8LL * h->sm_count));
     FMPT_CUDA(h, launch_chain(ozd_reduce, blocks, 256, 0, h->stream, ra));
