@@ -5,9 +5,8 @@
 // that matters, and what decides their speed is how evenly they spread the
 // multiply-adds over the 608 sub-partitions.  Large problems use a 64x64 tile with a
 // 4x4 register block per thread (gemm_kernel).  Small ones (the D <= 128
-// contractions of TDVP and of the first DMRG bonds) give every warp an 8x4 tile
-// straight from L1/L2 (gemm_warp) and may split K over the grid; a cost model picks
-// the split.  Every split writes its
+// contractions of TDVP and of the first DMRG bonds) give every warp an 8x4 tile and a
+// cp.async ring of its own (gemm_warp) and may split K over the grid.  Every split writes its
 // partial product to a workspace; the last split of a tile to finish (an atomic
 // count per tile) sums the tile's partials in split order, so the result does
 // not depend on scheduling, applies alpha/beta and resets the count.  Where no
@@ -28,12 +27,13 @@ __device__ __forceinline__ int64_t a_index(int t, int r, int c, int64_t ld) {
 // C (or the split workspace) = op(A) op(B) over k in [k_lo, k_hi).
 // gridDim.z = batch * splits; with splits > 1 (batch == 1) the raw partial
 // product goes to ws + split * plane_ws (re, then im plane at + m*n).
-template <bool CPLX, int BMN>
+template <bool CPLX>
 __global__ void __launch_bounds__(NT) gemm_kernel(GemmArgs g, int splits, int kchunk,
                                                   double* __restrict__ ws,
                                                   int* __restrict__ tile_cnt) {
   if (gate_closed(g.gate)) return;
   chain_begin();
+  constexpr int BMN = 64;                      // tile edge
   constexpr int TPR = BMN / 16;                // outputs per thread along each dimension
   __shared__ double As[2][BK][BMN + 1];
   __shared__ double Bs[2][BK][BMN + 1];
@@ -241,14 +241,6 @@ __global__ void __launch_bounds__(NT) gemm_kernel(GemmArgs g, int splits, int kc
 // 17.7 and 18.2 us.
 constexpr int WM = 8, WN = 4, WWARPS = 2, WK1 = 32, WST1 = 4;
 
-// 8 bytes, zeros if !in
-__device__ __forceinline__ void cp_async8z(double* dst, const double* src, bool in) {
-  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src),
-               "r"(in ? 8 : 0)
-               : "memory");
-}
-
 // KP > 1 (complex, Arnoldi only): KP pairs of warps take a K piece of the tile each, and the
 // pieces are added in order.  At D <= 32 a tile's chain of multiply-adds is longer than
 // everything else (K = 96: 192 of them, 64 cycles each) while most sub-partitions are idle.
@@ -453,8 +445,11 @@ constexpr int kMaxSplitTiles = 1 << 14;
 template <bool CPLX>
 int launch(fmpt_handle* h, const GemmArgs& g) {
   const int sms = h->sm_count > 0 ? h->sm_count : 1;
-  // the K split that, with its best tile edge, puts the fewest multiply-adds on the busiest
-  // SM; a split adds the partials' round trip, priced as that many multiply-adds
+  // The K split: the one that, in square tiles of the best of three edges, puts the fewest
+  // multiply-adds on the busiest SM; a split adds the partials' round trip, priced as that many
+  // multiply-adds.  It is a rule about the order of the sums, not a model of the kernel below: the
+  // 32 and 16 wide tiles it was made for have become warp tiles, and a Lanczos vector's sign
+  // hangs on the last bit of the sums, so it stays as it was.
   const double cm = CPLX ? 4.0 : 1.0;
   int splits = 1;
   double best = 1e300;
@@ -467,7 +462,7 @@ int launch(fmpt_handle* h, const GemmArgs& g) {
       const int64_t per_sm = (blocks + sms - 1) / sms;
       double cost = (double)per_sm * e * e * kc * cm;
       if (s > 1) cost += 2.0e4 * cm + (double)s * e * e * cm * 4.0;
-      if (e == 16) cost *= 1.15;               // one output per thread: more loads per FMA
+      if (e == 16) cost *= 1.15;               // (more loads per FMA)
       if (cost < best * 0.98) {
         best = cost;
         splits = s;
@@ -532,7 +527,7 @@ int launch(fmpt_handle* h, const GemmArgs& g) {
     FMPT_CUDA(h, launch_chain(gemm_warp<CPLX, 1>, grid, 32 * WWARPS, 0, h->stream, g, splits, kchunk,
                               ws, cnt));
   else
-    FMPT_CUDA(h, launch_chain(gemm_kernel<CPLX, 64>, grid, NT, 0, h->stream, g, splits, kchunk, ws,
+    FMPT_CUDA(h, launch_chain(gemm_kernel<CPLX>, grid, NT, 0, h->stream, g, splits, kchunk, ws,
                               cnt));
   FMPT_LAUNCHED(h);
   if (splits > 1 && !cnt) {

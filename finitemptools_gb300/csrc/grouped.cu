@@ -278,14 +278,6 @@ __global__ void __launch_bounds__(GNT) grouped_kernel(const GKArgs a) {
 constexpr int QM = 8, QN = 4, QK = 16, QST = 3, QWARPS = 4, QBLOCKS = 4;
 constexpr int QSM = 32, QSN = 4;           // tile of a SUM phase
 
-// 8 bytes, zeros if !in
-__device__ __forceinline__ void cp_async8z(double* dst, const double* src, bool in) {
-  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src),
-               "r"(in ? 8 : 0)
-               : "memory");
-}
-
 // The segments of a tile: each lane holds one of the 32 around the last one asked for, so that
 // a tile waits for one load of its descriptors, not for one per segment.
 struct SegWindow {

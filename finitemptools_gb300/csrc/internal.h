@@ -145,6 +145,14 @@ __device__ __forceinline__ bool gate_closed(const int* gate) {
   return *gate != 0;
 }
 
+// 8 bytes by cp.async, zeros if !in
+__device__ __forceinline__ void cp_async8z(double* dst, const double* src, bool in) {
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src),
+               "r"(in ? 8 : 0)
+               : "memory");
+}
+
 // Conversions between FP32 and FP64 on the integer pipe: a conversion instruction runs on the
 // FP64 pipe of GB300, 64 cycles of its SM sub-partition, and the epilogues and layout kernels
 // that widen or narrow every element were bound by it.  Zeros and normal numbers here; the rest

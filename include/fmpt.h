@@ -269,7 +269,7 @@ int fmpt_op_set_projectors(fmpt_op* op, int nproj, const double* const* p);
 /* Lowest eigenpair by the reference's plain Lanczos
  * (auxiliary/simple_lanczos.jl:83-120): three-term recurrence, stop when
  * beta < btol, at most kmax Krylov vectors, lowest Ritz pair of the
- * tridiagonal matrix (solved on the device in FP64).  reorth != 0 adds full
+ * tridiagonal matrix (solved on the host in FP64).  reorth != 0 adds full
  * FP64 reorthogonalisation (not in the reference; off for parity runs).
  * eigval/info/niter are HOST outputs; xout is a device vector. */
 int fmpt_lanczos_ground(fmpt_op* op, const double* x0, int kmax, double btol, int reorth,
