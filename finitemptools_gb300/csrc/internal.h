@@ -24,8 +24,8 @@ struct fmpt_handle {
   double* pinned = nullptr;
   size_t pinned_len = 0;
   // Lanczos solve: the ends of its two latest steps, and pinned memory their kernels write
-  // (alpha, beta) pairs to; of its own, since a step thrown away on convergence may still
-  // be running when the solve returns (both created on first use)
+  // (alpha, beta) pairs to while the staging area above serves the calls in between (both
+  // created on first use)
   cudaEvent_t step_event[2] = {nullptr, nullptr};
   double* step_host = nullptr;
   int sm_count = 0;

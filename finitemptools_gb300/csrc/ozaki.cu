@@ -31,7 +31,7 @@
 // (0.25).  Error of a product of random matrices relative to its norm, against 113-bit
 // references: 2.6e-16 at K = 2048 (15 moduli), 5e-17 at K = 5120 (16); of the digit form, which
 // drops the products below 2^-60 of the row and column maxima, 1.2e-15 and 1.9e-15.  The GEMM
-// runs 1.75 PFLOP/s of BF16 work at D = 2048, 0.99 of the sustained cuBLAS rate.
+// runs 1.73 to 1.75 PFLOP/s of BF16 work at D = 2048, 0.98 to 0.99 of the sustained cuBLAS rate.
 // Complex operands use the real embedding [Re -Im; Im Re] x [Re; Im].
 //
 // Kernels: oz_rowmax* / oz_residues* (FP64 operand -> row exponents and NMOD K-major BF16
